@@ -1027,21 +1027,27 @@ static FastCuts make_cuts(const PairRule &rule, float box, float dmax) {
     fc.ds2 = fc.dsf * fc.dsf;
     const double dd = rule.dd;
     const double rmax = (double)dmax * rule.ds + 1.0;  // r units
-    // Relative FP32 error of d2 (one rounding in each difference, then the
-    // FMA chain) stays below ~2^-21, and of r = sqrt.approx(d2*ds^2) below
-    // ~2^-20: the windows below keep an 8x margin over those bounds.
-    const double e_plain_d2 = dd * std::ldexp(1.0, -17);
-    const double w_plain = rmax * std::ldexp(1.0, -17);
-    // image-shifted home point: |error of dx| <= L*2^-23 per axis
-    const double e_shift_d2 = e_plain_d2 + (double)dmax * (double)box * std::ldexp(1.0, -19);
-    const double w_shift = w_plain + rule.ds * (double)box * std::ldexp(1.0, -19);
+    // FP32 error bounds, u = 2^-24 (the windows below keep more than twice them):
+    //  * unshifted: each difference is off by u of itself, its square by 2u, the
+    //    three roundings of the sum by 3u: d2 is off by 5u.  r = sqrt.approx(d2 *
+    //    ds2), with ds2 off by 3u, the product by u and the root by 2u, is off by
+    //    (5 + 3 + 1) / 2 + 2 = 6.5u, and r + 256 rounds by half of its 2^-15 unit.
+    //  * image-shifted: (shift - home) rounds by at most 2uL per axis, which
+    //    moves the separation vector by at most sqrt(3) 2uL = 3.5uL: r by
+    //    3.5uL ds, d2 by 6.9uL dmax.
+    // Windows of eight times the bounds (and 3 units more) sent 14% of the
+    // recheck votes to the FP64 rule where these send 3%.
+    const double e_plain_d2 = dd * std::ldexp(1.0, -20);
+    const double w_plain = rmax * std::ldexp(1.0, -20);
+    const double e_shift_d2 = e_plain_d2 + (double)dmax * (double)box * std::ldexp(1.0, -20);
+    const double w_shift = w_plain + rule.ds * (double)box * std::ldexp(1.0, -21);
     fc.lo[0] = (float)(dd - e_plain_d2);
     fc.hi[0] = (float)(dd + e_plain_d2);
     fc.lo[1] = (float)(dd - e_shift_d2);
     fc.hi[1] = (float)(dd + e_shift_d2);
-    // + quantisation of the fixed-point readout (2^-16)
-    fc.w[0] = std::min(8000u, (unsigned)std::ceil((w_plain + std::ldexp(1.0, -16)) * 32768.0) + 1u);
-    fc.w[1] = std::min(8000u, (unsigned)std::ceil((w_shift + std::ldexp(1.0, -16)) * 32768.0) + 1u);
+    // + the rounding of the fixed-point readout (2^-16)
+    fc.w[0] = std::min(8000u, (unsigned)std::ceil((w_plain + std::ldexp(1.0, -16)) * 32768.0));
+    fc.w[1] = std::min(8000u, (unsigned)std::ceil((w_shift + std::ldexp(1.0, -16)) * 32768.0));
     fc.tiny = 1e-30f;
     return fc;
 }

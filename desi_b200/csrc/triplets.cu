@@ -825,6 +825,29 @@ static int64_t max_stencil_scan(const CellGrid &g, int P, const std::vector<RowD
     return best;
 }
 
+// FP32 windows of the triplet kernels (u = 2^-24, R = dmax, L = box).  A list
+// entry, candidate - (anchor - shift), is off by u of itself (at most uR), and
+// where an axis is image-shifted by 2uL more; the third side's difference of
+// two entries adds u of itself.  Its vector is thus off by at most
+// sqrt(3) (2uR + 4uL) = 3.5uR + 6.9uL (no L term without a periodic box), and
+// d2 and r carry the pair kernel's 5u and 6.5u beside that (make_cuts).  The
+// windows keep more than twice these bounds; the anchor's sides, with one
+// entry's error, lie well inside.
+static TripCuts trip_cuts(const PairRule &rule, float box, float dmax, bool bpc) {
+    TripCuts c;
+    const double dd = rule.dd, R = (double)dmax, L = bpc ? (double)box : 0.0;
+    const double rmax = R * rule.ds + 1.0;
+    const double e_d2 = dd * std::ldexp(1.0, -19) + R * L * std::ldexp(1.0, -19);
+    const double wr = rmax * std::ldexp(1.0, -20) + rule.ds * (R * std::ldexp(1.0, -21) + L * std::ldexp(1.0, -20));
+    c.dsf = (float)rule.ds;
+    c.ds2 = c.dsf * c.dsf;
+    c.lo = (float)(dd - e_d2);
+    c.hi = (float)(dd + e_d2);
+    // + the rounding of the fixed-point readout (2^-16)
+    c.w = std::min(8000u, (unsigned)std::ceil((wr + std::ldexp(1.0, -16)) * 32768.0));
+    return c;
+}
+
 // Arguments of one isotropic triplet histogram over the cell structures of
 // x (and y for XXY) at P partitions: catalogs, side rules, FP32 windows and
 // the shared-memory layout (smem: dynamic bytes).  The buffers (rows,
@@ -855,21 +878,7 @@ static void trip_setup(pcf_ctx *ctx, const pcf_grid *X, const pcf_grid *Y, int P
     A.ctrl = ctx->d_abort;
     A.status = ctx->d_status;
     A.mixed = mixed ? 1 : 0;
-    {
-        // windows: the FP32 side |v_k - v_j| carries up to three roundings of
-        // coordinate differences (plus the image shift of the anchor when
-        // periodic); the bounds below keep a >= 8x margin
-        const double dd = rXX.dd;
-        const double rmax = (double)dmax * rXX.ds + 1.0;
-        const double Lx = bpc ? (double)X->box : (double)dmax;
-        const double e_d2 = dd * std::ldexp(1.0, -17) + (double)dmax * Lx * std::ldexp(1.0, -18);
-        const double wr = rmax * std::ldexp(1.0, -17) + rXX.ds * Lx * std::ldexp(1.0, -18);
-        A.fc.dsf = (float)rXX.ds;
-        A.fc.ds2 = A.fc.dsf * A.fc.dsf;
-        A.fc.lo = (float)(dd - e_d2);
-        A.fc.hi = (float)(dd + e_d2);
-        A.fc.w = std::min(8000u, (unsigned)std::ceil((wr + std::ldexp(1.0, -16)) * 32768.0) + 1u);
-    }
+    A.fc = trip_cuts(rXX, X->box, dmax, bpc);
     const int n3 = bins * bins * bins;
     // histogram + 32 dummy slots (the adds of 0 of lanes without a triangle)
     const size_t u_bytes = ((size_t)(n3 + 32) * 4 + 15) & ~(size_t)15;
@@ -1258,18 +1267,7 @@ static pcf_status count_triplets_ordered(pcf_ctx *ctx, const pcf_grid *x_, const
     A.ctrl = ctx->d_abort;
     A.status = ctx->d_status;
     if (gates) A.gate = gate_geometry(X->box, dmax, X->user_P);
-    {
-        const double dd = rXX.dd;
-        const double rmax = (double)dmax * rXX.ds + 1.0;
-        const double Lx = bpc ? (double)X->box : (double)dmax;
-        const double e_d2 = dd * std::ldexp(1.0, -17) + (double)dmax * Lx * std::ldexp(1.0, -18);
-        const double wr = rmax * std::ldexp(1.0, -17) + rXX.ds * Lx * std::ldexp(1.0, -18);
-        A.fc.dsf = (float)rXX.ds;
-        A.fc.ds2 = A.fc.dsf * A.fc.dsf;
-        A.fc.lo = (float)(dd - e_d2);
-        A.fc.hi = (float)(dd + e_d2);
-        A.fc.w = std::min(8000u, (unsigned)std::ceil((wr + std::ldexp(1.0, -16)) * 32768.0) + 1u);
-    }
+    A.fc = trip_cuts(rXX, X->box, dmax, bpc);
     const bool weighted = !(X->unit_weights && (!mixed || Y->unit_weights));
     const size_t ent = 16 + 2 + (weighted ? 4 : 0) + (gates ? 4 : 0);
     const size_t room = 227 * 1024 - 256 - (gates ? 64 * sizeof(GateBlock) + 128 + 64 : 0);
