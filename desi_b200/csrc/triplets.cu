@@ -7,21 +7,22 @@
 // *triple* with a global FP64 atomic per triangle and spell out 64 image
 // combinations.  Here:
 //
-//  * A persistent CTA takes one anchor point i at a time.  It scans the
-//    anchor's neighbour cells (the pair stencil, periodic images by index
-//    wrap) and compacts into shared memory the X neighbours j > i (list J)
+//  * A persistent CTA takes one anchor point i at a time.  It lists the point
+//    ranges of the anchor's neighbour rows (the pair stencil, periodic images
+//    by index wrap), deals the candidates of all of them to its warps 32 at a
+//    time, and compacts into shared memory the X neighbours j > i (list J)
 //    and, for XXY, all Y neighbours (list K), each with its FP32 image
-//    displacement from i and its exact side bin (FP32 fast path + FP64
-//    recheck, as in the pair kernel).
+//    displacement from i (in bins) and its exact side bin (FP32 fast path +
+//    FP64 recheck, as in the pair kernel).
 //  * It then runs the pairs of that list: XXX pairs (j < k) of J, XXY all of
 //    J x K.  The third side is |v_k - v_j| -- the consistent embedding of
 //    count123 (3isoBPC_k.cuh:56-75) -- tested and binned in FP32 with the
 //    same edge-window recheck.  Each unordered XXX triangle is seen once (i
 //    its lowest index), each unordered XX pair of an XXY triangle once.
-//  * Counts go to a shared u32 histogram U[b_ij][b_jk][b_ki] (one
-//    orientation per triangle); the finalize pass symmetrises it into the
-//    reference's ordered-triple histogram: XXX sums the 6 axis
-//    permutations, XXY the two orders of the XX pair (b_jk <-> b_ki).
+//  * Counts go to a shared u32 histogram (one orientation per triangle); the
+//    finalize pass symmetrises it into the reference's ordered-triple
+//    histogram: XXX sums the 6 axis permutations, XXY the two orders of the
+//    XX pair (b_jk <-> b_ki).
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -41,14 +42,17 @@ constexpr float kMagic = 256.0f;
 constexpr int kFracBits = 15;
 constexpr unsigned kFracMask = (1u << kFracBits) - 1u;
 constexpr unsigned kBinBias = 0x43800000u >> kFracBits;  // bits(256 + r) >> 15 = this + floor(r)
-#ifndef PCF_TRIP_GROUP
-#define PCF_TRIP_GROUP 2  // third-side steps between recheck votes
-#endif
-
 struct TripCuts {
     float dsf, ds2;
-    float lo, hi;  // d2 window around dd (image-aware bound for periodic boxes)
-    unsigned w;    // edge window, 2^-15 units of r
+    float lo, hi;    // d2 window around dd (image-aware bound for periodic boxes)
+    float lo3, hi3;  // the same in bins^2 (third sides: list entries are in bins)
+    unsigned w;      // edge window, 2^-15 units of r
+    // tiles (tri_tiles): the window with the distance from dmax to the last
+    // bin edge, where that is small (far = 0); else the window around dmax as
+    // values of r + 256 + w
+    unsigned wt;
+    int far;
+    float qlo, qhi;
 };
 
 struct Cat {
@@ -141,9 +145,15 @@ __device__ __forceinline__ int fast_bin(float d2, const TripCuts &c, int bins) {
     return -1;
 }
 
-// Appends the neighbours of anchor (hx,hy,hz) found in catalog C to a list.
-// only_after >= 0 keeps candidates with index > only_after (X list of XXX /
-// XXY).  Entries: {dx, dy, dz, bits(idx << 8 | bin)}.
+// The same for a third side, from the squared difference of two list entries
+// (in bins^2).
+__device__ __forceinline__ int fast_bin3(float r2, const TripCuts &c, int bins) {
+    if (!(r2 < c.hi3)) return -2;
+    const unsigned q = __float_as_uint(sqrt_approx(r2) + kMagic) & 0x7FFFFFu;
+    if (r2 < c.lo3 && fix_safe(q, c.w)) return min((int)(q >> kFracBits), bins - 1);
+    return -1;
+}
+
 // Angle bin of the anisotropic 3-point histograms for the side anchor->point:
 // t = (int)((1 + dz/d) * (float)(bins/2)) (3ani_k.cuh:79-91), dz signed, or
 // with periodic boxes dz = |z2-z1| - L*f (3aniBPC_k.cuh:57,73); -1 when >= bins.
@@ -162,109 +172,314 @@ __device__ __noinline__ int exact_angle(float ax, float ay, float az, float bx, 
     return (t >= 0 && t < bins) ? t : -1;
 }
 
-// ginfo (PCF_REF_NODE_GATES): per entry, its node on the reference's grid
-// and the axes of its image relative to the anchor (gate_pack).
-template <bool ANG>
-__device__ void build_list(const TripArgs &A, const Cat &C, float hx, float hy, float hz, int hcell_ix,
-                           int hcell_iy, int hcell_iz, int only_after, const PairRule &rule,
-                           float4 *list, float *wlist, int cap, int *s_n, unsigned &n_rechk,
-                           unsigned short *ang = nullptr, int step = 1, unsigned *ginfo = nullptr) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int P = A.P;
-    for (int r = 0; r < A.n_rows; ++r) {
+// The candidate ranges of an anchor's stencil rows, two per row (a periodic
+// row may wrap in z): first point with the image shifts (2 bits per axis
+// above bit 24: 0 -L, 1 none, 2 +L) and the number of candidates before it.
+constexpr int kSegs = kTThreads;
+struct SegTable {
+    int first[kSegs], before[kSegs];
+    int wsum[kTWarps];
+};
+
+// Ranges of rows [rb, rb + kSegs / 2), one per thread, in catalog C around the
+// anchor's cell; only_after >= 0 keeps the points after that index.  Returns
+// the number of candidates.  Called by the whole CTA; ends synchronised, and
+// needs no barrier before it (the table is written after its first barrier).
+__device__ __forceinline__ int seg_table(const TripArgs &A, const Cat &C, int cix, int ciy, int ciz,
+                                         int only_after, int rb, SegTable &T) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int r = rb + (tid >> 1), P = A.P;
+    int a = 0, len = 0;
+    if (r < A.n_rows) {
         const RowDesc rw = A.rows[r];
-        int nx = hcell_ix + rw.dx, ny = hcell_iy + rw.dy;
-        float sx = 0.f, sy = 0.f;
+        int nx = cix + rw.dx, ny = ciy + rw.dy, ix = 1, iy = 1, iz = 1;
+        bool ok = true;
         if (A.bpc) {
-            if (nx < 0) { nx += P; sx = -A.box; } else if (nx >= P) { nx -= P; sx = A.box; }
-            if (ny < 0) { ny += P; sy = -A.box; } else if (ny >= P) { ny -= P; sy = A.box; }
-        } else if (nx < 0 || nx >= P || ny < 0 || ny >= P) {
-            continue;
+            if (nx < 0) { nx += P; ix = 0; } else if (nx >= P) { nx -= P; ix = 2; }
+            if (ny < 0) { ny += P; iy = 0; } else if (ny >= P) { ny -= P; iy = 2; }
+        } else {
+            ok = nx >= 0 && nx < P && ny >= 0 && ny < P;
         }
-        const int col = (nx * P + ny) * P;
-        const int zlo = hcell_iz - rw.kz, zhi = hcell_iz + rw.kz;
-        int ra[2], rb[2];
-        float rz[2] = {0.f, 0.f};
-        ra[0] = C.cstart[col + max(zlo, 0)];
-        rb[0] = C.cstart[col + min(zhi, P - 1) + 1];
-        ra[1] = rb[1] = 0;
-        if (A.bpc) {
-            if (zlo < 0) { ra[1] = C.cstart[col + zlo + P]; rb[1] = C.cstart[col + P]; rz[1] = -A.box; }
-            else if (zhi >= P) { ra[1] = C.cstart[col]; rb[1] = C.cstart[col + zhi - P + 1]; rz[1] = A.box; }
+        if (ok) {
+            const int col = (nx * P + ny) * P;
+            int zlo = ciz - rw.kz, zhi = ciz + rw.kz;
+            if (tid & 1) {  // the part past the box's z face, through its image
+                ok = A.bpc && (zlo < 0 || zhi >= P);
+                iz = zlo < 0 ? 0 : 2;
+                if (zlo < 0) { zlo += P; zhi = P - 1; } else { zlo = 0; zhi -= P; }
+            } else {
+                zlo = max(zlo, 0);
+                zhi = min(zhi, P - 1);
+            }
+            if (ok) {
+                a = C.cstart[col + zlo];
+                const int b = C.cstart[col + zhi + 1];
+                if (only_after >= 0) a = max(a, only_after + 1);
+                len = max(b - a, 0);
+                a |= (ix | (iy << 2) | (iz << 4)) << 24;
+            }
         }
-        for (int sgi = 0; sgi < 2; ++sgi) {
-            int a = ra[sgi];
-            const int b = rb[sgi];
-            if (only_after >= 0) a = max(a, only_after + 1);
-            if (a >= b) continue;
-            const float ex = hx - sx, ey = hy - sy, ez = hz - rz[sgi];
-            // warps take 32-candidate chunks
-            for (int base = a + warp * 32; base < b; base += kTWarps * 32) {
-                const int c = base + lane;
-                int bin = -2;
-                float vx = 0.f, vy = 0.f, vz = 0.f;
-                if (c < b) {
-                    vx = C.x[c] - ex;
-                    vy = C.y[c] - ey;
-                    vz = C.z[c] - ez;
-                    const float d2 = fmaf(vz, vz, fmaf(vy, vy, vx * vx));
-                    bin = fast_bin(d2, A.fc, rule.bins);
-                    if (bin == -1) {
-                        ++n_rechk;
-                        bin = exact_side(hx, hy, hz, C.x[c], C.y[c], C.z[c], A.bpc, A.box, rule);
-                    }
+    }
+    int x = len;
+    #pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(kFull, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) T.wsum[warp] = x;
+    __syncthreads();
+    int ws = T.wsum[lane & (kTWarps - 1)], w = ws;
+    #pragma unroll
+    for (int o = 1; o < kTWarps; o <<= 1) {
+        const int y = __shfl_up_sync(kFull, w, o);
+        if ((lane & (kTWarps - 1)) >= o) w += y;
+    }
+    const int total = __shfl_sync(kFull, w, kTWarps - 1);
+    T.first[tid] = a;
+    T.before[tid] = x - len + __shfl_sync(kFull, w - ws, warp);
+    __syncthreads();
+    return total;
+}
+
+// Appends the neighbours of anchor (hx,hy,hz) found in catalog C to a list.
+// Entries: {dx, dy, dz in bins, bits(idx << 8 | bin)}.  ang: their angle bins
+// (ANG).  ginfo (PCF_REF_NODE_GATES): per entry, its node on the reference's
+// grid and the axes of its image relative to the anchor (gate_pack).
+//
+// All rows' candidates form one index space that the warps share 32 at a time
+// (the range of an index by binary search): a row holds 10 to 100 candidates,
+// so a loop over rows kept 1 to 3 of 16 warps busy and cost a dependent
+// cell-table load per row.
+template <bool ANG>
+__device__ void build_list(const TripArgs &A, const Cat &C, float hx, float hy, float hz, int cix, int ciy,
+                           int ciz, int only_after, const PairRule &rule, float4 *list, float *wlist,
+                           int cap, int *s_n, unsigned &n_rechk, SegTable &T, unsigned char *ang = nullptr,
+                           unsigned *ginfo = nullptr) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int rb = 0; rb < A.n_rows; rb += kSegs / 2) {
+        const int total = seg_table(A, C, cix, ciy, ciz, only_after, rb, T);
+        const int nseg = 2 * min(kSegs / 2, A.n_rows - rb);
+        const int top = 1 << (31 - __clz(nseg));
+        // candidate of index q: its point, or -1 past the end; image axes in sh
+        auto locate = [&](int q, int &sh) -> int {
+            if (q >= total) return -1;
+            int s = 0;
+            for (int o = top; o > 0; o >>= 1)
+                if (s + o < nseg && T.before[s + o] <= q) s += o;
+            const int f = T.first[s];
+            sh = f >> 24;
+            return (f & 0xFFFFFF) + q - T.before[s];
+        };
+        int sh = 0, c = locate(warp * 32 + lane, sh);
+        float px = 0.f, py = 0.f, pz = 0.f;
+        if (c >= 0) { px = C.x[c]; py = C.y[c]; pz = C.z[c]; }
+        for (int base = warp * 32; base < total; base += kTThreads) {
+            // the next chunk's points are on their way while this one is tested
+            int shn = 0;
+            const int cn = locate(base + kTThreads + lane, shn);
+            float nx = 0.f, ny = 0.f, nz = 0.f;
+            if (cn >= 0) { nx = C.x[cn]; ny = C.y[cn]; nz = C.z[cn]; }
+            int bin = -2, tang = 0;
+            float vx = 0.f, vy = 0.f, vz = 0.f;
+            if (c >= 0) {
+                vx = px - (hx - (float)((sh & 3) - 1) * A.box);
+                vy = py - (hy - (float)(((sh >> 2) & 3) - 1) * A.box);
+                vz = pz - (hz - (float)((sh >> 4) - 1) * A.box);
+                const float d2 = fmaf(vz, vz, fmaf(vy, vy, vx * vx));
+                bin = fast_bin(d2, A.fc, rule.bins);
+                if (bin == -1) {
+                    ++n_rechk;
+                    bin = exact_side(hx, hy, hz, px, py, pz, A.bpc, A.box, rule);
                 }
-                int tang = 0;
                 if (ANG && bin >= 0) {
-                    tang = exact_angle(hx, hy, hz, C.x[c], C.y[c], C.z[c], A.bpc, A.box, rule.bins,
+                    tang = exact_angle(hx, hy, hz, px, py, pz, A.bpc, A.box, rule.bins,
                                        (float)rule.bins / 2.0f);
                     if (tang < 0) bin = -2;  // the side can close no triangle
                 }
-                const bool keep = bin >= 0;
-                const unsigned m = __ballot_sync(kFull, keep);
-                int off = 0;
-                if (lane == 0 && m) off = atomicAdd(s_n, __popc(m));
-                off = __shfl_sync(kFull, off, 0);
-                if (keep) {
-                    const int pos = off + __popc(m & ((1u << lane) - 1u));
-                    if (pos < cap) {  // step -1: the list grows downwards from `list`
-                        list[step * pos] = make_float4(vx, vy, vz, __int_as_float((c << 8) | bin));
-                        if (wlist) wlist[pos] = C.w[c];
-                        if (ANG) ang[pos] = (unsigned short)(bin | (tang << 8));
-                        if (ginfo)
-                            ginfo[pos] = gate_pack(A.gate, C.x[c], C.y[c], C.z[c],
-                                                   (sx != 0.f ? 1u : 0u) | (sy != 0.f ? 2u : 0u) |
-                                                       (rz[sgi] != 0.f ? 4u : 0u));
-                    }
+            }
+            const bool keep = bin >= 0;
+            const unsigned m = __ballot_sync(kFull, keep);
+            int off = 0;
+            if (lane == 0 && m) off = atomicAdd(s_n, __popc(m));
+            off = __shfl_sync(kFull, off, 0);
+            if (keep) {
+                const int pos = off + __popc(m & ((1u << lane) - 1u));
+                if (pos < cap) {
+                    list[pos] = make_float4(vx * A.fc.dsf, vy * A.fc.dsf, vz * A.fc.dsf,
+                                            __int_as_float((c << 8) | bin));
+                    if (wlist) wlist[pos] = C.w[c];
+                    if (ANG) ang[pos] = (unsigned char)tang;
+                    if (ginfo)
+                        ginfo[pos] = gate_pack(A.gate, px, py, pz,
+                                               ((sh & 3) != 1 ? 1u : 0u) | (((sh >> 2) & 3) != 1 ? 2u : 0u) |
+                                                   ((sh >> 4) != 1 ? 4u : 0u));
                 }
             }
+            c = cn;
+            sh = shn;
+            px = nx;
+            py = ny;
+            pz = nz;
         }
     }
 }
 
-// Adds the shared histogram U (nb3 u32) into the u64 histogram g and clears
-// it (whole CTA).
-__device__ __forceinline__ void flush_hist(unsigned *U, int nb3, unsigned long long *g) {
+// The shared histogram U of the unit-weight counts: bins^2 rows [b_ij][b_ki]
+// of bins + 1 counters over b_jk, the last of which takes the tests out of
+// range and is never read.
+__host__ __device__ __forceinline__ int u_words(int bins) { return bins * bins * (bins + 1); }
+
+// Adds U into the u64 histogram g (bins^3, [b_ij][b_ki][b_jk]) and clears it
+// (whole CTA); returns the triangles this thread added.
+__device__ __forceinline__ unsigned long long flush_hist(unsigned *U, int bins, unsigned long long *g) {
     __syncthreads();
-    for (int k = threadIdx.x; k < nb3; k += kTThreads) {
+    unsigned long long n = 0;
+    const int nu = u_words(bins);
+    for (int k = threadIdx.x; k < nu; k += kTThreads) {
         const unsigned v = U[k];
         if (v) {
-            atomicAdd(g + k, (unsigned long long)v);
+            const int row = k / (bins + 1), c = k - row * (bins + 1);
             U[k] = 0u;
+            if (c < bins) {
+                atomicAdd(g + row * bins + c, (unsigned long long)v);
+                n += v;
+            }
         }
     }
     __syncthreads();
+    return n;
 }
 
 // Per-CTA state of the anchor loop.
 struct TripCta {
     unsigned *U;                      // shared histogram (hist_in_smem)
     unsigned char *lists;             // shared neighbour lists
+    SegTable *segs;
     int *s_nJ, *s_nK, *s_unit;        // shared counters
     unsigned n_rechk;
     unsigned long long n_tri;
     unsigned long long since;         // pair tests since U's last flush
 };
+
+// A list position past the end: farther than dmax from every entry, and a
+// tile's j from a padded k too (they carry opposite signs).
+constexpr float kFarAway = 1e15f;
+constexpr int kTile = 8;    // j per tile
+constexpr int kChunkK = 32; // K lists are padded to whole chunks of one k per lane
+
+// Pass 2 of the unit-weight counts into U: tiles of kTile consecutive j
+// against the K list, one k per lane.  A step loads one k and tests it
+// against the tile's j, two at a time in packed FP32.
+//
+// What bounds it is the shared-memory pipe, with instruction issue close
+// behind: a reduction of 32 scattered counters costs 2.9 cycles of the SM
+// (conflicts), a 16-byte list load 4.  Tiles divide the loads by kTile, and the
+// step is kept branch-free and short: every test adds 1 to a counter, tests out
+// of range (their r clamped to bins + 1/2) to the row's last one, and tests
+// within the window of a bin edge as the fast path has them; the rare vote that
+// finds one in the window corrects the count by the FP64 rule afterwards.  The
+// constant increment also lets the hardware add lanes that hit one counter
+// together (32 cycles for a register operand where all lanes collide, 1 for the
+// constant).
+// FAR: dmax lies more than the window below the last bin's edge (bins / dmax
+// rounded down to 1e-6, large dmax), so it needs a window of its own.
+template <bool MIXED, bool FAR>
+__device__ __forceinline__ void tri_tiles(const TripArgs &A, TripCta &C, const float4 *__restrict__ LJ,
+                                          const float4 *__restrict__ LK, int nJ, int nK, float hx, float hy,
+                                          float hz) {
+    const int lane = threadIdx.x & 31;
+    const int bins = A.rXX.bins, rowlen = bins + 1;
+    unsigned *U = C.U;
+    const unsigned Us = (unsigned)__cvta_generic_to_shared(U) - 4u * kBinBias;
+    const unsigned w2s = (2u * A.fc.wt) << (32 - kFracBits);
+    const float mgw = kMagic + (float)A.fc.wt * 0x1p-15f;
+    const float qout = kMagic + (float)bins + 0.5f;
+    const float qlo = A.fc.qlo, qhi = A.fc.qhi, qedge = kMagic + (float)bins;
+    const unsigned kstride = 4u * (unsigned)rowlen, jstride = kstride * (unsigned)bins;
+    const int ntile = (nJ + kTile - 1) / kTile, nchunk = (nK + kChunkK - 1) / kChunkK;
+    // units: tiles (XXX: the longest rows first), split along K while there
+    // are few tiles per warp
+    int segs = 1;
+    if (MIXED)
+        while (segs < nchunk && ntile * segs < 8 * kTWarps) segs <<= 1;
+    const int units = ntile * segs;
+    for (;;) {
+        int u0 = 0;
+        if (lane == 0) u0 = atomicAdd(C.s_unit, 1);
+        u0 = __shfl_sync(kFull, u0, 0);
+        if (u0 >= units) break;
+        const int tile = u0 / segs, sg = u0 - tile * segs, j0 = tile * kTile;
+        float2 JX[kTile / 2], JY[kTile / 2], JZ[kTile / 2];
+        unsigned jb[kTile];
+        #pragma unroll
+        for (int q = 0; q < kTile; ++q) {
+            float4 e = make_float4(-kFarAway, -kFarAway, -kFarAway, 0.f);
+            if (j0 + q < nJ) e = LJ[j0 + q];
+            (q & 1 ? JX[q / 2].y : JX[q / 2].x) = -e.x;
+            (q & 1 ? JY[q / 2].y : JY[q / 2].x) = -e.y;
+            (q & 1 ? JZ[q / 2].y : JZ[q / 2].x) = -e.z;
+            jb[q] = Us + (unsigned)(__float_as_int(e.w) & 255) * jstride;
+        }
+        // the canonical rule for test (j0 + q, k), counted as u by the fast path
+        auto settle = [&](int q, int k, unsigned u) {
+            ++C.n_rechk;
+            const float4 ej = LJ[j0 + q], ek = LK[k];
+            const int jidx = (int)((unsigned)__float_as_int(ej.w) >> 8);
+            const int kidx = (int)((unsigned)__float_as_int(ek.w) >> 8);
+            const Cat &CK = MIXED ? A.Y : A.X;
+            const int b = exact_third(hx, hy, hz, A.X.x[jidx], A.X.y[jidx], A.X.z[jidx], CK.x[kidx],
+                                      CK.y[kidx], CK.z[kidx], A.bpc, A.box, MIXED ? A.rXY : A.rXX);
+            unsigned *row = U + ((__float_as_int(ej.w) & 255) * bins + (__float_as_int(ek.w) & 255)) * rowlen;
+            const int fast = (int)((u >> kFracBits) - kBinBias);
+            if (b != fast) {
+                atomicSub(row + fast, 1u);
+                if (b >= 0) atomicAdd(row + b, 1u);
+            }
+        };
+        // head (XXX): the chunk that holds the tile itself, where k <= j is no test
+        auto step = [&](int k, bool head) {
+            const float4 e = LK[k];
+            const float2 KX = make_float2(e.x, e.x), KY = make_float2(e.y, e.y), KZ = make_float2(e.z, e.z);
+            const unsigned kb = (unsigned)(__float_as_int(e.w) & 255) * kstride;
+            unsigned u[kTile], near = 0xffffffffu;
+            #pragma unroll
+            for (int p = 0; p < kTile / 2; ++p) {
+                const float2 DX = __fadd2_rn(KX, JX[p]), DY = __fadd2_rn(KY, JY[p]), DZ = __fadd2_rn(KZ, JZ[p]);
+                const float2 R2 = __ffma2_rn(DZ, DZ, __ffma2_rn(DY, DY, __fmul2_rn(DX, DX)));
+                float2 Q = __fadd2_rn(make_float2(sqrt_approx(R2.x), sqrt_approx(R2.y)), make_float2(mgw, mgw));
+                if (head) {
+                    if (k <= j0 + 2 * p) Q.x = qout;
+                    if (k <= j0 + 2 * p + 1) Q.y = qout;
+                }
+                if (FAR) {  // inside dmax's window: the unread counter, marked for the FP64 rule
+                    u[2 * p] = __float_as_uint(Q.x < qlo ? Q.x : Q.x < qhi ? qedge : qout);
+                    u[2 * p + 1] = __float_as_uint(Q.y < qlo ? Q.y : Q.y < qhi ? qedge : qout);
+                } else {
+                    u[2 * p] = __float_as_uint(fminf(Q.x, qout));
+                    u[2 * p + 1] = __float_as_uint(fminf(Q.y, qout));
+                }
+                // bits above the fraction shifted out: below w2s in the window
+                near = min(near, min(u[2 * p] << (32 - kFracBits), u[2 * p + 1] << (32 - kFracBits)));
+                asm volatile("red.shared.add.u32 [%0], 1;" ::"r"(jb[2 * p] + kb + 4u * (u[2 * p] >> kFracBits)));
+                asm volatile("red.shared.add.u32 [%0], 1;" ::"r"(jb[2 * p + 1] + kb + 4u * (u[2 * p + 1] >> kFracBits)));
+            }
+            if (__any_sync(kFull, near < w2s)) {
+                #pragma unroll
+                for (int q = 0; q < kTile; ++q)
+                    if ((u[q] << (32 - kFracBits)) < w2s) settle(q, k, u[q]);
+            }
+        };
+        const int c0 = MIXED ? (int)((long long)nchunk * sg / segs) : j0 / kChunkK;
+        const int c1 = MIXED ? (int)((long long)nchunk * (sg + 1) / segs) : nchunk;
+        int k = c0 * kChunkK + lane;
+        const int kend = c1 * kChunkK;
+        if (!MIXED && c0 < c1) {
+            step(k, true);
+            k += kChunkK;
+        }
+        for (; k < kend; k += kChunkK) step(k, false);
+    }
+}
 
 // All triangles of anchor i of job A: pass 1 builds the anchor's
 // neighbour lists in shared memory (or, past their capacity, in this CTA's
@@ -272,13 +487,9 @@ struct TripCta {
 template <bool MIXED, bool WEIGHTED>
 __device__ __forceinline__ void tri_anchor(const TripArgs &A, int i, TripCta &C) {
     const int bins = A.rXX.bins;
-    const int nb3 = bins * bins * bins;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    unsigned *U = C.U;
-    int &s_nJ = *C.s_nJ, &s_nK = *C.s_nK, &s_unit = *C.s_unit;
+    int &s_nJ = *C.s_nJ, &s_nK = *C.s_nK;
     unsigned &n_rechk = C.n_rechk;
-    unsigned long long &n_tri = C.n_tri;
-    unsigned long long &since = C.since;
     float4 *sJ = reinterpret_cast<float4 *>(C.lists);
     float4 *sK = sJ + A.capJ;
     float *swJ = reinterpret_cast<float *>(sK + (MIXED ? A.capK : 0));
@@ -287,245 +498,142 @@ __device__ __forceinline__ void tri_anchor(const TripArgs &A, int i, TripCta &C)
     float4 *gK = A.gK ? A.gK + (size_t)blockIdx.x * A.gcap : nullptr;
     float *gwJ = A.gwJ ? A.gwJ + (size_t)blockIdx.x * A.gcap : nullptr;
     float *gwK = A.gwK ? A.gwK + (size_t)blockIdx.x * A.gcap : nullptr;
-    auto flush_u = [&]() { flush_hist(U, nb3, A.g_count); };
-        const float hx = A.X.x[i], hy = A.X.y[i], hz = A.X.z[i];
-        const float hw = WEIGHTED ? A.X.w[i] : 1.f;
-        const int P = A.P;
-        const int cix = min(max((int)__fdiv_rn(hx, A.cell), 0), P - 1);
-        const int ciy = min(max((int)__fdiv_rn(hy, A.cell), 0), P - 1);
-        const int ciz = min(max((int)__fdiv_rn(hz, A.cell), 0), P - 1);
-        // pass 1: lists into shared memory (sizes counted even past capacity).
-        // Pooled (XXY, unit weights, shared histogram): one buffer of capJ
-        // entries, J from the front and K from the back, so the anchor
-        // overflows only when both together exceed it.
-        const bool pool = MIXED && !WEIGHTED && A.hist_in_smem;
-        build_list<false>(A, A.X, hx, hy, hz, cix, ciy, ciz, i, A.rXX, sJ, WEIGHTED ? swJ : nullptr,
-                          A.capJ, &s_nJ, n_rechk);
-        int capK = A.capK;
+    const float hx = A.X.x[i], hy = A.X.y[i], hz = A.X.z[i];
+    const float hw = WEIGHTED ? A.X.w[i] : 1.f;
+    const int P = A.P;
+    const int cix = min(max((int)__fdiv_rn(hx, A.cell), 0), P - 1);
+    const int ciy = min(max((int)__fdiv_rn(hy, A.cell), 0), P - 1);
+    const int ciz = min(max((int)__fdiv_rn(hz, A.cell), 0), P - 1);
+    // pass 1: lists into shared memory (sizes counted even past capacity).
+    // Pooled (unit weights, shared histogram): one buffer of capJ entries, J
+    // and behind it K, each list that is walked in chunks padded to them.
+    const bool pool = !WEIGHTED && A.hist_in_smem;
+    auto padded = [](int n) { return (n + kChunkK - 1) / kChunkK * kChunkK; };
+    build_list<false>(A, A.X, hx, hy, hz, cix, ciy, ciz, i, A.rXX, sJ, WEIGHTED ? swJ : nullptr, A.capJ,
+                      &s_nJ, n_rechk, *C.segs);
+    int capK = A.capK;
+    __syncthreads();
+    int nJ = s_nJ;
+    if (MIXED) {
         if (pool) {
-            __syncthreads();
-            capK = max(0, A.capJ - s_nJ);
+            sK = sJ + min(nJ, A.capJ);
+            capK = max(0, A.capJ - nJ);
         }
-        if (MIXED)
-            build_list<false>(A, A.Y, hx, hy, hz, cix, ciy, ciz, -1, A.rXY, pool ? sJ + A.capJ - 1 : sK,
-                              WEIGHTED ? swK : nullptr, capK, &s_nK, n_rechk, nullptr, pool ? -1 : 1);
+        build_list<false>(A, A.Y, hx, hy, hz, cix, ciy, ciz, -1, A.rXY, sK, WEIGHTED ? swK : nullptr, capK,
+                          &s_nK, n_rechk, *C.segs);
         __syncthreads();
-        int nJ = s_nJ, nK = MIXED ? s_nK : nJ;
-        const float4 *LJ = sJ;
-        const float4 *LK = MIXED ? sK : sJ;
-        const float *WJ = swJ, *WK = MIXED ? swK : swJ;
-        if (nJ > A.capJ || (MIXED && nK > capK)) {
-            // overflow: rebuild the lists in this CTA's global scratch (L2)
-            __syncthreads();
-            if (tid == 0) { s_nJ = 0; s_nK = 0; }
-            __syncthreads();
-            build_list<false>(A, A.X, hx, hy, hz, cix, ciy, ciz, i, A.rXX, gJ,
-                              WEIGHTED ? gwJ : nullptr, A.gcap, &s_nJ, n_rechk);
-            if (MIXED)
-                build_list<false>(A, A.Y, hx, hy, hz, cix, ciy, ciz, -1, A.rXY, gK,
-                                  WEIGHTED ? gwK : nullptr, A.gcap, &s_nK, n_rechk);
-            __threadfence_block();
-            __syncthreads();
-            nJ = min(s_nJ, A.gcap);
-            nK = MIXED ? min(s_nK, A.gcap) : nJ;
-            LJ = gJ;
-            LK = MIXED ? gK : gJ;
-            WJ = gwJ;
-            WK = MIXED ? gwK : gwJ;
-        }
-        // K entry k is LK[kstepK * k]: the pooled K list grows downwards from
-        // the end of the shared buffer
-        int kstepK = 1;
-        if (pool && LJ == sJ) {
-            LK = sJ + A.capJ - 1;
-            kstepK = -1;
-        }
-        // Flush budget of the shared histogram: this anchor adds at most
-        // `tests` times.  Flush first if the total could pass the budget; an
-        // anchor whose tests alone exceed it counts into global memory.
-        bool smem_hist = !WEIGHTED && A.hist_in_smem;
-        if (smem_hist) {
-            const unsigned long long tests =
-                MIXED ? (unsigned long long)nJ * (unsigned long long)nK
-                      : (unsigned long long)nJ * (unsigned long long)(nJ > 0 ? nJ - 1 : 0) / 2;
-            if (tests > A.flush_budget) {
-                smem_hist = false;
-            } else {
-                if (since + tests > A.flush_budget) {
-                    flush_u();
-                    since = 0;
-                }
-                since += tests;
-            }
-        }
-        // pass 2: pairs of neighbours.  Rows j are dealt to warps in the
-        // order 0, n-1, 1, n-2, ... (XXX rows shrink with j).
-        if (smem_hist) {
-            // the lists' address space is fixed per instantiation, so the
-            // shared-memory case (all but overflowing anchors) uses shared loads
-            // LKx[kstep * k] is K entry k (kstep -1: the pooled, downward K list)
-            auto pass2 = [&](const float4 *__restrict__ LJx, const float4 *__restrict__ LKx, int kstep) {
-            // Unit weights, shared histogram: two k per lane per step in packed
-            // FP32, unpredicated shared reductions (a lane without a triangle
-            // adds 0 to its dummy slot past the histogram), one recheck vote
-            // per group of steps.
-            const PairRule &r3 = MIXED ? A.rXY : A.rXX;
-            const unsigned Us = (unsigned)__cvta_generic_to_shared(U);
-            const unsigned dummy = Us + (unsigned)(nb3 + lane) * 4u;
-            const float lo = A.fc.lo, hi = A.fc.hi;
-            const unsigned w2 = 2u * A.fc.w;
-            const float mgw = kMagic + (float)A.fc.w * 0x1p-15f;
-            const float2 DS2 = make_float2(A.fc.ds2, A.fc.ds2);
-            // Work units handed out dynamically (a shared counter), so warps
-            // finish together: XXX rows j in order (largest first), XXY rows
-            // split into `segs` segments of the K list when rows are few.
-            const int segs = (MIXED && nJ < 8 * kTWarps) ? 4 : 1;
-            const int units = nJ * segs;
-            for (;;) {
-                int u = 0;
-                if (lane == 0) u = atomicAdd(&s_unit, 1);
-                u = __shfl_sync(kFull, u, 0);
-                if (u >= units) break;
-                const int jj = u / segs, sg = u - jj * segs;
-                const int kbeg = MIXED ? (int)((long long)nK * sg / segs) : jj + 1;
-                const int kend = MIXED ? (int)((long long)nK * (sg + 1) / segs) : nK;
-                const float4 ej = LJx[jj];
-                const int bj = __float_as_int(ej.w) & 255;
-                const int jidx = (int)((unsigned)__float_as_int(ej.w) >> 8);
-                // slot = bj*bins^2 + b_jk*bins + b_k, with bits(r+256..) >> 15 = kBinBias + b_jk
-                const unsigned base_j = Us + 4u * (unsigned)(bj * bins * bins - (int)kBinBias * bins);
-                const float2 NJX = make_float2(-ej.x, -ej.x), NJY = make_float2(-ej.y, -ej.y),
-                             NJZ = make_float2(-ej.z, -ej.z);
-                struct Ev {
-                    unsigned a0, a1;
-                    bool f0, f1, r0, r1;
-                };
-                // k0 and (if v1) k0 + 32
-                auto eval = [&](int k0, bool v1) -> Ev {
-                    const float4 e0 = LKx[kstep * k0];
-                    const float4 e1 = LKx[kstep * (v1 ? k0 + 32 : k0)];
-                    const float2 DX = __fadd2_rn(make_float2(e0.x, e1.x), NJX);
-                    const float2 DY = __fadd2_rn(make_float2(e0.y, e1.y), NJY);
-                    const float2 DZ = __fadd2_rn(make_float2(e0.z, e1.z), NJZ);
-                    float2 D2 = __fmul2_rn(DX, DX);
-                    D2 = __ffma2_rn(DY, DY, D2);
-                    D2 = __ffma2_rn(DZ, DZ, D2);
-                    const float2 UU = __fmul2_rn(D2, DS2);
-                    const float2 Q = __fadd2_rn(make_float2(sqrt_approx(UU.x), sqrt_approx(UU.y)),
-                                                make_float2(mgw, mgw));
-                    const unsigned u0 = __float_as_uint(Q.x), u1 = __float_as_uint(Q.y);
-                    Ev e;
-                    e.f0 = (D2.x < lo) && (u0 & kFracMask) >= w2;
-                    e.f1 = v1 && (D2.y < lo) && (u1 & kFracMask) >= w2;
-                    e.r0 = !e.f0 && D2.x < hi;
-                    e.r1 = v1 && !e.f1 && D2.y < hi;
-                    e.a0 = base_j + 4u * ((u0 >> kFracBits) * (unsigned)bins + (unsigned)(__float_as_int(e0.w) & 255));
-                    e.a1 = base_j + 4u * ((u1 >> kFracBits) * (unsigned)bins + (unsigned)(__float_as_int(e1.w) & 255));
-                    return e;
-                };
-                auto core = [&](int k0, bool v1) -> bool {
-                    const Ev e = eval(k0, v1);
-                    asm volatile("red.shared.add.u32 [%0], %1;" :: "r"(e.f0 ? e.a0 : dummy), "r"((unsigned)e.f0));
-                    asm volatile("red.shared.add.u32 [%0], %1;" :: "r"(e.f1 ? e.a1 : dummy), "r"((unsigned)e.f1));
-                    n_tri += (unsigned)e.f0 + (unsigned)e.f1;
-                    return e.r0 || e.r1;
-                };
-                // third side by the canonical FP64 rule
-                auto slow = [&](int kk) {
-                    ++n_rechk;
-                    const float4 ek = LKx[kstep * kk];
-                    const int kidx = (int)((unsigned)__float_as_int(ek.w) >> 8);
-                    const Cat &CK = MIXED ? A.Y : A.X;
-                    const int bjk = exact_third(hx, hy, hz, A.X.x[jidx], A.X.y[jidx], A.X.z[jidx],
-                                                CK.x[kidx], CK.y[kidx], CK.z[kidx], A.bpc, A.box, r3);
-                    if (bjk >= 0) {
-                        atomicAdd(U + bj * bins * bins + bjk * bins + (__float_as_int(ek.w) & 255), 1u);
-                        ++n_tri;
-                    }
-                };
-                auto settle = [&](bool any, int k0, int nsteps, bool v1) {
-                    if (__any_sync(__activemask(), any)) {
-                        for (int q = 0; q < nsteps; ++q) {
-                            const Ev e = eval(k0 + 64 * q, v1);
-                            if (e.r0) slow(k0 + 64 * q);
-                            if (e.r1) slow(k0 + 64 * q + 32);
-                        }
-                    }
-                };
-                int kk = kbeg + lane;
-                constexpr int G = PCF_TRIP_GROUP;
-                for (; kk + 64 * (G - 1) + 32 < kend; kk += 64 * G) {
-                    bool any = false;
-                    #pragma unroll
-                    for (int q = 0; q < G; ++q) any |= core(kk + 64 * q, true);
-                    settle(any, kk, G, true);
-                }
-                for (; kk + 32 < kend; kk += 64) settle(core(kk, true), kk, 1, true);
-                if (kk < kend) settle(core(kk, false), kk, 1, false);
-            }
-            };
-            if (LJ == sJ) {
-                if (pool) pass2(sJ, sJ + A.capJ - 1, -1);
-                else pass2(sJ, MIXED ? sK : sJ, 1);
-            } else {
-                pass2(gJ, MIXED ? gK : gJ, 1);
-            }
+    }
+    int nK = MIXED ? s_nK : nJ;
+    const float4 *LJ = sJ;
+    const float4 *LK = MIXED ? sK : sJ;
+    const float *WJ = swJ, *WK = MIXED ? swK : swJ;
+    const bool spill = nJ > A.capJ || (MIXED && nK > capK) || (pool && padded(nK) > (MIXED ? capK : A.capJ));
+    if (spill) {
+        // overflow: rebuild the lists in this CTA's global scratch (L2)
+        __syncthreads();
+        if (tid == 0) { s_nJ = 0; s_nK = 0; }
+        __syncthreads();
+        build_list<false>(A, A.X, hx, hy, hz, cix, ciy, ciz, i, A.rXX, gJ, WEIGHTED ? gwJ : nullptr, A.gcap,
+                          &s_nJ, n_rechk, *C.segs);
+        if (MIXED)
+            build_list<false>(A, A.Y, hx, hy, hz, cix, ciy, ciz, -1, A.rXY, gK, WEIGHTED ? gwK : nullptr,
+                              A.gcap, &s_nK, n_rechk, *C.segs);
+        __threadfence_block();
+        __syncthreads();
+        nJ = min(s_nJ, A.gcap);
+        nK = MIXED ? min(s_nK, A.gcap) : nJ;
+        LJ = gJ;
+        LK = MIXED ? gK : gJ;
+        WJ = gwJ;
+        WK = MIXED ? gwK : gwJ;
+    }
+    // Flush budget of the shared histogram: this anchor adds at most
+    // `tests` times.  Flush first if the total could pass the budget; an
+    // anchor whose tests alone exceed it counts into global memory.
+    bool smem_hist = !WEIGHTED && A.hist_in_smem;
+    if (smem_hist) {
+        const unsigned long long tests =
+            MIXED ? (unsigned long long)nJ * (unsigned long long)nK
+                  : (unsigned long long)nJ * (unsigned long long)(nJ > 0 ? nJ - 1 : 0) / 2;
+        if (tests > A.flush_budget) {
+            smem_hist = false;
         } else {
-        for (int rr = warp; rr < nJ; rr += kTWarps) {
-            const int half = rr >> 1;
-            const int jj = MIXED ? rr : ((rr & 1) ? nJ - 1 - half : half);
-            const float4 ej = LJ[jj];
-            const int bj = __float_as_int(ej.w) & 255;
-            const int jidx = (int)((unsigned)__float_as_int(ej.w) >> 8);
-            const double wij = WEIGHTED ? (double)hw * (double)WJ[jj] : 1.0;
-            const int ubase = bj * bins * bins;
-            const int k0 = MIXED ? 0 : jj + 1;
-            for (int kk = k0 + lane; kk < nK; kk += 32) {
-                const float4 ek = LK[kstepK * kk];
-                const float dx = ek.x - ej.x, dy = ek.y - ej.y, dz = ek.z - ej.z;
-                const float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-                const PairRule &r3 = MIXED ? A.rXY : A.rXX;
-                int bjk = fast_bin(d2, A.fc, bins);
-                if (bjk == -1) {
-                    ++n_rechk;
-                    const int kidx = (int)((unsigned)__float_as_int(ek.w) >> 8);
-                    const Cat &CK = MIXED ? A.Y : A.X;
-                    bjk = exact_third(hx, hy, hz, A.X.x[jidx], A.X.y[jidx], A.X.z[jidx],
-                                      CK.x[kidx], CK.y[kidx], CK.z[kidx], A.bpc, A.box, r3);
-                }
-                if (bjk >= 0) {
-                    const int bk = __float_as_int(ek.w) & 255;
-                    const int slot = ubase + bjk * bins + bk;
-                    ++n_tri;
-                    if (WEIGHTED) {
-                        atomicAdd(A.g_wsum + slot, wij * (double)WK[kk]);
-                    } else {  // (the shared histogram took the anchor above if it could)
-                        atomicAdd(A.g_count + slot, 1ull);
-                    }
-                }
+            if (C.since + tests > A.flush_budget) {
+                C.n_tri += flush_hist(C.U, bins, A.g_count);
+                C.since = 0;
+            }
+            C.since += tests;
+        }
+    }
+    // pass 2: pairs of neighbours
+    if (smem_hist) {
+        float4 *pad = spill ? (MIXED ? gK : gJ) : (MIXED ? sK : sJ);
+        for (int k = nK + tid; k < padded(nK); k += kTThreads)
+            pad[k] = make_float4(kFarAway, kFarAway, kFarAway, 0.f);
+        __syncthreads();
+        // the lists' address space is fixed per instantiation, so the
+        // shared-memory case (all but overflowing anchors) uses shared loads
+        if (spill) {
+            if (A.fc.far) tri_tiles<MIXED, true>(A, C, gJ, MIXED ? gK : gJ, nJ, nK, hx, hy, hz);
+            else tri_tiles<MIXED, false>(A, C, gJ, MIXED ? gK : gJ, nJ, nK, hx, hy, hz);
+        } else {
+            if (A.fc.far) tri_tiles<MIXED, true>(A, C, sJ, MIXED ? sK : sJ, nJ, nK, hx, hy, hz);
+            else tri_tiles<MIXED, false>(A, C, sJ, MIXED ? sK : sJ, nJ, nK, hx, hy, hz);
+        }
+        return;
+    }
+    // rows j dealt to warps in the order 0, n-1, 1, n-2, ... (XXX rows shrink with j)
+    for (int rr = warp; rr < nJ; rr += kTWarps) {
+        const int half = rr >> 1;
+        const int jj = MIXED ? rr : ((rr & 1) ? nJ - 1 - half : half);
+        const float4 ej = LJ[jj];
+        const int bj = __float_as_int(ej.w) & 255;
+        const int jidx = (int)((unsigned)__float_as_int(ej.w) >> 8);
+        const double wij = WEIGHTED ? (double)hw * (double)WJ[jj] : 1.0;
+        const int ubase = bj * bins * bins;
+        const int k0 = MIXED ? 0 : jj + 1;
+        for (int kk = k0 + lane; kk < nK; kk += 32) {
+            const float4 ek = LK[kk];
+            const float dx = ek.x - ej.x, dy = ek.y - ej.y, dz = ek.z - ej.z;
+            const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+            const PairRule &r3 = MIXED ? A.rXY : A.rXX;
+            int bjk = fast_bin3(r2, A.fc, bins);
+            if (bjk == -1) {
+                ++n_rechk;
+                const int kidx = (int)((unsigned)__float_as_int(ek.w) >> 8);
+                const Cat &CK = MIXED ? A.Y : A.X;
+                bjk = exact_third(hx, hy, hz, A.X.x[jidx], A.X.y[jidx], A.X.z[jidx], CK.x[kidx], CK.y[kidx],
+                                  CK.z[kidx], A.bpc, A.box, r3);
+            }
+            if (bjk >= 0) {
+                const int bk = __float_as_int(ek.w) & 255;
+                const int slot = ubase + bk * bins + bjk;
+                ++C.n_tri;
+                if (WEIGHTED) atomicAdd(A.g_wsum + slot, wij * (double)WK[kk]);
+                else atomicAdd(A.g_count + slot, 1ull);
             }
         }
-        }
+    }
 }
 
 template <bool MIXED, bool WEIGHTED>
 __global__ void __launch_bounds__(kTThreads, 1) k_triplets(const TripArgs A) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int bins = A.rXX.bins;
-    const int nb3 = bins * bins * bins;
-    // histogram + 32 dummy slots (see the unit-weight pass 2)
-    const size_t u_bytes = A.hist_in_smem ? (((size_t)(nb3 + 32) * 4 + 15) & ~(size_t)15) : 0;
+    const size_t u_bytes = A.hist_in_smem ? (((size_t)u_words(bins) * 4 + 15) & ~(size_t)15) : 0;
+    __shared__ SegTable s_segs;
     __shared__ int s_anchor, s_nJ, s_nK, s_unit;
     __shared__ unsigned s_stop;
     const int tid = threadIdx.x, lane = tid & 31;
-    TripCta C{reinterpret_cast<unsigned *>(smem), smem + u_bytes, &s_nJ, &s_nK, &s_unit, 0u, 0ull, 0ull};
+    TripCta C{reinterpret_cast<unsigned *>(smem), smem + u_bytes, &s_segs, &s_nJ, &s_nK, &s_unit, 0u, 0ull, 0ull};
     if (A.hist_in_smem)
-        for (int k = tid; k < nb3 + 32; k += kTThreads) C.U[k] = 0u;
+        for (int k = tid; k < u_words(bins); k += kTThreads) C.U[k] = 0u;
     long long taken = 0;  // anchors this CTA took (iteration cap: nX + 1)
-    __syncthreads();
+    int ticket = 0;       // thread 0: the next anchor, taken while the last one is counted
+    if (tid == 0) ticket = (int)atomicAdd(A.counter, 1ull);
     for (;;) {
         if (tid == 0) {
-            s_anchor = (int)atomicAdd(A.counter, 1ull);
+            s_anchor = ticket;
             s_nJ = 0;
             s_nK = 0;
             s_unit = 0;
@@ -537,13 +645,11 @@ __global__ void __launch_bounds__(kTThreads, 1) k_triplets(const TripArgs A) {
         __syncthreads();
         const int i = s_anchor;
         if (i >= A.nX || s_stop) break;
+        if (tid == 0) ticket = (int)atomicAdd(A.counter, 1ull);
         tri_anchor<MIXED, WEIGHTED>(A, i, C);
         __syncthreads();
     }
-    if (A.hist_in_smem) {
-        for (int k = tid; k < nb3; k += kTThreads)
-            if (C.U[k]) atomicAdd(A.g_count + k, (unsigned long long)C.U[k]);
-    }
+    if (A.hist_in_smem) C.n_tri += flush_hist(C.U, bins, A.g_count);
     unsigned long long rr = C.n_rechk, nt = C.n_tri;
     for (int off = 16; off > 0; off >>= 1) {
         rr += __shfl_down_sync(kFull, rr, off);
@@ -574,24 +680,24 @@ struct TripBatch {
 template <bool MIXED, bool WEIGHTED>
 __global__ void __launch_bounds__(kTThreads, 1) k_triplets_batch(const __grid_constant__ TripBatch B) {
     extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ SegTable s_segs;
     __shared__ long long s_anchor;
     __shared__ int s_nJ, s_nK, s_unit;
     __shared__ unsigned s_stop;
     const int tid = threadIdx.x, lane = tid & 31;
     const TripArgs &J0 = B.job[0];
     const int bins = J0.rXX.bins;
-    const int nb3 = bins * bins * bins;
     const bool in_smem = J0.hist_in_smem != 0;
-    const size_t u_bytes = in_smem ? (((size_t)(nb3 + 32) * 4 + 15) & ~(size_t)15) : 0;
-    TripCta C{reinterpret_cast<unsigned *>(smem), smem + u_bytes, &s_nJ, &s_nK, &s_unit, 0u, 0ull, 0ull};
+    const size_t u_bytes = in_smem ? (((size_t)u_words(bins) * 4 + 15) & ~(size_t)15) : 0;
+    TripCta C{reinterpret_cast<unsigned *>(smem), smem + u_bytes, &s_segs, &s_nJ, &s_nK, &s_unit, 0u, 0ull, 0ull};
     if (in_smem)
-        for (int k = tid; k < nb3 + 32; k += kTThreads) C.U[k] = 0u;
+        for (int k = tid; k < u_words(bins); k += kTThreads) C.U[k] = 0u;
     int cur = -1;  // the CTA's current job (uniform: every thread follows s_anchor)
-    long long taken = 0;
-    __syncthreads();
+    long long taken = 0, ticket = 0;  // ticket (thread 0): taken while the last anchor is counted
+    if (tid == 0) ticket = (long long)atomicAdd(B.counter, 1ull);
     for (;;) {
         if (tid == 0) {
-            s_anchor = (long long)atomicAdd(B.counter, 1ull);
+            s_anchor = ticket;
             s_nJ = 0;
             s_nK = 0;
             s_unit = 0;
@@ -603,12 +709,13 @@ __global__ void __launch_bounds__(kTThreads, 1) k_triplets_batch(const __grid_co
         __syncthreads();
         const long long g = s_anchor;
         if (g >= B.n_anchors || s_stop) break;
+        if (tid == 0) ticket = (long long)atomicAdd(B.counter, 1ull);
         // the job of anchor g (a CTA's anchors only move forward in the queue)
         if (cur < 0 || g >= B.job[cur].anchor_begin + B.job[cur].nX) {
             int j = cur < 0 ? 0 : cur;
             while (j + 1 < B.n_jobs && g >= B.job[j + 1].anchor_begin) ++j;
             if (cur >= 0 && in_smem && C.since) {
-                flush_hist(C.U, nb3, B.job[cur].g_count);
+                C.n_tri += flush_hist(C.U, bins, B.job[cur].g_count);
                 C.since = 0;
             }
             cur = j;
@@ -617,10 +724,7 @@ __global__ void __launch_bounds__(kTThreads, 1) k_triplets_batch(const __grid_co
         tri_anchor<MIXED, WEIGHTED>(A, (int)(g - A.anchor_begin), C);
         __syncthreads();
     }
-    if (in_smem && cur >= 0) {
-        for (int k = tid; k < nb3; k += kTThreads)
-            if (C.U[k]) atomicAdd(B.job[cur].g_count + k, (unsigned long long)C.U[k]);
-    }
+    if (in_smem && cur >= 0) C.n_tri += flush_hist(C.U, bins, B.job[cur].g_count);
     unsigned long long rr = C.n_rechk, nt = C.n_tri;
     for (int off = 16; off > 0; off >>= 1) {
         rr += __shfl_down_sync(kFull, rr, off);
@@ -648,14 +752,14 @@ __global__ void __launch_bounds__(kTThreads, 1) k_triplets_ani(const TripArgs A)
     const int bins = A.rXX.bins;
     float4 *sJ = reinterpret_cast<float4 *>(smem);
     float4 *sK = sJ + A.capJ;
-    unsigned short *aJ = reinterpret_cast<unsigned short *>(sK + (MIXED ? A.capK : 0));
-    unsigned short *aK = aJ + A.capJ;
-    float *swJ = reinterpret_cast<float *>(aK + (MIXED ? A.capK : 0) + 8);
+    float *swJ = reinterpret_cast<float *>(sK + (MIXED ? A.capK : 0));
     float *swK = swJ + (WEIGHTED ? A.capJ : 0);
-    // node / image words of the gated counts, 16-byte aligned past the weights
-    unsigned *gJ = reinterpret_cast<unsigned *>(
-        (reinterpret_cast<uintptr_t>(swK + (WEIGHTED && MIXED ? A.capK : 0)) + 15) & ~(uintptr_t)15);
-    unsigned *gK = gJ + A.capJ;
+    // node / image words of the gated counts, then the angle bins
+    unsigned *gJ = reinterpret_cast<unsigned *>(swK + (WEIGHTED && MIXED ? A.capK : 0));
+    unsigned *gK = gJ + (GATES ? A.capJ : 0);
+    unsigned char *aJ = reinterpret_cast<unsigned char *>(gK + (GATES && MIXED ? A.capK : 0));
+    unsigned char *aK = aJ + A.capJ;
+    __shared__ SegTable s_segs;
     __shared__ int s_anchor, s_nJ, s_nK;
     __shared__ unsigned s_stop;
     __shared__ GateBlock s_gates[GATES ? 64 : 1];
@@ -692,11 +796,10 @@ __global__ void __launch_bounds__(kTThreads, 1) k_triplets_ani(const TripArgs A)
         const int ciy = min(max((int)__fdiv_rn(hy, A.cell), 0), P - 1);
         const int ciz = min(max((int)__fdiv_rn(hz, A.cell), 0), P - 1);
         build_list<!ISO3>(A, A.X, hx, hy, hz, cix, ciy, ciz, -1, A.rXX, sJ, WEIGHTED ? swJ : nullptr,
-                          A.capJ, &s_nJ, n_rechk, aJ, 1, GATES ? gJ : nullptr);
+                          A.capJ, &s_nJ, n_rechk, s_segs, aJ, GATES ? gJ : nullptr);
         if (MIXED)
-            build_list<!ISO3>(A, A.Y, hx, hy, hz, cix, ciy, ciz, -1, A.rXY, sK,
-                              WEIGHTED ? swK : nullptr, A.capK, &s_nK, n_rechk, aK, 1,
-                              GATES ? gK : nullptr);
+            build_list<!ISO3>(A, A.Y, hx, hy, hz, cix, ciy, ciz, -1, A.rXY, sK, WEIGHTED ? swK : nullptr,
+                              A.capK, &s_nK, n_rechk, s_segs, aK, GATES ? gK : nullptr);
         GateNode n1{};
         if (GATES) n1 = gate_unpack(A.gate, gate_pack(A.gate, hx, hy, hz, 0u));
         __syncthreads();
@@ -708,13 +811,13 @@ __global__ void __launch_bounds__(kTThreads, 1) k_triplets_ani(const TripArgs A)
             continue;
         }
         const float4 *LK = MIXED ? sK : sJ;
-        const unsigned short *AK = MIXED ? aK : aJ;
+        const unsigned char *AK = MIXED ? aK : aJ;
         const float *WK = MIXED ? swK : swJ;
         for (int jj = warp; jj < nJ; jj += kTWarps) {
             const float4 ej = sJ[jj];
             const int jidx = (int)((unsigned)__float_as_int(ej.w) >> 8);
-            const unsigned short pj = ISO3 ? (unsigned short)(__float_as_int(ej.w) & 255) : aJ[jj];
-            const long long base = ISO3 ? (long long)pj * B2 : (long long)(pj & 255) * B4 + (long long)(pj >> 8) * B;
+            const int bj = __float_as_int(ej.w) & 255;
+            const long long base = ISO3 ? (long long)bj * B2 : (long long)bj * B4 + (long long)aJ[jj] * B;
             const double wij = WEIGHTED ? (double)hw * (double)swJ[jj] : 1.0;
             GateNode n2{};
             if (GATES) n2 = gate_unpack(A.gate, gJ[jj]);
@@ -723,9 +826,9 @@ __global__ void __launch_bounds__(kTThreads, 1) k_triplets_ani(const TripArgs A)
                 if (!MIXED && kk == jj) continue;
                 const float4 ek = LK[kk];
                 const float dx = ek.x - ej.x, dy = ek.y - ej.y, dz = ek.z - ej.z;
-                const float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+                const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
                 const PairRule &r3 = MIXED ? A.rXY : A.rXX;
-                int c = fast_bin(d2, A.fc, bins);
+                int c = fast_bin3(r2, A.fc, bins);
                 if (c == -1) {
                     ++n_rechk;
                     const int kidx = (int)((unsigned)__float_as_int(ek.w) >> 8);
@@ -743,8 +846,7 @@ __global__ void __launch_bounds__(kTThreads, 1) k_triplets_ani(const TripArgs A)
                     if (ISO3) {
                         slot = base + (long long)c * B + (__float_as_int(ek.w) & 255);
                     } else {
-                        const unsigned short pk = AK[kk];
-                        slot = base + (long long)(pk & 255) * B3 + (long long)c * B2 + (pk >> 8);
+                        slot = base + (long long)(__float_as_int(ek.w) & 255) * B3 + (long long)c * B2 + AK[kk];
                     }
                     n_tri += (unsigned long long)mult;
                     if (WEIGHTED) atomicAdd(A.g_wsum + slot, wij * (double)WK[kk] * (double)mult);
@@ -771,7 +873,8 @@ __global__ void k_to_double(const unsigned long long *__restrict__ c, const doub
     if (t < n) out[t] = weighted ? w[t] : (double)c[t];
 }
 
-// Ordered-triple histogram from the oriented counts U[b_ij][b_jk][b_ki].
+// Ordered-triple histogram from the oriented counts U[b_ij][b_ki][b_jk] (both
+// sums below are the same for U[b_ij][b_jk][b_ki]).
 __global__ void k_trip_finalize(const unsigned long long *__restrict__ cnt,
                                 const double *__restrict__ ws, int weighted, int mixed, int bins,
                                 double *__restrict__ out) {
@@ -826,25 +929,38 @@ static int64_t max_stencil_scan(const CellGrid &g, int P, const std::vector<RowD
 }
 
 // FP32 windows of the triplet kernels (u = 2^-24, R = dmax, L = box).  A list
-// entry, candidate - (anchor - shift), is off by u of itself (at most uR), and
-// where an axis is image-shifted by 2uL more; the third side's difference of
-// two entries adds u of itself.  Its vector is thus off by at most
-// sqrt(3) (2uR + 4uL) = 3.5uR + 6.9uL (no L term without a periodic box), and
-// d2 and r carry the pair kernel's 5u and 6.5u beside that (make_cuts).  The
-// windows keep more than twice these bounds; the anchor's sides, with one
-// entry's error, lie well inside.
+// entry, candidate - (anchor - shift), is off by u of itself (at most uR), where
+// an axis is image-shifted by 2uL more, and by u of itself again when scaled to
+// bins; the third side's difference of two entries adds u of itself.  Its vector
+// is thus off by at most sqrt(3) (4uR + 4uL) = 6.9uR + 6.9uL (no L term without a
+// periodic box), and d2 and r carry the pair kernel's 5u and 6.5u (make_cuts) and
+// the scale's u beside that.  The windows keep more than twice these bounds; the
+// anchor's sides, with one entry's error, lie well inside.
 static TripCuts trip_cuts(const PairRule &rule, float box, float dmax, bool bpc) {
     TripCuts c;
     const double dd = rule.dd, R = (double)dmax, L = bpc ? (double)box : 0.0;
     const double rmax = R * rule.ds + 1.0;
-    const double e_d2 = dd * std::ldexp(1.0, -19) + R * L * std::ldexp(1.0, -19);
-    const double wr = rmax * std::ldexp(1.0, -20) + rule.ds * (R * std::ldexp(1.0, -21) + L * std::ldexp(1.0, -20));
+    const double e_d2 = dd * std::ldexp(1.0, -18) + R * L * std::ldexp(1.0, -19);
+    const double wr = rmax * std::ldexp(1.0, -20) + rule.ds * (R + L) * std::ldexp(1.0, -20);
     c.dsf = (float)rule.ds;
     c.ds2 = c.dsf * c.dsf;
     c.lo = (float)(dd - e_d2);
     c.hi = (float)(dd + e_d2);
+    c.lo3 = (float)((dd - e_d2) * rule.ds * rule.ds);
+    c.hi3 = (float)((dd + e_d2) * rule.ds * rule.ds);
     // + the rounding of the fixed-point readout (2^-16)
     c.w = std::min(8000u, (unsigned)std::ceil((wr + std::ldexp(1.0, -16)) * 32768.0));
+    // dmax lies `gap` units below the last bin's edge: ds is rounded down to
+    // 1e-6, so gap is at most dmax * 0.033.  Up to 8 units (dmax of about 250)
+    // the window takes it in (a vote then finds a recheck in 5% of the steps
+    // instead of 3%); beyond, a window of its own costs four instructions a test.
+    const double edge = std::sqrt(dd) * rule.ds;
+    const double gap = std::ceil(std::max(0.0, (double)rule.bins - edge) * 32768.0);
+    c.far = gap > 8.0 ? 1 : 0;
+    c.wt = c.w + (c.far ? 0u : (unsigned)gap);
+    // r in [edge - w, edge + w] as values of r + 256 + w, one unit wider
+    c.qlo = (float)(256.0 + edge) - 0x1p-15f;
+    c.qhi = (float)(256.0 + edge) + (float)(2u * c.w + 1u) * 0x1p-15f;
     return c;
 }
 
@@ -879,10 +995,8 @@ static void trip_setup(pcf_ctx *ctx, const pcf_grid *X, const pcf_grid *Y, int P
     A.status = ctx->d_status;
     A.mixed = mixed ? 1 : 0;
     A.fc = trip_cuts(rXX, X->box, dmax, bpc);
-    const int n3 = bins * bins * bins;
-    // histogram + 32 dummy slots (the adds of 0 of lanes without a triangle)
-    const size_t u_bytes = ((size_t)(n3 + 32) * 4 + 15) & ~(size_t)15;
-    const size_t smem_max = 227 * 1024 - 64;
+    const size_t u_bytes = ((size_t)u_words(bins) * 4 + 15) & ~(size_t)15;
+    const size_t smem_max = 227 * 1024 - 128 - sizeof(SegTable);
     A.hist_in_smem = (!weighted && u_bytes <= 150 * 1024) ? 1 : 0;
     const size_t hist_b = A.hist_in_smem ? u_bytes : 0;
     const size_t ent = 16 + (weighted ? 4 : 0);
@@ -890,7 +1004,7 @@ static void trip_setup(pcf_ctx *ctx, const pcf_grid *X, const pcf_grid *Y, int P
     if (mixed && !(A.hist_in_smem && !weighted)) {
         A.capJ = (int)(room / ent / 3);
         A.capK = (int)(room / ent) - A.capJ;
-    } else {  // XXX, or XXY with one pooled buffer (J up, K down; see tri_anchor)
+    } else {  // XXX, or XXY with one pooled buffer (see tri_anchor)
         A.capJ = (int)(room / ent);
         A.capK = 0;
     }
@@ -1278,7 +1392,9 @@ static pcf_status count_triplets_ordered(pcf_ctx *ctx, const pcf_grid *x_, const
         A.capJ = (int)(room / ent) - 8;
         A.capK = 0;
     }
-    const size_t smem = (size_t)(A.capJ + A.capK) * ent + 64;
+    // (an entry's angle bin takes one of the two bytes `ent` counts: the row
+    // table has the rest)
+    const size_t smem = (size_t)(A.capJ + A.capK) * (ent - 1) + 64;
     const int64_t n5 = nh;
     PlanSlot *sl = nullptr;
     s = stage_plan(ctx, plan, &sl);
