@@ -36,20 +36,19 @@
 namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
-constexpr int kTThreads = 512;  // 16 warps, one CTA per SM
+constexpr int kTThreads = 768;  // 24 warps, one CTA per SM (16 warps left 30% of issue slots empty, 24 leave 20%)
 constexpr int kTWarps = kTThreads / 32;
 constexpr float kMagic = 256.0f;
 constexpr int kFracBits = 15;
 constexpr unsigned kFracMask = (1u << kFracBits) - 1u;
-constexpr unsigned kBinBias = 0x43800000u >> kFracBits;  // bits(256 + r) >> 15 = this + floor(r)
 struct TripCuts {
     float dsf, ds2;
     float lo, hi;    // d2 window around dd (image-aware bound for periodic boxes)
     float lo3, hi3;  // the same in bins^2 (third sides: list entries are in bins)
     unsigned w;      // edge window, 2^-15 units of r
-    // tiles (tri_tiles): the window with the distance from dmax to the last
-    // bin edge, where that is small (far = 0); else the window around dmax as
-    // values of r + 256 + w
+    // tiles (tri_tiles): the window in 2^-16 units with the distance from dmax
+    // to the last bin edge, where that is small (far = 0); else the window
+    // around dmax as values of r + 128 + w
     unsigned wt;
     int far;
     float qlo, qhi;
@@ -228,11 +227,12 @@ __device__ __forceinline__ int seg_table(const TripArgs &A, const Cat &C, int ci
     }
     if (lane == 31) T.wsum[warp] = x;
     __syncthreads();
-    int ws = T.wsum[lane & (kTWarps - 1)], w = ws;
+    const int ws = lane < kTWarps ? T.wsum[lane] : 0;
+    int w = ws;
     #pragma unroll
     for (int o = 1; o < kTWarps; o <<= 1) {
         const int y = __shfl_up_sync(kFull, w, o);
-        if ((lane & (kTWarps - 1)) >= o) w += y;
+        if (lane >= o) w += y;
     }
     const int total = __shfl_sync(kFull, w, kTWarps - 1);
     T.first[tid] = a;
@@ -241,23 +241,33 @@ __device__ __forceinline__ int seg_table(const TripArgs &A, const Cat &C, int ci
     return total;
 }
 
-// Appends the neighbours of anchor (hx,hy,hz) found in catalog C to a list.
-// Entries: {dx, dy, dz in bins, bits(idx << 8 | bin)}.  ang: their angle bins
-// (ANG).  ginfo (PCF_REF_NODE_GATES): per entry, its node on the reference's
-// grid and the axes of its image relative to the anchor (gate_pack).
+// Per-CTA scratch of the list builds.
+struct ListScratch {
+    SegTable seg;
+    int kept[2][kTWarps];  // entries of each warp's chunk, alternating rounds
+};
+
+// Lists the neighbours of anchor (hx,hy,hz) found in catalog C, in the order of
+// the stencil's cells, and returns their number; entries past cap are not
+// written.  Entries: {dx, dy, dz in bins, bits(idx << 8 | bin)}.  ang: their
+// angle bins (ANG).  ginfo (PCF_REF_NODE_GATES): per entry, its node on the
+// reference's grid and the axes of its image relative to the anchor
+// (gate_pack).  Called by the whole CTA; ends synchronised.
 //
-// All rows' candidates form one index space that the warps share 32 at a time
+// All rows' candidates form one index space that the CTA takes 768 at a time
 // (the range of an index by binary search): a row holds 10 to 100 candidates,
-// so a loop over rows kept 1 to 3 of 16 warps busy and cost a dependent
-// cell-table load per row.
+// so a loop over rows kept 1 to 3 warps busy and cost a dependent
+// cell-table load per row.  The order is kept (a barrier per round) so that
+// runs of entries stay close in space, for the culling of tri_tiles.
 template <bool ANG>
-__device__ void build_list(const TripArgs &A, const Cat &C, float hx, float hy, float hz, int cix, int ciy,
-                           int ciz, int only_after, const PairRule &rule, float4 *list, float *wlist,
-                           int cap, int *s_n, unsigned &n_rechk, SegTable &T, unsigned char *ang = nullptr,
-                           unsigned *ginfo = nullptr) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+__device__ int build_list(const TripArgs &A, const Cat &C, float hx, float hy, float hz, int cix, int ciy,
+                          int ciz, int only_after, const PairRule &rule, float4 *list, float *wlist, int cap,
+                          unsigned &n_rechk, ListScratch &S, unsigned char *ang = nullptr,
+                          unsigned *ginfo = nullptr) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    int n = 0, par = 0;
     for (int rb = 0; rb < A.n_rows; rb += kSegs / 2) {
-        const int total = seg_table(A, C, cix, ciy, ciz, only_after, rb, T);
+        const int total = seg_table(A, C, cix, ciy, ciz, only_after, rb, S.seg);
         const int nseg = 2 * min(kSegs / 2, A.n_rows - rb);
         const int top = 1 << (31 - __clz(nseg));
         // candidate of index q: its point, or -1 past the end; image axes in sh
@@ -265,18 +275,18 @@ __device__ void build_list(const TripArgs &A, const Cat &C, float hx, float hy, 
             if (q >= total) return -1;
             int s = 0;
             for (int o = top; o > 0; o >>= 1)
-                if (s + o < nseg && T.before[s + o] <= q) s += o;
-            const int f = T.first[s];
+                if (s + o < nseg && S.seg.before[s + o] <= q) s += o;
+            const int f = S.seg.first[s];
             sh = f >> 24;
-            return (f & 0xFFFFFF) + q - T.before[s];
+            return (f & 0xFFFFFF) + q - S.seg.before[s];
         };
-        int sh = 0, c = locate(warp * 32 + lane, sh);
+        int sh = 0, c = locate(tid, sh);
         float px = 0.f, py = 0.f, pz = 0.f;
         if (c >= 0) { px = C.x[c]; py = C.y[c]; pz = C.z[c]; }
-        for (int base = warp * 32; base < total; base += kTThreads) {
-            // the next chunk's points are on their way while this one is tested
+        for (int base = 0; base < total; base += kTThreads) {
+            // the next round's points are on their way while this one is tested
             int shn = 0;
-            const int cn = locate(base + kTThreads + lane, shn);
+            const int cn = locate(base + kTThreads + tid, shn);
             float nx = 0.f, ny = 0.f, nz = 0.f;
             if (cn >= 0) { nx = C.x[cn]; ny = C.y[cn]; nz = C.z[cn]; }
             int bin = -2, tang = 0;
@@ -299,21 +309,27 @@ __device__ void build_list(const TripArgs &A, const Cat &C, float hx, float hy, 
             }
             const bool keep = bin >= 0;
             const unsigned m = __ballot_sync(kFull, keep);
-            int off = 0;
-            if (lane == 0 && m) off = atomicAdd(s_n, __popc(m));
-            off = __shfl_sync(kFull, off, 0);
-            if (keep) {
-                const int pos = off + __popc(m & ((1u << lane) - 1u));
-                if (pos < cap) {
-                    list[pos] = make_float4(vx * A.fc.dsf, vy * A.fc.dsf, vz * A.fc.dsf,
-                                            __int_as_float((c << 8) | bin));
-                    if (wlist) wlist[pos] = C.w[c];
-                    if (ANG) ang[pos] = (unsigned char)tang;
-                    if (ginfo)
-                        ginfo[pos] = gate_pack(A.gate, px, py, pz,
-                                               ((sh & 3) != 1 ? 1u : 0u) | (((sh >> 2) & 3) != 1 ? 2u : 0u) |
-                                                   ((sh >> 4) != 1 ? 4u : 0u));
-                }
+            if (lane == 0) S.kept[par][warp] = __popc(m);
+            __syncthreads();
+            const int wk = lane < kTWarps ? S.kept[par][lane] : 0;
+            int x = wk;
+            #pragma unroll
+            for (int o = 1; o < kTWarps; o <<= 1) {
+                const int y = __shfl_up_sync(kFull, x, o);
+                if (lane >= o) x += y;
+            }
+            const int pos = n + __shfl_sync(kFull, x - wk, warp) + __popc(m & ((1u << lane) - 1u));
+            n += __shfl_sync(kFull, x, kTWarps - 1);
+            par ^= 1;
+            if (keep && pos < cap) {
+                list[pos] = make_float4(vx * A.fc.dsf, vy * A.fc.dsf, vz * A.fc.dsf,
+                                        __int_as_float((c << 8) | bin));
+                if (wlist) wlist[pos] = C.w[c];
+                if (ANG) ang[pos] = (unsigned char)tang;
+                if (ginfo)
+                    ginfo[pos] = gate_pack(A.gate, px, py, pz,
+                                           ((sh & 3) != 1 ? 1u : 0u) | (((sh >> 2) & 3) != 1 ? 2u : 0u) |
+                                               ((sh >> 4) != 1 ? 4u : 0u));
             }
             c = cn;
             sh = shn;
@@ -322,6 +338,8 @@ __device__ void build_list(const TripArgs &A, const Cat &C, float hx, float hy, 
             pz = nz;
         }
     }
+    __syncthreads();
+    return n;
 }
 
 // The shared histogram U of the unit-weight counts: bins^2 rows [b_ij][b_ki]
@@ -350,12 +368,19 @@ __device__ __forceinline__ unsigned long long flush_hist(unsigned *U, int bins, 
     return n;
 }
 
+// The extent of one chunk of the K list (in bins).
+struct ChunkBox {
+    float lo[3], hi[3];
+};
+
 // Per-CTA state of the anchor loop.
 struct TripCta {
     unsigned *U;                      // shared histogram (hist_in_smem)
     unsigned char *lists;             // shared neighbour lists
-    SegTable *segs;
-    int *s_nJ, *s_nK, *s_unit;        // shared counters
+    ListScratch *scr;
+    ChunkBox *boxes;                  // kMaxBoxes chunks of the K list
+    uint2 *queue;                     // 64 tests per warp on their way to the FP64 rule
+    int *s_unit;                      // shared counter
     unsigned n_rechk;
     unsigned long long n_tri;
     unsigned long long since;         // pair tests since U's last flush
@@ -364,39 +389,98 @@ struct TripCta {
 // A list position past the end: farther than dmax from every entry, and a
 // tile's j from a padded k too (they carry opposite signs).
 constexpr float kFarAway = 1e15f;
-constexpr int kTile = 8;    // j per tile
-constexpr int kChunkK = 32; // K lists are padded to whole chunks of one k per lane
+constexpr int kTile = 8;        // j per tile
+constexpr int kChunkK = 32;     // K lists are padded to whole chunks of one k per lane
+constexpr int kMaxBoxes = 256;  // chunks of a K list that take part in the culling
+// Fixed-point readout of a third side: bits(128 + r) >> 16 = kSideBias + bin
+constexpr float kSideMagic = 128.0f;
+constexpr int kSideBits = 16;
+constexpr unsigned kSideBias = 0x43000000u >> kSideBits;
+
+// Pads the K list to whole chunks and finds the chunks' extents.  Whole CTA;
+// ends synchronised.
+__device__ __forceinline__ void finish_k(TripCta &C, float4 *L, int nK) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int nchunk = (nK + kChunkK - 1) / kChunkK;
+    for (int c = warp; c < nchunk; c += kTWarps) {
+        const int k = c * kChunkK + lane;
+        float4 e = make_float4(kFarAway, kFarAway, kFarAway, 0.f);
+        if (k < nK) e = L[k];
+        else L[k] = e;
+        if (c < kMaxBoxes) {
+            const float v[3] = {e.x, e.y, e.z};
+            #pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                float lo = v[a], hi = k < nK ? v[a] : -kFarAway;
+                #pragma unroll
+                for (int o = 16; o > 0; o >>= 1) {
+                    lo = fminf(lo, __shfl_xor_sync(kFull, lo, o));
+                    hi = fmaxf(hi, __shfl_xor_sync(kFull, hi, o));
+                }
+                if (lane == 0) {
+                    C.boxes[c].lo[a] = lo;
+                    C.boxes[c].hi[a] = hi;
+                }
+            }
+        }
+    }
+    __syncthreads();
+}
+
+// The canonical rule for up to 32 tests that fell into a window, one per lane
+// (queue entries: j | fast bin << 24, k); corrects their counts in U.
+template <bool MIXED>
+__device__ __noinline__ void settle(const TripArgs &A, unsigned *U, const float4 *LJ, const float4 *LK,
+                                    const uint2 *queue, int n, float hx, float hy, float hz) {
+    const int lane = threadIdx.x & 31;
+    if (lane >= n) return;
+    const uint2 t = queue[lane];
+    const int bins = A.rXX.bins, fast = (int)(t.x >> 24);
+    const float4 ej = LJ[t.x & 0xFFFFFFu], ek = LK[t.y];
+    const int jidx = (int)((unsigned)__float_as_int(ej.w) >> 8);
+    const int kidx = (int)((unsigned)__float_as_int(ek.w) >> 8);
+    const Cat &CK = MIXED ? A.Y : A.X;
+    const int b = exact_third(hx, hy, hz, A.X.x[jidx], A.X.y[jidx], A.X.z[jidx], CK.x[kidx], CK.y[kidx],
+                              CK.z[kidx], A.bpc, A.box, MIXED ? A.rXY : A.rXX);
+    if (b == fast) return;
+    unsigned *row = U + ((__float_as_int(ej.w) & 255) * bins + (__float_as_int(ek.w) & 255)) * (bins + 1);
+    atomicSub(row + fast, 1u);
+    if (b >= 0) atomicAdd(row + b, 1u);
+}
 
 // Pass 2 of the unit-weight counts into U: tiles of kTile consecutive j
 // against the K list, one k per lane.  A step loads one k and tests it
-// against the tile's j, two at a time in packed FP32.
+// against the tile's j.
 //
-// What bounds it is the shared-memory pipe, with instruction issue close
-// behind: a reduction of 32 scattered counters costs 2.9 cycles of the SM
-// (conflicts), a 16-byte list load 4.  Tiles divide the loads by kTile, and the
-// step is kept branch-free and short: every test adds 1 to a counter, tests out
-// of range (their r clamped to bins + 1/2) to the row's last one, and tests
-// within the window of a bin edge as the fast path has them; the rare vote that
-// finds one in the window corrects the count by the FP64 rule afterwards.  The
-// constant increment also lets the hardware add lanes that hit one counter
-// together (32 cycles for a register operand where all lanes collide, 1 for the
-// constant).
+// What bounds it is instruction issue.  Tiles divide the list loads by kTile,
+// and the step is kept branch-free and short: every test adds 1 to a counter,
+// tests out of range (their r clamped to bins + 1/2) to the row's last one, and
+// tests within the window of a bin edge as the fast path has them; those are
+// queued (a rare vote finds them) and, 32 at a time, corrected by the FP64
+// rule.  The constant increment lets the hardware add lanes that hit one
+// counter together (32 cycles for a register operand where all lanes collide,
+// 1 for the constant).  The separations are scalar FP32: packed pairs issue
+// half as many FP instructions, but the moves that assemble the pairs come to
+// as many again, all on the FMA pipe's heavy half.
+// Half of all tests between two neighbours of one anchor are out of range: a
+// chunk whose extent is out of the tile's reach is skipped whole (the rounded
+// differences are monotone, so no test inside could have been in range).
 // FAR: dmax lies more than the window below the last bin's edge (bins / dmax
 // rounded down to 1e-6, large dmax), so it needs a window of its own.
 template <bool MIXED, bool FAR>
 __device__ __forceinline__ void tri_tiles(const TripArgs &A, TripCta &C, const float4 *__restrict__ LJ,
                                           const float4 *__restrict__ LK, int nJ, int nK, float hx, float hy,
                                           float hz) {
-    const int lane = threadIdx.x & 31;
-    const int bins = A.rXX.bins, rowlen = bins + 1;
-    unsigned *U = C.U;
-    const unsigned Us = (unsigned)__cvta_generic_to_shared(U) - 4u * kBinBias;
-    const unsigned w2s = (2u * A.fc.wt) << (32 - kFracBits);
-    const float mgw = kMagic + (float)A.fc.wt * 0x1p-15f;
-    const float qout = kMagic + (float)bins + 0.5f;
-    const float qlo = A.fc.qlo, qhi = A.fc.qhi, qedge = kMagic + (float)bins;
-    const unsigned kstride = 4u * (unsigned)rowlen, jstride = kstride * (unsigned)bins;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int bins = A.rXX.bins;
+    const float mgw = kSideMagic + (float)A.fc.wt * 0x1p-16f, qout = kSideMagic + (float)bins + 0.5f;
+    const float qlo = A.fc.qlo, qhi = A.fc.qhi, qedge = kSideMagic + (float)bins;
+    const unsigned w2 = 2u * A.fc.wt;
+    const unsigned Us = (unsigned)__cvta_generic_to_shared(C.U) - 4u * kSideBias;
+    const unsigned kstride = 4u * (unsigned)(bins + 1), jstride = kstride * (unsigned)bins;
     const int ntile = (nJ + kTile - 1) / kTile, nchunk = (nK + kChunkK - 1) / kChunkK;
+    uint2 *queue = C.queue + warp * 64;
+    int queued = 0;
     // units: tiles (XXX: the longest rows first), split along K while there
     // are few tiles per warp
     int segs = 1;
@@ -409,76 +493,85 @@ __device__ __forceinline__ void tri_tiles(const TripArgs &A, TripCta &C, const f
         u0 = __shfl_sync(kFull, u0, 0);
         if (u0 >= units) break;
         const int tile = u0 / segs, sg = u0 - tile * segs, j0 = tile * kTile;
-        float2 JX[kTile / 2], JY[kTile / 2], JZ[kTile / 2];
+        float JX[kTile], JY[kTile], JZ[kTile];
         unsigned jb[kTile];
+        float blo[3] = {kFarAway, kFarAway, kFarAway}, bhi[3] = {-kFarAway, -kFarAway, -kFarAway};
         #pragma unroll
         for (int q = 0; q < kTile; ++q) {
             float4 e = make_float4(-kFarAway, -kFarAway, -kFarAway, 0.f);
-            if (j0 + q < nJ) e = LJ[j0 + q];
-            (q & 1 ? JX[q / 2].y : JX[q / 2].x) = -e.x;
-            (q & 1 ? JY[q / 2].y : JY[q / 2].x) = -e.y;
-            (q & 1 ? JZ[q / 2].y : JZ[q / 2].x) = -e.z;
+            if (j0 + q < nJ) {
+                e = LJ[j0 + q];
+                blo[0] = fminf(blo[0], e.x);
+                bhi[0] = fmaxf(bhi[0], e.x);
+                blo[1] = fminf(blo[1], e.y);
+                bhi[1] = fmaxf(bhi[1], e.y);
+                blo[2] = fminf(blo[2], e.z);
+                bhi[2] = fmaxf(bhi[2], e.z);
+            }
+            JX[q] = e.x;
+            JY[q] = e.y;
+            JZ[q] = e.z;
             jb[q] = Us + (unsigned)(__float_as_int(e.w) & 255) * jstride;
         }
-        // the canonical rule for test (j0 + q, k), counted as u by the fast path
-        auto settle = [&](int q, int k, unsigned u) {
-            ++C.n_rechk;
-            const float4 ej = LJ[j0 + q], ek = LK[k];
-            const int jidx = (int)((unsigned)__float_as_int(ej.w) >> 8);
-            const int kidx = (int)((unsigned)__float_as_int(ek.w) >> 8);
-            const Cat &CK = MIXED ? A.Y : A.X;
-            const int b = exact_third(hx, hy, hz, A.X.x[jidx], A.X.y[jidx], A.X.z[jidx], CK.x[kidx],
-                                      CK.y[kidx], CK.z[kidx], A.bpc, A.box, MIXED ? A.rXY : A.rXX);
-            unsigned *row = U + ((__float_as_int(ej.w) & 255) * bins + (__float_as_int(ek.w) & 255)) * rowlen;
-            const int fast = (int)((u >> kFracBits) - kBinBias);
-            if (b != fast) {
-                atomicSub(row + fast, 1u);
-                if (b >= 0) atomicAdd(row + b, 1u);
-            }
-        };
         // head (XXX): the chunk that holds the tile itself, where k <= j is no test
         auto step = [&](int k, bool head) {
             const float4 e = LK[k];
-            const float2 KX = make_float2(e.x, e.x), KY = make_float2(e.y, e.y), KZ = make_float2(e.z, e.z);
             const unsigned kb = (unsigned)(__float_as_int(e.w) & 255) * kstride;
-            unsigned u[kTile], near = 0xffffffffu;
+            unsigned u[kTile], nearest = 0xffffffffu;  // the smallest fractions, two 16-bit lanes
             #pragma unroll
-            for (int p = 0; p < kTile / 2; ++p) {
-                const float2 DX = __fadd2_rn(KX, JX[p]), DY = __fadd2_rn(KY, JY[p]), DZ = __fadd2_rn(KZ, JZ[p]);
-                const float2 R2 = __ffma2_rn(DZ, DZ, __ffma2_rn(DY, DY, __fmul2_rn(DX, DX)));
-                float2 Q = __fadd2_rn(make_float2(sqrt_approx(R2.x), sqrt_approx(R2.y)), make_float2(mgw, mgw));
-                if (head) {
-                    if (k <= j0 + 2 * p) Q.x = qout;
-                    if (k <= j0 + 2 * p + 1) Q.y = qout;
-                }
-                if (FAR) {  // inside dmax's window: the unread counter, marked for the FP64 rule
-                    u[2 * p] = __float_as_uint(Q.x < qlo ? Q.x : Q.x < qhi ? qedge : qout);
-                    u[2 * p + 1] = __float_as_uint(Q.y < qlo ? Q.y : Q.y < qhi ? qedge : qout);
-                } else {
-                    u[2 * p] = __float_as_uint(fminf(Q.x, qout));
-                    u[2 * p + 1] = __float_as_uint(fminf(Q.y, qout));
-                }
-                // bits above the fraction shifted out: below w2s in the window
-                near = min(near, min(u[2 * p] << (32 - kFracBits), u[2 * p + 1] << (32 - kFracBits)));
-                asm volatile("red.shared.add.u32 [%0], 1;" ::"r"(jb[2 * p] + kb + 4u * (u[2 * p] >> kFracBits)));
-                asm volatile("red.shared.add.u32 [%0], 1;" ::"r"(jb[2 * p + 1] + kb + 4u * (u[2 * p + 1] >> kFracBits)));
+            for (int q = 0; q < kTile; ++q) {
+                const float dx = __fsub_rn(e.x, JX[q]), dy = __fsub_rn(e.y, JY[q]), dz = __fsub_rn(e.z, JZ[q]);
+                const float r2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
+                float s = __fadd_rn(sqrt_approx(r2), mgw);
+                if (head && k <= j0 + q) s = qout;
+                // FAR: inside dmax's window the unread counter, marked for the FP64 rule
+                if (FAR) s = s < qlo ? s : s < qhi ? qedge : qout;
+                else s = fminf(s, qout);
+                u[q] = __float_as_uint(s);
+                asm volatile("red.shared.add.u32 [%0], 1;" ::"r"(jb[q] + kb + 4u * (u[q] >> kSideBits)));
+                if ((q & 3) == 3)
+                    nearest = __vimin3_u16x2(nearest, __byte_perm(u[q - 3], u[q - 2], 0x5410),
+                                             __byte_perm(u[q - 1], u[q], 0x5410));
             }
-            if (__any_sync(kFull, near < w2s)) {
+            if (__any_sync(kFull, min(nearest & 0xFFFFu, nearest >> 16) < w2)) {
                 #pragma unroll
-                for (int q = 0; q < kTile; ++q)
-                    if ((u[q] << (32 - kFracBits)) < w2s) settle(q, k, u[q]);
+                for (int q = 0; q < kTile; ++q) {
+                    const bool hit = (u[q] & 0xFFFFu) < w2;
+                    const unsigned m = __ballot_sync(kFull, hit);
+                    if (!m) continue;
+                    if (hit)
+                        queue[queued + __popc(m & ((1u << lane) - 1u))] =
+                            make_uint2((unsigned)(j0 + q) | (((u[q] >> kSideBits) - kSideBias) << 24), (unsigned)k);
+                    C.n_rechk += hit;
+                    queued += __popc(m);
+                    __syncwarp();
+                    if (queued >= 32) {
+                        queued -= 32;
+                        settle<MIXED>(A, C.U, LJ, LK, queue + queued, 32, hx, hy, hz);
+                        __syncwarp();
+                    }
+                }
             }
         };
-        const int c0 = MIXED ? (int)((long long)nchunk * sg / segs) : j0 / kChunkK;
+        int c = MIXED ? (int)((long long)nchunk * sg / segs) : j0 / kChunkK;
         const int c1 = MIXED ? (int)((long long)nchunk * (sg + 1) / segs) : nchunk;
-        int k = c0 * kChunkK + lane;
-        const int kend = c1 * kChunkK;
-        if (!MIXED && c0 < c1) {
-            step(k, true);
-            k += kChunkK;
+        if (!MIXED) step(c++ * kChunkK + lane, true);
+        for (; c < c1; c += 32) {
+            bool in = c + lane < c1;
+            if (in && c + lane < kMaxBoxes) {
+                const ChunkBox &b = C.boxes[c + lane];
+                float g[3];
+                #pragma unroll
+                for (int a = 0; a < 3; ++a)
+                    g[a] = fmaxf(0.f, fmaxf(__fsub_rn(b.lo[a], bhi[a]), __fsub_rn(blo[a], b.hi[a])));
+                in = !(fmaf(g[2], g[2], fmaf(g[1], g[1], __fmul_rn(g[0], g[0]))) >= A.fc.hi3);
+            }
+            unsigned todo = __ballot_sync(kFull, in);
+            for (int k = c * kChunkK + lane; todo; k += kChunkK, todo >>= 1)
+                if (todo & 1u) step(k, false);
         }
-        for (; k < kend; k += kChunkK) step(k, false);
     }
+    if (queued) settle<MIXED>(A, C.U, LJ, LK, queue, queued, hx, hy, hz);
 }
 
 // All triangles of anchor i of job A: pass 1 builds the anchor's
@@ -488,7 +581,6 @@ template <bool MIXED, bool WEIGHTED>
 __device__ __forceinline__ void tri_anchor(const TripArgs &A, int i, TripCta &C) {
     const int bins = A.rXX.bins;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    int &s_nJ = *C.s_nJ, &s_nK = *C.s_nK;
     unsigned &n_rechk = C.n_rechk;
     float4 *sJ = reinterpret_cast<float4 *>(C.lists);
     float4 *sK = sJ + A.capJ;
@@ -509,39 +601,29 @@ __device__ __forceinline__ void tri_anchor(const TripArgs &A, int i, TripCta &C)
     // and behind it K, each list that is walked in chunks padded to them.
     const bool pool = !WEIGHTED && A.hist_in_smem;
     auto padded = [](int n) { return (n + kChunkK - 1) / kChunkK * kChunkK; };
-    build_list<false>(A, A.X, hx, hy, hz, cix, ciy, ciz, i, A.rXX, sJ, WEIGHTED ? swJ : nullptr, A.capJ,
-                      &s_nJ, n_rechk, *C.segs);
-    int capK = A.capK;
-    __syncthreads();
-    int nJ = s_nJ;
+    int nJ = build_list<false>(A, A.X, hx, hy, hz, cix, ciy, ciz, i, A.rXX, sJ, WEIGHTED ? swJ : nullptr, A.capJ,
+                               n_rechk, *C.scr);
+    int capK = A.capK, nK = nJ;
     if (MIXED) {
         if (pool) {
             sK = sJ + min(nJ, A.capJ);
             capK = max(0, A.capJ - nJ);
         }
-        build_list<false>(A, A.Y, hx, hy, hz, cix, ciy, ciz, -1, A.rXY, sK, WEIGHTED ? swK : nullptr, capK,
-                          &s_nK, n_rechk, *C.segs);
-        __syncthreads();
+        nK = build_list<false>(A, A.Y, hx, hy, hz, cix, ciy, ciz, -1, A.rXY, sK, WEIGHTED ? swK : nullptr, capK,
+                               n_rechk, *C.scr);
     }
-    int nK = MIXED ? s_nK : nJ;
     const float4 *LJ = sJ;
     const float4 *LK = MIXED ? sK : sJ;
     const float *WJ = swJ, *WK = MIXED ? swK : swJ;
     const bool spill = nJ > A.capJ || (MIXED && nK > capK) || (pool && padded(nK) > (MIXED ? capK : A.capJ));
     if (spill) {
-        // overflow: rebuild the lists in this CTA's global scratch (L2)
-        __syncthreads();
-        if (tid == 0) { s_nJ = 0; s_nK = 0; }
-        __syncthreads();
-        build_list<false>(A, A.X, hx, hy, hz, cix, ciy, ciz, i, A.rXX, gJ, WEIGHTED ? gwJ : nullptr, A.gcap,
-                          &s_nJ, n_rechk, *C.segs);
+        // overflow: the lists in this CTA's global scratch (L2), which holds any anchor's
+        nJ = min(A.gcap, build_list<false>(A, A.X, hx, hy, hz, cix, ciy, ciz, i, A.rXX, gJ,
+                                           WEIGHTED ? gwJ : nullptr, A.gcap, n_rechk, *C.scr));
+        nK = nJ;
         if (MIXED)
-            build_list<false>(A, A.Y, hx, hy, hz, cix, ciy, ciz, -1, A.rXY, gK, WEIGHTED ? gwK : nullptr,
-                              A.gcap, &s_nK, n_rechk, *C.segs);
-        __threadfence_block();
-        __syncthreads();
-        nJ = min(s_nJ, A.gcap);
-        nK = MIXED ? min(s_nK, A.gcap) : nJ;
+            nK = min(A.gcap, build_list<false>(A, A.Y, hx, hy, hz, cix, ciy, ciz, -1, A.rXY, gK,
+                                               WEIGHTED ? gwK : nullptr, A.gcap, n_rechk, *C.scr));
         LJ = gJ;
         LK = MIXED ? gK : gJ;
         WJ = gwJ;
@@ -567,16 +649,14 @@ __device__ __forceinline__ void tri_anchor(const TripArgs &A, int i, TripCta &C)
     }
     // pass 2: pairs of neighbours
     if (smem_hist) {
-        float4 *pad = spill ? (MIXED ? gK : gJ) : (MIXED ? sK : sJ);
-        for (int k = nK + tid; k < padded(nK); k += kTThreads)
-            pad[k] = make_float4(kFarAway, kFarAway, kFarAway, 0.f);
-        __syncthreads();
         // the lists' address space is fixed per instantiation, so the
         // shared-memory case (all but overflowing anchors) uses shared loads
         if (spill) {
+            finish_k(C, MIXED ? gK : gJ, nK);
             if (A.fc.far) tri_tiles<MIXED, true>(A, C, gJ, MIXED ? gK : gJ, nJ, nK, hx, hy, hz);
             else tri_tiles<MIXED, false>(A, C, gJ, MIXED ? gK : gJ, nJ, nK, hx, hy, hz);
         } else {
+            finish_k(C, MIXED ? sK : sJ, nK);
             if (A.fc.far) tri_tiles<MIXED, true>(A, C, sJ, MIXED ? sK : sJ, nJ, nK, hx, hy, hz);
             else tri_tiles<MIXED, false>(A, C, sJ, MIXED ? sK : sJ, nJ, nK, hx, hy, hz);
         }
@@ -617,15 +697,17 @@ __device__ __forceinline__ void tri_anchor(const TripArgs &A, int i, TripCta &C)
 }
 
 template <bool MIXED, bool WEIGHTED>
-__global__ void __launch_bounds__(kTThreads, 1) k_triplets(const TripArgs A) {
+__global__ void __launch_bounds__(kTThreads, 1) k_triplets(const __grid_constant__ TripArgs A) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int bins = A.rXX.bins;
     const size_t u_bytes = A.hist_in_smem ? (((size_t)u_words(bins) * 4 + 15) & ~(size_t)15) : 0;
-    __shared__ SegTable s_segs;
-    __shared__ int s_anchor, s_nJ, s_nK, s_unit;
+    __shared__ ListScratch s_scr;
+    __shared__ ChunkBox s_boxes[kMaxBoxes];
+    __shared__ uint2 s_queue[64 * kTWarps];
+    __shared__ int s_anchor, s_unit;
     __shared__ unsigned s_stop;
     const int tid = threadIdx.x, lane = tid & 31;
-    TripCta C{reinterpret_cast<unsigned *>(smem), smem + u_bytes, &s_segs, &s_nJ, &s_nK, &s_unit, 0u, 0ull, 0ull};
+    TripCta C{reinterpret_cast<unsigned *>(smem), smem + u_bytes, &s_scr, s_boxes, s_queue, &s_unit, 0u, 0ull, 0ull};
     if (A.hist_in_smem)
         for (int k = tid; k < u_words(bins); k += kTThreads) C.U[k] = 0u;
     long long taken = 0;  // anchors this CTA took (iteration cap: nX + 1)
@@ -634,8 +716,6 @@ __global__ void __launch_bounds__(kTThreads, 1) k_triplets(const TripArgs A) {
     for (;;) {
         if (tid == 0) {
             s_anchor = ticket;
-            s_nJ = 0;
-            s_nK = 0;
             s_unit = 0;
             unsigned stop = (A.ctrl && ctrl_load(A.ctrl)) ? PCF_GAVE_UP_ABORT : 0u;
             if (++taken > (long long)A.nX + 1) stop |= PCF_GAVE_UP_CAP;
@@ -680,16 +760,18 @@ struct TripBatch {
 template <bool MIXED, bool WEIGHTED>
 __global__ void __launch_bounds__(kTThreads, 1) k_triplets_batch(const __grid_constant__ TripBatch B) {
     extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ SegTable s_segs;
+    __shared__ ListScratch s_scr;
+    __shared__ ChunkBox s_boxes[kMaxBoxes];
+    __shared__ uint2 s_queue[64 * kTWarps];
     __shared__ long long s_anchor;
-    __shared__ int s_nJ, s_nK, s_unit;
+    __shared__ int s_unit;
     __shared__ unsigned s_stop;
     const int tid = threadIdx.x, lane = tid & 31;
     const TripArgs &J0 = B.job[0];
     const int bins = J0.rXX.bins;
     const bool in_smem = J0.hist_in_smem != 0;
     const size_t u_bytes = in_smem ? (((size_t)u_words(bins) * 4 + 15) & ~(size_t)15) : 0;
-    TripCta C{reinterpret_cast<unsigned *>(smem), smem + u_bytes, &s_segs, &s_nJ, &s_nK, &s_unit, 0u, 0ull, 0ull};
+    TripCta C{reinterpret_cast<unsigned *>(smem), smem + u_bytes, &s_scr, s_boxes, s_queue, &s_unit, 0u, 0ull, 0ull};
     if (in_smem)
         for (int k = tid; k < u_words(bins); k += kTThreads) C.U[k] = 0u;
     int cur = -1;  // the CTA's current job (uniform: every thread follows s_anchor)
@@ -698,8 +780,6 @@ __global__ void __launch_bounds__(kTThreads, 1) k_triplets_batch(const __grid_co
     for (;;) {
         if (tid == 0) {
             s_anchor = ticket;
-            s_nJ = 0;
-            s_nK = 0;
             s_unit = 0;
             unsigned stop = (J0.ctrl && ctrl_load(J0.ctrl)) ? PCF_GAVE_UP_ABORT : 0u;
             if (++taken > B.n_anchors + 1) stop |= PCF_GAVE_UP_CAP;
@@ -759,8 +839,8 @@ __global__ void __launch_bounds__(kTThreads, 1) k_triplets_ani(const TripArgs A)
     unsigned *gK = gJ + (GATES ? A.capJ : 0);
     unsigned char *aJ = reinterpret_cast<unsigned char *>(gK + (GATES && MIXED ? A.capK : 0));
     unsigned char *aK = aJ + A.capJ;
-    __shared__ SegTable s_segs;
-    __shared__ int s_anchor, s_nJ, s_nK;
+    __shared__ ListScratch s_scr;
+    __shared__ int s_anchor;
     __shared__ unsigned s_stop;
     __shared__ GateBlock s_gates[GATES ? 64 : 1];
     __shared__ signed char s_gate_by[GATES ? 64 : 1][2];
@@ -779,8 +859,6 @@ __global__ void __launch_bounds__(kTThreads, 1) k_triplets_ani(const TripArgs A)
     for (;;) {
         if (tid == 0) {
             s_anchor = (int)atomicAdd(A.counter, 1ull);
-            s_nJ = 0;
-            s_nK = 0;
             unsigned stop = (A.ctrl && ctrl_load(A.ctrl)) ? PCF_GAVE_UP_ABORT : 0u;
             if (++taken > (long long)A.nX + 1) stop |= PCF_GAVE_UP_CAP;
             if (stop && A.status) ctrl_store(A.status, stop);
@@ -795,15 +873,15 @@ __global__ void __launch_bounds__(kTThreads, 1) k_triplets_ani(const TripArgs A)
         const int cix = min(max((int)__fdiv_rn(hx, A.cell), 0), P - 1);
         const int ciy = min(max((int)__fdiv_rn(hy, A.cell), 0), P - 1);
         const int ciz = min(max((int)__fdiv_rn(hz, A.cell), 0), P - 1);
-        build_list<!ISO3>(A, A.X, hx, hy, hz, cix, ciy, ciz, -1, A.rXX, sJ, WEIGHTED ? swJ : nullptr,
-                          A.capJ, &s_nJ, n_rechk, s_segs, aJ, GATES ? gJ : nullptr);
-        if (MIXED)
-            build_list<!ISO3>(A, A.Y, hx, hy, hz, cix, ciy, ciz, -1, A.rXY, sK, WEIGHTED ? swK : nullptr,
-                              A.capK, &s_nK, n_rechk, s_segs, aK, GATES ? gK : nullptr);
+        const int nJ = build_list<!ISO3>(A, A.X, hx, hy, hz, cix, ciy, ciz, -1, A.rXX, sJ,
+                                         WEIGHTED ? swJ : nullptr, A.capJ, n_rechk, s_scr, aJ,
+                                         GATES ? gJ : nullptr);
+        const int nK = MIXED ? build_list<!ISO3>(A, A.Y, hx, hy, hz, cix, ciy, ciz, -1, A.rXY, sK,
+                                                 WEIGHTED ? swK : nullptr, A.capK, n_rechk, s_scr, aK,
+                                                 GATES ? gK : nullptr)
+                             : nJ;
         GateNode n1{};
         if (GATES) n1 = gate_unpack(A.gate, gate_pack(A.gate, hx, hy, hz, 0u));
-        __syncthreads();
-        const int nJ = s_nJ, nK = MIXED ? s_nK : s_nJ;
         if (nJ > A.capJ || (MIXED && nK > A.capK)) {
             // lists beyond shared memory: flagged for the host, anchor skipped
             if (tid == 0) atomicAdd(A.g_stats + 3, 1ull);
@@ -950,17 +1028,18 @@ static TripCuts trip_cuts(const PairRule &rule, float box, float dmax, bool bpc)
     c.hi3 = (float)((dd + e_d2) * rule.ds * rule.ds);
     // + the rounding of the fixed-point readout (2^-16)
     c.w = std::min(8000u, (unsigned)std::ceil((wr + std::ldexp(1.0, -16)) * 32768.0));
-    // dmax lies `gap` units below the last bin's edge: ds is rounded down to
-    // 1e-6, so gap is at most dmax * 0.033.  Up to 8 units (dmax of about 250)
-    // the window takes it in (a vote then finds a recheck in 5% of the steps
-    // instead of 3%); beyond, a window of its own costs four instructions a test.
+    // The tiles' window, in units of 2^-16: 1.25 times the bound and the rounding
+    // of the readout (a test in it costs about 40 instructions of its warp).  dmax lies `gap` units below the last bin's edge: ds is rounded down to
+    // 1e-6, so gap is at most dmax * 0.066.  Up to 16 units (dmax of about 250)
+    // the window takes it in; beyond, dmax gets a window of its own.
     const double edge = std::sqrt(dd) * rule.ds;
-    const double gap = std::ceil(std::max(0.0, (double)rule.bins - edge) * 32768.0);
-    c.far = gap > 8.0 ? 1 : 0;
-    c.wt = c.w + (c.far ? 0u : (unsigned)gap);
-    // r in [edge - w, edge + w] as values of r + 256 + w, one unit wider
-    c.qlo = (float)(256.0 + edge) - 0x1p-15f;
-    c.qhi = (float)(256.0 + edge) + (float)(2u * c.w + 1u) * 0x1p-15f;
+    const double gap = std::ceil(std::max(0.0, (double)rule.bins - edge) * 65536.0);
+    c.far = gap > 16.0 ? 1 : 0;
+    const double bound = (rmax * 7.5 + rule.ds * (R + L) * 6.93) / 256.0;
+    c.wt = std::min(16000u, (unsigned)std::ceil(bound * 1.25 + 0.5 + (c.far ? 0.0 : gap)));
+    // r in [edge - w, edge + w] as values of r + 128 + w, one unit wider
+    c.qlo = (float)(128.0 + edge) - 0x1p-16f;
+    c.qhi = (float)(128.0 + edge) + (float)(2u * c.wt + 1u) * 0x1p-16f;
     return c;
 }
 
@@ -996,7 +1075,8 @@ static void trip_setup(pcf_ctx *ctx, const pcf_grid *X, const pcf_grid *Y, int P
     A.mixed = mixed ? 1 : 0;
     A.fc = trip_cuts(rXX, X->box, dmax, bpc);
     const size_t u_bytes = ((size_t)u_words(bins) * 4 + 15) & ~(size_t)15;
-    const size_t smem_max = 227 * 1024 - 128 - sizeof(SegTable);
+    const size_t smem_max = 227 * 1024 - 128 - sizeof(ListScratch) - sizeof(ChunkBox) * kMaxBoxes -
+                            sizeof(uint2) * 64 * kTWarps;
     A.hist_in_smem = (!weighted && u_bytes <= 150 * 1024) ? 1 : 0;
     const size_t hist_b = A.hist_in_smem ? u_bytes : 0;
     const size_t ent = 16 + (weighted ? 4 : 0);
