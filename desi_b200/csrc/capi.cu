@@ -429,6 +429,28 @@ static pcf_status hist_scratch(pcf_ctx *ctx, int nb, unsigned long long **cnt, d
     return PCF_OK;
 }
 
+// The launch parameters of one pair histogram that follow from its arguments.
+static PairLaunch pair_launch(pcf_ctx *ctx, const pcf_grid *a, const pcf_grid *b, int kind, int bins, float dmax,
+                              uint32_t flags, bool weighted) {
+    const bool ani = kind != PCF_ISO, both = kind == PCF_BOTH, bpc = (flags & PCF_BPC) != 0, cross = b != nullptr;
+    PairLaunch pl;
+    pl.ani = ani;
+    pl.both = both;
+    pl.bpc = bpc;
+    pl.self = !cross;
+    pl.weighted = weighted;
+    pl.rule = make_pair_rule(bins, dmax, flags, ani && !both, bpc, cross);
+    if (both) pl.flags2 = make_pair_rule(bins, dmax, flags, true, bpc, cross).flags;
+    pl.mult = cross ? 1.0 : 2.0;
+    const pcf_grid *gs[2] = {a, cross ? b : a};
+    set_weight_fix(pl, gs, 2);
+    pl.wunscale = weight_unscale(a, cross ? b : a);
+    pl.ctrl = ctx->d_abort;
+    pl.status = ctx->d_status;
+    pl.variant = ctx->pair_variant;
+    return pl;
+}
+
 // One pair histogram; ds_override > 0 replaces the bin scale (the fine
 // histograms of the analytic path use (float)bins / dmax).
 static pcf_status count_pairs_impl(pcf_ctx *ctx, int kind, const pcf_grid *a_, const pcf_grid *b_,
@@ -460,16 +482,22 @@ static pcf_status count_pairs_impl(pcf_ctx *ctx, int kind, const pcf_grid *a_, c
                                           std::max<int64_t>(a->n, cross ? b->n : 0), a->box, dmax));
         if (it != ctx->tune.end()) te = it->second;
     }
-    // Both kinds run as the two single-kind launches written into one layout
-    // unless the autotuner found one pass faster for this call class (a
-    // tuned or forced scheme).  One pass saves the isotropic launch's
-    // candidate tests, but its isotropic copy takes the anisotropic copy's
-    // per-warp scheme, where lanes contend for few hot bins, and its extra
-    // shared memory can cost resident CTAs.  Measured (200k x 32 randoms,
-    // dmax 120, one batch each): exact weights, 40 bins: one pass 273 ms vs
-    // 74 + 146 ms; 48 bins: 500 vs 68 + 267 ms; signed weights (per-warp FP64
-    // copies either way), 40 bins: 381 vs 133 + 216 ms.
-    if (both && te.hist_mode < 0) {
+    // Both kinds of a call come from one pass over the candidates where
+    // k_pairs_lean counts them.  Otherwise they run as the two single-kind
+    // launches written into one layout unless the autotuner found one pass
+    // faster for this call class (a tuned or forced scheme): one pass of the
+    // general kernel saves the isotropic launch's candidate tests, but its
+    // isotropic copy takes the anisotropic copy's per-warp scheme, where lanes
+    // contend for few hot bins, and its extra shared memory can cost resident
+    // CTAs (signed weights, 40 bins, 200k points against 32 randoms: 381 vs 133 +
+    // 216 ms).
+    bool one_pass = te.hist_mode >= 0;
+    if (both && !one_pass) {
+        PairLaunch pl = pair_launch(ctx, a, b, kind, bins, dmax, flags, weighted);
+        pl.count = stats != nullptr;
+        one_pass = pair_lean(pl, a->box);
+    }
+    if (both && !one_pass) {
         pcf_stats si{}, sa{};
         pcf_status s = count_pairs_impl(ctx, PCF_ISO, a_, b_, bins, dmax, flags, hist,
                                         stats ? &si : nullptr, 0.0);
@@ -501,26 +529,10 @@ static pcf_status count_pairs_impl(pcf_ctx *ctx, int kind, const pcf_grid *a_, c
     double *d_ws, *d_out;
     s = hist_scratch(ctx, nb, &d_cnt, &d_ws, &d_stats, &d_out);
     if (s != PCF_OK) return s;
-    PairLaunch pl;
-    pl.ani = ani;
-    pl.both = both;
-    pl.bpc = bpc;
-    pl.self = !cross;
-    pl.weighted = weighted;
+    PairLaunch pl = pair_launch(ctx, a, b, kind, bins, dmax, flags, weighted);
     pl.hist_mode = te.hist_mode;
-    pl.rule = make_pair_rule(bins, dmax, flags, ani && !both, bpc, cross);
-    if (both) pl.flags2 = make_pair_rule(bins, dmax, flags, true, bpc, cross).flags;
     if (ds_override > 0) pl.rule.ds = ds_override;
-    pl.mult = cross ? 1.0 : 2.0;
-    {
-        const pcf_grid *gs[2] = {a, cross ? b : a};
-        set_weight_fix(pl, gs, 2);
-        pl.wunscale = weight_unscale(a, cross ? b : a);
-    }
     pl.count = stats != nullptr && !ctx->tune_timing;
-    pl.ctrl = ctx->d_abort;
-    pl.status = ctx->d_status;
-    pl.variant = ctx->pair_variant;
     pl.tile_cap = tile_cap;
     pl.chunk_cap = te.chunk;
     s = launch_pairs(ctx, plan, *a->cells, cross ? *b->cells : *a->cells, a->box, pl, d_cnt, d_ws,

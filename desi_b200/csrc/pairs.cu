@@ -33,6 +33,7 @@
 //  * A launch produces the isotropic histogram, the anisotropic one, or both
 //    from one pass over the candidates (PCF_BOTH).
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstring>
 #include <map>
@@ -81,6 +82,7 @@ constexpr int kLimbs = 3;
 #define PCF_GROUP_ANI 2
 #endif
 constexpr int kChunkMax = 8;            // work items per ticket, at most
+constexpr int kLeanWideBins = 120;      // bins up to which k_pairs_lean reads out 16 fraction bits
 
 // Fast-path cut constants for one range type (0: unshifted, 1: image-shifted).
 struct FastCuts {
@@ -89,6 +91,9 @@ struct FastCuts {
     float lo[2];      // d2 below lo (and >= tiny) is safely inside dmax
     float hi[2];      // d2 at or above hi is safely outside dmax
     unsigned w[2];    // edge window in 2^-15 units of r
+    // k_pairs_lean: the edge window in units of its readout, dmax included; 0
+    // where it does not apply (see make_cuts)
+    unsigned wl[2];
     float tiny;
 };
 
@@ -394,6 +399,51 @@ struct WarpState {
     int cj, slot;
 };
 
+// The candidate ranges of stencil row rw for home tile t of job J, whose
+// points lie in [zmn, zmx].
+__device__ __forceinline__ RowRange row_range(const PairArgs &A, const PairJob &J, const RowDesc rw, const TileDesc &t,
+                                              float zmn, float zmx) {
+    RowRange rr{0, 0, 0, 0, 0.f, 0.f, 0.f, 0};
+    int nx = t.ix + rw.dx, ny = t.iy + rw.dy;
+    const int P = J.P;
+    bool ok = true;
+    if (A.bpc) {
+        if (nx < 0) { nx += P; rr.sx = -A.box; } else if (nx >= P) { nx -= P; rr.sx = A.box; }
+        if (ny < 0) { ny += P; rr.sy = -A.box; } else if (ny >= P) { ny -= P; rr.sy = A.box; }
+    } else if (nx < 0 || nx >= P || ny < 0 || ny >= P) {
+        ok = false;
+    }
+    if (ok) {
+        const int col = (nx * P + ny) * P;
+        // the row's cells, clipped to those the home points reach in z:
+        // a candidate within dmax of a home point has z in (zmn - dmax,
+        // zmx + dmax), so its cell lies in [zcut_lo, zcut_hi] (with
+        // 1e-3 of a cell to spare for the rounding of z / cell here
+        // and in the grid build; the tile's own cells always stay);
+        // periodic images follow the same cell arithmetic past 0 and P
+        const float rcell = (float)P / A.box;
+        const int zcut_lo = min((int)floorf((zmn - A.zreach) * rcell - 1e-3f), (int)t.z0);
+        const int zcut_hi = max((int)floorf((zmx + A.zreach) * rcell + 1e-3f), (int)t.z1);
+        const int zhi = min(t.z1 + rw.kz, zcut_hi);
+        rr.kind = rw.kind;
+        const int *cs = J.cand.cstart;
+        if (rw.kind == 1) {  // forward half of the home column (XX): j > home index
+            rr.a0 = t.start;
+            rr.b0 = cs[col + min(zhi, P - 1) + 1];
+            if (A.bpc && zhi >= P) { rr.a1 = cs[col]; rr.b1 = cs[col + zhi - P + 1]; rr.sz1 = A.box; }
+        } else {
+            const int zlo = max(t.z0 - rw.kz, zcut_lo);
+            rr.a0 = cs[col + max(zlo, 0)];
+            rr.b0 = cs[col + min(zhi, P - 1) + 1];
+            if (A.bpc) {
+                if (zlo < 0) { rr.a1 = cs[col + zlo + P]; rr.b1 = cs[col + P]; rr.sz1 = -A.box; }
+                else if (zhi >= P) { rr.a1 = cs[col]; rr.b1 = cs[col + zhi - P + 1]; rr.sz1 = A.box; }
+            }
+        }
+    }
+    return rr;
+}
+
 // COUNT: also count the in-range pairs (weighted histograms, statistics on).
 // HM is the scheme of the anisotropic copy for K_ANI / K_BOTH launches.
 template <int KIND, bool WEIGHTED, int HM, bool COUNT, int VAR = 0>
@@ -560,46 +610,7 @@ __global__ void __launch_bounds__(kThreads, MinBlocks<KIND, HM, VAR>::value) k_p
         // Candidate ranges of all rows of the item, one row per lane, so the
         // dependent cell-table loads of different rows overlap.
         if (lane < nrows) {
-            RowRange rr{0, 0, 0, 0, 0.f, 0.f, 0.f, 0};
-            const RowDesc rw = J.rows[row_begin + lane];
-            int nx = t.ix + rw.dx, ny = t.iy + rw.dy;
-            const int P = J.P;
-            bool ok = true;
-            if (A.bpc) {
-                if (nx < 0) { nx += P; rr.sx = -A.box; } else if (nx >= P) { nx -= P; rr.sx = A.box; }
-                if (ny < 0) { ny += P; rr.sy = -A.box; } else if (ny >= P) { ny -= P; rr.sy = A.box; }
-            } else if (nx < 0 || nx >= P || ny < 0 || ny >= P) {
-                ok = false;
-            }
-            if (ok) {
-                const int col = (nx * P + ny) * P;
-                // the row's cells, clipped to those the home points reach in z:
-                // a candidate within dmax of a home point has z in (zmn - dmax,
-                // zmx + dmax), so its cell lies in [zcut_lo, zcut_hi] (with
-                // 1e-3 of a cell to spare for the rounding of z / cell here
-                // and in the grid build; the tile's own cells always stay);
-                // periodic images follow the same cell arithmetic past 0 and P
-                const float rcell = (float)P / A.box;
-                const int zcut_lo = min((int)floorf((zmn - A.zreach) * rcell - 1e-3f), (int)t.z0);
-                const int zcut_hi = max((int)floorf((zmx + A.zreach) * rcell + 1e-3f), (int)t.z1);
-                const int zhi = min(t.z1 + rw.kz, zcut_hi);
-                rr.kind = rw.kind;
-                const int *cs = J.cand.cstart;
-                if (rw.kind == 1) {  // forward half of the home column (XX): j > home index
-                    rr.a0 = t.start;
-                    rr.b0 = cs[col + min(zhi, P - 1) + 1];
-                    if (A.bpc && zhi >= P) { rr.a1 = cs[col]; rr.b1 = cs[col + zhi - P + 1]; rr.sz1 = A.box; }
-                } else {
-                    const int zlo = max(t.z0 - rw.kz, zcut_lo);
-                    rr.a0 = cs[col + max(zlo, 0)];
-                    rr.b0 = cs[col + min(zhi, P - 1) + 1];
-                    if (A.bpc) {
-                        if (zlo < 0) { rr.a1 = cs[col + zlo + P]; rr.b1 = cs[col + P]; rr.sz1 = -A.box; }
-                        else if (zhi >= P) { rr.a1 = cs[col]; rr.b1 = cs[col + zhi - P + 1]; rr.sz1 = A.box; }
-                    }
-                }
-            }
-            ws.rows[lane] = rr;
+            ws.rows[lane] = row_range(A, J, J.rows[row_begin + lane], t, zmn, zmx);
         }
         __syncwarp();
         const float4 *__restrict__ cpk = J.cand.pk;
@@ -906,6 +917,8 @@ __global__ void __launch_bounds__(kThreads, MinBlocks<KIND, HM, VAR>::value) k_p
     }
 }
 
+#include "pairs_lean.cuh"
+
 // Several histograms: out[s*nb + k] = mult[s] * hist[s*nb + k].
 __global__ void k_finalize_slots(const unsigned long long *__restrict__ cnt,
                                  const double *__restrict__ ws, int weighted,
@@ -1048,6 +1061,21 @@ static FastCuts make_cuts(const PairRule &rule, float box, float dmax) {
     // + the rounding of the fixed-point readout (2^-16)
     fc.w[0] = std::min(8000u, (unsigned)std::ceil((w_plain + std::ldexp(1.0, -16)) * 32768.0));
     fc.w[1] = std::min(8000u, (unsigned)std::ceil((w_shift + std::ldexp(1.0, -16)) * 32768.0));
+    // k_pairs_lean's windows, in units of its readout (2^-16 up to 120 bins, else
+    // 2^-15): 1.25 times the bounds above and the readout's rounding.  dmax lies
+    // `gap` units below the last bin's edge (bins / dmax is rounded down to
+    // 1e-6, so gap is at most dmax * 0.066); the windows take it in up to 16
+    // units, a dmax of about 250.  Beyond that, and where coordinates are so
+    // large against a bin that the window would take a tenth of it, the general
+    // kernel counts.
+    const double unit = rule.bins <= kLeanWideBins ? 65536.0 : 32768.0;
+    const double edge = std::sqrt(dd) * rule.ds;
+    const double gap = std::ceil(std::max(0.0, (double)rule.bins - edge) * unit);
+    const double rel = rmax * 6.5 * std::ldexp(1.0, -24), shift = rule.ds * (double)box * 3.47 * std::ldexp(1.0, -24);
+    const double w0 = std::ceil(1.25 * rel * unit + 0.5 + gap), w1 = std::ceil(1.25 * (rel + shift) * unit + 0.5 + gap);
+    const bool lean = rule.bins <= 255 && gap * (65536.0 / unit) <= 16.0 && w1 < 0.05 * unit;
+    fc.wl[0] = lean ? (unsigned)w0 : 0u;
+    fc.wl[1] = lean ? (unsigned)w1 : 0u;
     fc.tiny = 1e-30f;
     return fc;
 }
@@ -1071,39 +1099,11 @@ static int pair_variant(const PairLaunch &pl, int hm, int n_jobs = 1) {
     return (v == 3 && n_jobs != 1) ? 0 : v;  // shared copies hold one job's adds only
 }
 
-template <int KIND, bool W, int HM, bool C, int VAR = 0>
-static cudaError_t launch_one(const PairArgs &A, size_t smem, long long n_items, cudaStream_t st,
-                              int sm_count, int device) {
-    auto kfn = k_pairs<KIND, W, HM, C, VAR>;
-    // occupancy queries cost microseconds: cached per (device, shared-memory
-    // size) and instantiation, under a lock (several host threads launch)
-    struct Occ {
-        std::mutex mu;
-        std::map<std::pair<int, size_t>, int> per_sm;
-    };
-    static Occ occ;
-    cudaError_t e = ensure_smem_limit(reinterpret_cast<const void *>(kfn), device, smem);
-    if (e != cudaSuccess) return e;
-    int per_sm = 0;
-    {
-        std::lock_guard<std::mutex> lk(occ.mu);
-        auto it = occ.per_sm.find({device, smem});
-        if (it != occ.per_sm.end()) {
-            per_sm = it->second;
-        } else {
-            int per = 0;
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kfn, kThreads, smem);
-            if (e != cudaSuccess) return e;
-            per_sm = std::max(1, per);
-            occ.per_sm[{device, smem}] = per_sm;
-        }
-    }
-    const long long want = (n_items + kWarps - 1) / kWarps;
-    const int grid = (int)std::max(1LL, std::min<long long>(want, (long long)sm_count * per_sm));
-    // runs of k items per ticket while a queue holds >= 32 runs per warp (k at
-    // most 8, or the tuned cap that A.kchunk carries in)
+// The ticket shape of a launch of `warps` warps: runs of k items per ticket
+// while a queue holds >= 32 runs per warp (k at most 8, or the tuned cap that
+// A.kchunk carries in).
+static PairArgs with_tickets(const PairArgs &A, long long n_items, long long warps) {
     PairArgs B = A;
-    const long long warps = (long long)grid * kWarps;
     const long long cap = A.kchunk > 0 ? std::min<long long>(A.kchunk, kChunkMax) : kChunkMax;
     B.kchunk = (int)std::max(1LL, std::min<long long>(cap, n_items / (warps * 32)));
     B.n_chunked = B.kchunk > 1 ? std::max(0LL, n_items - 2 * warps) : 0;
@@ -1111,6 +1111,40 @@ static cudaError_t launch_one(const PairArgs &A, size_t smem, long long n_items,
     // a warp can take at most every ticket of the queue plus the one that
     // finds it empty
     B.max_tickets = B.t_chunked + (n_items - B.n_chunked) + 2;
+    return B;
+}
+
+// CTAs of `kfn` per SM (occupancy queries cost microseconds: cached per device
+// and shared-memory size, under a lock, as several host threads launch).
+struct OccCache {
+    std::mutex mu;
+    std::map<std::pair<int, size_t>, int> per_sm;
+    cudaError_t get(const void *kfn, int threads, int device, size_t smem, int *out) {
+        std::lock_guard<std::mutex> lk(mu);
+        auto it = per_sm.find({device, smem});
+        if (it == per_sm.end()) {
+            int per = 0;
+            const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kfn, threads, smem);
+            if (e != cudaSuccess) return e;
+            it = per_sm.insert({{device, smem}, std::max(1, per)}).first;
+        }
+        *out = it->second;
+        return cudaSuccess;
+    }
+};
+
+template <int KIND, bool W, int HM, bool C, int VAR = 0>
+static cudaError_t launch_one(const PairArgs &A, size_t smem, long long n_items, cudaStream_t st,
+                              int sm_count, int device) {
+    auto kfn = k_pairs<KIND, W, HM, C, VAR>;
+    static OccCache occ;
+    cudaError_t e = ensure_smem_limit(reinterpret_cast<const void *>(kfn), device, smem);
+    int per_sm = 0;
+    if (e == cudaSuccess) e = occ.get(reinterpret_cast<const void *>(kfn), kThreads, device, smem, &per_sm);
+    if (e != cudaSuccess) return e;
+    const long long want = (n_items + kWarps - 1) / kWarps;
+    const int grid = (int)std::max(1LL, std::min<long long>(want, (long long)sm_count * per_sm));
+    const PairArgs B = with_tickets(A, n_items, (long long)grid * kWarps);
     kfn<<<grid, kThreads, smem, st>>>(B);
     return cudaGetLastError();
 }
@@ -1160,9 +1194,74 @@ static int pair_scheme(const PairLaunch &pl) {
     return hm;
 }
 
-// Chooses the histogram mode of one launch and starts the kernel.
+template <int KIND, bool W, bool C, int FB, int NC>
+static cudaError_t launch_lean(const PairArgs &A, cudaStream_t st, int sm_count, int device) {
+    auto kfn = k_pairs_lean<KIND, W, C, FB, NC>;
+    const size_t smem = (size_t)LeanCopies<KIND, W, NC>::bytes(A.rule.bins);
+    static OccCache occ;
+    cudaError_t e = ensure_smem_limit(reinterpret_cast<const void *>(kfn), device, smem);
+    int per_sm = 0;
+    if (e == cudaSuccess) e = occ.get(reinterpret_cast<const void *>(kfn), LeanShape<W>::threads, device, smem, &per_sm);
+    if (e != cudaSuccess) return e;
+    constexpr int kLWarps = LeanShape<W>::warps;
+    const long long want = (A.n_items + kLWarps - 1) / kLWarps;
+    const int grid = (int)std::max(1LL, std::min<long long>(want, (long long)sm_count * per_sm));
+    kfn<<<grid, LeanShape<W>::threads, smem, st>>>(with_tickets(A, A.n_items, (long long)grid * kLWarps));
+    return cudaGetLastError();
+}
+
+// Columns per isotropic bin of a lean launch (32, 16 or 8): the most that let
+// two CTAs share an SM, else 8; 0 where not even that fits one CTA.
+static int lean_columns(const PairLaunch &pl) {
+    const int bins = pl.rule.bins;
+    const int kLWarps = pl.weighted ? LeanShape<true>::warps : LeanShape<false>::warps;
+    const size_t fixed = sizeof(LeanWarp) * kLWarps + sizeof(PairJob) + 2048;
+    const size_t ani = !pl.ani ? 0 : pl.weighted ? LeanCopies<K_ANI, true, 32>::ani(bins) : LeanCopies<K_ANI, false, 32>::ani(bins);
+    const bool cols = pl.weighted && (!pl.ani || pl.both);
+    for (int nc = 32; nc >= 8; nc >>= 1) {
+        const size_t iso = cols ? (size_t)kLWarps * (bins + 1) * 8 * nc : (size_t)kLWarps * (bins + 1) * 4;
+        const size_t room = nc > 8 && cols ? 114 * 1024 : 227 * 1024;
+        if (fixed + iso + ani <= room) return nc;
+    }
+    return 0;
+}
+
+// k_pairs_lean takes every launch of unit weights or exact integer weights that
+// its windows and its copies fit, unless a histogram scheme or a kernel variant
+// was asked for: it is the faster one at every size and bin count measured
+// (pairs_lean.cuh has both sides).
+bool pair_lean(const PairLaunch &pl, float box) {
+    if (pl.hist_mode >= 0 || pl.variant != 0 || (pl.weighted && !pl.wfix)) return false;
+    return make_cuts(pl.rule, box, std::sqrt((float)pl.rule.dd)).wl[0] != 0 && lean_columns(pl) != 0;
+}
+
+template <int KIND, int FB>
+static cudaError_t dispatch_lean(const PairArgs &A, const PairLaunch &pl, cudaStream_t st, int sm_count, int device) {
+    if (!pl.weighted) return launch_lean<KIND, false, false, FB, 32>(A, st, sm_count, device);
+    const int nc = KIND == K_ANI ? 32 : lean_columns(pl);
+    if (pl.count) {
+        if (nc == 32) return launch_lean<KIND, true, true, FB, 32>(A, st, sm_count, device);
+        if (nc == 16) return launch_lean<KIND, true, true, FB, KIND == K_ANI ? 32 : 16>(A, st, sm_count, device);
+        return launch_lean<KIND, true, true, FB, KIND == K_ANI ? 32 : 8>(A, st, sm_count, device);
+    }
+    if (nc == 32) return launch_lean<KIND, true, false, FB, 32>(A, st, sm_count, device);
+    if (nc == 16) return launch_lean<KIND, true, false, FB, KIND == K_ANI ? 32 : 16>(A, st, sm_count, device);
+    return launch_lean<KIND, true, false, FB, KIND == K_ANI ? 32 : 8>(A, st, sm_count, device);
+}
+
+// Chooses the kernel and histogram mode of one launch and starts it.
 static cudaError_t dispatch_pairs(PairArgs A, const PairLaunch &pl, cudaStream_t st,
                                   int sm_count, int device) {
+    if (pair_lean(pl, A.box)) {
+        A.budget = pl.weighted ? pl.lean_budget : 1 << 30;  // adds a column absorbs between flushes
+        const bool wide = pl.rule.bins <= kLeanWideBins;
+        if (pl.both) return wide ? dispatch_lean<K_BOTH, 16>(A, pl, st, sm_count, device)
+                                 : dispatch_lean<K_BOTH, 15>(A, pl, st, sm_count, device);
+        if (pl.ani) return wide ? dispatch_lean<K_ANI, 16>(A, pl, st, sm_count, device)
+                                : dispatch_lean<K_ANI, 15>(A, pl, st, sm_count, device);
+        return wide ? dispatch_lean<K_ISO, 16>(A, pl, st, sm_count, device)
+                    : dispatch_lean<K_ISO, 15>(A, pl, st, sm_count, device);
+    }
     const int hm = pair_scheme(pl);
     const size_t smem = hm == H_GLOBAL ? 0 : scheme_bytes(pl, hm, A.n_jobs);
     // budget: adds one shared counter absorbs between flushes; chunk:
@@ -1258,6 +1357,8 @@ void set_weight_fix(PairLaunch &pl, const pcf_grid *const *gs, int n) {
     if (budget < 4096) return;
     pl.wfix = true;
     pl.wbudget = (int)budget;
+    // two limbs with carries: the upper takes at most hi + 1 per add
+    pl.lean_budget = (int)std::min<unsigned long long>(1u << 30, 0xFFFFFFFFull / (hi + 1));
 }
 
 double weight_unscale(const pcf_grid *home, const pcf_grid *cand) {

@@ -385,6 +385,7 @@ struct PairLaunch {
                          // (weighted iso); -1 automatic
     bool wfix = false;   // exact integer weight products available (set_weight_fix)
     int wbudget = 0;     // limb adds between flushes of a fixed-point copy
+    int lean_budget = 0; // adds between flushes of a two-limb column (pairs_lean.cuh)
     double wunscale = 0.0;  // single-job launches: weight_unscale(home, cand)
     bool count = true;   // weighted launches: count in-range pairs (statistics)
     // queue control (pcf_ctx_abort): the abort word the kernel polls at every
@@ -398,6 +399,8 @@ struct PairLaunch {
 // Enables the fixed-point weighted histograms when every grid of the launch
 // has exact integer weights and any product fits the three-limb budget.
 void set_weight_fix(PairLaunch &pl, const pcf_grid *const *gs, int n);
+// Whether a launch runs k_pairs_lean (pairs_lean.cuh).
+bool pair_lean(const PairLaunch &pl, float box);
 // 2^-(wshift_home + wshift_cand): converts a fixed-point sum back to w*w units.
 double weight_unscale(const pcf_grid *home, const pcf_grid *cand);
 std::string tune_key(int kind, bool bpc, bool cross, bool weighted, int bins, int64_t n, float box,
