@@ -390,14 +390,20 @@ class PcfServer:
                 s.ctx.close()
 
     # -- a timed stream ----------------------------------------------------
-    def run_stream(self, reqs: list[Request]) -> dict:
-        """Submit requests at their arrival times; wait for all; report."""
+    def run_stream(self, reqs: list[Request], tick_s: float = 0.005) -> dict:
+        """Submit requests at their arrival times; wait for all; report.
+        Arrivals within tick_s after the one that is due are submitted with
+        it: each wake-up of this thread takes the interpreter lock from the
+        slots, and small requests now take less than a millisecond."""
         a0 = _lib.alloc_counters()
         t0 = time.perf_counter()
+        due = -1.0
         for r in sorted(reqs, key=lambda r: r.arrival):
-            delay = t0 + r.arrival - time.perf_counter()
-            if delay > 0:
-                time.sleep(delay)
+            if r.arrival > due:
+                due = r.arrival + tick_s
+                delay = t0 + r.arrival - time.perf_counter()
+                if delay > 0:
+                    time.sleep(delay)
             self.submit(r)
         results = [r.future.result() for r in reqs]
         t1 = time.perf_counter()
