@@ -1054,27 +1054,28 @@ pcf_status grid_finish(pcf_ctx *ctx, const pcf_grid *g_) {
     return PCF_OK;
 }
 
-// Cells per side for a counting call: cell size about dmax/4 (so the
-// stencil hugs the dmax sphere), coarsened while cells would hold fewer
-// than ~6 points on average, and kept so that a periodic stencil never
-// wraps onto itself (2k+1 <= P).
+// Cells per side for a counting call: `refine` cells per dmax, as many as keep
+// the stencil at `refine` cells each way (plan_rows adds a margin to dmax, so a
+// cell of exactly dmax / refine would need one more: 2iso of 1.5M points at dmax
+// 20 took 2757 us at 55 cells per side, 1340 us at 54).  Without a caller's
+// choice, 4 or 3 cells per dmax while a cell holds 12 points on average, else 2
+// while it holds 6, else 1 (us per DD + DR, isotropic: 300000 points, box 1000,
+// dmax 100: 1325 at 3 cells, 1620 at 4; 10^6 points: 10083 and 9738; 2000 points,
+// box 250, dmax 80: 55, 59, 98 and 136 at 1, 2, 3 and 4).  Triplet counts, where
+// a candidate costs an anchor's CTA more, take 4 or 3 from 6 points on.  A periodic stencil never wraps onto
+// itself (2k + 2 <= P).
 int choose_partitions(int64_t n, float box, float dmax, int kind, bool bpc, int refine) {
+    double least = 6.0;  // points per cell at 3 cells per dmax or more
     if (refine <= 0) {
         const char *e = getenv("PCF_REFINE");  // experiment / autotuner override
         refine = e ? atoi(e) : 4;
         if (refine < 1 || refine > 16) refine = 4;
+        if (!e && kind != kTripletCells) least = 12.0;
     }
     double L = box, R = dmax;
-    int P = (int)std::floor(L / (R / refine));
-    // mean occupancy floor
-    while (P > 1) {
-        double occ = (double)n / ((double)P * P * P);
-        if (occ >= 6.0) break;
-        int nr = refine - 1;
-        if (nr < 1) break;
-        refine = nr;
-        P = (int)std::floor(L / (R / refine));
-    }
+    auto cells = [&](int r) { return (int)std::floor(L * (r - 1e-4) / (R + 8.0 * L * 1.2e-7) * (1.0 - 1e-9)); };
+    int P = cells(refine);
+    while (P > 1 && refine > 1 && (double)n / ((double)P * P * P) < (refine > 2 ? least : 6.0)) P = cells(--refine);
     P = std::max(1, std::min(P, 256));
     if (bpc) {
         // need 2k+1 <= P with k = ceil(R / (L/P)) (+1 for the tile span)
@@ -1085,7 +1086,6 @@ int choose_partitions(int64_t n, float box, float dmax, int kind, bool bpc, int 
             ++P;
         }
     }
-    (void)kind;
     return P;
 }
 

@@ -342,7 +342,9 @@ cudaError_t ensure_smem_limit(const void *fn, int device, size_t bytes);
 // grid_finish first; it is a no-op for a finished grid.
 pcf_status grid_ensure_cells(pcf_ctx *ctx, pcf_grid *g, int P, bool defer = false);
 pcf_status grid_finish(pcf_ctx *ctx, const pcf_grid *g);
-int choose_partitions(int64_t n, float box, float dmax, int kind, bool bpc, int npoint_kind);
+// kind: a histogram kind, or kTripletCells.
+constexpr int kTripletCells = 3;
+int choose_partitions(int64_t n, float box, float dmax, int kind, bool bpc, int refine);
 
 // Stencil of one pair launch (host).  Work items are implicit: item i is
 // (tile i / n_chunks, rows [c*rows_per_item, ...) of chunk c = i % n_chunks).

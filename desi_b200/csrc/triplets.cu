@@ -1131,7 +1131,7 @@ extern "C" pcf_status pcf_count_triplets(pcf_ctx *ctx, int kind, const pcf_grid 
     if (X->n >= (1 << 24) || (Y && Y->n >= (1 << 24))) return PCF_ERR_UNSUPPORTED;
     if (ctx_abort_requested(ctx) != PCF_OK) return PCF_ERR_TIMEOUT;
     int P = 0;
-    pcf_status s = prepare_grids(ctx, X, Y, dmax, PCF_ISO, bpc, &P);
+    pcf_status s = prepare_grids(ctx, X, Y, dmax, kTripletCells, bpc, &P);
     if (s != PCF_OK) return s;
     const CellGrid &gx = *X->cells;
     const CellGrid &gy = mixed ? *Y->cells : gx;
@@ -1250,7 +1250,7 @@ extern "C" pcf_status pcf_batch_triplets(pcf_ctx *ctx, const pcf_grid *d_, const
     }
     if (D->n >= (1 << 24)) return PCF_ERR_UNSUPPORTED;
     int P = 0;
-    pcf_status s = prepare_grids(ctx, big, nullptr, dmax, PCF_ISO, bpc, &P);
+    pcf_status s = prepare_grids(ctx, big, nullptr, dmax, kTripletCells, bpc, &P);
     if (s != PCF_OK) return s;
     // every structure queued before the first is completed
     if ((s = grid_ensure_cells(ctx, D, P, true)) != PCF_OK) return s;
@@ -1436,7 +1436,7 @@ static pcf_status count_triplets_ordered(pcf_ctx *ctx, const pcf_grid *x_, const
     if (X->n >= (1 << 24) || (Y && Y->n >= (1 << 24))) return PCF_ERR_UNSUPPORTED;
     if (ctx_abort_requested(ctx) != PCF_OK) return PCF_ERR_TIMEOUT;
     int P = 0;
-    pcf_status s = prepare_grids(ctx, X, Y, dmax, PCF_ISO, bpc, &P);
+    pcf_status s = prepare_grids(ctx, X, Y, dmax, kTripletCells, bpc, &P);
     if (s != PCF_OK) return s;
     const CellGrid &gx = *X->cells;
     const CellGrid &gy = mixed ? *Y->cells : gx;
