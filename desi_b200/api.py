@@ -8,7 +8,9 @@ Every call goes to the CUDA library; errors raise :class:`PcfError`.
 """
 from __future__ import annotations
 
+import collections
 import ctypes
+import weakref
 
 import numpy as np
 
@@ -41,6 +43,38 @@ def as_points(a) -> np.ndarray:
     return a
 
 
+class _Results:
+    """Arrays for large histograms (256 KB to 16 MB) over blocks that come back
+    when the last view of an array is gone: a new array's pages are brought in
+    one fault at a time (2 MB: 0.3 to 1 ms, as long as its count).  Keeps at most
+    four blocks each of four sizes.  deque operations are atomic, so blocks may
+    come back from any thread."""
+
+    LOW, HIGH = 256 << 10, 16 << 20
+
+    def __init__(self):
+        self._spare = {}
+
+    def take(self, n: int) -> np.ndarray:
+        size = 8 * n
+        if not self.LOW <= size <= self.HIGH:
+            return np.zeros(n, np.float64)
+        spare = self._spare.get(size)
+        if spare is None:
+            if len(self._spare) >= 4:
+                self._spare = {}
+            spare = self._spare.setdefault(size, collections.deque(maxlen=4))
+        try:
+            block = spare.pop()
+        except IndexError:
+            block = (ctypes.c_char * size)()
+        # every view's base is this array (its own base is no array), so it
+        # outlives them all
+        out = np.frombuffer(block, np.float64)
+        weakref.finalize(out, spare.append, block).atexit = False
+        return out
+
+
 class Context:
     """One CUDA stream on one device; owns the grids it builds."""
 
@@ -50,6 +84,7 @@ class Context:
         _check(None, self._lib.pcf_ctx_create(device, ctypes.byref(h)), "pcf_ctx_create")
         self.handle = h
         self.device = device
+        self._results = _Results()
 
     @property
     def stream(self) -> int:
@@ -156,7 +191,7 @@ class Context:
             f |= PCF_DEVICE_OUT
             out, outp = None, ctypes.c_void_p(out_device_ptr)
         else:
-            out = np.zeros(nb, np.float64)
+            out = self._results.take(nb)
             outp = out.ctypes.data_as(ctypes.c_void_p)
         rc = self._lib.pcf_count_triplets(self.handle, PCF_ANI if ani else PCF_ISO, x.handle,
                                           y.handle if y is not None else None, int(bins),
@@ -186,7 +221,7 @@ class Context:
             self.handle, d.handle, int(bins), float(dmax), int(ptt), int(bn_ref), int(wrap),
             ddd.ctypes.data_as(ctypes.c_void_p) if ddd is not None else None,
             ddr.ctypes.data_as(ctypes.c_void_p), rrr.ctypes.data_as(ctypes.c_void_p),
-            ctypes.byref(st))
+            ctypes.byref(st) if stats else None)
         _check(self.handle, rc, "pcf_analytic_3iso")
         s = (bins, bins, bins)
         res = (ddd.reshape(s) if ddd is not None else None, ddr.reshape(s), rrr.reshape(s))

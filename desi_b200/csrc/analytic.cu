@@ -270,7 +270,7 @@ extern "C" pcf_status pcf_analytic_3iso(pcf_ctx *ctx, const pcf_grid *d_, int bi
     // DDD, counted (XXX3iso_BPC)
     if (ddd) {
         pcf_stats st{};
-        s = pcf_count_triplets(ctx, PCF_ISO, D, nullptr, bins, dmax, PCF_BPC, ddd, &st);
+        s = pcf_count_triplets(ctx, PCF_ISO, D, nullptr, bins, dmax, PCF_BPC, ddd, stats ? &st : nullptr);
         if (s != PCF_OK) return s;
         kernel_ms += st.kernel_ms;
     }
@@ -295,7 +295,7 @@ extern "C" pcf_status pcf_analytic_3iso(pcf_ctx *ctx, const pcf_grid *d_, int bi
         const float dsf = (float)nbf / dmax;
         pcf_stats st{};
         s = pcf_count_pairs_ds(ctx, D, (int)nbf, dmax, (double)dsf, PCF_BPC | PCF_DEVICE_OUT,
-                               pass ? dd_ffr : dd_ff, &st);
+                               pass ? dd_ffr : dd_ff, stats ? &st : nullptr);  // statistics make a call wait
         if (s != PCF_OK) return s;
         kernel_ms += st.kernel_ms;
     }
@@ -320,9 +320,13 @@ extern "C" pcf_status pcf_analytic_3iso(pcf_ctx *ctx, const pcf_grid *d_, int bi
     k_refine<<<(unsigned)n3, 256, 0, st>>>(bins, bn_ref, dr, alpha_ref, ffr, partial, d_ddr, d_rrr);
     PCF_CU(ctx, cudaGetLastError());
     ctx->launches += 6;
-    PCF_CU(ctx, cudaMemcpyAsync(ddr, d_ddr, sizeof(double) * n3, cudaMemcpyDeviceToHost, st));
-    PCF_CU(ctx, cudaMemcpyAsync(rrr, d_rrr, sizeof(double) * n3, cudaMemcpyDeviceToHost, st));
-    PCF_CU(ctx, cudaStreamSynchronize(st));
+    std::vector<char> spill;
+    const char *hb = nullptr;
+    s = fetch_block(ctx, d_ddr, sizeof(double) * 2 * n3, spill, &hb);  // [ddr | rrr]
+    if (s == PCF_OK) s = ctx_queue_status(ctx);
+    if (s != PCF_OK) return s;
+    memcpy(ddr, hb, sizeof(double) * n3);
+    memcpy(rrr, hb + sizeof(double) * n3, sizeof(double) * n3);
     if (stats) {
         stats->kernel_ms = kernel_ms;
         stats->partitions = D->cells ? D->cells->P : 0;

@@ -188,7 +188,7 @@ extern "C" pcf_status pcf_batch_pairs(pcf_ctx *ctx, int kind, const pcf_grid *d_
         int64_t total = 0;
         for (auto &j : js) {
             const auto &rp = rows[j.P];
-            total += (int64_t)j.hc->tiles.size() * (int64_t)(j.self ? rp.first.size() : rp.second.size());
+            total += j.hc->n_tiles * (int64_t)(j.self ? rp.first.size() : rp.second.size());
         }
         // plan buffer: row tables | jobs | mults
         std::map<int, std::pair<size_t, size_t>> roff;  // [P] -> (self, cross) byte offsets
@@ -218,7 +218,7 @@ extern "C" pcf_status pcf_batch_pairs(pcf_ctx *ctx, int kind, const pcf_grid *d_
             j.wunscale = weight_unscale(js[k].h, js[k].c);
             j.tiles = h.d_tiles.as<TileDesc>();
             j.rows = reinterpret_cast<const RowDesc *>(dp + (js[k].self ? roff[js[k].P].first : roff[js[k].P].second));
-            shape_job(j, (int64_t)h.tiles.size(), (int)(js[k].self ? rp.first.size() : rp.second.size()),
+            shape_job(j, h.n_tiles, (int)(js[k].self ? rp.first.size() : rp.second.size()),
                       total, ctx->sm_count);
             j.slot = k;
             j.item_begin = item;
@@ -228,7 +228,7 @@ extern "C" pcf_status pcf_batch_pairs(pcf_ctx *ctx, int kind, const pcf_grid *d_
             j.rule_flags2 = 0;  // single-kind jobs
             j.pad = 0;
             j.P = js[k].P;
-            item += (long long)h.tiles.size() * j.n_chunks;
+            item += (long long)h.n_tiles * j.n_chunks;
             mult[k] = js[k].mult;
             bg->keep.push_back(js[k].hc);
             bg->keep.push_back(js[k].cc);
@@ -292,18 +292,19 @@ extern "C" pcf_status pcf_batch_pairs(pcf_ctx *ctx, int kind, const pcf_grid *d_
         ctx->launches += 2;
     }
     // results
-    std::vector<double> host((size_t)bg->nb * bg->nslots);
-    unsigned long long hs[4] = {0, 0, 0, 0};
-    PCF_CU(ctx, cudaMemcpyAsync(host.data(), bg->d_out, sizeof(double) * host.size(), cudaMemcpyDeviceToHost, st));
-    PCF_CU(ctx, cudaMemcpyAsync(hs, bg->d_stats, sizeof(hs), cudaMemcpyDeviceToHost, st));
-    PCF_CU(ctx, cudaStreamSynchronize(st));
-    s = ctx_queue_status(ctx);
+    std::vector<char> spill;
+    const char *hb = nullptr;
+    s = fetch_block(ctx, bg->d_stats, 128 + sizeof(double) * (size_t)bg->nb * bg->nslots, spill, &hb);
+    if (s == PCF_OK) s = ctx_queue_status(ctx);
     if (s != PCF_OK) return s;
+    unsigned long long hs[4];
+    memcpy(hs, hb, sizeof(hs));
+    const double *host = reinterpret_cast<const double *>(hb + 128);  // [stats | counter | out]
     int k = 0;
-    if (dd) memcpy(dd, host.data() + (size_t)(k++) * nb, sizeof(double) * nb);
+    if (dd) memcpy(dd, host + (size_t)(k++) * nb, sizeof(double) * nb);
     for (int i = 0; i < n_rand; ++i) {
-        if (rr) memcpy(rr + (size_t)i * nb, host.data() + (size_t)(k++) * nb, sizeof(double) * nb);
-        if (dr) memcpy(dr + (size_t)i * nb, host.data() + (size_t)(k++) * nb, sizeof(double) * nb);
+        if (rr) memcpy(rr + (size_t)i * nb, host + (size_t)(k++) * nb, sizeof(double) * nb);
+        if (dr) memcpy(dr + (size_t)i * nb, host + (size_t)(k++) * nb, sizeof(double) * nb);
     }
     if (stats) {
         float ms = 0.f;

@@ -46,7 +46,7 @@ pcf_status pcf_ctx_create(int device, pcf_ctx **out) {
     c->device = device;
     for (DevBuf *b : {&c->scratch_a, &c->scratch_b, &c->scratch_c, &c->d_hist, &c->d_flag})
         b->pool = c->scratch_pool;
-    for (PlanSlot &sl : c->slots) sl.d_rows.pool = sl.d_counter.pool = c->scratch_pool;
+    for (PlanSlot &sl : c->slots) sl.d.pool = c->scratch_pool;
     if (cudaSetDevice(device) != cudaSuccess ||
         cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreate(&c->ev0) != cudaSuccess || cudaEventCreate(&c->ev1) != cudaSuccess) {
@@ -167,7 +167,7 @@ pcf_status pcf_ctx_profile(pcf_ctx *ctx, int enable) {
     ctx->profile = enable != 0;
     ctx->prof_used = 0;
     ctx->prof_grid_used = 0;
-    ctx->prof_grid_points = 0;
+    ctx->prof_grid_points = ctx->prof_grid_builds = 0;
     return PCF_OK;
 }
 
@@ -183,10 +183,10 @@ pcf_status pcf_ctx_profile_read_grid(pcf_ctx *ctx, double *total_ms, int64_t *bu
         tot += ms;
     }
     if (total_ms) *total_ms = tot;
-    if (builds) *builds = (int64_t)ctx->prof_grid_used;
+    if (builds) *builds = ctx->prof_grid_builds;
     if (points) *points = ctx->prof_grid_points;
     ctx->prof_grid_used = 0;
-    ctx->prof_grid_points = 0;
+    ctx->prof_grid_points = ctx->prof_grid_builds = 0;
     return PCF_OK;
 }
 
@@ -240,15 +240,6 @@ cudaError_t ensure_smem_limit(const void *fn, int device, size_t bytes) {
 
 extern "C" {
 
-static bool is_device_ptr(const void *p) {
-    cudaPointerAttributes a;
-    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
-}
-
 pcf_status pcf_grid_build(pcf_ctx *ctx, const pcf_point *pts, int64_t n, float box,
                           int partitions, pcf_grid **out) {
     if (!ctx || !pts || !out || n < 1 || !(box > 0.f) || partitions < 0 || partitions > 320)
@@ -258,18 +249,18 @@ pcf_status pcf_grid_build(pcf_ctx *ctx, const pcf_point *pts, int64_t n, float b
     cudaSetDevice(ctx->device);
     std::unique_ptr<pcf_grid> g(new pcf_grid);
     g->pool = ctx->pool;
-    g->raw.pool = ctx->pool;
+    g->raw.pool = g->flags.pool = ctx->pool;
     g->n = n;
     g->box = box;
     PCF_CU(ctx, g->raw.ensure(sizeof(float4) * (size_t)n));
-    PCF_CU(ctx, cudaMemcpyAsync(g->raw.p, pts, sizeof(float4) * (size_t)n,
-                                is_device_ptr(pts) ? cudaMemcpyDeviceToDevice
-                                                   : cudaMemcpyHostToDevice,
-                                ctx->stream));
     g->user_P = partitions;
-    int P = partitions > 0 ? partitions : choose_partitions(n, box, box / 8.f, PCF_ISO, false, 4);
     g->owner = ctx;
-    pcf_status s = grid_ensure_cells(ctx, g.get(), P, ctx->grid_defer);
+    // the caller's partitions are gridded here; without them the first count
+    // that uses the grid chooses (a structure made before it is known for which
+    // dmax would be thrown away)
+    pcf_status s = grid_take(ctx, g.get(), pts);
+    if (s == PCF_OK && partitions > 0) s = grid_ensure_cells(ctx, g.get(), partitions, true);
+    if (s == PCF_OK && !ctx->grid_defer) s = grid_finish(ctx, g.get());
     if (s != PCF_OK) return s;
     *out = g.release();
     return PCF_OK;
@@ -287,9 +278,9 @@ pcf_status pcf_grid_free(pcf_ctx *ctx, pcf_grid *g) {
 pcf_status pcf_grid_info(const pcf_grid *g, int64_t *n, float *box, int *partitions,
                          int64_t *nonempty_cells, int *unit_weights) {
     if (!g) return PCF_ERR_INVALID_ARG;
-    if (g->owner) {  // a deferred build completes here
+    if (g->owner) {  // a queued build completes here
         cudaSetDevice(g->owner->device);
-        pcf_status s = grid_finish(g->owner, g);
+        pcf_status s = grid_default_cells(g->owner, const_cast<pcf_grid *>(g));
         if (s != PCF_OK) return s;
     }
     if (n) *n = g->n;
@@ -297,8 +288,10 @@ pcf_status pcf_grid_info(const pcf_grid *g, int64_t *n, float *box, int *partiti
     if (partitions) *partitions = g->cells ? g->cells->P : 0;
     if (nonempty_cells) {
         int64_t c = 0;
-        if (g->cells) {
-            const auto &h = g->cells->h_start;
+        if (g->cells && g->owner) {
+            std::vector<int> h;
+            pcf_status s = grid_host_starts(g->owner, g, h);
+            if (s != PCF_OK) return s;
             for (size_t i = 0; i + 1 < h.size(); ++i) c += h[i + 1] > h[i];
         }
         *nonempty_cells = c;
@@ -309,10 +302,10 @@ pcf_status pcf_grid_info(const pcf_grid *g, int64_t *n, float *box, int *partiti
 
 pcf_status pcf_grid_download(pcf_ctx *ctx, const pcf_grid *g, pcf_point *pts_out,
                              int32_t *cell_start_out) {
-    if (!ctx || !g || !g->cells) return PCF_ERR_INVALID_ARG;
+    if (!ctx || !g) return PCF_ERR_INVALID_ARG;
     cudaSetDevice(ctx->device);
     {
-        pcf_status s0 = grid_finish(ctx, g);
+        pcf_status s0 = grid_default_cells(ctx, const_cast<pcf_grid *>(g));
         if (s0 != PCF_OK) return s0;
     }
     std::vector<float> planes;
@@ -334,8 +327,12 @@ pcf_status pcf_grid_download(pcf_ctx *ctx, const pcf_grid *g, pcf_point *pts_out
             o[4 * i + 3] = planes[3 * n + i];
         }
     }
-    if (cell_start_out)
-        memcpy(cell_start_out, g->cells->h_start.data(), sizeof(int) * g->cells->h_start.size());
+    if (cell_start_out) {
+        std::vector<int> h;
+        pcf_status s0 = grid_host_starts(ctx, g, h);
+        if (s0 != PCF_OK) return s0;
+        memcpy(cell_start_out, h.data(), sizeof(int) * h.size());
+    }
     return PCF_OK;
 }
 
@@ -519,7 +516,7 @@ static pcf_status count_pairs_impl(pcf_ctx *ctx, int kind, const pcf_grid *a_, c
     if (s != PCF_OK) return s;
     const int tile_cap = te.tile == 16 ? 16 : kTileCap;
     if (tile_cap == 16) {
-        s = ensure_half_tiles(ctx, *a->cells);
+        s = ensure_half_tiles(ctx, *a->cells, a->n);
         if (s != PCF_OK) return s;
     }
     PairPlan plan;
@@ -533,34 +530,28 @@ static pcf_status count_pairs_impl(pcf_ctx *ctx, int kind, const pcf_grid *a_, c
     pl.hist_mode = te.hist_mode;
     if (ds_override > 0) pl.rule.ds = ds_override;
     pl.count = stats != nullptr && !ctx->tune_timing;
+    pl.timed = stats != nullptr;
     pl.tile_cap = tile_cap;
     pl.chunk_cap = te.chunk;
     s = launch_pairs(ctx, plan, *a->cells, cross ? *b->cells : *a->cells, a->box, pl, d_cnt, d_ws,
                      d_stats);
     if (s != PCF_OK) return s;
     const bool dev_out = (flags & PCF_DEVICE_OUT) != 0;
-    s = finalize_hist(ctx, d_cnt, d_ws, pl.weighted, pl.mult, nb, dev_out ? hist : d_out);
+    OutPath o;
+    s = out_open(ctx, nb, dev_out, hist, d_out, &o);
+    if (s != PCF_OK) return s;
+    s = finalize_hist(ctx, d_cnt, d_ws, pl.weighted, pl.mult, nb, o.to, d_stats, stats || !dev_out ? o.stats : nullptr);
     if (s != PCF_OK) return s;
     if (stats || !dev_out) {
-        // results come back through the context's page-locked buffer: copies
-        // into pageable memory go through the driver's staging, where the
-        // request server's concurrent slots were seen to stall one another
-        const size_t hb = dev_out ? 0 : sizeof(double) * nb;
-        const size_t cb = (stats && !pl.weighted) ? sizeof(unsigned long long) * nb : 0;
-        s = pcf_ensure_pinned(ctx, hb + cb + 64);
-        if (s != PCF_OK) return s;
-        char *hp = static_cast<char *>(ctx->h_pinned);
-        if (hb) PCF_CU(ctx, cudaMemcpyAsync(hp, d_out, hb, cudaMemcpyDeviceToHost, ctx->stream));
-        if (cb) PCF_CU(ctx, cudaMemcpyAsync(hp + hb, d_cnt, cb, cudaMemcpyDeviceToHost, ctx->stream));
-        PCF_CU(ctx, cudaMemcpyAsync(hp + hb + cb, d_stats, 32, cudaMemcpyDeviceToHost, ctx->stream));
-        PCF_CU(ctx, cudaStreamSynchronize(ctx->stream));
-        s = ctx_queue_status(ctx);
-        if (s != PCF_OK) return s;
-        if (hb) memcpy(hist, hp, hb);
         unsigned long long hs[4];
-        memcpy(hs, hp + hb + cb, sizeof(hs));
-        if (cb) {  // unit weights: pairs = sum of the counts
-            const unsigned long long *cnt = reinterpret_cast<const unsigned long long *>(hp + hb);
+        s = out_close(ctx, o, nb, dev_out, hist, hs);
+        if (s != PCF_OK) return s;
+        if (stats && !pl.weighted) {  // unit weights: pairs = sum of the counts
+            std::vector<char> spill;
+            const char *h = nullptr;
+            s = fetch_block(ctx, d_cnt, sizeof(unsigned long long) * (size_t)nb, spill, &h);
+            if (s != PCF_OK) return s;
+            const unsigned long long *cnt = reinterpret_cast<const unsigned long long *>(h);
             hs[2] = 0;
             for (int q = 0; q < nb; ++q) hs[2] += cnt[q];
         }

@@ -151,12 +151,28 @@ PinnedPool::~PinnedPool() {
     for (auto &kv : free_blocks) cudaFreeHost(kv.second);
 }
 
-CellGrid::~CellGrid() {
-    if (ready) {  // the stage may still feed the tile table's copy
+HostNote::~HostNote() {
+    if (ready) {  // the device may still write into the block
         cudaEventSynchronize(ready);
         cudaEventDestroy(ready);
     }
-    if (stage && pinned) pinned->put(stage, stage_bytes);
+    if (block && pinned) pinned->put(block, bytes);
+}
+
+cudaError_t HostNote::open(const std::shared_ptr<PinnedPool> &pool, size_t n) {
+    pinned = pool;
+    cudaError_t e = block ? cudaSuccess : pinned->get(n, &block, &bytes);
+    if (e == cudaSuccess && !ready) e = cudaEventCreateWithFlags(&ready, cudaEventDisableTiming);
+    return e;
+}
+
+cudaError_t HostNote::wait(void *to, size_t n) {
+    const cudaError_t e = cudaEventSynchronize(ready);
+    if (e != cudaSuccess) return e;
+    memcpy(to, block, n);
+    pinned->put(block, bytes);
+    block = nullptr;
+    return cudaSuccess;
 }
 
 cudaError_t DevBuf::ensure(size_t n) {
@@ -258,6 +274,7 @@ __device__ __forceinline__ void flush_flags(unsigned f, unsigned wmax, unsigned 
     }
 }
 
+// flags (null: not wanted): the catalog's flags, zeroed by the caller.
 __global__ void k_cell_ids(const float4 *__restrict__ pts, int64_t n, int P, float cell, float box,
                            int *__restrict__ cid, int *__restrict__ rank,
                            int *__restrict__ counts, int *__restrict__ flags) {
@@ -265,12 +282,55 @@ __global__ void k_cell_ids(const float4 *__restrict__ pts, int64_t n, int P, flo
     unsigned f = 0u, wmax = 0u, wminc = 0u;
     if (i < n) {
         const float4 p = pts[i];
-        point_flags(p, box, f, wmax, wminc);
+        if (flags) point_flags(p, box, f, wmax, wminc);
         const int c = cell_of_point(p, P, cell);
         cid[i] = c;
         rank[i] = atomicAdd(&counts[c], 1);
     }
-    flush_flags(f, wmax, wminc, flags);
+    if (flags) flush_flags(f, wmax, wminc, flags);
+}
+
+// Takes a catalog in: copies it to dst (unless it is already there, dst ==
+// pts) and checks it.  One read and one write of the points, where a copy and a
+// check of their own read them twice.  With one block the flags are stored, and
+// go to the host's block as well; with more they are merged into zeroed words.
+constexpr int kIntakeThreads = 256, kIntakeUnroll = 8, kIntakeOneBlock = 4096;
+__global__ void __launch_bounds__(kIntakeThreads) k_intake(const float4 *pts, float4 *dst, int64_t n, float box,
+                                                           int *__restrict__ flags, unsigned *host) {
+    unsigned f = 0u, wmax = 0u, wminc = 0u;
+    const int64_t step = (int64_t)gridDim.x * kIntakeThreads;
+    for (int64_t i = (int64_t)blockIdx.x * kIntakeThreads + threadIdx.x; i < n; i += kIntakeUnroll * step) {
+        float4 p[kIntakeUnroll];
+        #pragma unroll
+        for (int u = 0; u < kIntakeUnroll; ++u)
+            if (i + u * step < n) p[u] = pts[i + u * step];
+        #pragma unroll
+        for (int u = 0; u < kIntakeUnroll; ++u) {
+            if (i + u * step >= n) break;
+            point_flags(p[u], box, f, wmax, wminc);
+            if (dst != pts) dst[i + u * step] = p[u];
+        }
+    }
+    if (gridDim.x > 1) {
+        flush_flags(f, wmax, wminc, flags);
+        return;
+    }
+    __shared__ unsigned s_f[3];
+    if (threadIdx.x < 3) s_f[threadIdx.x] = 0u;
+    __syncthreads();
+    f = __reduce_or_sync(0xffffffffu, f);
+    wmax = __reduce_max_sync(0xffffffffu, wmax);
+    wminc = __reduce_max_sync(0xffffffffu, wminc);
+    if ((threadIdx.x & 31) == 0) {
+        atomicOr(&s_f[0], f);
+        atomicMax(&s_f[1], wmax);
+        atomicMax(&s_f[2], wminc);
+    }
+    __syncthreads();
+    if (threadIdx.x < 3) {
+        flags[threadIdx.x] = (int)s_f[threadIdx.x];
+        host[threadIdx.x] = s_f[threadIdx.x];
+    }
 }
 
 // Exclusive scan of one 1024-element chunk per block; the chunk total goes to
@@ -509,15 +569,13 @@ __device__ void block_excl_scan4(int *a, int q, int *wsum) {
 }
 
 __global__ void __launch_bounds__(kBktThreads) k_bkt_count(const float4 *__restrict__ pts, int64_t n,
-                                                           int64_t span, int P, float cell, float box,
-                                                           int Q, float rq, int K, int *__restrict__ M,
-                                                           int *__restrict__ flags) {
+                                                           int64_t span, int P, float cell, int Q, float rq,
+                                                           int K, int *__restrict__ M) {
     extern __shared__ int hist[];
     for (int k = threadIdx.x; k < K; k += blockDim.x) hist[k] = 0;
     __syncthreads();
     const int64_t i0 = (int64_t)blockIdx.x * span, i1 = min(n, i0 + span);
     const int64_t T = blockDim.x;
-    unsigned f = 0u, wmax = 0u, wminc = 0u;
     int64_t i = i0 + threadIdx.x;
     for (; i + (kBktUnroll - 1) * T < i1; i += kBktUnroll * T) {
         if (threadIdx.x == 0) {  // the next block of the slice into L2 meanwhile
@@ -528,17 +586,10 @@ __global__ void __launch_bounds__(kBktThreads) k_bkt_count(const float4 *__restr
 #pragma unroll
         for (int u = 0; u < kBktUnroll; ++u) p[u] = pts[i + u * T];
 #pragma unroll
-        for (int u = 0; u < kBktUnroll; ++u) {
-            point_flags(p[u], box, f, wmax, wminc);
-            atomicAdd(&hist[div_q(cell_of_point(p[u], P, cell), Q, rq)], 1);
-        }
+        for (int u = 0; u < kBktUnroll; ++u) atomicAdd(&hist[div_q(cell_of_point(p[u], P, cell), Q, rq)], 1);
     }
-    for (; i < i1; i += T) {
-        const float4 p = pts[i];
-        point_flags(p, box, f, wmax, wminc);
-        atomicAdd(&hist[div_q(cell_of_point(p, P, cell), Q, rq)], 1);
-    }
-    flush_flags(f, wmax, wminc, flags);  // ends with the block's histogram complete
+    for (; i < i1; i += T) atomicAdd(&hist[div_q(cell_of_point(pts[i], P, cell), Q, rq)], 1);
+    __syncthreads();
     const int64_t G = gridDim.x;
     for (int k = threadIdx.x; k < K; k += blockDim.x) M[k * G + blockIdx.x] = hist[k];
 }
@@ -751,6 +802,158 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kSortThreads)
     }
 }
 
+// Home tiles of column (ix, iy): runs of at most `cap` consecutive points that
+// span at most two adjacent cells [z0, z1], so a warp's lanes stay busy when
+// cells hold fewer than 32 points.  Two cells keep a periodic stencil within the
+// box: the counts require 2k + 2 <= P for k neighbour cells per side, and a row
+// covers z0 - k .. z1 + k.  Writes them to out (null: only counts).
+__device__ int column_tiles(const int *start, int P, int col, int cap, TileDesc *out) {
+    const int *hs = start + (int64_t)col * P;
+    const int end = hs[P];
+    int p = hs[0], iz = 0, n = 0;
+    while (p < end) {
+        while (hs[iz + 1] <= p) ++iz;  // cell of point p
+        const int m = min(cap, hs[min(iz + 2, P)] - p);
+        if (out) {
+            int z1 = iz;
+            while (hs[z1 + 1] < p + m) ++z1;  // cell of the tile's last point
+            TileDesc t;
+            t.start = p;
+            t.count = m;
+            t.ix = (int16_t)(col / P);
+            t.iy = (int16_t)(col % P);
+            t.z0 = (int16_t)iz;
+            t.z1 = (int16_t)z1;
+            out[n] = t;
+        }
+        ++n;
+        p += m;
+    }
+    return n;
+}
+
+// The tile table by one block (P^2 columns, at most 4 per thread): counts per
+// column in `cnt` (shared), their scan, then the tiles; their number goes to the
+// host's block.  Whole block.
+__device__ void block_tiles(const int *start, int P, int cap, TileDesc *tiles, int *host, int *cnt,
+                            int *wsum) {
+    const int ncol = P * P;
+    for (int c = threadIdx.x; c < ncol; c += blockDim.x) cnt[c] = column_tiles(start, P, c, cap, nullptr);
+    __syncthreads();
+    const int last = cnt[ncol - 1];
+    __syncthreads();
+    block_excl_scan4(cnt, ncol, wsum);
+    for (int c = threadIdx.x; c < ncol; c += blockDim.x) column_tiles(start, P, c, cap, tiles + cnt[c]);
+    if (threadIdx.x == 0) *host = cnt[ncol - 1] + last;
+}
+constexpr int kTileBlockColumns = 1024;
+__global__ void __launch_bounds__(1024) k_tiles_block(const int *__restrict__ start, int P, int cap, TileDesc *tiles,
+                                                      int *host) {
+    __shared__ int cnt[kTileBlockColumns], wsum[32];
+    block_tiles(start, P, cap, tiles, host, cnt, wsum);
+}
+// The same over many blocks: counts per column (entry P^2: 0), then, after a
+// scan, the tiles.
+__global__ void k_tile_cols(const int *__restrict__ start, int P, int cap, int *__restrict__ cnt) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c <= P * P) cnt[c] = c < P * P ? column_tiles(start, P, c, cap, nullptr) : 0;
+}
+__global__ void k_tile_fill(const int *__restrict__ start, int P, int cap, const int *__restrict__ off,
+                            TileDesc *__restrict__ tiles, int *host) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c < P * P) column_tiles(start, P, c, cap, tiles + off[c]);
+    if (c == 0) *host = off[P * P];
+}
+
+// The whole build of a small catalog by one block: cell counts and ranks in
+// shared memory, their scan, the cell-ordered copies with their padding, and the
+// tile table.  One launch where the per-point build takes seven of 2 to 4 us
+// each: 6 us against 24 for 1000 points.
+constexpr int kSmallPoints = 4096, kSmallCells = 4096, kSmallThreads = 1024;
+__global__ void __launch_bounds__(kSmallThreads) k_build_small(const float4 *__restrict__ pts, int n, int P, float cell,
+                                                               int *__restrict__ cell_start, float *__restrict__ soa,
+                                                               size_t plane, float4 *__restrict__ pk, int pk_to,
+                                                               unsigned *__restrict__ qw, const int *__restrict__ flags,
+                                                               int cap, TileDesc *tiles, int *host) {
+    __shared__ int cnt[kSmallCells + 1], cols[256], wsum[32];  // P^3 <= 4096: at most 256 columns
+    __shared__ unsigned short perm[kSmallPoints];
+    const int ncell = P * P * P, tid = threadIdx.x;
+    constexpr int kPer = kSmallPoints / kSmallThreads;
+    for (int c = tid; c < ncell; c += kSmallThreads) cnt[c] = 0;
+    // padding past point n (the copies below write the rest)
+    for (int64_t d = n + tid; d < (int64_t)plane; d += kSmallThreads) {
+        for (int a = 0; a < 4; ++a) soa[a * plane + d] = 0.f;
+        qw[d] = 0u;
+    }
+    for (int k = 2 * (n / 2) + tid; k < pk_to; k += kSmallThreads) pk[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+    __syncthreads();
+    int c[kPer], rank[kPer];
+    #pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+        const int i = tid + u * kSmallThreads;
+        if (i < n) c[u] = cell_of_point(pts[i], P, cell);
+    }
+    #pragma unroll
+    for (int u = 0; u < kPer; ++u)
+        if (tid + u * kSmallThreads < n) rank[u] = atomicAdd(&cnt[c[u]], 1);
+    __syncthreads();
+    block_excl_scan4(cnt, ncell, wsum);
+    #pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+        const int i = tid + u * kSmallThreads;
+        if (i < n) perm[cnt[c[u]] + rank[u]] = (unsigned short)i;
+    }
+    if (tid == 0) cnt[ncell] = n;
+    for (int k = tid; k < ncell; k += kSmallThreads) cell_start[k] = cnt[k];
+    if (tid == 0) cell_start[ncell] = n;
+    int emin, emax;
+    const unsigned *uf = reinterpret_cast<const unsigned *>(flags);
+    const bool fix = weight_fix_range(uf[0], uf[1], uf[2], &emin, &emax);
+    __syncthreads();
+    // in cell order, so that the writes coalesce: scattered, 13 words of every
+    // point went through one SM's store path one at a time (3000 points: 20.6 us)
+    #pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+        const int d = tid + u * kSmallThreads;
+        if (d >= n) continue;
+        const float4 p = pts[perm[d]];
+        soa[d] = p.x;
+        soa[plane + d] = p.y;
+        soa[2 * plane + d] = p.z;
+        soa[3 * plane + d] = p.w;
+        qw[d] = fix ? weight_q(p.w, emin) : 0u;
+        pk_put(pk, d, p);
+    }
+    block_tiles(cnt, P, cap, tiles, host, cols, wsum);
+}
+
+// Largest number of candidates of any cell's stencil (rows: the stencil's).
+__global__ void k_stencil_max(const int *__restrict__ start, int P, const RowDesc *__restrict__ rows, int n_rows,
+                              int bpc, int *__restrict__ out) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    int n = 0;
+    if (c < P * P * P) {
+        const int iz = c % P, iy = (c / P) % P, ix = c / (P * P);
+        for (int r = 0; r < n_rows; ++r) {
+            const RowDesc rw = rows[r];
+            int nx = ix + rw.dx, ny = iy + rw.dy;
+            if (bpc) {
+                nx += nx < 0 ? P : nx >= P ? -P : 0;
+                ny += ny < 0 ? P : ny >= P ? -P : 0;
+            } else if (nx < 0 || nx >= P || ny < 0 || ny >= P) {
+                continue;
+            }
+            const int *cs = start + (int64_t)(nx * P + ny) * P;
+            const int zlo = iz - rw.kz, zhi = iz + rw.kz;
+            n += cs[min(zhi, P - 1) + 1] - cs[max(zlo, 0)];
+            if (bpc && zlo < 0) n += cs[P] - cs[zlo + P];
+            if (bpc && zhi >= P) n += cs[zhi - P + 1] - cs[0];
+        }
+    }
+    n = __reduce_max_sync(0xffffffffu, (unsigned)n);
+    if ((threadIdx.x & 31) == 0) atomicMax(out, n);
+}
+
 // Zero the padding past the catalog: the SoA planes' and integer weights'
 // entries n .. plane - 1 and the pair blocks from the one holding point n
 // (an odd n leaves that block's second half empty).
@@ -769,11 +972,11 @@ __global__ void k_tails(float *__restrict__ soa, size_t plane, int64_t n, float4
 
 int launch_grid_build(const float4 *raw, int64_t n, int P, float cell, float box, int *cid,
                       int *rank, int *perm, int *counts, int *cell_start, int *scan_tmp, float *soa,
-                      size_t plane, float4 *pk, unsigned *qw, int *flags, cudaStream_t st) {
+                      size_t plane, float4 *pk, unsigned *qw, int *flags, bool checked, cudaStream_t st) {
     const int64_t ncell = (int64_t)P * P * P;
     const int thr = 256;
     const unsigned blocks = (unsigned)((n + thr - 1) / thr);
-    k_cell_ids<<<blocks, thr, 0, st>>>(raw, n, P, cell, box, cid, rank, counts, flags);
+    k_cell_ids<<<blocks, thr, 0, st>>>(raw, n, P, cell, box, cid, rank, counts, checked ? nullptr : flags);
     int launches = 1 + scan_exclusive(counts, cell_start, ncell + 1, scan_tmp, st);
     k_perm<<<blocks, thr, 0, st>>>(n, cid, rank, cell_start, perm);
     k_gather<<<blocks, thr, 0, st>>>(raw, n, perm, soa, plane, pk, qw, flags);
@@ -831,15 +1034,14 @@ static int sort_clusters(int device) {
     return num;
 }
 
-int launch_grid_build_buckets(const float4 *raw, int64_t n, int P, float cell, float box, int G, int Q,
-                              int K, int *M, int *Mx, int *scan_tmp, float4 *S, int *cell_start,
-                              float *soa, size_t plane, float4 *pk, unsigned *qw, int *flags,
-                              int device, cudaStream_t st) {
+int launch_grid_build_buckets(const float4 *raw, int64_t n, int P, float cell, int G, int Q, int K, int *M,
+                              int *Mx, int *scan_tmp, float4 *S, int *cell_start, float *soa, size_t plane,
+                              float4 *pk, unsigned *qw, const int *flags, int device, cudaStream_t st) {
     const int ncell = P * P * P;
     const int64_t span = (n + G - 1) / G;
     const size_t hs = sizeof(int) * (size_t)K;
     const float rq = 1.0f / (float)Q;
-    k_bkt_count<<<G, kBktThreads, hs, st>>>(raw, n, span, P, cell, box, Q, rq, K, M, flags);
+    k_bkt_count<<<G, kBktThreads, hs, st>>>(raw, n, span, P, cell, Q, rq, K, M);
     int launches = 1 + scan_exclusive(M, Mx, (int64_t)G * K, scan_tmp, st);
     k_bkt_scatter<<<G, kBktThreads, scatter_smem(K), st>>>(raw, n, span, P, cell, Q, rq, K, Mx, S);
     const int nclus = std::min(K, sort_clusters(device));
@@ -901,14 +1103,67 @@ pcf_status pcf_ensure_pinned(pcf_ctx *ctx, size_t bytes) {
     return PCF_OK;
 }
 
+pcf_status out_open(pcf_ctx *ctx, int64_t nb, bool dev_out, double *hist, double *d_out, OutPath *o) {
+    const size_t bytes = sizeof(double) * (size_t)nb;
+    const bool staged = !dev_out && bytes <= kStagedOut;
+    const pcf_status s = pcf_ensure_pinned(ctx, 64 + (staged ? bytes : 0));
+    if (s != PCF_OK) return s;
+    char *hp = static_cast<char *>(ctx->h_pinned);
+    o->stats = reinterpret_cast<unsigned long long *>(hp);
+    o->staged = staged ? reinterpret_cast<double *>(hp + 64) : nullptr;
+    o->to = dev_out ? hist : bytes <= kDirectOut ? o->staged : d_out;
+    return PCF_OK;
+}
+
+pcf_status out_close(pcf_ctx *ctx, const OutPath &o, int64_t nb, bool dev_out, double *hist,
+                     unsigned long long *hs) {
+    const size_t bytes = sizeof(double) * (size_t)nb;
+    double *at = o.staged ? o.staged : hist;
+    if (!dev_out && o.to != at) {
+        PCF_CU(ctx, cudaMemcpyAsync(at, o.to, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+        if (o.staged) {
+            // bring the result's pages in while the device is still counting (a new
+            // array's 486 pages of 2 MB: 0.8 ms after the kernel); what they hold stays
+            volatile char *h = reinterpret_cast<volatile char *>(hist);
+            for (size_t i = 0; i < bytes; i += 4096) h[i] = h[i];
+        }
+    }
+    PCF_CU(ctx, cudaStreamSynchronize(ctx->stream));
+    const pcf_status s = ctx_queue_status(ctx);
+    if (s != PCF_OK) return s;
+    if (o.staged) memcpy(hist, o.staged, bytes);
+    if (hs) memcpy(hs, o.stats, 4 * sizeof(*hs));
+    return PCF_OK;
+}
+
+pcf_status fetch_block(pcf_ctx *ctx, const void *d, size_t bytes, std::vector<char> &spill, const char **host) {
+    char *to;
+    if (bytes <= kStagedOut) {
+        const pcf_status s = pcf_ensure_pinned(ctx, bytes);
+        if (s != PCF_OK) return s;
+        to = static_cast<char *>(ctx->h_pinned);
+    } else {
+        spill.resize(bytes);
+        to = spill.data();
+    }
+    PCF_CU(ctx, cudaMemcpyAsync(to, d, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+    PCF_CU(ctx, cudaStreamSynchronize(ctx->stream));
+    *host = to;
+    return PCF_OK;
+}
+
 // Build (or rebuild) the cell structure of g for P cells per side.
 // A grid keeps the cell structures of the last few partition counts it was
 // counted at, so classes of histograms tuned to different partitions do not
 // rebuild (and synchronise) on every switch.
+pcf_status launch_tiles(pcf_ctx *ctx, const CellGrid &cg, int cap, TileDesc *tiles, int *host);
+pcf_status grid_profile_begin(pcf_ctx *ctx, int64_t n, cudaEvent_t *end);
 pcf_status grid_ensure_cells(pcf_ctx *ctx, pcf_grid *g, int P, bool defer) {
     if (g->cells && g->cells->P == P) return defer ? PCF_OK : grid_finish(ctx, g);
-    pcf_status s0 = grid_finish(ctx, g);  // the current structure, before it is replaced
-    if (s0 != PCF_OK) return s0;
+    if (g->cells) {  // the current structure, before it is replaced
+        const pcf_status s0 = grid_finish(ctx, g);
+        if (s0 != PCF_OK) return s0;
+    }
     if (P < 1 || P > 320) return PCF_ERR_INVALID_ARG;
     for (size_t i = 0; i < g->cell_cache.size(); ++i) {
         if (g->cell_cache[i]->P != P) continue;
@@ -934,6 +1189,7 @@ pcf_status grid_ensure_cells(pcf_ctx *ctx, pcf_grid *g, int P, bool defer) {
     PCF_CU(ctx, cg->qw.ensure(sizeof(unsigned) * cg->plane));
     PCF_CU(ctx, cg->cell_start.ensure(sizeof(int) * (size_t)(ncell + 1)));
     int Q = 0, K = 0;
+    const bool small = n <= kSmallPoints && ncell <= kSmallCells && ctx->grid_build == 0;
     const int G = ctx->sm_count;
     // the bucketed build pays a fixed cost per bucket (a cluster of four
     // CTAs and three cluster barriers): below ~6M points the per-point build,
@@ -949,61 +1205,55 @@ pcf_status grid_ensure_cells(pcf_ctx *ctx, pcf_grid *g, int P, bool defer) {
         PCF_CU(ctx, ctx->scratch_b.ensure(sizeof(int) * 2 * mat));
         PCF_CU(ctx, ctx->scratch_c.ensure(sizeof(int) * (mat / 256 + 256)));
         PCF_CU(ctx, grid_bucket_attrs(ctx->device, K));
-    } else {
+    } else if (!small) {
         // scratch: cid, rank, perm (n each); counts (ncell + 1); scan tmp.
         PCF_CU(ctx, ctx->scratch_a.ensure(sizeof(int) * (size_t)n * 3));
         PCF_CU(ctx, ctx->scratch_b.ensure(sizeof(int) * (size_t)(ncell + 1)));
         PCF_CU(ctx, ctx->scratch_c.ensure(sizeof(int) * (size_t)((ncell + 1) / 256 + 256)));
     }
-    PCF_CU(ctx, ctx->d_flag.ensure(sizeof(int) * 4));
-    int *flags = ctx->d_flag.as<int>();
-    if (!buckets) PCF_CU(ctx, cudaMemsetAsync(ctx->scratch_b.p, 0, sizeof(int) * (size_t)(ncell + 1), st));
-    PCF_CU(ctx, cudaMemsetAsync(flags, 0, sizeof(int) * 3, st));
-    cudaEvent_t pg0 = nullptr, pg1 = nullptr;  // kernel-time log of grid builds
-    if (ctx->profile) {
-        if (ctx->prof_grid_used == ctx->prof_grid_events.size()) {
-            cudaEvent_t e0, e1;
-            PCF_CU(ctx, cudaEventCreate(&e0));
-            PCF_CU(ctx, cudaEventCreate(&e1));
-            ctx->prof_grid_events.push_back({e0, e1});
-        }
-        pg0 = ctx->prof_grid_events[ctx->prof_grid_used].first;
-        pg1 = ctx->prof_grid_events[ctx->prof_grid_used].second;
-        ++ctx->prof_grid_used;
-        ctx->prof_grid_points += n;
-        PCF_CU(ctx, cudaEventRecord(pg0, st));
+    const int *flags = g->flags.as<int>();
+    if (!buckets && !small)
+        PCF_CU(ctx, cudaMemsetAsync(ctx->scratch_b.p, 0, sizeof(int) * (size_t)(ncell + 1), st));
+    // tiles <= n / kTileCap + the non-empty cells + 1
+    const int64_t tile_max = std::min<int64_t>(ncell, n) + n / kTileCap + 2;
+    cg->d_tiles.pool = g->pool;
+    PCF_CU(ctx, cg->d_tiles.ensure(sizeof(TileDesc) * (size_t)tile_max));
+    PCF_CU(ctx, cg->note.open(ctx->pinned));
+    int *host = static_cast<int *>(cg->note.block);
+    cudaEvent_t pg1 = nullptr;
+    {
+        pcf_status ps = grid_profile_begin(ctx, n, &pg1);
+        if (ps != PCF_OK) return ps;
     }
-    ctx->launches += launch_grid_tails(cg->soa.as<float>(), cg->plane, n, cg->pk.as<float4>(),
-                                       cg->qw.as<unsigned>(), st);
-    if (buckets) {
-        int *M = ctx->scratch_b.as<int>();
-        ctx->launches += launch_grid_build_buckets(
-            g->raw.as<float4>(), n, P, cg->cell, g->box, G, Q, K, M, M + mat, ctx->scratch_c.as<int>(),
-            ctx->scratch_a.as<float4>(), cg->cell_start.as<int>(), cg->soa.as<float>(), cg->plane,
-            cg->pk.as<float4>(), cg->qw.as<unsigned>(), flags, ctx->device, st);
+    if (small) {
+        k_build_small<<<1, kSmallThreads, 0, st>>>(g->raw.as<float4>(), (int)n, P, cg->cell, cg->cell_start.as<int>(),
+                                                   cg->soa.as<float>(), cg->plane, cg->pk.as<float4>(),
+                                                   2 * (int)pk_blocks(n), cg->qw.as<unsigned>(), flags, kTileCap,
+                                                   cg->d_tiles.as<TileDesc>(), host);
+        ++ctx->launches;
     } else {
-        int *cid = ctx->scratch_a.as<int>();
-        ctx->launches += launch_grid_build(g->raw.as<float4>(), n, P, cg->cell, g->box, cid, cid + n,
-                                           cid + 2 * n, ctx->scratch_b.as<int>(), cg->cell_start.as<int>(),
-                                           ctx->scratch_c.as<int>(), cg->soa.as<float>(), cg->plane,
-                                           cg->pk.as<float4>(), cg->qw.as<unsigned>(), flags, st);
+        ctx->launches += launch_grid_tails(cg->soa.as<float>(), cg->plane, n, cg->pk.as<float4>(),
+                                           cg->qw.as<unsigned>(), st);
+        if (buckets) {
+            int *M = ctx->scratch_b.as<int>();
+            ctx->launches += launch_grid_build_buckets(
+                g->raw.as<float4>(), n, P, cg->cell, G, Q, K, M, M + mat, ctx->scratch_c.as<int>(),
+                ctx->scratch_a.as<float4>(), cg->cell_start.as<int>(), cg->soa.as<float>(), cg->plane,
+                cg->pk.as<float4>(), cg->qw.as<unsigned>(), flags, ctx->device, st);
+        } else {
+            int *cid = ctx->scratch_a.as<int>();
+            ctx->launches += launch_grid_build(g->raw.as<float4>(), n, P, cg->cell, g->box, cid, cid + n,
+                                               cid + 2 * n, ctx->scratch_b.as<int>(), cg->cell_start.as<int>(),
+                                               ctx->scratch_c.as<int>(), cg->soa.as<float>(), cg->plane,
+                                               cg->pk.as<float4>(), cg->qw.as<unsigned>(), g->flags.as<int>(),
+                                               true, st);
+        }
+        const pcf_status ps = launch_tiles(ctx, *cg, kTileCap, cg->d_tiles.as<TileDesc>(), host);
+        if (ps != PCF_OK) return ps;
     }
     PCF_CU(ctx, cudaGetLastError());
     if (pg1) PCF_CU(ctx, cudaEventRecord(pg1, st));
-    // this build's own page-locked block: the cell table and flags come back
-    // into it, and the tile table later goes out from it (pageable copies go
-    // through the driver's staging, where concurrent contexts were seen to
-    // stall one another); sized for both (tiles <= n / kTileCap + the
-    // non-empty cells + 1)
-    const size_t sb = sizeof(int) * (size_t)(ncell + 1);
-    const size_t tile_max = sizeof(TileDesc) * (size_t)(std::min<int64_t>(ncell, n) + n / kTileCap + 2);
-    cg->pinned = ctx->pinned;
-    PCF_CU(ctx, ctx->pinned->get(std::max(sb + 64, tile_max), &cg->stage, &cg->stage_bytes));
-    char *hp = static_cast<char *>(cg->stage);
-    PCF_CU(ctx, cudaMemcpyAsync(hp, cg->cell_start.p, sb, cudaMemcpyDeviceToHost, st));
-    PCF_CU(ctx, cudaMemcpyAsync(hp + sb, flags, 3 * sizeof(unsigned), cudaMemcpyDeviceToHost, st));
-    PCF_CU(ctx, cudaEventCreateWithFlags(&cg->ready, cudaEventDisableTiming));
-    PCF_CU(ctx, cudaEventRecord(cg->ready, st));
+    PCF_CU(ctx, cudaEventRecord(cg->note.ready, st));
     cg->pending = true;
     if (g->cells) {
         g->cell_cache.push_back(std::move(g->cells));
@@ -1013,11 +1263,107 @@ pcf_status grid_ensure_cells(pcf_ctx *ctx, pcf_grid *g, int P, bool defer) {
     return defer ? PCF_OK : grid_finish(ctx, g);
 }
 
-// Completes a queued build: waits for its cell table, checks the catalog's
-// flags, sets the weight range and sends the tile table.  A catalog found
-// invalid stays marked, so every later use reports it.
+// The tile table of cg at `cap` points per tile, on the context's stream; the
+// number of tiles goes to *host (page-locked).  Built on the device: sent to the
+// host, made there and sent back, the tables of 6M + 9M points in 100^3 cells
+// took 12 ms of a 31 ms call.
+pcf_status launch_tiles(pcf_ctx *ctx, const CellGrid &cg, int cap, TileDesc *tiles, int *host) {
+    const int P = cg.P, ncol = P * P;
+    cudaStream_t st = ctx->stream;
+    const int *start = cg.cell_start.as<int>();
+    if (ncol <= kTileBlockColumns) {
+        k_tiles_block<<<1, 1024, 0, st>>>(start, P, cap, tiles, host);
+        ++ctx->launches;
+    } else {
+        PCF_CU(ctx, ctx->scratch_b.ensure(sizeof(int) * 2 * (size_t)(ncol + 1)));
+        PCF_CU(ctx, ctx->scratch_c.ensure(sizeof(int) * (size_t)((ncol + 1) / 256 + 256)));
+        int *cnt = ctx->scratch_b.as<int>(), *off = cnt + ncol + 1;
+        k_tile_cols<<<(ncol + 1 + 127) / 128, 128, 0, st>>>(start, P, cap, cnt);
+        ctx->launches += 2 + scan_exclusive(cnt, off, ncol + 1, ctx->scratch_c.as<int>(), st);
+        k_tile_fill<<<(ncol + 127) / 128, 128, 0, st>>>(start, P, cap, off, tiles, host);
+    }
+    PCF_CU(ctx, cudaGetLastError());
+    return PCF_OK;
+}
+
+// Begins an entry of the kernel-time log of grid builds (n points; 0: part of
+// the same catalog's build); *end: the event to record behind the kernels, or
+// null while the log is off.
+pcf_status grid_profile_begin(pcf_ctx *ctx, int64_t n, cudaEvent_t *end) {
+    *end = nullptr;
+    if (!ctx->profile) return PCF_OK;
+    if (ctx->prof_grid_used == ctx->prof_grid_events.size()) {
+        cudaEvent_t e0, e1;
+        PCF_CU(ctx, cudaEventCreate(&e0));
+        PCF_CU(ctx, cudaEventCreate(&e1));
+        ctx->prof_grid_events.push_back({e0, e1});
+    }
+    const auto &e = ctx->prof_grid_events[ctx->prof_grid_used++];
+    ctx->prof_grid_builds += n > 0;
+    ctx->prof_grid_points += n;
+    PCF_CU(ctx, cudaEventRecord(e.first, ctx->stream));
+    *end = e.second;
+    return PCF_OK;
+}
+
+// Copies the caller's points into g->raw and checks them, on the context's
+// stream.  Device memory of this device, 16-byte aligned, is copied by the
+// kernel that checks it, and so are a few points from the host, which it reads in
+// a page-locked block (a copy from pageable memory costs the host 11 us);
+// everything else by a copy first.
+pcf_status grid_take(pcf_ctx *ctx, pcf_grid *g, const pcf_point *pts) {
+    cudaStream_t st = ctx->stream;
+    const int64_t n = g->n;
+    float4 *raw = g->raw.as<float4>();
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, pts) != cudaSuccess) {
+        cudaGetLastError();
+        at.type = cudaMemoryTypeUnregistered;
+    }
+    const bool direct = at.type == cudaMemoryTypeDevice && at.device == ctx->device && ((uintptr_t)pts & 15) == 0;
+    const bool device = at.type == cudaMemoryTypeDevice || at.type == cudaMemoryTypeManaged;
+    const bool one = n <= kIntakeOneBlock, staged = one && !device;
+    PCF_CU(ctx, g->flags.ensure(64));
+    PCF_CU(ctx, g->note.open(ctx->pinned, staged ? 64 + sizeof(float4) * (size_t)n : 64));
+    const float4 *from = direct ? reinterpret_cast<const float4 *>(pts) : raw;
+    if (staged) {
+        char *b = static_cast<char *>(g->note.block) + 64;
+        memcpy(b, pts, sizeof(float4) * (size_t)n);
+        from = reinterpret_cast<const float4 *>(b);
+    } else if (!direct) {
+        PCF_CU(ctx, cudaMemcpyAsync(raw, pts, sizeof(float4) * (size_t)n,
+                                    device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, st));
+    }
+    if (!one) PCF_CU(ctx, cudaMemsetAsync(g->flags.p, 0, 64, st));
+    cudaEvent_t pe = nullptr;
+    const pcf_status ps = grid_profile_begin(ctx, 0, &pe);
+    if (ps != PCF_OK) return ps;
+    const int64_t per = (int64_t)kIntakeThreads * kIntakeUnroll;
+    const int blocks = one ? 1 : (int)std::min<int64_t>((n + per - 1) / per, (int64_t)ctx->sm_count * 8);
+    k_intake<<<blocks, kIntakeThreads, 0, st>>>(from, raw, n, g->box, g->flags.as<int>(),
+                                                static_cast<unsigned *>(g->note.block));
+    PCF_CU(ctx, cudaGetLastError());
+    ++ctx->launches;
+    if (pe) PCF_CU(ctx, cudaEventRecord(pe, st));
+    if (!one)
+        PCF_CU(ctx, cudaMemcpyAsync(g->note.block, g->flags.p, 3 * sizeof(unsigned), cudaMemcpyDeviceToHost, st));
+    PCF_CU(ctx, cudaEventRecord(g->note.ready, st));
+    g->unchecked = true;
+    return PCF_OK;
+}
+
+// Completes what is queued of g: the catalog's flags (a catalog found invalid
+// stays marked, so every later use reports it) and weight range, and the tile
+// count of its current cell structure.
 pcf_status grid_finish(pcf_ctx *ctx, const pcf_grid *g_) {
     pcf_grid *g = const_cast<pcf_grid *>(g_);
+    if (g->unchecked) {
+        g->unchecked = false;
+        unsigned hf[3];
+        PCF_CU(ctx, g->note.wait(hf, sizeof(hf)));
+        if (hf[0] & 1u) g->bad = PCF_ERR_OUT_OF_BOX;
+        else set_weight_range(g, hf);
+    }
     if (g->bad != PCF_OK) {
         ctx->last_error = "a coordinate lies outside [0, box)";
         return g->bad;
@@ -1025,32 +1371,41 @@ pcf_status grid_finish(pcf_ctx *ctx, const pcf_grid *g_) {
     CellGrid *cg = g->cells.get();
     if (!cg || !cg->pending) return PCF_OK;
     cg->pending = false;
-    PCF_CU(ctx, cudaEventSynchronize(cg->ready));
-    const int64_t ncell = (int64_t)cg->P * cg->P * cg->P;
-    const size_t sb = sizeof(int) * (size_t)(ncell + 1);
-    const char *hp = static_cast<const char *>(cg->stage);
-    cg->h_start.assign(reinterpret_cast<const int *>(hp), reinterpret_cast<const int *>(hp) + ncell + 1);
-    unsigned hf[3];
-    memcpy(hf, hp + sb, sizeof(hf));
-    if (hf[0] & 1u) {
-        g->bad = PCF_ERR_OUT_OF_BOX;
-        ctx->last_error = "a coordinate lies outside [0, box)";
-        return PCF_ERR_OUT_OF_BOX;
-    }
-    set_weight_range(g, hf);
-    build_tiles(*cg, kTileCap, cg->tiles);
-    cg->d_tiles.pool = g->pool;
-    PCF_CU(ctx, cg->d_tiles.ensure(sizeof(TileDesc) * std::max<size_t>(1, cg->tiles.size())));
-    if (!cg->tiles.empty()) {
-        const size_t tb = sizeof(TileDesc) * cg->tiles.size();
-        if (tb > cg->stage_bytes) {  // cannot happen: the staging is sized by the bound above
-            ctx->last_error = "tile table larger than its staging block";
-            return PCF_ERR_CUDA;
-        }
-        memcpy(cg->stage, cg->tiles.data(), tb);  // the cell table's copy into it has completed
-        PCF_CU(ctx, cudaMemcpyAsync(cg->d_tiles.p, cg->stage, tb, cudaMemcpyHostToDevice, ctx->stream));
-        PCF_CU(ctx, cudaEventRecord(cg->ready, ctx->stream));
-    }
+    int nt = 0;
+    PCF_CU(ctx, cg->note.wait(&nt, sizeof(nt)));
+    cg->n_tiles = nt;
+    return PCF_OK;
+}
+
+// The cell table of g's current structure on the host (grid_info, download).
+pcf_status grid_host_starts(pcf_ctx *ctx, const pcf_grid *g, std::vector<int> &out) {
+    const CellGrid &c = *g->cells;
+    out.resize((size_t)c.P * c.P * c.P + 1);
+    PCF_CU(ctx, cudaMemcpyAsync(out.data(), c.cell_start.p, sizeof(int) * out.size(), cudaMemcpyDeviceToHost, ctx->stream));
+    PCF_CU(ctx, cudaStreamSynchronize(ctx->stream));
+    return PCF_OK;
+}
+
+// The structure that a grid shows before any count has chosen one.
+pcf_status grid_default_cells(pcf_ctx *ctx, pcf_grid *g) {
+    const pcf_status s = grid_finish(ctx, g);
+    if (s != PCF_OK || g->cells) return s;
+    const int P = g->user_P > 0 ? g->user_P : choose_partitions(g->n, g->box, g->box / 8.f, PCF_ISO, false, 4);
+    return grid_ensure_cells(ctx, g, P);
+}
+
+pcf_status stencil_max(pcf_ctx *ctx, const CellGrid &g, const RowDesc *d_rows, int n_rows, bool bpc, int64_t *out) {
+    PCF_CU(ctx, ctx->d_flag.ensure(64));
+    int *d = ctx->d_flag.as<int>();
+    PCF_CU(ctx, cudaMemsetAsync(d, 0, sizeof(int), ctx->stream));
+    const int ncell = g.P * g.P * g.P;
+    k_stencil_max<<<(ncell + 127) / 128, 128, 0, ctx->stream>>>(g.cell_start.as<int>(), g.P, d_rows, n_rows, bpc ? 1 : 0, d);
+    PCF_CU(ctx, cudaGetLastError());
+    ++ctx->launches;
+    int v = 0;
+    PCF_CU(ctx, cudaMemcpyAsync(&v, d, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    PCF_CU(ctx, cudaStreamSynchronize(ctx->stream));
+    *out = v;
     return PCF_OK;
 }
 
@@ -1089,21 +1444,17 @@ int choose_partitions(int64_t n, float box, float dmax, int kind, bool bpc, int 
     return P;
 }
 
-pcf_status ensure_half_tiles(pcf_ctx *ctx, CellGrid &g) {
-    if (g.have_half) return PCF_OK;
-    build_tiles(g, 16, g.tiles_half);
+pcf_status ensure_half_tiles(pcf_ctx *ctx, CellGrid &g, int64_t n) {
+    if (g.n_tiles_half >= 0) return PCF_OK;
+    const int64_t ncell = (int64_t)g.P * g.P * g.P;
     g.d_tiles_half.pool = g.d_tiles.pool;
-    PCF_CU(ctx, g.d_tiles_half.ensure(sizeof(TileDesc) * std::max<size_t>(1, g.tiles_half.size())));
-    if (!g.tiles_half.empty()) {
-        // the page-locked buffer may still feed an earlier copy: wait first
-        PCF_CU(ctx, cudaStreamSynchronize(ctx->stream));
-        const size_t tb = sizeof(TileDesc) * g.tiles_half.size();
-        pcf_status ps = pcf_ensure_pinned(ctx, tb);
-        if (ps != PCF_OK) return ps;
-        memcpy(ctx->h_pinned, g.tiles_half.data(), tb);
-        PCF_CU(ctx, cudaMemcpyAsync(g.d_tiles_half.p, ctx->h_pinned, tb, cudaMemcpyHostToDevice,
-                                    ctx->stream));
-    }
-    g.have_half = true;
+    PCF_CU(ctx, g.d_tiles_half.ensure(sizeof(TileDesc) * (size_t)(std::min<int64_t>(ncell, n) + n / 16 + 2)));
+    PCF_CU(ctx, g.note.open(ctx->pinned));
+    const pcf_status s = launch_tiles(ctx, g, 16, g.d_tiles_half.as<TileDesc>(), static_cast<int *>(g.note.block));
+    if (s != PCF_OK) return s;
+    PCF_CU(ctx, cudaEventRecord(g.note.ready, ctx->stream));
+    int nt = 0;
+    PCF_CU(ctx, g.note.wait(&nt, sizeof(nt)));
+    g.n_tiles_half = nt;
     return PCF_OK;
 }

@@ -135,10 +135,10 @@ extern "C" pcf_status pcf_count_pairs_noalloc(const pcf_point *a, int64_t na, co
 
     const float cell = box / (float)P;
     launch_grid_build(reinterpret_cast<const float4 *>(a), na, P, cell, box, A.cid, A.rank, A.perm,
-                      A.counts, A.start, scan_tmp, nullptr, 0, A.pk, nullptr, d_flags, st);
+                      A.counts, A.start, scan_tmp, nullptr, 0, A.pk, nullptr, d_flags, false, st);
     if (cross)
         launch_grid_build(reinterpret_cast<const float4 *>(b), nb, P, cell, box, B.cid, B.rank,
-                          B.perm, B.counts, B.start, scan_tmp, nullptr, 0, B.pk, nullptr, d_flags, st);
+                          B.perm, B.counts, B.start, scan_tmp, nullptr, 0, B.pk, nullptr, d_flags, false, st);
     launch_tile_build(A.start, P, tile_counts, tile_offsets, scan_tmp, tiles, st);
     if ((e = cudaGetLastError()) != cudaSuccess) return fail(e);
     if ((e = cudaMemcpyAsync(d_rows, rows.data(), sizeof(RowDesc) * rows.size(),

@@ -930,10 +930,13 @@ __global__ void k_finalize_slots(const unsigned long long *__restrict__ cnt,
     out[t] = mult[s] * (weighted ? ws[t] : (double)cnt[t]);
 }
 
-// out[k] = mult * hist[k] (u64 counts or FP64 sums).
+// out[k] = mult * hist[k] (u64 counts or FP64 sums); with host_stats, the four
+// statistics words too.
 __global__ void k_finalize(const unsigned long long *__restrict__ cnt, const double *__restrict__ ws,
-                           int weighted, double mult, int nb, double *__restrict__ out) {
+                           int weighted, double mult, int nb, double *__restrict__ out,
+                           const unsigned long long *__restrict__ stats, unsigned long long *host_stats) {
     int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (host_stats && k < 4) host_stats[k] = stats[k];
     if (k >= nb) return;
     double v = weighted ? ws[k] : (double)cnt[k];
     out[k] = mult * v;
@@ -944,40 +947,6 @@ __global__ void k_finalize(const unsigned long long *__restrict__ cnt, const dou
 // ---------------------------------------------------------------------------
 // Host planning.
 // ---------------------------------------------------------------------------
-// Home tiles: up to kTileCap consecutive points of one (ix, iy) column,
-// spanning at most two adjacent cells [z0, z1], so a warp's lanes stay busy
-// when cells hold fewer than 32 points.  Two cells keep a periodic stencil
-// within the box: the counts require 2k + 2 <= P for k neighbour cells per
-// side, and a row covers z0 - k .. z1 + k.
-void build_tiles(const CellGrid &g, int cap, std::vector<TileDesc> &out) {
-    const int P = g.P;
-    const std::vector<int> &hs = g.h_start;
-    out.clear();
-    for (int ix = 0; ix < P; ++ix)
-        for (int iy = 0; iy < P; ++iy) {
-            const int col = (ix * P + iy) * P;
-            int iz = 0;
-            int p = hs[col];
-            const int end = hs[col + P];
-            while (p < end) {
-                while (hs[col + iz + 1] <= p) ++iz;  // cell of point p
-                const int limit = hs[col + std::min(iz + 2, P)];
-                const int n = std::min(cap, limit - p);
-                int z1 = iz;
-                while (hs[col + z1 + 1] < p + n) ++z1;  // cell of the tile's last point
-                TileDesc t;
-                t.start = p;
-                t.count = n;
-                t.ix = (int16_t)ix;
-                t.iy = (int16_t)iy;
-                t.z0 = (int16_t)iz;
-                t.z1 = (int16_t)z1;
-                out.push_back(t);
-                p += n;
-            }
-        }
-}
-
 void plan_rows(int P, float box, float dmax, bool ani, bool self, std::vector<RowDesc> &rows) {
     const double cell = (double)box / P;
     const double R = (double)dmax;
@@ -1022,7 +991,7 @@ void plan_pairs(const CellGrid &home, float box, float dmax, bool ani, bool self
     plan.cell = (float)((double)box / P);
     plan_rows(P, box, dmax, ani, self, plan.rows);
     // ~16 items per resident warp keeps the tail short; at most 32 rows each
-    const int64_t nt = (int64_t)home.tiles_for(tile_cap).size();
+    const int64_t nt = home.tiles_for(tile_cap);
     const int64_t nr = (int64_t)plan.rows.size();
     const int64_t want = std::max<int64_t>(1, (int64_t)resident_warps * 16);
     int rpi = (int)std::min<int64_t>(32, std::max<int64_t>(1, (nt * nr) / want));
@@ -1418,27 +1387,32 @@ cudaError_t launch_pairs_view(const PairView &home, const PairView &cand, const 
 
 // Copies the stencil rows into the next staging slot (pinned host ->
 // device).  Waits only for the kernel that used that slot two launches ago.
-pcf_status stage_plan(pcf_ctx *ctx, const PairPlan &plan, PlanSlot **out) {
+pcf_status stage_plan(pcf_ctx *ctx, const PairPlan &plan, PlanSlot **out, PairJob *job, PairJob **d_job) {
     cudaStream_t st = ctx->stream;
     ctx->slot ^= 1;
     PlanSlot &sl = ctx->slots[ctx->slot];
     if (!sl.done) PCF_CU(ctx, cudaEventCreateWithFlags(&sl.done, cudaEventDisableTiming));
     if (sl.used) PCF_CU(ctx, cudaEventSynchronize(sl.done));
     const size_t rb = plan.rows.size() * sizeof(RowDesc);
-    const size_t jb = sizeof(PairJob) * 4;
-    if (sl.h_bytes < rb + jb + 256) {
+    const size_t roff = (64 + rb + 255) & ~(size_t)255, all = roff + (job ? sizeof(PairJob) : 0);
+    if (sl.h_bytes < all) {
         if (sl.h_pinned) cudaFreeHost(sl.h_pinned);
         sl.h_pinned = nullptr;
         sl.h_bytes = 0;
-        const size_t want = std::max<size_t>((rb + jb) * 2 + 256, 1 << 16);
+        const size_t want = std::max<size_t>(all * 2, 1 << 16);
         PCF_CU(ctx, counted_malloc_host(&sl.h_pinned, want));
         sl.h_bytes = want;
     }
-    PCF_CU(ctx, sl.d_rows.ensure(rb + jb + 256));
-    PCF_CU(ctx, sl.d_counter.ensure(64));
-    memcpy(sl.h_pinned, plan.rows.data(), rb);
-    PCF_CU(ctx, cudaMemcpyAsync(sl.d_rows.p, sl.h_pinned, rb, cudaMemcpyHostToDevice, st));
-    PCF_CU(ctx, cudaMemsetAsync(sl.d_counter.p, 0, 64, st));
+    PCF_CU(ctx, sl.d.ensure(all));
+    char *h = static_cast<char *>(sl.h_pinned);
+    memset(h, 0, 64);
+    memcpy(h + 64, plan.rows.data(), rb);
+    if (job) {
+        job->rows = sl.rows();
+        memcpy(h + roff, job, sizeof(PairJob));
+        *d_job = reinterpret_cast<PairJob *>(sl.d.as<char>() + roff);
+    }
+    PCF_CU(ctx, cudaMemcpyAsync(sl.d.p, h, job ? all : 64 + rb, cudaMemcpyHostToDevice, st));
     sl.used = true;
     *out = &sl;
     return PCF_OK;
@@ -1465,14 +1439,11 @@ pcf_status launch_pairs(pcf_ctx *ctx, const PairPlan &plan, const CellGrid &home
     cudaStream_t st = ctx->stream;
     if (plan.n_items == 0) return PCF_OK;
     PlanSlot *sl = nullptr;
-    pcf_status ps = stage_plan(ctx, plan, &sl);
-    if (ps != PCF_OK) return ps;
-    // the one job of this launch, staged behind the rows in the same slot
-    PairJob job;
+    PairJob job, *d_job = nullptr;
     job.home = pair_view(home, pl.wfix);
     job.cand = pair_view(cand, pl.wfix);
     job.tiles = home.d_tiles_for(pl.tile_cap);
-    job.rows = sl->d_rows.as<RowDesc>();
+    job.rows = nullptr;
     job.n_rows = (int)plan.rows.size();
     job.rows_per_item = plan.rows_per_item;
     job.n_chunks = plan.n_chunks;
@@ -1483,14 +1454,11 @@ pcf_status launch_pairs(pcf_ctx *ctx, const PairPlan &plan, const CellGrid &home
     job.pad = 0;
     job.P = plan.P;
     job.wunscale = pl.wunscale;
-    const size_t roff = (plan.rows.size() * sizeof(RowDesc) + 255) & ~(size_t)255;
-    char *hjob = static_cast<char *>(sl->h_pinned) + roff;
-    memcpy(hjob, &job, sizeof(PairJob));
-    PairJob *d_job = reinterpret_cast<PairJob *>(sl->d_rows.as<char>() + roff);
-    PCF_CU(ctx, cudaMemcpyAsync(d_job, hjob, sizeof(PairJob), cudaMemcpyHostToDevice, st));
-    const PairArgs A = make_args(d_job, 1, plan.n_items, sl->d_counter.as<unsigned long long>(),
+    pcf_status ps = stage_plan(ctx, plan, &sl, &job, &d_job);
+    if (ps != PCF_OK) return ps;
+    const PairArgs A = make_args(d_job, 1, plan.n_items, sl->counter(),
                                  plan.P, box, pl, d_count, d_wsum, d_stats);
-    PCF_CU(ctx, cudaEventRecord(ctx->ev0, st));
+    if (pl.timed) PCF_CU(ctx, cudaEventRecord(ctx->ev0, st));
     cudaEvent_t pe0 = nullptr, pe1 = nullptr;
     if (ctx->profile) {
         pcf_status q = profile_events(ctx, &pe0, &pe1);
@@ -1498,7 +1466,7 @@ pcf_status launch_pairs(pcf_ctx *ctx, const PairPlan &plan, const CellGrid &home
         PCF_CU(ctx, cudaEventRecord(pe0, st));
     }
     PCF_CU(ctx, dispatch_pairs(A, pl, st, ctx->sm_count, ctx->device));
-    PCF_CU(ctx, cudaEventRecord(ctx->ev1, st));
+    if (pl.timed) PCF_CU(ctx, cudaEventRecord(ctx->ev1, st));
     if (pe1) PCF_CU(ctx, cudaEventRecord(pe1, st));
     PCF_CU(ctx, cudaEventRecord(sl->done, st));
     ++ctx->launches;
@@ -1516,14 +1484,15 @@ cudaError_t launch_finalize_slots(const unsigned long long *d_count, const doubl
 
 cudaError_t launch_finalize(const unsigned long long *d_count, const double *d_wsum, bool weighted,
                             double mult, int nb, double *d_out, cudaStream_t st) {
-    k_finalize<<<(nb + 255) / 256, 256, 0, st>>>(d_count, d_wsum, weighted ? 1 : 0, mult, nb, d_out);
+    k_finalize<<<(nb + 255) / 256, 256, 0, st>>>(d_count, d_wsum, weighted ? 1 : 0, mult, nb, d_out, nullptr, nullptr);
     return cudaGetLastError();
 }
 
 pcf_status finalize_hist(pcf_ctx *ctx, const unsigned long long *d_count, const double *d_wsum,
-                         bool weighted, double mult, int nb, double *d_out) {
+                         bool weighted, double mult, int nb, double *out, const unsigned long long *d_stats,
+                         unsigned long long *host_stats) {
     k_finalize<<<(nb + 255) / 256, 256, 0, ctx->stream>>>(d_count, d_wsum, weighted ? 1 : 0, mult,
-                                                          nb, d_out);
+                                                          nb, out, d_stats, host_stats);
     PCF_CU(ctx, cudaGetLastError());
     ++ctx->launches;
     return PCF_OK;

@@ -161,10 +161,9 @@ struct DevBuf {
 
 constexpr int kTileCap = 32;  // home points per warp item
 
-// Page-locked host blocks for the grid builds' staging (the cell table read
-// back, the tile table sent), reused by size; shared by a context and its
-// cell structures, so a structure that outlives its context still returns
-// its block.
+// Page-locked host blocks for what the grid builds report, reused by size;
+// shared by a context and its cell structures, so a structure that outlives its
+// context still returns its block.
 struct PinnedPool {
     std::mutex mu;
     std::multimap<size_t, void *> free_blocks;
@@ -173,18 +172,24 @@ struct PinnedPool {
     ~PinnedPool();
 };
 
+// A few words that kernels or copies of a context's stream leave in page-locked
+// memory, and the event behind them.
+struct HostNote {
+    std::shared_ptr<PinnedPool> pinned;
+    void *block = nullptr;
+    size_t bytes = 0;
+    cudaEvent_t ready = nullptr;
+    // a block of at least n bytes to write to, and the event
+    cudaError_t open(const std::shared_ptr<PinnedPool> &pool, size_t n = 64);
+    cudaError_t wait(void *to, size_t n);  // waits, copies n bytes, returns the block
+    HostNote() = default;
+    HostNote(const HostNote &) = delete;
+    HostNote &operator=(const HostNote &) = delete;
+    ~HostNote();
+};
+
 struct CellGrid {
     int P = 0;
-    // a build whose cell table is still on its way to the host (deferred
-    // builds): `ready` follows its copy into `stage`; grid_finish completes
-    // it.  `stage` (from `pinned`) then feeds the tile table's copy and is
-    // returned once `ready`, recorded after that copy, has passed.
-    bool pending = false;
-    cudaEvent_t ready = nullptr;
-    void *stage = nullptr;
-    size_t stage_bytes = 0;
-    std::shared_ptr<PinnedPool> pinned;
-    ~CellGrid();
     uint64_t serial = 0;          // unique per build (keys captured graphs)
     float cell = 0.f;             // box / P
     DevBuf soa;                   // x | y | z | w planes, n + kSoaPad floats each
@@ -192,21 +197,24 @@ struct CellGrid {
     DevBuf pk;                    // pair-packed blocks (PairView), pk_blocks(n) x 32 B
     DevBuf qw;                    // exact integer weights (u32 x (n + kSoaPad)), when wfix_ok
     DevBuf cell_start;            // int x (P^3 + 1)
-    std::vector<int> h_start;     // host copy of cell_start
-    std::vector<TileDesc> tiles;  // home tiles: <= 32 points of one column, <= 2 cells
+    int64_t n_tiles = 0;          // home tiles: <= 32 points of one column, <= 2 cells
     DevBuf d_tiles;
     // the same with at most 16 points per tile (an autotuner candidate),
-    // built on first use
-    std::vector<TileDesc> tiles_half;
+    // built on first use (-1: not yet)
+    int64_t n_tiles_half = -1;
     DevBuf d_tiles_half;
-    bool have_half = false;
     // largest stencil population of a cell per (dmax, periodic), memoised
-    // for the triplet launches (a host pass over every cell and row)
+    // for the triplet launches
     mutable std::vector<std::pair<std::pair<float, bool>, int64_t>> stencil_memo;
-    const std::vector<TileDesc> &tiles_for(int cap) const { return cap == 16 ? tiles_half : tiles; }
+    int64_t tiles_for(int cap) const { return cap == 16 ? n_tiles_half : n_tiles; }
     const TileDesc *d_tiles_for(int cap) const {
         return (cap == 16 ? d_tiles_half : d_tiles).as<TileDesc>();
     }
+    // a build whose tile count is still on its way to the host: grid_finish
+    // completes it.  Declared behind the buffers: its end waits for the build
+    // before they are freed.
+    bool pending = false;
+    HostNote note;
     const float *x() const { return soa.as<float>(); }
     const float *y() const { return soa.as<float>() + plane; }
     const float *z() const { return soa.as<float>() + 2 * plane; }
@@ -235,6 +243,9 @@ struct pcf_grid {
     int wshift = 0;
     unsigned long long wqmax = 0;
     DevBuf raw;                   // float4 x n, input order
+    DevBuf flags;                 // the catalog's flags (three words; grid.cu), as found when it was taken in
+    HostNote note;                // their way to the host
+    bool unchecked = false;       // ... not yet read there (grid_finish)
     int user_P = 0;               // partitions fixed by the caller at build (0: automatic)
     // cell structures are shared: a captured batch graph keeps the ones it reads alive
     std::shared_ptr<CellGrid> cells;                    // the current cell structure
@@ -249,7 +260,9 @@ constexpr int kCellCache = 2;  // cell structures kept besides the current one
 struct PlanSlot {
     void *h_pinned = nullptr;
     size_t h_bytes = 0;
-    DevBuf d_rows, d_counter;
+    DevBuf d;                    // 8 zeroed counters | stencil rows | one pair job
+    unsigned long long *counter() const { return d.as<unsigned long long>(); }
+    RowDesc *rows() const { return reinterpret_cast<RowDesc *>(d.as<char>() + 64); }
     cudaEvent_t done = nullptr;  // recorded after the kernel that read this slot
     bool used = false;
 };
@@ -288,7 +301,7 @@ struct pcf_ctx {
     // the same for grid builds (counting sort + scatter kernels)
     std::vector<std::pair<cudaEvent_t, cudaEvent_t>> prof_grid_events;
     size_t prof_grid_used = 0;
-    int64_t prof_grid_points = 0;
+    int64_t prof_grid_points = 0, prof_grid_builds = 0;
     int device = 0;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -336,12 +349,17 @@ cudaError_t ensure_smem_limit(const void *fn, int device, size_t bytes);
         if (_e != cudaSuccess) return pcf_fail(ctx, _e, #call); \
     } while (0)
 
-// defer: return once the build is queued (its cell table read back
-// asynchronously); grid_finish then completes it (host cell table, catalog
-// checks, tile table).  Every use of a grid's host-side fields goes through
-// grid_finish first; it is a no-op for a finished grid.
+// defer: return once the build is queued; grid_finish then completes it (the
+// catalog's checks, the tile count).  Every use of a grid's host-side fields goes
+// through grid_finish first; it is a no-op for a finished grid.
 pcf_status grid_ensure_cells(pcf_ctx *ctx, pcf_grid *g, int P, bool defer = false);
 pcf_status grid_finish(pcf_ctx *ctx, const pcf_grid *g);
+// Copies and checks the caller's points (queued; grid_finish reads the checks).
+pcf_status grid_take(pcf_ctx *ctx, pcf_grid *g, const pcf_point *pts);
+pcf_status grid_default_cells(pcf_ctx *ctx, pcf_grid *g);
+pcf_status grid_host_starts(pcf_ctx *ctx, const pcf_grid *g, std::vector<int> &out);
+// Largest stencil population of any cell (rows on the device); waits for it.
+pcf_status stencil_max(pcf_ctx *ctx, const CellGrid &g, const RowDesc *d_rows, int n_rows, bool bpc, int64_t *out);
 // kind: a histogram kind, or kTripletCells.
 constexpr int kTripletCells = 3;
 int choose_partitions(int64_t n, float box, float dmax, int kind, bool bpc, int refine);
@@ -357,11 +375,8 @@ struct PairPlan {
     int64_t n_items = 0;
 };
 
-// Home tiles of a gridded catalog: runs of at most `cap` (<= kTileCap)
-// consecutive points of one column within two adjacent cells (pairs.cu).
-void build_tiles(const CellGrid &g, int cap, std::vector<TileDesc> &out);
-// The 16-point tile table of a cell structure, built and uploaded on first use.
-pcf_status ensure_half_tiles(pcf_ctx *ctx, CellGrid &g);
+// The 16-point tile table of a cell structure of n points, built on first use.
+pcf_status ensure_half_tiles(pcf_ctx *ctx, CellGrid &g, int64_t n);
 // Stencil rows (dx, dy, kz) of cells that can hold a pair within dmax.
 void plan_rows(int P, float box, float dmax, bool ani, bool self, std::vector<RowDesc> &rows);
 // Builds the stencil and item shape of one pair launch.  self: XX half shell.
@@ -369,6 +384,26 @@ void plan_pairs(const CellGrid &home, float box, float dmax, bool ani, bool self
                 int resident_warps, int tile_cap = kTileCap);
 
 pcf_status pcf_ensure_pinned(pcf_ctx *ctx, size_t bytes);
+// The way of a call's nb doubles and its four statistics words to the host.  The
+// last kernel of the call writes `stats` and, up to kDirectOut bytes, `to`
+// straight into the context's page-locked block: two copies behind the kernel
+// took 13 us of a call of 75.  Larger results (2 MB: 50 us by copy, 75 to 99
+// written by the kernel) are copied there from d_out, those past kStagedOut
+// straight to the caller.
+constexpr size_t kDirectOut = (size_t)256 << 10, kStagedOut = (size_t)16 << 20;
+struct OutPath {
+    double *to = nullptr;              // where the last kernel writes
+    double *staged = nullptr;          // page-locked, null: hist itself
+    unsigned long long *stats = nullptr;
+};
+pcf_status out_open(pcf_ctx *ctx, int64_t nb, bool dev_out, double *hist, double *d_out, OutPath *o);
+// Waits for the call, then copies into hist (host results).  hs: four words.
+pcf_status out_close(pcf_ctx *ctx, const OutPath &o, int64_t nb, bool dev_out, double *hist,
+                     unsigned long long *hs);
+// Reads `bytes` at d, behind the context's stream, into host memory that stays
+// until the next call on the context (spill: what the page-locked block is too
+// small for).
+pcf_status fetch_block(pcf_ctx *ctx, const void *d, size_t bytes, std::vector<char> &spill, const char **host);
 // PCF_ERR_TIMEOUT if an abort is requested (before a call launches) or if a
 // kernel gave up its queue (after the call's work is complete), else PCF_OK.
 pcf_status ctx_abort_requested(pcf_ctx *ctx);
@@ -390,6 +425,7 @@ struct PairLaunch {
     int lean_budget = 0; // adds between flushes of a two-limb column (pairs_lean.cuh)
     double wunscale = 0.0;  // single-job launches: weight_unscale(home, cand)
     bool count = true;   // weighted launches: count in-range pairs (statistics)
+    bool timed = true;   // ctx->ev0 and ev1 around the kernel (statistics)
     // queue control (pcf_ctx_abort): the abort word the kernel polls at every
     // ticket and the status word it sets when it gives up; null: no polling
     const unsigned *ctrl = nullptr;
@@ -411,7 +447,8 @@ pcf_status launch_pairs(pcf_ctx *ctx, const PairPlan &plan, const CellGrid &home
                         const CellGrid &cand, float box, const PairLaunch &pl,
                         unsigned long long *d_count, double *d_wsum, unsigned long long *d_stats);
 pcf_status finalize_hist(pcf_ctx *ctx, const unsigned long long *d_count, const double *d_wsum,
-                         bool weighted, double mult, int nb, double *d_out);
+                         bool weighted, double mult, int nb, double *out, const unsigned long long *d_stats,
+                         unsigned long long *host_stats);
 // One histogram of a pair launch: home / candidate catalogs, stencil rows,
 // and the implicit items [item_begin, item_begin + n_tiles * n_chunks).
 struct PairJob {
@@ -451,11 +488,12 @@ unsigned reference_pair_rule(bool ani, bool bpc, bool cross);
 // Counting sort of n points into P^3 cells on explicit buffers; returns the
 // number of kernels launched (counts must be zeroed, P^3 + 1 entries).
 // soa and qw may be null; pk (pk_blocks(n) blocks, zeroed by the caller) is
-// always written, qw only when the weights allow exact integers.  cid, rank
+// always written, qw only when the weights allow exact integers (flags: checked, the catalog's; else
+// zeroed words that the build sets).  cid, rank
 // and perm: n ints of scratch each.
 int launch_grid_build(const float4 *raw, int64_t n, int P, float cell, float box, int *cid,
                       int *rank, int *perm, int *counts, int *cell_start, int *scan_tmp, float *soa,
-                      size_t plane, float4 *pk, unsigned *qw, int *flags, cudaStream_t st);
+                      size_t plane, float4 *pk, unsigned *qw, int *flags, bool checked, cudaStream_t st);
 // Bucketed counting sort (the build for catalogs of 6M to ~134M points, or
 // any size when forced): Q cells per bucket, K buckets; false when the
 // catalog needs more buckets than the shared arrays hold (the per-point
@@ -465,11 +503,10 @@ bool grid_bucket_plan(int64_t n, int P, int *Q, int *K);
 // ints of each of the two CTA x bucket matrices (G CTAs)
 size_t grid_bucket_scratch_ints(int G, int K);
 cudaError_t grid_bucket_attrs(int device, int K);
-// M, Mx: grid_bucket_scratch_ints each; S: n float4 of scratch; flags zeroed.
-int launch_grid_build_buckets(const float4 *raw, int64_t n, int P, float cell, float box, int G, int Q,
-                              int K, int *M, int *Mx, int *scan_tmp, float4 *S, int *cell_start,
-                              float *soa, size_t plane, float4 *pk, unsigned *qw, int *flags,
-                              int device, cudaStream_t st);
+// M, Mx: grid_bucket_scratch_ints each; S: n float4 of scratch.
+int launch_grid_build_buckets(const float4 *raw, int64_t n, int P, float cell, int G, int Q, int K, int *M,
+                              int *Mx, int *scan_tmp, float4 *S, int *cell_start, float *soa, size_t plane,
+                              float4 *pk, unsigned *qw, const int *flags, int device, cudaStream_t st);
 // Zeroes the padding past point n of the SoA planes, integer weights and pair
 // blocks (the builds write entries 0 .. n-1); runs before the build.
 int launch_grid_tails(float *soa, size_t plane, int64_t n, float4 *pk, unsigned *qw, cudaStream_t st);
@@ -481,7 +518,10 @@ void set_weight_range(pcf_grid *g, const unsigned flags[3]);
 int launch_tile_build(const int *cell_start, int P, int *tile_counts, int *tile_offsets,
                       int *scan_tmp, TileDesc *tiles, cudaStream_t st);
 PairRule make_pair_rule(int bins, float dmax, uint32_t flags, bool ani, bool bpc, bool cross);
-pcf_status stage_plan(pcf_ctx *ctx, const PairPlan &plan, PlanSlot **out);
+// Sends the plan's rows, zeroed counters and, with job (whose rows it sets), one
+// pair job at *d_job to a slot, in one copy.
+pcf_status stage_plan(pcf_ctx *ctx, const PairPlan &plan, PlanSlot **out, PairJob *job = nullptr,
+                      PairJob **d_job = nullptr);
 // XX iso pair histogram with an explicit bin scale (analytic path).
 pcf_status pcf_count_pairs_ds(pcf_ctx *ctx, const pcf_grid *a, int bins, float dmax, double ds,
                               uint32_t flags, double *hist, pcf_stats *stats);

@@ -946,8 +946,10 @@ __global__ void __launch_bounds__(kTThreads, 1) k_triplets_ani(const TripArgs A)
 }
 
 __global__ void k_to_double(const unsigned long long *__restrict__ c, const double *__restrict__ w,
-                            int weighted, long long n, double *__restrict__ out) {
+                            int weighted, long long n, double *__restrict__ out,
+                            const unsigned long long *__restrict__ stats, unsigned long long *host_stats) {
     long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < 4) host_stats[t] = stats[t];
     if (t < n) out[t] = weighted ? w[t] : (double)c[t];
 }
 
@@ -955,9 +957,11 @@ __global__ void k_to_double(const unsigned long long *__restrict__ c, const doub
 // sums below are the same for U[b_ij][b_jk][b_ki]).
 __global__ void k_trip_finalize(const unsigned long long *__restrict__ cnt,
                                 const double *__restrict__ ws, int weighted, int mixed, int bins,
-                                double *__restrict__ out) {
+                                double *__restrict__ out, const unsigned long long *__restrict__ stats,
+                                unsigned long long *host_stats) {
     const int n3 = bins * bins * bins;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (host_stats && t < 4) host_stats[t] = stats[t];
     if (t >= n3) return;
     const int a = t / (bins * bins), b = (t / bins) % bins, c = t % bins;
     auto U = [&](int x, int y, int z) -> double {
@@ -972,38 +976,22 @@ __global__ void k_trip_finalize(const unsigned long long *__restrict__ cnt,
 
 }  // namespace
 
-// Largest stencil population of any cell of g: bounds an anchor's lists
-// (memoised per cell structure, dmax and periodicity: the rows are fixed by
-// them and the structure's P).
-static int64_t max_stencil_scan(const CellGrid &g, int P, const std::vector<RowDesc> &rows, bool bpc);
-static int64_t max_stencil(const CellGrid &g, float dmax, const std::vector<RowDesc> &rows, bool bpc) {
+// Bound of an anchor's list in a catalog of n points gridded as g: n itself
+// while overflow lists of that size are small, else the largest stencil
+// population of any cell (memoised per cell structure, dmax and periodicity: the
+// rows are fixed by them and the structure's P).
+static pcf_status list_bound(pcf_ctx *ctx, const CellGrid &g, int64_t n, float dmax, const RowDesc *d_rows, int n_rows,
+                             bool bpc, int64_t *out) {
+    *out = n;
+    if (n <= 8192) return PCF_OK;
     for (const auto &m : g.stencil_memo)
-        if (m.first.first == dmax && m.first.second == bpc) return m.second;
-    const int64_t v = max_stencil_scan(g, g.P, rows, bpc);
-    g.stencil_memo.push_back({{dmax, bpc}, v});
-    return v;
-}
-static int64_t max_stencil_scan(const CellGrid &g, int P, const std::vector<RowDesc> &rows, bool bpc) {
-    const std::vector<int> &cs = g.h_start;
-    int64_t best = 0;
-    for (int ix = 0; ix < P; ++ix)
-        for (int iy = 0; iy < P; ++iy)
-            for (int iz = 0; iz < P; ++iz) {
-                int64_t n = 0;
-                for (const RowDesc &rw : rows) {
-                    int nx = ix + rw.dx, ny = iy + rw.dy;
-                    if (bpc) { nx = (nx + P) % P; ny = (ny + P) % P; }
-                    else if (nx < 0 || nx >= P || ny < 0 || ny >= P) continue;
-                    const int col = (nx * P + ny) * P;
-                    const int zlo = iz - rw.kz, zhi = iz + rw.kz;
-                    const int lo = std::max(zlo, 0), hi = std::min(zhi, P - 1);
-                    if (lo <= hi) n += cs[col + hi + 1] - cs[col + lo];
-                    if (bpc && zlo < 0) n += cs[col + P] - cs[col + zlo + P];
-                    if (bpc && zhi >= P) n += cs[col + zhi - P + 1] - cs[col];
-                }
-                best = std::max(best, n);
-            }
-    return best;
+        if (m.first.first == dmax && m.first.second == bpc) {
+            *out = m.second;
+            return PCF_OK;
+        }
+    const pcf_status s = stencil_max(ctx, g, d_rows, n_rows, bpc, out);
+    if (s == PCF_OK) g.stencil_memo.push_back({{dmax, bpc}, *out});
+    return s;
 }
 
 // FP32 windows of the triplet kernels (u = 2^-24, R = dmax, L = box).  A list
@@ -1142,18 +1130,19 @@ extern "C" pcf_status pcf_count_triplets(pcf_ctx *ctx, int kind, const pcf_grid 
     size_t smem = 0;
     trip_setup(ctx, X, Y, P, (int)plan.rows.size(), bins, dmax, flags, weighted, A, smem);
     const int n3 = bins * bins * bins;
-    // overflow lists: bounded by the largest stencil population of any cell
-    const int64_t gmax = std::max<int64_t>(max_stencil(gx, dmax, plan.rows, bpc),
-                                           mixed ? max_stencil(gy, dmax, plan.rows, bpc) : 0) + 32;
-    const int grid = ctx->sm_count;
-    s = trip_overflow(ctx, gmax, mixed, weighted, grid, A);
-    if (s != PCF_OK) return s;
     // rows + counter through the plan slot
     PlanSlot *sl = nullptr;
     s = stage_plan(ctx, plan, &sl);
     if (s != PCF_OK) return s;
-    A.rows = sl->d_rows.as<RowDesc>();
-    A.counter = sl->d_counter.as<unsigned long long>();
+    A.rows = sl->rows();
+    A.counter = sl->counter();
+    // overflow lists
+    int64_t bx = 0, by = 0;
+    s = list_bound(ctx, gx, X->n, dmax, A.rows, A.n_rows, bpc, &bx);
+    if (s == PCF_OK && mixed) s = list_bound(ctx, gy, Y->n, dmax, A.rows, A.n_rows, bpc, &by);
+    const int grid = ctx->sm_count;
+    if (s == PCF_OK) s = trip_overflow(ctx, std::max(bx, by) + 32, mixed, weighted, grid, A);
+    if (s != PCF_OK) return s;
     // histogram scratch: [u64 n3][f64 n3][stats 8][f64 out n3]
     PCF_CU(ctx, ctx->d_hist.ensure((size_t)n3 * 24 + 64));
     char *hp = ctx->d_hist.as<char>();
@@ -1180,24 +1169,18 @@ extern "C" pcf_status pcf_count_triplets(pcf_ctx *ctx, int kind, const pcf_grid 
     PCF_CU(ctx, cudaEventRecord(sl->done, ctx->stream));
     ++ctx->launches;
     const bool dev_out = (flags & PCF_DEVICE_OUT) != 0;
+    OutPath o;
+    s = out_open(ctx, n3, dev_out, hist, d_out, &o);
+    if (s != PCF_OK) return s;
     k_trip_finalize<<<(n3 + 255) / 256, 256, 0, ctx->stream>>>(A.g_count, A.g_wsum, weighted ? 1 : 0,
-                                                                mixed ? 1 : 0, bins,
-                                                                dev_out ? hist : d_out);
+                                                                mixed ? 1 : 0, bins, o.to, A.g_stats,
+                                                                stats || !dev_out ? o.stats : nullptr);
     PCF_CU(ctx, cudaGetLastError());
     ++ctx->launches;
-    if (stats || !dev_out) {  // through the context's page-locked buffer (see count_pairs_impl)
-        const size_t hb = dev_out ? 0 : sizeof(double) * n3;
-        s = pcf_ensure_pinned(ctx, hb + 64);
-        if (s != PCF_OK) return s;
-        char *hp = static_cast<char *>(ctx->h_pinned);
-        if (hb) PCF_CU(ctx, cudaMemcpyAsync(hp, d_out, hb, cudaMemcpyDeviceToHost, ctx->stream));
-        PCF_CU(ctx, cudaMemcpyAsync(hp + hb, A.g_stats, 32, cudaMemcpyDeviceToHost, ctx->stream));
-        PCF_CU(ctx, cudaStreamSynchronize(ctx->stream));
-        s = ctx_queue_status(ctx);
-        if (s != PCF_OK) return s;
-        if (hb) memcpy(hist, hp, hb);
+    if (stats || !dev_out) {
         unsigned long long hs[4];
-        memcpy(hs, hp + hb, sizeof(hs));
+        s = out_close(ctx, o, n3, dev_out, hist, hs);
+        if (s != PCF_OK) return s;
         if (stats) {
             float ms = 0.f;
             cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
@@ -1278,12 +1261,22 @@ extern "C" pcf_status pcf_batch_triplets(pcf_ctx *ctx, const pcf_grid *d_, const
     long long anchors = 0;
     bool any_mixed = false;
     int64_t gmax = 0;
-    std::map<const pcf_grid *, int64_t> stencil;  // per grid
-    auto stencil_of = [&](const pcf_grid *g) {
-        auto it = stencil.find(g);
-        if (it != stencil.end()) return it->second;
-        return stencil[g] = max_stencil(*g->cells, dmax, plan.rows, bpc);
-    };
+    // rows + counters through the plan slot
+    PlanSlot *sl = nullptr;
+    s = stage_plan(ctx, plan, &sl);
+    if (s != PCF_OK) return s;
+    for (pcf_grid *g : R) {
+        int64_t b = 0;
+        s = list_bound(ctx, *g->cells, g->n, dmax, sl->rows(), (int)plan.rows.size(), bpc, &b);
+        if (s != PCF_OK) return s;
+        gmax = std::max(gmax, b);
+    }
+    {
+        int64_t b = 0;
+        s = list_bound(ctx, *D->cells, D->n, dmax, sl->rows(), (int)plan.rows.size(), bpc, &b);
+        if (s != PCF_OK) return s;
+        gmax = std::max(gmax, b);
+    }
     for (int k = 0; k < nj; ++k) {
         size_t sm = 0;
         trip_setup(ctx, jobs[k].x, jobs[k].y, P, (int)plan.rows.size(), bins, dmax, flags, weighted,
@@ -1292,18 +1285,13 @@ extern "C" pcf_status pcf_batch_triplets(pcf_ctx *ctx, const pcf_grid *d_, const
         args[k].anchor_begin = anchors;
         anchors += jobs[k].x->n;
         any_mixed = any_mixed || jobs[k].y;
-        gmax = std::max<int64_t>(gmax, stencil_of(jobs[k].x));
-        if (jobs[k].y) gmax = std::max<int64_t>(gmax, stencil_of(jobs[k].y));
     }
     const int grid = ctx->sm_count;
     TripArgs ov;
     s = trip_overflow(ctx, gmax + 32, any_mixed, weighted, grid, ov);
     if (s != PCF_OK) return s;
 
-    // rows + counter through the plan slot; histograms per job
-    PlanSlot *sl = nullptr;
-    s = stage_plan(ctx, plan, &sl);
-    if (s != PCF_OK) return s;
+    // histograms per job
     const size_t nh = (size_t)nj * n3;
     PCF_CU(ctx, ctx->d_hist.ensure(nh * 24 + 64));
     char *hp = ctx->d_hist.as<char>();
@@ -1319,8 +1307,8 @@ extern "C" pcf_status pcf_batch_triplets(pcf_ctx *ctx, const pcf_grid *d_, const
         A.gK = ov.gK;
         A.gwJ = ov.gwJ;
         A.gwK = ov.gwK;
-        A.rows = sl->d_rows.as<RowDesc>();
-        A.counter = sl->d_counter.as<unsigned long long>();
+        A.rows = sl->rows();
+        A.counter = sl->counter();
         A.g_count = cnt + (size_t)k * n3;
         A.g_wsum = wsum + (size_t)k * n3;
         A.g_stats = gstats;
@@ -1348,7 +1336,7 @@ extern "C" pcf_status pcf_batch_triplets(pcf_ctx *ctx, const pcf_grid *d_, const
         PCF_CU(ctx, cudaEventRecord(pe0, ctx->stream));
     }
     PCF_CU(ctx, cudaEventRecord(ctx->ev0, ctx->stream));
-    unsigned long long *ctr = sl->d_counter.as<unsigned long long>();
+    unsigned long long *ctr = sl->counter();
     std::unique_ptr<TripBatch> tb(new TripBatch);
     for (size_t q = 0; q < groups.size(); ++q) {
         memset(tb.get(), 0, sizeof(TripBatch));
@@ -1375,19 +1363,18 @@ extern "C" pcf_status pcf_batch_triplets(pcf_ctx *ctx, const pcf_grid *d_, const
     for (int k = 0; k < nj; ++k) {
         k_trip_finalize<<<(n3 + 255) / 256, 256, 0, ctx->stream>>>(
             cnt + (size_t)k * n3, wsum + (size_t)k * n3, weighted ? 1 : 0, jobs[k].y ? 1 : 0, bins,
-            d_out + (size_t)k * n3);
+            d_out + (size_t)k * n3, nullptr, nullptr);
         PCF_CU(ctx, cudaGetLastError());
         ++ctx->launches;
     }
-    std::vector<double> host(nh);
-    unsigned long long hs[4] = {0, 0, 0, 0};
-    PCF_CU(ctx, cudaMemcpyAsync(host.data(), d_out, sizeof(double) * nh, cudaMemcpyDeviceToHost,
-                                ctx->stream));
-    PCF_CU(ctx, cudaMemcpyAsync(hs, gstats, sizeof(hs), cudaMemcpyDeviceToHost, ctx->stream));
-    PCF_CU(ctx, cudaStreamSynchronize(ctx->stream));
-    s = ctx_queue_status(ctx);
+    std::vector<char> spill;
+    const char *hb = nullptr;
+    s = fetch_block(ctx, gstats, 64 + sizeof(double) * nh, spill, &hb);  // [stats | out]
+    if (s == PCF_OK) s = ctx_queue_status(ctx);
     if (s != PCF_OK) return s;
-    for (int k = 0; k < nj; ++k) memcpy(jobs[k].out, host.data() + (size_t)k * n3, sizeof(double) * n3);
+    unsigned long long hs[4];
+    memcpy(hs, hb, sizeof(hs));
+    for (int k = 0; k < nj; ++k) memcpy(jobs[k].out, hb + 64 + (size_t)k * n3 * sizeof(double), sizeof(double) * n3);
     if (stats) {
         float ms = 0.f;
         cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
@@ -1479,8 +1466,8 @@ static pcf_status count_triplets_ordered(pcf_ctx *ctx, const pcf_grid *x_, const
     PlanSlot *sl = nullptr;
     s = stage_plan(ctx, plan, &sl);
     if (s != PCF_OK) return s;
-    A.rows = sl->d_rows.as<RowDesc>();
-    A.counter = sl->d_counter.as<unsigned long long>();
+    A.rows = sl->rows();
+    A.counter = sl->counter();
     PCF_CU(ctx, ctx->d_hist.ensure((size_t)n5 * 16 + 128));
     char *hp = ctx->d_hist.as<char>();
     A.g_count = reinterpret_cast<unsigned long long *>(hp);
@@ -1504,17 +1491,16 @@ static pcf_status count_triplets_ordered(pcf_ctx *ctx, const pcf_grid *x_, const
     PCF_CU(ctx, cudaGetLastError());
     PCF_CU(ctx, cudaEventRecord(ctx->ev1, ctx->stream));
     PCF_CU(ctx, cudaEventRecord(sl->done, ctx->stream));
-    k_to_double<<<(unsigned)((n5 + 255) / 256), 256, 0, ctx->stream>>>(A.g_count, A.g_wsum,
-                                                                       weighted ? 1 : 0, n5, d_out);
+    const bool dev_out = (flags & PCF_DEVICE_OUT) != 0;
+    OutPath o;
+    s = out_open(ctx, n5, dev_out, hist, d_out, &o);
+    if (s != PCF_OK) return s;
+    k_to_double<<<(unsigned)((n5 + 255) / 256), 256, 0, ctx->stream>>>(A.g_count, A.g_wsum, weighted ? 1 : 0, n5, o.to,
+                                                                       A.g_stats, o.stats);
     PCF_CU(ctx, cudaGetLastError());
     ctx->launches += 2;
-    const bool dev_out = (flags & PCF_DEVICE_OUT) != 0;
-    unsigned long long hs[4] = {0, 0, 0, 0};
-    PCF_CU(ctx, cudaMemcpyAsync(hs, A.g_stats, sizeof(hs), cudaMemcpyDeviceToHost, ctx->stream));
-    PCF_CU(ctx, cudaMemcpyAsync(hist, d_out, sizeof(double) * n5,
-                                dev_out ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, ctx->stream));
-    PCF_CU(ctx, cudaStreamSynchronize(ctx->stream));
-    s = ctx_queue_status(ctx);
+    unsigned long long hs[4];
+    s = out_close(ctx, o, n5, dev_out, hist, hs);
     if (s != PCF_OK) return s;
     if (hs[3]) {
         ctx->last_error = "neighbour lists of the anisotropic triplet kernel exceed shared memory";

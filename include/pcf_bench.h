@@ -46,15 +46,16 @@ pcf_status pcf_microbench(pcf_ctx *ctx, int which, double *result);
  *                              Results are the same in every variant.
  *   PCF_OPT_GRID_BUILD         the grid build: 0 (default) by size (the
  *                              bucketed counting sort from 6M points, the
- *                              per-point one below), 1 per-point, 2
+ *                              per-point one below, one block up to 4096
+ *                              points and cells), 1 per-point, 2
  *                              bucketed wherever its shared arrays allow.
  *                              Grids are the same either way up to the
  *                              order of points inside a cell.
  *   PCF_OPT_GRID_DEFER         0 (default): pcf_grid_build returns a
- *                              complete grid, or the catalog's error.  1:
- *                              it returns once the build is queued; the
- *                              first call that uses the grid completes it
- *                              (waiting only for this build's cell table)
+ *                              checked catalog, or its error.  1: it
+ *                              returns once the copy and the check are
+ *                              queued; the first call that uses the grid
+ *                              waits for them
  *                              and reports a catalog error such as
  *                              PCF_ERR_OUT_OF_BOX, as does every later use.
  *                              Building several grids before counting then
