@@ -214,3 +214,59 @@ __device__ __forceinline__ int gate_mult(const GateGeom &g, const GateNode &n1, 
     }
     return m;
 }
+
+// Whether the block of images (f2, f3) holds the geometry of those images: one
+// block, edge flags as its images, and on each pair the distance test through the
+// image that joins the pair (f2, f3 and, between nodes 2 and 3, their difference).
+__device__ inline bool gate_regular(int f2, int f3, const GateBlock *blocks, const signed char (*by_image)[2]) {
+    const signed char *blk = by_image[f2 | (f3 << 3)];
+    if (blk[0] < 0 || blk[1] >= 0) return false;
+    const GateBlock &B = blocks[blk[0]];
+    if (B.a2 != f2 || B.a3 != f3 || B.f2 != f2 || B.f3 != f3) return false;
+    unsigned pairs = 0;
+    for (int t = 0; t < 3; ++t) {
+        const GateTest &T = B.t[t];
+        int axes = 0, na = 0;
+        for (int a = 0; a < 3; ++a)
+            if (T.ax[a] >= 0) { axes |= 1 << T.ax[a]; ++na; }
+        const int want = T.pair == 0 ? f2 : T.pair == 1 ? (f2 ^ f3) : f3;
+        if (axes != want || na != __popc((unsigned)want) || T.k != na) return false;
+        pairs |= 1u << T.pair;
+    }
+    return pairs == 7u;
+}
+
+// Whether a regular block counts every triangle in range (squared sides up to dd)
+// exactly once on this node grid, wherever its points lie in their nodes and
+// however the gate's FP32 arithmetic rounds (u = 2^-24):
+//  * a node corner is off by at most 2uL of the point's cell edge (the division's
+//    and the product's rounding), a difference of two by uL more, and P s is L
+//    within uL: tol = 16uL covers any axis and sqrt(3) times it;
+//  * a test's value is off by at most 42 u L^2 (its terms reach 6 L^2): err.
+// Edge flags: every node that a point within reach of a face can lie in passes its
+// comparison (evaluated as the gate does).  Tests: of two points in range, the
+// node offset (a, b, c) has its nearest corners, (|a| - 1)+ and so on, in range;
+// each such offset's own length must stay inside the gate's (dmax + s sqrt(3)).
+// That fails only where dmax lies within about 1e-4 of a length that makes an
+// offset along a diagonal touch the bound.
+inline bool gates_hold(const GateGeom &g, double dd) {
+    const double u = std::ldexp(1.0, -24), L = g.L, s = g.s, tol = 16.0 * u * L, err = 64.0 * u * L * L;
+    const double R = std::sqrt(dd) * (1.0 + 1e-6) + tol;
+    if (!(2.0 * R < L)) return false;
+    for (int i = 0; i < g.P; ++i) {
+        const float n = (float)i * g.s;
+        if ((double)n - tol < R && !(n <= g.fd)) return false;
+        if (((double)i + 1.0) * s + tol > L - R && !(n >= g.fdn)) return false;
+    }
+    const int K = (int)(R / s) + 3;
+    auto gap = [&](int a) { return std::max(0.0, (double)(a - 1) * s - tol); };
+    for (int a = 0; a <= K; ++a)
+        for (int b = 0; b <= a; ++b) {
+            const double rest = R * R - gap(a) * gap(a) - gap(b) * gap(b);
+            if (rest < 0) break;
+            const double c = std::floor((std::sqrt(rest) + tol) / s) + 1.0;  // largest |c| in range
+            const double len = s * std::sqrt((double)a * a + (double)b * b + c * c) + tol;
+            if (len * len + err > (double)g.M) return false;
+        }
+    return true;
+}

@@ -252,14 +252,15 @@ struct ListScratch {
 // written.  Entries: {dx, dy, dz in bins, bits(idx << 8 | bin)}.  ang: their
 // angle bins (ANG).  ginfo (PCF_REF_NODE_GATES): per entry, its node on the
 // reference's grid and the axes of its image relative to the anchor
-// (gate_pack).  Called by the whole CTA; ends synchronised.
+// (gate_pack).  WRAPPED: only the neighbours through an image.  Called by the
+// whole CTA; ends synchronised.
 //
 // All rows' candidates form one index space that the CTA takes 768 at a time
 // (the range of an index by binary search): a row holds 10 to 100 candidates,
 // so a loop over rows kept 1 to 3 warps busy and cost a dependent
 // cell-table load per row.  The order is kept (a barrier per round) so that
 // runs of entries stay close in space, for the culling of tri_tiles.
-template <bool ANG>
+template <bool ANG, bool WRAPPED = false>
 __device__ int build_list(const TripArgs &A, const Cat &C, float hx, float hy, float hz, int cix, int ciy,
                           int ciz, int only_after, const PairRule &rule, float4 *list, float *wlist, int cap,
                           unsigned &n_rechk, ListScratch &S, unsigned char *ang = nullptr,
@@ -291,7 +292,7 @@ __device__ int build_list(const TripArgs &A, const Cat &C, float hx, float hy, f
             if (cn >= 0) { nx = C.x[cn]; ny = C.y[cn]; nz = C.z[cn]; }
             int bin = -2, tang = 0;
             float vx = 0.f, vy = 0.f, vz = 0.f;
-            if (c >= 0) {
+            if (c >= 0 && !(WRAPPED && sh == (1 | (1 << 2) | (1 << 4)))) {
                 vx = px - (hx - (float)((sh & 3) - 1) * A.box);
                 vy = py - (hy - (float)(((sh >> 2) & 3) - 1) * A.box);
                 vz = pz - (hz - (float)((sh >> 4) - 1) * A.box);
@@ -945,6 +946,129 @@ __global__ void __launch_bounds__(kTThreads, 1) k_triplets_ani(const TripArgs A)
     }
 }
 
+// Node-gated isotropic counts (unit weights) as corrections of the plain ones.
+// Where gates_hold, a regular block (node_gates.cuh) counts each of its triangles
+// once, so the gated histogram is the plain one, which k_triplets makes from
+// unordered triangles, plus (multiplicity - 1) of the ordered triangles whose
+// images (F2, F3) have no regular block: eight of the 64 combinations, both points
+// through an image and two axes involved.  This kernel evaluates those alone, from
+// the anchors near two or more faces and their neighbours through an image.
+// Evaluating every ordered triangle's gates, with a global atomic each, took 50.7 ms
+// for 4096 and 4100 points (DDD, RRR, DDR, DRR; bins 30, dmax 80 of 250).
+// Histogram: A.g_count, bins^3 signed, [b(d12)][b(d23)][b(d31)]; g_stats[1]: their sum.
+template <bool MIXED>
+__global__ void __launch_bounds__(kTThreads, 1) k_gate_fix(const __grid_constant__ TripArgs A, float reach) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    float4 *sJ = reinterpret_cast<float4 *>(smem), *sK = sJ + A.capJ;
+    unsigned *gJ = reinterpret_cast<unsigned *>(sK + A.capK), *gK = gJ + A.capJ;
+    // the third points by image: indices in `by`, those of images f at s_class[f] ..
+    unsigned short *by = reinterpret_cast<unsigned short *>(gK + A.capK);
+    __shared__ int s_class[9], s_fill[8];
+    __shared__ ListScratch s_scr;
+    __shared__ int s_anchor;
+    __shared__ unsigned s_stop;
+    __shared__ GateBlock s_gates[64];
+    __shared__ signed char s_gate_by[64][2];
+    __shared__ unsigned s_irr[8];  // per F2: the F3 without a regular block
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, bins = A.rXX.bins;
+    if (tid < 8) s_irr[tid] = 0u;
+    if (tid < 64) {
+        s_gates[tid] = kGateBlocks[tid];
+        s_gate_by[tid][0] = kGateByImage[tid][0];
+        s_gate_by[tid][1] = kGateByImage[tid][1];
+    }
+    __syncthreads();
+    if (tid < 64 && !gate_regular(tid & 7, tid >> 3, s_gates, s_gate_by)) atomicOr(&s_irr[tid & 7], 1u << (tid >> 3));
+    unsigned n_rechk = 0;
+    long long n_fix = 0, taken = 0;
+    for (;;) {
+        if (tid == 0) {
+            s_anchor = (int)atomicAdd(A.counter, 1ull);
+            unsigned stop = (A.ctrl && ctrl_load(A.ctrl)) ? PCF_GAVE_UP_ABORT : 0u;
+            if (++taken > (long long)A.nX + 1) stop |= PCF_GAVE_UP_CAP;
+            if (stop && A.status) ctrl_store(A.status, stop);
+            s_stop = stop;
+        }
+        __syncthreads();
+        const int i = s_anchor;
+        if (i >= A.nX || s_stop) break;
+        const float hx = A.X.x[i], hy = A.X.y[i], hz = A.X.z[i];
+        const int near = (hx <= reach || hx >= A.box - reach) + (hy <= reach || hy >= A.box - reach) +
+                         (hz <= reach || hz >= A.box - reach);
+        if (near >= 2) {
+            const int P = A.P;
+            const int cix = min(max((int)__fdiv_rn(hx, A.cell), 0), P - 1);
+            const int ciy = min(max((int)__fdiv_rn(hy, A.cell), 0), P - 1);
+            const int ciz = min(max((int)__fdiv_rn(hz, A.cell), 0), P - 1);
+            const int nJ = build_list<false, true>(A, A.X, hx, hy, hz, cix, ciy, ciz, -1, A.rXX, sJ, nullptr, A.capJ,
+                                                   n_rechk, s_scr, nullptr, gJ);
+            const int nK = MIXED ? build_list<false, true>(A, A.Y, hx, hy, hz, cix, ciy, ciz, -1, A.rXY, sK, nullptr,
+                                                           A.capK, n_rechk, s_scr, nullptr, gK)
+                                 : nJ;
+            const bool fits = nJ <= A.capJ && (!MIXED || nK <= A.capK);
+            if (!fits && tid == 0) atomicAdd(A.g_stats + 3, 1ull);  // not reached: the host bounds the lists
+            const GateNode n1 = gate_unpack(A.gate, gate_pack(A.gate, hx, hy, hz, 0u));
+            const float4 *LK = MIXED ? sK : sJ;
+            const unsigned *GK = MIXED ? gK : gJ;
+            if (tid < 8) s_fill[tid] = 0;
+            __syncthreads();
+            for (int kk = tid; fits && kk < nK; kk += kTThreads) atomicAdd(&s_fill[GK[kk] >> 27 & 7u], 1);
+            __syncthreads();
+            if (tid == 0) {
+                int n = 0;
+                for (int f = 0; f < 8; ++f) {
+                    s_class[f] = n;
+                    n += s_fill[f];
+                    s_fill[f] = s_class[f];
+                }
+                s_class[8] = n;
+            }
+            __syncthreads();
+            for (int kk = tid; fits && kk < nK; kk += kTThreads)
+                by[atomicAdd(&s_fill[GK[kk] >> 27 & 7u], 1)] = (unsigned short)kk;
+            __syncthreads();
+            for (int jj = warp; fits && jj < nJ; jj += kTWarps) {
+                unsigned irr = s_irr[(gJ[jj] >> 27) & 7u];
+                if (!irr) continue;
+                const float4 ej = sJ[jj];
+                const GateNode n2 = gate_unpack(A.gate, gJ[jj]);
+                const int jidx = (int)((unsigned)__float_as_int(ej.w) >> 8), bj = __float_as_int(ej.w) & 255;
+                for (; irr; irr &= irr - 1u)
+                for (int q = s_class[__ffs(irr) - 1] + lane; q < s_class[__ffs(irr)]; q += 32) {
+                    const int kk = by[q];
+                    if (!MIXED && kk == jj) continue;
+                    const float4 ek = LK[kk];
+                    const float dx = ek.x - ej.x, dy = ek.y - ej.y, dz = ek.z - ej.z;
+                    int c = fast_bin3(fmaf(dz, dz, fmaf(dy, dy, dx * dx)), A.fc, bins);
+                    if (c == -1) {
+                        ++n_rechk;
+                        const int kidx = (int)((unsigned)__float_as_int(ek.w) >> 8);
+                        const Cat &CK = MIXED ? A.Y : A.X;
+                        c = exact_third(hx, hy, hz, A.X.x[jidx], A.X.y[jidx], A.X.z[jidx], CK.x[kidx], CK.y[kidx],
+                                        CK.z[kidx], A.bpc, A.box, MIXED ? A.rXY : A.rXX);
+                    }
+                    if (c < 0) continue;
+                    const int fix = gate_mult(A.gate, n1, n2, gate_unpack(A.gate, GK[kk]), s_gates, s_gate_by) - 1;
+                    if (fix == 0) continue;
+                    n_fix += fix;
+                    atomicAdd(A.g_count + ((long long)bj * bins + c) * bins + (__float_as_int(ek.w) & 255),
+                              (unsigned long long)(long long)fix);
+                }
+            }
+        }
+        __syncthreads();
+    }
+    unsigned long long rr = n_rechk;
+    for (int off = 16; off > 0; off >>= 1) {
+        rr += __shfl_down_sync(kFull, rr, off);
+        n_fix += __shfl_down_sync(kFull, n_fix, off);
+    }
+    if (lane == 0) {
+        if (rr) atomicAdd(A.g_stats + 0, rr);
+        if (n_fix) atomicAdd(A.g_stats + 1, (unsigned long long)n_fix);
+    }
+}
+
 __global__ void k_to_double(const unsigned long long *__restrict__ c, const double *__restrict__ w,
                             int weighted, long long n, double *__restrict__ out,
                             const unsigned long long *__restrict__ stats, unsigned long long *host_stats) {
@@ -953,12 +1077,13 @@ __global__ void k_to_double(const unsigned long long *__restrict__ c, const doub
     if (t < n) out[t] = weighted ? w[t] : (double)c[t];
 }
 
+// fix: the node gates' corrections of an unweighted count.
 // Ordered-triple histogram from the oriented counts U[b_ij][b_ki][b_jk] (both
 // sums below are the same for U[b_ij][b_jk][b_ki]).
 __global__ void k_trip_finalize(const unsigned long long *__restrict__ cnt,
                                 const double *__restrict__ ws, int weighted, int mixed, int bins,
                                 double *__restrict__ out, const unsigned long long *__restrict__ stats,
-                                unsigned long long *host_stats) {
+                                unsigned long long *host_stats, const unsigned long long *__restrict__ fix) {
     const int n3 = bins * bins * bins;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (host_stats && t < 4) host_stats[t] = stats[t];
@@ -968,6 +1093,14 @@ __global__ void k_trip_finalize(const unsigned long long *__restrict__ cnt,
         const int s = (x * bins + y) * bins + z;
         return weighted ? ws[s] : (double)cnt[s];
     };
+    if (fix) {  // k_gate_fix, in whole numbers
+        auto N = [&](int x, int y, int z) { return cnt[(x * bins + y) * bins + z]; };
+        const unsigned long long n =
+            mixed ? N(a, b, c) + N(a, c, b)
+                  : N(a, b, c) + N(b, c, a) + N(c, a, b) + N(a, c, b) + N(c, b, a) + N(b, a, c);
+        out[t] = (double)(n + fix[t]);
+        return;
+    }
     double v;
     if (mixed) v = U(a, b, c) + U(a, c, b);
     else v = U(a, b, c) + U(b, c, a) + U(c, a, b) + U(a, c, b) + U(c, b, a) + U(b, a, c);
@@ -977,13 +1110,13 @@ __global__ void k_trip_finalize(const unsigned long long *__restrict__ cnt,
 }  // namespace
 
 // Bound of an anchor's list in a catalog of n points gridded as g: n itself
-// while overflow lists of that size are small, else the largest stencil
+// up to `cheap` (while overflow lists of that size are small), else the largest stencil
 // population of any cell (memoised per cell structure, dmax and periodicity: the
 // rows are fixed by them and the structure's P).
 static pcf_status list_bound(pcf_ctx *ctx, const CellGrid &g, int64_t n, float dmax, const RowDesc *d_rows, int n_rows,
-                             bool bpc, int64_t *out) {
+                             bool bpc, int64_t *out, int64_t cheap = 8192) {
     *out = n;
-    if (n <= 8192) return PCF_OK;
+    if (n <= cheap) return PCF_OK;
     for (const auto &m : g.stencil_memo)
         if (m.first.first == dmax && m.first.second == bpc) {
             *out = m.second;
@@ -1098,14 +1231,42 @@ static pcf_status count_triplets_ordered(pcf_ctx *ctx, const pcf_grid *x_, const
                                          float dmax, uint32_t flags, double *hist, pcf_stats *stats,
                                          bool iso3);
 
+// Entries that the ordered counts' lists hold in shared memory; returns the bytes
+// of one (the row table of the list build takes one of them).
+static size_t ordered_caps(bool mixed, bool weighted, bool gates, TripArgs &A) {
+    const size_t ent = 16 + 2 + (weighted ? 4 : 0) + (gates ? 4 : 0);
+    const size_t room = 227 * 1024 - 256 - (gates ? 64 * sizeof(GateBlock) + 128 + 64 : 0);
+    if (mixed) {
+        A.capJ = (int)(room / ent / 3);
+        A.capK = (int)(room / ent) - A.capJ - 8;
+    } else {
+        A.capJ = (int)(room / ent) - 8;
+        A.capK = 0;
+    }
+    return ent;
+}
+
 extern "C" pcf_status pcf_count_triplets(pcf_ctx *ctx, int kind, const pcf_grid *x_,
                                          const pcf_grid *y_, int bins, float dmax, uint32_t flags,
                                          double *hist, pcf_stats *stats) {
     if (!ctx || !x_ || !hist || bins < 1 || !(dmax > 0.f)) return PCF_ERR_INVALID_ARG;
     if (kind == PCF_ANI) return pcf_count_triplets_ani(ctx, x_, y_, bins, dmax, flags, hist, stats);
     if (kind != PCF_ISO) return PCF_ERR_INVALID_ARG;
-    if (flags & PCF_REF_NODE_GATES)
-        return count_triplets_ordered(ctx, x_, y_, bins, dmax, flags, hist, stats, true);
+    // Node gates of unit-weight counts: corrections of the plain count where the
+    // gates hold on the grid's nodes; else (weights, whose corrections would
+    // cancel; long lists; a touching diagonal; invalid calls) every ordered triangle.
+    const bool gates = (flags & PCF_REF_NODE_GATES) != 0;
+    auto ordered = [&] { return count_triplets_ordered(ctx, x_, y_, bins, dmax, flags, hist, stats, true); };
+    GateGeom geom{};
+    if (gates) {
+        if (!(flags & PCF_BPC) || x_->user_P < 1 || x_->user_P > 512 || bins > 255 ||
+            (int64_t)bins * bins * bins > (1 << 26) ||
+            (y_ && (y_->user_P != x_->user_P || y_->box != x_->box)))
+            return ordered();
+        geom = gate_geometry(x_->box, dmax, x_->user_P);
+        if (!gates_hold(geom, make_pair_rule(bins, dmax, flags & ~PCF_DS_EXACT, false, true, false).dd))
+            return ordered();
+    }
     if (bins > 255 || (int64_t)bins * bins * bins > (1 << 26)) return PCF_ERR_UNSUPPORTED;
     cudaSetDevice(ctx->device);
     {
@@ -1126,6 +1287,7 @@ extern "C" pcf_status pcf_count_triplets(pcf_ctx *ctx, int kind, const pcf_grid 
     PairPlan plan;
     plan_pairs(gx, X->box, dmax, false, false, plan, ctx->sm_count * 24);
     const bool weighted = !(X->unit_weights && (!mixed || Y->unit_weights));
+    if (gates && weighted) return ordered();
     TripArgs A;
     size_t smem = 0;
     trip_setup(ctx, X, Y, P, (int)plan.rows.size(), bins, dmax, flags, weighted, A, smem);
@@ -1140,6 +1302,23 @@ extern "C" pcf_status pcf_count_triplets(pcf_ctx *ctx, int kind, const pcf_grid 
     int64_t bx = 0, by = 0;
     s = list_bound(ctx, gx, X->n, dmax, A.rows, A.n_rows, bpc, &bx);
     if (s == PCF_OK && mixed) s = list_bound(ctx, gy, Y->n, dmax, A.rows, A.n_rows, bpc, &by);
+    TripArgs F;  // the gates' corrections
+    size_t fix_smem = 0;
+    if (s == PCF_OK && gates) {
+        ordered_caps(mixed, false, true, F);
+        int64_t fx = bx, fy = by;
+        // an entry also has its place in the order by image (two bytes; the row
+        // table's share of `room` comes off here)
+        const int capJ = F.capJ - 300, capK = mixed ? F.capK : 0;
+        if (fx > capJ) s = list_bound(ctx, gx, X->n, dmax, A.rows, A.n_rows, bpc, &fx, capJ);
+        if (s == PCF_OK && mixed && fy > capK) s = list_bound(ctx, gy, Y->n, dmax, A.rows, A.n_rows, bpc, &fy, capK);
+        if (s == PCF_OK && (fx > capJ || (mixed && fy > capK))) return ordered();
+        F = A;
+        F.capJ = capJ;
+        F.capK = capK;
+        F.gate = geom;
+        fix_smem = (size_t)(capJ + capK) * 20 + 2 * (size_t)(mixed ? capK : capJ);
+    }
     const int grid = ctx->sm_count;
     if (s == PCF_OK) s = trip_overflow(ctx, std::max(bx, by) + 32, mixed, weighted, grid, A);
     if (s != PCF_OK) return s;
@@ -1151,6 +1330,8 @@ extern "C" pcf_status pcf_count_triplets(pcf_ctx *ctx, int kind, const pcf_grid 
     A.g_stats = reinterpret_cast<unsigned long long *>(hp + (size_t)n3 * 16);
     double *d_out = reinterpret_cast<double *>(hp + (size_t)n3 * 16 + 64);
     PCF_CU(ctx, cudaMemsetAsync(hp, 0, (size_t)n3 * 16 + 64, ctx->stream));
+    // unweighted: the sums' place holds the gates' corrections
+    unsigned long long *fix = gates ? reinterpret_cast<unsigned long long *>(A.g_wsum) : nullptr;
 
     auto kfn = mixed ? (weighted ? k_triplets<true, true> : k_triplets<true, false>)
                      : (weighted ? k_triplets<false, true> : k_triplets<false, false>);
@@ -1164,6 +1345,17 @@ extern "C" pcf_status pcf_count_triplets(pcf_ctx *ctx, int kind, const pcf_grid 
     PCF_CU(ctx, cudaEventRecord(ctx->ev0, ctx->stream));
     kfn<<<grid, kTThreads, smem, ctx->stream>>>(A);
     PCF_CU(ctx, cudaGetLastError());
+    if (gates) {
+        F.g_count = fix;
+        F.g_stats = A.g_stats;
+        F.counter = A.counter + 1;
+        auto ffn = mixed ? k_gate_fix<true> : k_gate_fix<false>;
+        PCF_CU(ctx, ensure_smem_limit(reinterpret_cast<const void *>(ffn), ctx->device, fix_smem));
+        const float reach = (float)(std::sqrt(A.rXX.dd) * (1.0 + 1e-6) + (double)A.box * 1e-6);
+        ffn<<<grid, kTThreads, fix_smem, ctx->stream>>>(F, reach);
+        PCF_CU(ctx, cudaGetLastError());
+        ++ctx->launches;
+    }
     PCF_CU(ctx, cudaEventRecord(ctx->ev1, ctx->stream));
     if (pe1) PCF_CU(ctx, cudaEventRecord(pe1, ctx->stream));
     PCF_CU(ctx, cudaEventRecord(sl->done, ctx->stream));
@@ -1174,17 +1366,19 @@ extern "C" pcf_status pcf_count_triplets(pcf_ctx *ctx, int kind, const pcf_grid 
     if (s != PCF_OK) return s;
     k_trip_finalize<<<(n3 + 255) / 256, 256, 0, ctx->stream>>>(A.g_count, A.g_wsum, weighted ? 1 : 0,
                                                                 mixed ? 1 : 0, bins, o.to, A.g_stats,
-                                                                stats || !dev_out ? o.stats : nullptr);
+                                                                stats || !dev_out || gates ? o.stats : nullptr, fix);
     PCF_CU(ctx, cudaGetLastError());
     ++ctx->launches;
-    if (stats || !dev_out) {
+    if (stats || !dev_out || gates) {
         unsigned long long hs[4];
         s = out_close(ctx, o, n3, dev_out, hist, hs);
         if (s != PCF_OK) return s;
+        if (gates && hs[3]) return PCF_ERR_UNSUPPORTED;
         if (stats) {
             float ms = 0.f;
             cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
             stats->pairs = (double)hs[2];  // unordered triangles (XXY: per unordered XX pair)
+            if (gates) stats->pairs = (double)(hs[2] * (mixed ? 2 : 6) + hs[1]);  // counts of ordered ones
             stats->candidates = 0;
             stats->rechecks = (double)hs[0];
             stats->kernel_ms = ms;
@@ -1363,7 +1557,7 @@ extern "C" pcf_status pcf_batch_triplets(pcf_ctx *ctx, const pcf_grid *d_, const
     for (int k = 0; k < nj; ++k) {
         k_trip_finalize<<<(n3 + 255) / 256, 256, 0, ctx->stream>>>(
             cnt + (size_t)k * n3, wsum + (size_t)k * n3, weighted ? 1 : 0, jobs[k].y ? 1 : 0, bins,
-            d_out + (size_t)k * n3, nullptr, nullptr);
+            d_out + (size_t)k * n3, nullptr, nullptr, nullptr);
         PCF_CU(ctx, cudaGetLastError());
         ++ctx->launches;
     }
@@ -1450,15 +1644,7 @@ static pcf_status count_triplets_ordered(pcf_ctx *ctx, const pcf_grid *x_, const
     if (gates) A.gate = gate_geometry(X->box, dmax, X->user_P);
     A.fc = trip_cuts(rXX, X->box, dmax, bpc);
     const bool weighted = !(X->unit_weights && (!mixed || Y->unit_weights));
-    const size_t ent = 16 + 2 + (weighted ? 4 : 0) + (gates ? 4 : 0);
-    const size_t room = 227 * 1024 - 256 - (gates ? 64 * sizeof(GateBlock) + 128 + 64 : 0);
-    if (mixed) {
-        A.capJ = (int)(room / ent / 3);
-        A.capK = (int)(room / ent) - A.capJ - 8;
-    } else {
-        A.capJ = (int)(room / ent) - 8;
-        A.capK = 0;
-    }
+    const size_t ent = ordered_caps(mixed, weighted, gates, A);
     // (an entry's angle bin takes one of the two bytes `ent` counts: the row
     // table has the rest)
     const size_t smem = (size_t)(A.capJ + A.capK) * (ent - 1) + 64;
