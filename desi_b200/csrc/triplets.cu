@@ -78,6 +78,7 @@ struct TripArgs {
     unsigned long long *g_count;  // bins^3 (unit weights)
     double *g_wsum;               // bins^3 (weighted)
     int hist_in_smem;
+    int list_bytes;          // shared memory of a group's lists
     unsigned long long *g_stats;
     // adds the shared u32 histogram absorbs between flushes into g_count
     // (a counter then never wraps: one slot gets at most that many adds)
@@ -174,19 +175,32 @@ __device__ __noinline__ int exact_angle(float ax, float ay, float az, float bx, 
 // The candidate ranges of an anchor's stencil rows, two per row (a periodic
 // row may wrap in z): first point with the image shifts (2 bits per axis
 // above bit 24: 0 -L, 1 none, 2 +L) and the number of candidates before it.
-constexpr int kSegs = kTThreads;
+//
+// The list builds and the counting of an anchor run in a group of NW warps, of
+// which a CTA holds one or more, each with anchors of its own: lane, warp and
+// thread numbers below are the group's, gsync its barrier.
+constexpr int kGroupWarps = 8;  // of a group, where a CTA or an SM holds several
+template <int NW>
 struct SegTable {
-    int first[kSegs], before[kSegs];
-    int wsum[kTWarps];
+    int first[NW * 32], before[NW * 32];
+    int wsum[NW];
 };
+template <int NW>
+__device__ __forceinline__ int group_tid() { return (int)(threadIdx.x % (NW * 32)); }
+template <int NW>
+__device__ __forceinline__ void gsync() {
+    if (NW == kTWarps) __syncthreads();
+    else asm volatile("bar.sync %0, %1;" ::"r"(1 + threadIdx.x / (NW * 32)), "n"(NW * 32) : "memory");
+}
 
-// Ranges of rows [rb, rb + kSegs / 2), one per thread, in catalog C around the
+// Ranges of rows [rb, rb + NW * 16), one per thread, in catalog C around the
 // anchor's cell; only_after >= 0 keeps the points after that index.  Returns
-// the number of candidates.  Called by the whole CTA; ends synchronised, and
+// the number of candidates.  Called by the whole group; ends synchronised, and
 // needs no barrier before it (the table is written after its first barrier).
+template <int NW>
 __device__ __forceinline__ int seg_table(const TripArgs &A, const Cat &C, int cix, int ciy, int ciz,
-                                         int only_after, int rb, SegTable &T) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+                                         int only_after, int rb, SegTable<NW> &T) {
+    const int tid = group_tid<NW>(), lane = tid & 31, warp = tid >> 5;
     const int r = rb + (tid >> 1), P = A.P;
     int a = 0, len = 0;
     if (r < A.n_rows) {
@@ -226,25 +240,26 @@ __device__ __forceinline__ int seg_table(const TripArgs &A, const Cat &C, int ci
         if (lane >= o) x += y;
     }
     if (lane == 31) T.wsum[warp] = x;
-    __syncthreads();
-    const int ws = lane < kTWarps ? T.wsum[lane] : 0;
+    gsync<NW>();
+    const int ws = lane < NW ? T.wsum[lane] : 0;
     int w = ws;
     #pragma unroll
-    for (int o = 1; o < kTWarps; o <<= 1) {
+    for (int o = 1; o < NW; o <<= 1) {
         const int y = __shfl_up_sync(kFull, w, o);
         if (lane >= o) w += y;
     }
-    const int total = __shfl_sync(kFull, w, kTWarps - 1);
+    const int total = __shfl_sync(kFull, w, NW - 1);
     T.first[tid] = a;
     T.before[tid] = x - len + __shfl_sync(kFull, w - ws, warp);
-    __syncthreads();
+    gsync<NW>();
     return total;
 }
 
-// Per-CTA scratch of the list builds.
+// Scratch of a group's list builds.
+template <int NW>
 struct ListScratch {
-    SegTable seg;
-    int kept[2][kTWarps];  // entries of each warp's chunk, alternating rounds
+    SegTable<NW> seg;
+    int kept[2][NW];  // entries of each warp's chunk, alternating rounds
 };
 
 // Lists the neighbours of anchor (hx,hy,hz) found in catalog C, in the order of
@@ -255,21 +270,21 @@ struct ListScratch {
 // (gate_pack).  WRAPPED: only the neighbours through an image.  Called by the
 // whole CTA; ends synchronised.
 //
-// All rows' candidates form one index space that the CTA takes 768 at a time
+// All rows' candidates form one index space that the group takes NW * 32 at a time
 // (the range of an index by binary search): a row holds 10 to 100 candidates,
 // so a loop over rows kept 1 to 3 warps busy and cost a dependent
 // cell-table load per row.  The order is kept (a barrier per round) so that
 // runs of entries stay close in space, for the culling of tri_tiles.
-template <bool ANG, bool WRAPPED = false>
+template <int NW, bool ANG, bool WRAPPED = false>
 __device__ int build_list(const TripArgs &A, const Cat &C, float hx, float hy, float hz, int cix, int ciy,
                           int ciz, int only_after, const PairRule &rule, float4 *list, float *wlist, int cap,
-                          unsigned &n_rechk, ListScratch &S, unsigned char *ang = nullptr,
+                          unsigned &n_rechk, ListScratch<NW> &S, unsigned char *ang = nullptr,
                           unsigned *ginfo = nullptr) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = group_tid<NW>(), lane = tid & 31, warp = tid >> 5;
     int n = 0, par = 0;
-    for (int rb = 0; rb < A.n_rows; rb += kSegs / 2) {
-        const int total = seg_table(A, C, cix, ciy, ciz, only_after, rb, S.seg);
-        const int nseg = 2 * min(kSegs / 2, A.n_rows - rb);
+    for (int rb = 0; rb < A.n_rows; rb += NW * 16) {
+        const int total = seg_table<NW>(A, C, cix, ciy, ciz, only_after, rb, S.seg);
+        const int nseg = 2 * min(NW * 16, A.n_rows - rb);
         const int top = 1 << (31 - __clz(nseg));
         // candidate of index q: its point, or -1 past the end; image axes in sh
         auto locate = [&](int q, int &sh) -> int {
@@ -284,10 +299,10 @@ __device__ int build_list(const TripArgs &A, const Cat &C, float hx, float hy, f
         int sh = 0, c = locate(tid, sh);
         float px = 0.f, py = 0.f, pz = 0.f;
         if (c >= 0) { px = C.x[c]; py = C.y[c]; pz = C.z[c]; }
-        for (int base = 0; base < total; base += kTThreads) {
+        for (int base = 0; base < total; base += NW * 32) {
             // the next round's points are on their way while this one is tested
             int shn = 0;
-            const int cn = locate(base + kTThreads + tid, shn);
+            const int cn = locate(base + NW * 32 + tid, shn);
             float nx = 0.f, ny = 0.f, nz = 0.f;
             if (cn >= 0) { nx = C.x[cn]; ny = C.y[cn]; nz = C.z[cn]; }
             int bin = -2, tang = 0;
@@ -311,16 +326,16 @@ __device__ int build_list(const TripArgs &A, const Cat &C, float hx, float hy, f
             const bool keep = bin >= 0;
             const unsigned m = __ballot_sync(kFull, keep);
             if (lane == 0) S.kept[par][warp] = __popc(m);
-            __syncthreads();
-            const int wk = lane < kTWarps ? S.kept[par][lane] : 0;
+            gsync<NW>();
+            const int wk = lane < NW ? S.kept[par][lane] : 0;
             int x = wk;
             #pragma unroll
-            for (int o = 1; o < kTWarps; o <<= 1) {
+            for (int o = 1; o < NW; o <<= 1) {
                 const int y = __shfl_up_sync(kFull, x, o);
                 if (lane >= o) x += y;
             }
             const int pos = n + __shfl_sync(kFull, x - wk, warp) + __popc(m & ((1u << lane) - 1u));
-            n += __shfl_sync(kFull, x, kTWarps - 1);
+            n += __shfl_sync(kFull, x, NW - 1);
             par ^= 1;
             if (keep && pos < cap) {
                 list[pos] = make_float4(vx * A.fc.dsf, vy * A.fc.dsf, vz * A.fc.dsf,
@@ -339,7 +354,7 @@ __device__ int build_list(const TripArgs &A, const Cat &C, float hx, float hy, f
             pz = nz;
         }
     }
-    __syncthreads();
+    gsync<NW>();
     return n;
 }
 
@@ -349,23 +364,28 @@ __device__ int build_list(const TripArgs &A, const Cat &C, float hx, float hy, f
 __host__ __device__ __forceinline__ int u_words(int bins) { return bins * bins * (bins + 1); }
 
 // Adds U into the u64 histogram g (bins^3, [b_ij][b_ki][b_jk]) and clears it
-// (whole CTA); returns the triangles this thread added.
+// (whole group); returns the triangles this thread added.  SHARED: other groups
+// may be counting into U meanwhile, so a counter is taken by an exchange, and one
+// that settle lowers after its count was taken reads as -1.
+template <int NW, bool SHARED>
 __device__ __forceinline__ unsigned long long flush_hist(unsigned *U, int bins, unsigned long long *g) {
-    __syncthreads();
+    gsync<NW>();
     unsigned long long n = 0;
     const int nu = u_words(bins);
-    for (int k = threadIdx.x; k < nu; k += kTThreads) {
-        const unsigned v = U[k];
+    for (int k = group_tid<NW>(); k < nu; k += NW * 32) {
+        unsigned v = U[k];
         if (v) {
             const int row = k / (bins + 1), c = k - row * (bins + 1);
-            U[k] = 0u;
+            if (SHARED) v = atomicExch(&U[k], 0u);
+            else U[k] = 0u;
             if (c < bins) {
-                atomicAdd(g + row * bins + c, (unsigned long long)v);
-                n += v;
+                const unsigned long long d = SHARED ? (unsigned long long)(long long)(int)v : v;
+                atomicAdd(g + row * bins + c, d);
+                n += d;
             }
         }
     }
-    __syncthreads();
+    gsync<NW>();
     return n;
 }
 
@@ -374,14 +394,16 @@ struct ChunkBox {
     float lo[3], hi[3];
 };
 
-// Per-CTA state of the anchor loop.
+// State of a group's anchor loop.
+template <int NW>
 struct TripCta {
     unsigned *U;                      // shared histogram (hist_in_smem)
     unsigned char *lists;             // shared neighbour lists
-    ListScratch *scr;
-    ChunkBox *boxes;                  // kMaxBoxes chunks of the K list
+    ListScratch<NW> *scr;
+    ChunkBox *boxes;                  // max_boxes<NW>() chunks of the K list
     uint2 *queue;                     // 64 tests per warp on their way to the FP64 rule
     int *s_unit;                      // shared counter
+    int slot;                         // of the overflow lists
     unsigned n_rechk;
     unsigned long long n_tri;
     unsigned long long since;         // pair tests since U's last flush
@@ -392,23 +414,26 @@ struct TripCta {
 constexpr float kFarAway = 1e15f;
 constexpr int kTile = 8;        // j per tile
 constexpr int kChunkK = 32;     // K lists are padded to whole chunks of one k per lane
-constexpr int kMaxBoxes = 256;  // chunks of a K list that take part in the culling
+constexpr int kMaxBoxes = 256;  // chunks of K lists that take part in the culling, over the groups
+template <int NW>
+__host__ __device__ constexpr int max_boxes() { return kMaxBoxes * NW / kTWarps; }
 // Fixed-point readout of a third side: bits(128 + r) >> 16 = kSideBias + bin
 constexpr float kSideMagic = 128.0f;
 constexpr int kSideBits = 16;
 constexpr unsigned kSideBias = 0x43000000u >> kSideBits;
 
-// Pads the K list to whole chunks and finds the chunks' extents.  Whole CTA;
+// Pads the K list to whole chunks and finds the chunks' extents.  Whole group;
 // ends synchronised.
-__device__ __forceinline__ void finish_k(TripCta &C, float4 *L, int nK) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+template <int NW>
+__device__ __forceinline__ void finish_k(TripCta<NW> &C, float4 *L, int nK) {
+    const int lane = threadIdx.x & 31, warp = group_tid<NW>() >> 5;
     const int nchunk = (nK + kChunkK - 1) / kChunkK;
-    for (int c = warp; c < nchunk; c += kTWarps) {
+    for (int c = warp; c < nchunk; c += NW) {
         const int k = c * kChunkK + lane;
         float4 e = make_float4(kFarAway, kFarAway, kFarAway, 0.f);
         if (k < nK) e = L[k];
         else L[k] = e;
-        if (c < kMaxBoxes) {
+        if (c < max_boxes<NW>()) {
             const float v[3] = {e.x, e.y, e.z};
             #pragma unroll
             for (int a = 0; a < 3; ++a) {
@@ -425,7 +450,7 @@ __device__ __forceinline__ void finish_k(TripCta &C, float4 *L, int nK) {
             }
         }
     }
-    __syncthreads();
+    gsync<NW>();
 }
 
 // The canonical rule for up to 32 tests that fell into a window, one per lane
@@ -468,11 +493,11 @@ __device__ __noinline__ void settle(const TripArgs &A, unsigned *U, const float4
 // differences are monotone, so no test inside could have been in range).
 // FAR: dmax lies more than the window below the last bin's edge (bins / dmax
 // rounded down to 1e-6, large dmax), so it needs a window of its own.
-template <bool MIXED, bool FAR>
-__device__ __forceinline__ void tri_tiles(const TripArgs &A, TripCta &C, const float4 *__restrict__ LJ,
+template <int NW, bool MIXED, bool FAR>
+__device__ __forceinline__ void tri_tiles(const TripArgs &A, TripCta<NW> &C, const float4 *__restrict__ LJ,
                                           const float4 *__restrict__ LK, int nJ, int nK, float hx, float hy,
                                           float hz) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, warp = group_tid<NW>() >> 5;
     const int bins = A.rXX.bins;
     const float mgw = kSideMagic + (float)A.fc.wt * 0x1p-16f, qout = kSideMagic + (float)bins + 0.5f;
     const float qlo = A.fc.qlo, qhi = A.fc.qhi, qedge = kSideMagic + (float)bins;
@@ -486,7 +511,7 @@ __device__ __forceinline__ void tri_tiles(const TripArgs &A, TripCta &C, const f
     // are few tiles per warp
     int segs = 1;
     if (MIXED)
-        while (segs < nchunk && ntile * segs < 8 * kTWarps) segs <<= 1;
+        while (segs < nchunk && ntile * segs < 8 * NW) segs <<= 1;
     const int units = ntile * segs;
     for (;;) {
         int u0 = 0;
@@ -559,7 +584,7 @@ __device__ __forceinline__ void tri_tiles(const TripArgs &A, TripCta &C, const f
         if (!MIXED) step(c++ * kChunkK + lane, true);
         for (; c < c1; c += 32) {
             bool in = c + lane < c1;
-            if (in && c + lane < kMaxBoxes) {
+            if (in && c + lane < max_boxes<NW>()) {
                 const ChunkBox &b = C.boxes[c + lane];
                 float g[3];
                 #pragma unroll
@@ -576,21 +601,21 @@ __device__ __forceinline__ void tri_tiles(const TripArgs &A, TripCta &C, const f
 }
 
 // All triangles of anchor i of job A: pass 1 builds the anchor's
-// neighbour lists in shared memory (or, past their capacity, in this CTA's
+// neighbour lists in shared memory (or, past their capacity, in the group's
 // global scratch), pass 2 counts the neighbour pairs.
-template <bool MIXED, bool WEIGHTED>
-__device__ __forceinline__ void tri_anchor(const TripArgs &A, int i, TripCta &C) {
+template <int NW, bool MIXED, bool WEIGHTED>
+__device__ __forceinline__ void tri_anchor(const TripArgs &A, int i, TripCta<NW> &C) {
     const int bins = A.rXX.bins;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = group_tid<NW>(), lane = tid & 31, warp = tid >> 5;
     unsigned &n_rechk = C.n_rechk;
     float4 *sJ = reinterpret_cast<float4 *>(C.lists);
     float4 *sK = sJ + A.capJ;
     float *swJ = reinterpret_cast<float *>(sK + (MIXED ? A.capK : 0));
     float *swK = swJ + (WEIGHTED ? A.capJ : 0);
-    float4 *gJ = A.gJ + (size_t)blockIdx.x * A.gcap;
-    float4 *gK = A.gK ? A.gK + (size_t)blockIdx.x * A.gcap : nullptr;
-    float *gwJ = A.gwJ ? A.gwJ + (size_t)blockIdx.x * A.gcap : nullptr;
-    float *gwK = A.gwK ? A.gwK + (size_t)blockIdx.x * A.gcap : nullptr;
+    float4 *gJ = A.gJ + (size_t)C.slot * A.gcap;
+    float4 *gK = A.gK ? A.gK + (size_t)C.slot * A.gcap : nullptr;
+    float *gwJ = A.gwJ ? A.gwJ + (size_t)C.slot * A.gcap : nullptr;
+    float *gwK = A.gwK ? A.gwK + (size_t)C.slot * A.gcap : nullptr;
     const float hx = A.X.x[i], hy = A.X.y[i], hz = A.X.z[i];
     const float hw = WEIGHTED ? A.X.w[i] : 1.f;
     const int P = A.P;
@@ -602,7 +627,7 @@ __device__ __forceinline__ void tri_anchor(const TripArgs &A, int i, TripCta &C)
     // and behind it K, each list that is walked in chunks padded to them.
     const bool pool = !WEIGHTED && A.hist_in_smem;
     auto padded = [](int n) { return (n + kChunkK - 1) / kChunkK * kChunkK; };
-    int nJ = build_list<false>(A, A.X, hx, hy, hz, cix, ciy, ciz, i, A.rXX, sJ, WEIGHTED ? swJ : nullptr, A.capJ,
+    int nJ = build_list<NW, false>(A, A.X, hx, hy, hz, cix, ciy, ciz, i, A.rXX, sJ, WEIGHTED ? swJ : nullptr, A.capJ,
                                n_rechk, *C.scr);
     int capK = A.capK, nK = nJ;
     if (MIXED) {
@@ -610,7 +635,7 @@ __device__ __forceinline__ void tri_anchor(const TripArgs &A, int i, TripCta &C)
             sK = sJ + min(nJ, A.capJ);
             capK = max(0, A.capJ - nJ);
         }
-        nK = build_list<false>(A, A.Y, hx, hy, hz, cix, ciy, ciz, -1, A.rXY, sK, WEIGHTED ? swK : nullptr, capK,
+        nK = build_list<NW, false>(A, A.Y, hx, hy, hz, cix, ciy, ciz, -1, A.rXY, sK, WEIGHTED ? swK : nullptr, capK,
                                n_rechk, *C.scr);
     }
     const float4 *LJ = sJ;
@@ -618,12 +643,12 @@ __device__ __forceinline__ void tri_anchor(const TripArgs &A, int i, TripCta &C)
     const float *WJ = swJ, *WK = MIXED ? swK : swJ;
     const bool spill = nJ > A.capJ || (MIXED && nK > capK) || (pool && padded(nK) > (MIXED ? capK : A.capJ));
     if (spill) {
-        // overflow: the lists in this CTA's global scratch (L2), which holds any anchor's
-        nJ = min(A.gcap, build_list<false>(A, A.X, hx, hy, hz, cix, ciy, ciz, i, A.rXX, gJ,
+        // overflow: the lists in the group's global scratch (L2), which holds any anchor's
+        nJ = min(A.gcap, build_list<NW, false>(A, A.X, hx, hy, hz, cix, ciy, ciz, i, A.rXX, gJ,
                                            WEIGHTED ? gwJ : nullptr, A.gcap, n_rechk, *C.scr));
         nK = nJ;
         if (MIXED)
-            nK = min(A.gcap, build_list<false>(A, A.Y, hx, hy, hz, cix, ciy, ciz, -1, A.rXY, gK,
+            nK = min(A.gcap, build_list<NW, false>(A, A.Y, hx, hy, hz, cix, ciy, ciz, -1, A.rXY, gK,
                                                WEIGHTED ? gwK : nullptr, A.gcap, n_rechk, *C.scr));
         LJ = gJ;
         LK = MIXED ? gK : gJ;
@@ -642,7 +667,7 @@ __device__ __forceinline__ void tri_anchor(const TripArgs &A, int i, TripCta &C)
             smem_hist = false;
         } else {
             if (C.since + tests > A.flush_budget) {
-                C.n_tri += flush_hist(C.U, bins, A.g_count);
+                C.n_tri += flush_hist<NW, NW != kTWarps>(C.U, bins, A.g_count);
                 C.since = 0;
             }
             C.since += tests;
@@ -654,17 +679,17 @@ __device__ __forceinline__ void tri_anchor(const TripArgs &A, int i, TripCta &C)
         // shared-memory case (all but overflowing anchors) uses shared loads
         if (spill) {
             finish_k(C, MIXED ? gK : gJ, nK);
-            if (A.fc.far) tri_tiles<MIXED, true>(A, C, gJ, MIXED ? gK : gJ, nJ, nK, hx, hy, hz);
-            else tri_tiles<MIXED, false>(A, C, gJ, MIXED ? gK : gJ, nJ, nK, hx, hy, hz);
+            if (A.fc.far) tri_tiles<NW, MIXED, true>(A, C, gJ, MIXED ? gK : gJ, nJ, nK, hx, hy, hz);
+            else tri_tiles<NW, MIXED, false>(A, C, gJ, MIXED ? gK : gJ, nJ, nK, hx, hy, hz);
         } else {
             finish_k(C, MIXED ? sK : sJ, nK);
-            if (A.fc.far) tri_tiles<MIXED, true>(A, C, sJ, MIXED ? sK : sJ, nJ, nK, hx, hy, hz);
-            else tri_tiles<MIXED, false>(A, C, sJ, MIXED ? sK : sJ, nJ, nK, hx, hy, hz);
+            if (A.fc.far) tri_tiles<NW, MIXED, true>(A, C, sJ, MIXED ? sK : sJ, nJ, nK, hx, hy, hz);
+            else tri_tiles<NW, MIXED, false>(A, C, sJ, MIXED ? sK : sJ, nJ, nK, hx, hy, hz);
         }
         return;
     }
     // rows j dealt to warps in the order 0, n-1, 1, n-2, ... (XXX rows shrink with j)
-    for (int rr = warp; rr < nJ; rr += kTWarps) {
+    for (int rr = warp; rr < nJ; rr += NW) {
         const int half = rr >> 1;
         const int jj = MIXED ? rr : ((rr & 1) ? nJ - 1 - half : half);
         const float4 ej = LJ[jj];
@@ -697,40 +722,47 @@ __device__ __forceinline__ void tri_anchor(const TripArgs &A, int i, TripCta &C)
     }
 }
 
-template <bool MIXED, bool WEIGHTED>
+template <bool MIXED, bool WEIGHTED, int NW>
 __global__ void __launch_bounds__(kTThreads, 1) k_triplets(const __grid_constant__ TripArgs A) {
+    constexpr int G = kTWarps / NW;
     extern __shared__ __align__(16) unsigned char smem[];
     const int bins = A.rXX.bins;
     const size_t u_bytes = A.hist_in_smem ? (((size_t)u_words(bins) * 4 + 15) & ~(size_t)15) : 0;
-    __shared__ ListScratch s_scr;
+    __shared__ ListScratch<NW> s_scr[G];
     __shared__ ChunkBox s_boxes[kMaxBoxes];
     __shared__ uint2 s_queue[64 * kTWarps];
-    __shared__ int s_anchor, s_unit;
-    __shared__ unsigned s_stop;
-    const int tid = threadIdx.x, lane = tid & 31;
-    TripCta C{reinterpret_cast<unsigned *>(smem), smem + u_bytes, &s_scr, s_boxes, s_queue, &s_unit, 0u, 0ull, 0ull};
+    __shared__ int s_anchor[G], s_unit[G];
+    __shared__ unsigned s_stop[G];
+    const int tid = group_tid<NW>(), lane = tid & 31, g = (int)threadIdx.x / (NW * 32);
+    TripCta<NW> C{reinterpret_cast<unsigned *>(smem), smem + u_bytes + (size_t)g * A.list_bytes, &s_scr[g],
+                  s_boxes + g * max_boxes<NW>(), s_queue + g * NW * 64, &s_unit[g], (int)blockIdx.x * G + g, 0u,
+                  0ull, 0ull};
     if (A.hist_in_smem)
-        for (int k = tid; k < u_words(bins); k += kTThreads) C.U[k] = 0u;
-    long long taken = 0;  // anchors this CTA took (iteration cap: nX + 1)
+        for (int k = threadIdx.x; k < u_words(bins); k += kTThreads) C.U[k] = 0u;
+    if (G > 1) __syncthreads();
+    long long taken = 0;  // anchors this group took (iteration cap: nX + 1)
     int ticket = 0;       // thread 0: the next anchor, taken while the last one is counted
     if (tid == 0) ticket = (int)atomicAdd(A.counter, 1ull);
     for (;;) {
         if (tid == 0) {
-            s_anchor = ticket;
-            s_unit = 0;
+            s_anchor[g] = ticket;
+            s_unit[g] = 0;
             unsigned stop = (A.ctrl && ctrl_load(A.ctrl)) ? PCF_GAVE_UP_ABORT : 0u;
             if (++taken > (long long)A.nX + 1) stop |= PCF_GAVE_UP_CAP;
             if (stop && A.status) ctrl_store(A.status, stop);
-            s_stop = stop;
+            s_stop[g] = stop;
         }
-        __syncthreads();
-        const int i = s_anchor;
-        if (i >= A.nX || s_stop) break;
+        gsync<NW>();
+        const int i = s_anchor[g];
+        if (i >= A.nX || s_stop[g]) break;
         if (tid == 0) ticket = (int)atomicAdd(A.counter, 1ull);
-        tri_anchor<MIXED, WEIGHTED>(A, i, C);
-        __syncthreads();
+        tri_anchor<NW, MIXED, WEIGHTED>(A, i, C);
+        gsync<NW>();
     }
-    if (A.hist_in_smem) C.n_tri += flush_hist(C.U, bins, A.g_count);
+    if (A.hist_in_smem) {
+        if (G > 1) __syncthreads();  // every group's counts are in
+        C.n_tri += flush_hist<kTWarps, (G > 1)>(C.U, bins, A.g_count);
+    }
     unsigned long long rr = C.n_rechk, nt = C.n_tri;
     for (int off = 16; off > 0; off >>= 1) {
         rr += __shfl_down_sync(kFull, rr, off);
@@ -761,7 +793,7 @@ struct TripBatch {
 template <bool MIXED, bool WEIGHTED>
 __global__ void __launch_bounds__(kTThreads, 1) k_triplets_batch(const __grid_constant__ TripBatch B) {
     extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ ListScratch s_scr;
+    __shared__ ListScratch<kTWarps> s_scr;
     __shared__ ChunkBox s_boxes[kMaxBoxes];
     __shared__ uint2 s_queue[64 * kTWarps];
     __shared__ long long s_anchor;
@@ -772,7 +804,7 @@ __global__ void __launch_bounds__(kTThreads, 1) k_triplets_batch(const __grid_co
     const int bins = J0.rXX.bins;
     const bool in_smem = J0.hist_in_smem != 0;
     const size_t u_bytes = in_smem ? (((size_t)u_words(bins) * 4 + 15) & ~(size_t)15) : 0;
-    TripCta C{reinterpret_cast<unsigned *>(smem), smem + u_bytes, &s_scr, s_boxes, s_queue, &s_unit, 0u, 0ull, 0ull};
+    TripCta<kTWarps> C{reinterpret_cast<unsigned *>(smem), smem + u_bytes, &s_scr, s_boxes, s_queue, &s_unit, (int)blockIdx.x, 0u, 0ull, 0ull};
     if (in_smem)
         for (int k = tid; k < u_words(bins); k += kTThreads) C.U[k] = 0u;
     int cur = -1;  // the CTA's current job (uniform: every thread follows s_anchor)
@@ -796,16 +828,16 @@ __global__ void __launch_bounds__(kTThreads, 1) k_triplets_batch(const __grid_co
             int j = cur < 0 ? 0 : cur;
             while (j + 1 < B.n_jobs && g >= B.job[j + 1].anchor_begin) ++j;
             if (cur >= 0 && in_smem && C.since) {
-                C.n_tri += flush_hist(C.U, bins, B.job[cur].g_count);
+                C.n_tri += flush_hist<kTWarps, false>(C.U, bins, B.job[cur].g_count);
                 C.since = 0;
             }
             cur = j;
         }
         const TripArgs &A = B.job[cur];
-        tri_anchor<MIXED, WEIGHTED>(A, (int)(g - A.anchor_begin), C);
+        tri_anchor<kTWarps, MIXED, WEIGHTED>(A, (int)(g - A.anchor_begin), C);
         __syncthreads();
     }
-    if (in_smem && cur >= 0) C.n_tri += flush_hist(C.U, bins, B.job[cur].g_count);
+    if (in_smem && cur >= 0) C.n_tri += flush_hist<kTWarps, false>(C.U, bins, B.job[cur].g_count);
     unsigned long long rr = C.n_rechk, nt = C.n_tri;
     for (int off = 16; off > 0; off >>= 1) {
         rr += __shfl_down_sync(kFull, rr, off);
@@ -827,8 +859,8 @@ __global__ void __launch_bounds__(kTThreads, 1) k_triplets_batch(const __grid_co
 // reference's node grid A.gate.  ISO3 (with GATES): the isotropic bins^3
 // histogram [b(d12)][b(d23)][b(d31)] of the same ordered triangles
 // (3isoBPC_k.cuh:191,940), from lists without angle bins.
-template <bool MIXED, bool WEIGHTED, bool GATES = false, bool ISO3 = false>
-__global__ void __launch_bounds__(kTThreads, 1) k_triplets_ani(const TripArgs A) {
+template <int NW, bool MIXED, bool WEIGHTED, bool GATES = false, bool ISO3 = false>
+__global__ void __launch_bounds__(NW * 32, kTWarps / NW) k_triplets_ani(const TripArgs A) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int bins = A.rXX.bins;
     float4 *sJ = reinterpret_cast<float4 *>(smem);
@@ -840,14 +872,14 @@ __global__ void __launch_bounds__(kTThreads, 1) k_triplets_ani(const TripArgs A)
     unsigned *gK = gJ + (GATES ? A.capJ : 0);
     unsigned char *aJ = reinterpret_cast<unsigned char *>(gK + (GATES && MIXED ? A.capK : 0));
     unsigned char *aK = aJ + A.capJ;
-    __shared__ ListScratch s_scr;
+    __shared__ ListScratch<NW> s_scr;
     __shared__ int s_anchor;
     __shared__ unsigned s_stop;
     __shared__ GateBlock s_gates[GATES ? 64 : 1];
     __shared__ signed char s_gate_by[GATES ? 64 : 1][2];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (GATES) {
-        for (int k = tid; k < 64; k += kTThreads) {
+        for (int k = tid; k < 64; k += NW * 32) {
             s_gates[k] = kGateBlocks[k];
             s_gate_by[k][0] = kGateByImage[k][0];
             s_gate_by[k][1] = kGateByImage[k][1];
@@ -874,10 +906,10 @@ __global__ void __launch_bounds__(kTThreads, 1) k_triplets_ani(const TripArgs A)
         const int cix = min(max((int)__fdiv_rn(hx, A.cell), 0), P - 1);
         const int ciy = min(max((int)__fdiv_rn(hy, A.cell), 0), P - 1);
         const int ciz = min(max((int)__fdiv_rn(hz, A.cell), 0), P - 1);
-        const int nJ = build_list<!ISO3>(A, A.X, hx, hy, hz, cix, ciy, ciz, -1, A.rXX, sJ,
+        const int nJ = build_list<NW, !ISO3>(A, A.X, hx, hy, hz, cix, ciy, ciz, -1, A.rXX, sJ,
                                          WEIGHTED ? swJ : nullptr, A.capJ, n_rechk, s_scr, aJ,
                                          GATES ? gJ : nullptr);
-        const int nK = MIXED ? build_list<!ISO3>(A, A.Y, hx, hy, hz, cix, ciy, ciz, -1, A.rXY, sK,
+        const int nK = MIXED ? build_list<NW, !ISO3>(A, A.Y, hx, hy, hz, cix, ciy, ciz, -1, A.rXY, sK,
                                                  WEIGHTED ? swK : nullptr, A.capK, n_rechk, s_scr, aK,
                                                  GATES ? gK : nullptr)
                              : nJ;
@@ -892,7 +924,7 @@ __global__ void __launch_bounds__(kTThreads, 1) k_triplets_ani(const TripArgs A)
         const float4 *LK = MIXED ? sK : sJ;
         const unsigned char *AK = MIXED ? aK : aJ;
         const float *WK = MIXED ? swK : swJ;
-        for (int jj = warp; jj < nJ; jj += kTWarps) {
+        for (int jj = warp; jj < nJ; jj += NW) {
             const float4 ej = sJ[jj];
             const int jidx = (int)((unsigned)__float_as_int(ej.w) >> 8);
             const int bj = __float_as_int(ej.w) & 255;
@@ -956,15 +988,15 @@ __global__ void __launch_bounds__(kTThreads, 1) k_triplets_ani(const TripArgs A)
 // Evaluating every ordered triangle's gates, with a global atomic each, took 50.7 ms
 // for 4096 and 4100 points (DDD, RRR, DDR, DRR; bins 30, dmax 80 of 250).
 // Histogram: A.g_count, bins^3 signed, [b(d12)][b(d23)][b(d31)]; g_stats[1]: their sum.
-template <bool MIXED>
-__global__ void __launch_bounds__(kTThreads, 1) k_gate_fix(const __grid_constant__ TripArgs A, float reach) {
+template <int NW, bool MIXED>
+__global__ void __launch_bounds__(NW * 32, kTWarps / NW) k_gate_fix(const __grid_constant__ TripArgs A, float reach) {
     extern __shared__ __align__(16) unsigned char smem[];
     float4 *sJ = reinterpret_cast<float4 *>(smem), *sK = sJ + A.capJ;
     unsigned *gJ = reinterpret_cast<unsigned *>(sK + A.capK), *gK = gJ + A.capJ;
     // the third points by image: indices in `by`, those of images f at s_class[f] ..
     unsigned short *by = reinterpret_cast<unsigned short *>(gK + A.capK);
     __shared__ int s_class[9], s_fill[8];
-    __shared__ ListScratch s_scr;
+    __shared__ ListScratch<NW> s_scr;
     __shared__ int s_anchor;
     __shared__ unsigned s_stop;
     __shared__ GateBlock s_gates[64];
@@ -1000,9 +1032,9 @@ __global__ void __launch_bounds__(kTThreads, 1) k_gate_fix(const __grid_constant
             const int cix = min(max((int)__fdiv_rn(hx, A.cell), 0), P - 1);
             const int ciy = min(max((int)__fdiv_rn(hy, A.cell), 0), P - 1);
             const int ciz = min(max((int)__fdiv_rn(hz, A.cell), 0), P - 1);
-            const int nJ = build_list<false, true>(A, A.X, hx, hy, hz, cix, ciy, ciz, -1, A.rXX, sJ, nullptr, A.capJ,
+            const int nJ = build_list<NW, false, true>(A, A.X, hx, hy, hz, cix, ciy, ciz, -1, A.rXX, sJ, nullptr, A.capJ,
                                                    n_rechk, s_scr, nullptr, gJ);
-            const int nK = MIXED ? build_list<false, true>(A, A.Y, hx, hy, hz, cix, ciy, ciz, -1, A.rXY, sK, nullptr,
+            const int nK = MIXED ? build_list<NW, false, true>(A, A.Y, hx, hy, hz, cix, ciy, ciz, -1, A.rXY, sK, nullptr,
                                                            A.capK, n_rechk, s_scr, nullptr, gK)
                                  : nJ;
             const bool fits = nJ <= A.capJ && (!MIXED || nK <= A.capK);
@@ -1012,7 +1044,7 @@ __global__ void __launch_bounds__(kTThreads, 1) k_gate_fix(const __grid_constant
             const unsigned *GK = MIXED ? gK : gJ;
             if (tid < 8) s_fill[tid] = 0;
             __syncthreads();
-            for (int kk = tid; fits && kk < nK; kk += kTThreads) atomicAdd(&s_fill[GK[kk] >> 27 & 7u], 1);
+            for (int kk = tid; fits && kk < nK; kk += NW * 32) atomicAdd(&s_fill[GK[kk] >> 27 & 7u], 1);
             __syncthreads();
             if (tid == 0) {
                 int n = 0;
@@ -1024,10 +1056,10 @@ __global__ void __launch_bounds__(kTThreads, 1) k_gate_fix(const __grid_constant
                 s_class[8] = n;
             }
             __syncthreads();
-            for (int kk = tid; fits && kk < nK; kk += kTThreads)
+            for (int kk = tid; fits && kk < nK; kk += NW * 32)
                 by[atomicAdd(&s_fill[GK[kk] >> 27 & 7u], 1)] = (unsigned short)kk;
             __syncthreads();
-            for (int jj = warp; fits && jj < nJ; jj += kTWarps) {
+            for (int jj = warp; fits && jj < nJ; jj += NW) {
                 unsigned irr = s_irr[(gJ[jj] >> 27) & 7u];
                 if (!irr) continue;
                 const float4 ej = sJ[jj];
@@ -1164,12 +1196,39 @@ static TripCuts trip_cuts(const PairRule &rule, float box, float dmax, bool bpc)
     return c;
 }
 
+// Shared memory of the isotropic kernels' lists and histogram.
+constexpr size_t kTripSmem = 227 * 1024 - 256 - sizeof(ListScratch<kTWarps>) - sizeof(ChunkBox) * kMaxBoxes -
+                             sizeof(uint2) * 64 * kTWarps;
+static size_t trip_hist_bytes(int bins, bool weighted) {
+    const size_t b = ((size_t)u_words(bins) * 4 + 15) & ~(size_t)15;
+    return !weighted && b <= 150 * 1024 ? b : 0;
+}
+
+// Groups of warps per CTA, each with anchors of its own.  Three overlap the
+// latencies of one anchor's list builds (about 6 us, most of the time of a short
+// list) with the counting of others; their lists share the room, and lists that
+// spill into global memory cost more than that.  us, 1 -> 3 groups (XXX
+// clustered, XXX, XXY): 1000 points, dmax 45 of 250, 20 bins 42 39 55 -> 29 23 35;
+// 4100: 153 136 254 -> 86 71 176; 16000: 969 817 2848 -> 698 524 1755; 30 bins, dmax 80: 4100: 279
+// 257 852 -> 221 193 567; 8000: 986 883 2939 -> 952 805 2468; 16000, where they
+// spill: 5057 4401 15533 -> 5652 4770 18544.  Weighted counts, bound by their
+// atomics in global memory: 1000 points 53 41 76 -> 78 35 86, 4100 190 131 373 ->
+// 180 73 384, so they keep one.  (Four groups of 6 warps and two of 12 lie between.)
+static int trip_groups(const pcf_grid *X, const pcf_grid *Y, int bins, float dmax, bool weighted) {
+    const size_t hist = trip_hist_bytes(bins, weighted);
+    if (weighted || !hist) return 1;
+    const double L = X->box, in = std::min(1.0, 4.18879 * (double)dmax * dmax * dmax / (L * L * L));
+    const double list = Y ? (0.5 * (double)X->n + (double)Y->n) * in : (double)X->n * in;
+    constexpr int G = kTWarps / kGroupWarps;
+    return list <= (double)((kTripSmem - hist) / G / 16) ? G : 1;
+}
+
 // Arguments of one isotropic triplet histogram over the cell structures of
 // x (and y for XXY) at P partitions: catalogs, side rules, FP32 windows and
 // the shared-memory layout (smem: dynamic bytes).  The buffers (rows,
 // counter, histograms, overflow lists) are the caller's.
 static void trip_setup(pcf_ctx *ctx, const pcf_grid *X, const pcf_grid *Y, int P, int n_rows, int bins,
-                       float dmax, uint32_t flags, bool weighted, TripArgs &A, size_t &smem) {
+                       float dmax, uint32_t flags, bool weighted, TripArgs &A, size_t &smem, int groups = 1) {
     const bool bpc = (flags & PCF_BPC) != 0, mixed = Y != nullptr;
     const CellGrid &gx = *X->cells;
     const CellGrid &gy = mixed ? *Y->cells : gx;
@@ -1195,13 +1254,10 @@ static void trip_setup(pcf_ctx *ctx, const pcf_grid *X, const pcf_grid *Y, int P
     A.status = ctx->d_status;
     A.mixed = mixed ? 1 : 0;
     A.fc = trip_cuts(rXX, X->box, dmax, bpc);
-    const size_t u_bytes = ((size_t)u_words(bins) * 4 + 15) & ~(size_t)15;
-    const size_t smem_max = 227 * 1024 - 128 - sizeof(ListScratch) - sizeof(ChunkBox) * kMaxBoxes -
-                            sizeof(uint2) * 64 * kTWarps;
-    A.hist_in_smem = (!weighted && u_bytes <= 150 * 1024) ? 1 : 0;
-    const size_t hist_b = A.hist_in_smem ? u_bytes : 0;
+    const size_t hist_b = trip_hist_bytes(bins, weighted);
+    A.hist_in_smem = hist_b > 0 ? 1 : 0;
     const size_t ent = 16 + (weighted ? 4 : 0);
-    const size_t room = smem_max - hist_b;
+    const size_t room = (kTripSmem - hist_b) / groups;
     if (mixed && !(A.hist_in_smem && !weighted)) {
         A.capJ = (int)(room / ent / 3);
         A.capK = (int)(room / ent) - A.capJ;
@@ -1209,7 +1265,9 @@ static void trip_setup(pcf_ctx *ctx, const pcf_grid *X, const pcf_grid *Y, int P
         A.capJ = (int)(room / ent);
         A.capK = 0;
     }
-    smem = hist_b + (size_t)(A.capJ + A.capK) * ent;
+    A.list_bytes = (int)(((size_t)(A.capJ + A.capK) * ent + 15) & ~(size_t)15);
+    if (groups > 1) A.flush_budget = std::min<unsigned long long>(A.flush_budget, 1ull << 30) / (unsigned)groups;
+    smem = hist_b + (size_t)A.list_bytes * groups;
 }
 
 // Per-CTA overflow lists for lists of up to gcap entries (J, K and weights).
@@ -1231,11 +1289,16 @@ static pcf_status count_triplets_ordered(pcf_ctx *ctx, const pcf_grid *x_, const
                                          float dmax, uint32_t flags, double *hist, pcf_stats *stats,
                                          bool iso3);
 
-// Entries that the ordered counts' lists hold in shared memory; returns the bytes
-// of one (the row table of the list build takes one of them).
-static size_t ordered_caps(bool mixed, bool weighted, bool gates, TripArgs &A) {
+// Entries that the ordered counts' lists hold in shared memory with `ctas` CTAs
+// per SM; returns the bytes of one (the row table of the list build takes one of
+// them).  Several small CTAs overlap one's list builds with another's counting;
+// they are taken where no list can be longer than theirs hold, which leaves the
+// calls that the large one refuses as they are.
+static size_t ordered_caps(bool mixed, bool weighted, bool gates, int ctas, TripArgs &A) {
     const size_t ent = 16 + 2 + (weighted ? 4 : 0) + (gates ? 4 : 0);
-    const size_t room = 227 * 1024 - 256 - (gates ? 64 * sizeof(GateBlock) + 128 + 64 : 0);
+    const size_t fixed = 256 + (gates ? 64 * sizeof(GateBlock) + 128 + 64 : 0);
+    const size_t room = ctas == 1 ? 227 * 1024 - fixed
+                                  : 228 * 1024 / ctas - 1024 - 256 - sizeof(ListScratch<kGroupWarps>) - fixed;
     if (mixed) {
         A.capJ = (int)(room / ent / 3);
         A.capK = (int)(room / ent) - A.capJ - 8;
@@ -1290,7 +1353,8 @@ extern "C" pcf_status pcf_count_triplets(pcf_ctx *ctx, int kind, const pcf_grid 
     if (gates && weighted) return ordered();
     TripArgs A;
     size_t smem = 0;
-    trip_setup(ctx, X, Y, P, (int)plan.rows.size(), bins, dmax, flags, weighted, A, smem);
+    const int groups = trip_groups(X, Y, bins, dmax, weighted);
+    trip_setup(ctx, X, Y, P, (int)plan.rows.size(), bins, dmax, flags, weighted, A, smem, groups);
     const int n3 = bins * bins * bins;
     // rows + counter through the plan slot
     PlanSlot *sl = nullptr;
@@ -1304,15 +1368,23 @@ extern "C" pcf_status pcf_count_triplets(pcf_ctx *ctx, int kind, const pcf_grid 
     if (s == PCF_OK && mixed) s = list_bound(ctx, gy, Y->n, dmax, A.rows, A.n_rows, bpc, &by);
     TripArgs F;  // the gates' corrections
     size_t fix_smem = 0;
+    int fix_ctas = kTWarps / kGroupWarps;
     if (s == PCF_OK && gates) {
-        ordered_caps(mixed, false, true, F);
-        int64_t fx = bx, fy = by;
-        // an entry also has its place in the order by image (two bytes; the row
-        // table's share of `room` comes off here)
-        const int capJ = F.capJ - 300, capK = mixed ? F.capK : 0;
-        if (fx > capJ) s = list_bound(ctx, gx, X->n, dmax, A.rows, A.n_rows, bpc, &fx, capJ);
-        if (s == PCF_OK && mixed && fy > capK) s = list_bound(ctx, gy, Y->n, dmax, A.rows, A.n_rows, bpc, &fy, capK);
-        if (s == PCF_OK && (fx > capJ || (mixed && fy > capK))) return ordered();
+        int capJ = 0, capK = 0;
+        for (;; fix_ctas = 1) {
+            ordered_caps(mixed, false, true, fix_ctas, F);
+            // an entry also has its place in the order by image (two bytes; the row
+            // table's share of the room comes off here)
+            capJ = F.capJ - 300;
+            capK = mixed ? F.capK : 0;
+            int64_t fx = bx, fy = by;
+            if (fx > capJ) s = list_bound(ctx, gx, X->n, dmax, A.rows, A.n_rows, bpc, &fx, capJ);
+            if (s == PCF_OK && mixed && fy > capK)
+                s = list_bound(ctx, gy, Y->n, dmax, A.rows, A.n_rows, bpc, &fy, capK);
+            if (s != PCF_OK) return s;
+            if (fx <= capJ && (!mixed || fy <= capK)) break;
+            if (fix_ctas == 1) return ordered();
+        }
         F = A;
         F.capJ = capJ;
         F.capK = capK;
@@ -1320,7 +1392,7 @@ extern "C" pcf_status pcf_count_triplets(pcf_ctx *ctx, int kind, const pcf_grid 
         fix_smem = (size_t)(capJ + capK) * 20 + 2 * (size_t)(mixed ? capK : capJ);
     }
     const int grid = ctx->sm_count;
-    if (s == PCF_OK) s = trip_overflow(ctx, std::max(bx, by) + 32, mixed, weighted, grid, A);
+    if (s == PCF_OK) s = trip_overflow(ctx, std::max(bx, by) + 32, mixed, weighted, grid * groups, A);
     if (s != PCF_OK) return s;
     // histogram scratch: [u64 n3][f64 n3][stats 8][f64 out n3]
     PCF_CU(ctx, ctx->d_hist.ensure((size_t)n3 * 24 + 64));
@@ -1333,8 +1405,11 @@ extern "C" pcf_status pcf_count_triplets(pcf_ctx *ctx, int kind, const pcf_grid 
     // unweighted: the sums' place holds the gates' corrections
     unsigned long long *fix = gates ? reinterpret_cast<unsigned long long *>(A.g_wsum) : nullptr;
 
-    auto kfn = mixed ? (weighted ? k_triplets<true, true> : k_triplets<true, false>)
-                     : (weighted ? k_triplets<false, true> : k_triplets<false, false>);
+    auto pick = [&](auto one, auto several) { return groups > 1 ? several : one; };
+    auto kfn = mixed ? (weighted ? pick(k_triplets<true, true, kTWarps>, k_triplets<true, true, kGroupWarps>)
+                                 : pick(k_triplets<true, false, kTWarps>, k_triplets<true, false, kGroupWarps>))
+                     : (weighted ? pick(k_triplets<false, true, kTWarps>, k_triplets<false, true, kGroupWarps>)
+                                 : pick(k_triplets<false, false, kTWarps>, k_triplets<false, false, kGroupWarps>));
     PCF_CU(ctx, ensure_smem_limit(reinterpret_cast<const void *>(kfn), ctx->device, smem));
     cudaEvent_t pe0 = nullptr, pe1 = nullptr;
     if (ctx->profile) {
@@ -1349,10 +1424,12 @@ extern "C" pcf_status pcf_count_triplets(pcf_ctx *ctx, int kind, const pcf_grid 
         F.g_count = fix;
         F.g_stats = A.g_stats;
         F.counter = A.counter + 1;
-        auto ffn = mixed ? k_gate_fix<true> : k_gate_fix<false>;
+        const bool few = fix_ctas == 1;
+        auto ffn = mixed ? (few ? k_gate_fix<kTWarps, true> : k_gate_fix<kGroupWarps, true>)
+                         : (few ? k_gate_fix<kTWarps, false> : k_gate_fix<kGroupWarps, false>);
         PCF_CU(ctx, ensure_smem_limit(reinterpret_cast<const void *>(ffn), ctx->device, fix_smem));
         const float reach = (float)(std::sqrt(A.rXX.dd) * (1.0 + 1e-6) + (double)A.box * 1e-6);
-        ffn<<<grid, kTThreads, fix_smem, ctx->stream>>>(F, reach);
+        ffn<<<grid * fix_ctas, kTThreads / fix_ctas, fix_smem, ctx->stream>>>(F, reach);
         PCF_CU(ctx, cudaGetLastError());
         ++ctx->launches;
     }
@@ -1582,6 +1659,19 @@ extern "C" pcf_status pcf_batch_triplets(pcf_ctx *ctx, const pcf_grid *d_, const
     return PCF_OK;
 }
 
+template <int NW>
+static void (*ordered_kernel(bool mixed, bool weighted, bool gates, bool iso3))(const TripArgs) {
+    if (iso3)
+        return mixed ? (weighted ? k_triplets_ani<NW, true, true, true, true> : k_triplets_ani<NW, true, false, true, true>)
+                     : (weighted ? k_triplets_ani<NW, false, true, true, true>
+                                 : k_triplets_ani<NW, false, false, true, true>);
+    if (gates)
+        return mixed ? (weighted ? k_triplets_ani<NW, true, true, true> : k_triplets_ani<NW, true, false, true>)
+                     : (weighted ? k_triplets_ani<NW, false, true, true> : k_triplets_ani<NW, false, false, true>);
+    return mixed ? (weighted ? k_triplets_ani<NW, true, true> : k_triplets_ani<NW, true, false>)
+                 : (weighted ? k_triplets_ani<NW, false, true> : k_triplets_ani<NW, false, false>);
+}
+
 // Anisotropic triplets (bins^5).  The histogram lives in global memory (u64
 // counts or FP64 sums); lists stay in shared memory (an anchor whose lists
 // do not fit makes the call fail with PCF_ERR_UNSUPPORTED).
@@ -1644,16 +1734,24 @@ static pcf_status count_triplets_ordered(pcf_ctx *ctx, const pcf_grid *x_, const
     if (gates) A.gate = gate_geometry(X->box, dmax, X->user_P);
     A.fc = trip_cuts(rXX, X->box, dmax, bpc);
     const bool weighted = !(X->unit_weights && (!mixed || Y->unit_weights));
-    const size_t ent = ordered_caps(mixed, weighted, gates, A);
-    // (an entry's angle bin takes one of the two bytes `ent` counts: the row
-    // table has the rest)
-    const size_t smem = (size_t)(A.capJ + A.capK) * (ent - 1) + 64;
     const int64_t n5 = nh;
     PlanSlot *sl = nullptr;
     s = stage_plan(ctx, plan, &sl);
     if (s != PCF_OK) return s;
     A.rows = sl->rows();
     A.counter = sl->counter();
+    int ctas = kTWarps / kGroupWarps;
+    size_t ent = ordered_caps(mixed, weighted, gates, ctas, A);
+    int64_t bx = 0, by = 0;
+    s = list_bound(ctx, gx, X->n, dmax, A.rows, A.n_rows, bpc, &bx, A.capJ);
+    if (s == PCF_OK && mixed) s = list_bound(ctx, gy, Y->n, dmax, A.rows, A.n_rows, bpc, &by, A.capK);
+    if (s != PCF_OK) return s;
+    if (bx > A.capJ || (mixed && by > A.capK)) {
+        ctas = 1;
+        ent = ordered_caps(mixed, weighted, gates, ctas, A);
+    }
+    // (an entry's angle bin takes one of the two bytes `ent` counts)
+    const size_t smem = (size_t)(A.capJ + A.capK) * (ent - 1) + 64;
     PCF_CU(ctx, ctx->d_hist.ensure((size_t)n5 * 16 + 128));
     char *hp = ctx->d_hist.as<char>();
     A.g_count = reinterpret_cast<unsigned long long *>(hp);
@@ -1661,19 +1759,11 @@ static pcf_status count_triplets_ordered(pcf_ctx *ctx, const pcf_grid *x_, const
     A.g_stats = reinterpret_cast<unsigned long long *>(hp + (size_t)n5 * 8);
     double *d_out = reinterpret_cast<double *>(hp + (size_t)n5 * 8 + 128);
     PCF_CU(ctx, cudaMemsetAsync(hp, 0, (size_t)n5 * 8 + 128, ctx->stream));
-    void (*kfn)(const TripArgs);
-    if (iso3)
-        kfn = mixed ? (weighted ? k_triplets_ani<true, true, true, true> : k_triplets_ani<true, false, true, true>)
-                    : (weighted ? k_triplets_ani<false, true, true, true> : k_triplets_ani<false, false, true, true>);
-    else if (gates)
-        kfn = mixed ? (weighted ? k_triplets_ani<true, true, true> : k_triplets_ani<true, false, true>)
-                    : (weighted ? k_triplets_ani<false, true, true> : k_triplets_ani<false, false, true>);
-    else
-        kfn = mixed ? (weighted ? k_triplets_ani<true, true> : k_triplets_ani<true, false>)
-                    : (weighted ? k_triplets_ani<false, true> : k_triplets_ani<false, false>);
+    const auto kfn = ctas == 1 ? ordered_kernel<kTWarps>(mixed, weighted, gates, iso3)
+                               : ordered_kernel<kGroupWarps>(mixed, weighted, gates, iso3);
     PCF_CU(ctx, ensure_smem_limit(reinterpret_cast<const void *>(kfn), ctx->device, smem));
     PCF_CU(ctx, cudaEventRecord(ctx->ev0, ctx->stream));
-    kfn<<<ctx->sm_count, kTThreads, smem, ctx->stream>>>(A);
+    kfn<<<ctx->sm_count * ctas, kTThreads / ctas, smem, ctx->stream>>>(A);
     PCF_CU(ctx, cudaGetLastError());
     PCF_CU(ctx, cudaEventRecord(ctx->ev1, ctx->stream));
     PCF_CU(ctx, cudaEventRecord(sl->done, ctx->stream));
