@@ -78,6 +78,10 @@ struct TripArgs {
     unsigned long long *g_count;  // bins^3 (unit weights)
     double *g_wsum;               // bins^3 (weighted)
     int hist_in_smem;
+    // weighted: the catalogs' weights are exact integers q (Cat::w holds their
+    // bits), w_i w_j w_k = q_i q_j q_k * wunscale
+    int wfix;
+    double wunscale;
     int list_bytes;          // shared memory of a group's lists
     unsigned long long *g_stats;
     // adds the shared u32 histogram absorbs between flushes into g_count
@@ -362,6 +366,43 @@ __device__ int build_list(const TripArgs &A, const Cat &C, float hx, float hy, f
 // of bins + 1 counters over b_jk, the last of which takes the tests out of
 // range and is never read.
 __host__ __device__ __forceinline__ int u_words(int bins) { return bins * bins * (bins + 1); }
+
+// The shared histogram of the weighted counts: sums of exact integer weight
+// products, three 32-bit limbs each, over [b_ij] and the unordered pair of b_ki and
+// b_jk, which the final sums take together.  FP64 adds in global memory queued in
+// L2; FP64 adds to shared memory, loops of compare-and-swaps, lay between (us, XXX
+// clustered, XXX, XXY of 4100 points, 25 bins, dmax 70: 633 424 1316, 557 342 786, and
+// 377 310 682 by limbs; 8000 points 3790 2987 8535, 3222 1861 4779, 2111 1618 3980).
+__host__ __device__ __forceinline__ int w_slots(int bins) { return bins * (bins * (bins + 1) / 2); }
+__device__ __forceinline__ int w_slot(int bins, int bij, int bki, int bjk) {
+    const int lo = min(bki, bjk), hi = max(bki, bjk);
+    return bij * (bins * (bins + 1) / 2) + hi * (hi + 1) / 2 + lo;
+}
+// Bytes of a shared histogram, rounded up to 16.
+__host__ __device__ __forceinline__ size_t hist_bytes(int bins, bool weighted) {
+    const size_t b = weighted ? (size_t)w_slots(bins) * 12 : (size_t)u_words(bins) * 4;
+    return (b + 15) & ~(size_t)15;
+}
+// Adds it into g (bins^3, at [b_ij][lo][hi]) and clears it (whole group; others may
+// be adding meanwhile: the limbs are taken one by one, and what a carry brings to
+// one afterwards stays for the next flush).
+template <int NW>
+__device__ __forceinline__ void flush_limbs(unsigned *U, int bins, double unscale, double *g) {
+    gsync<NW>();
+    const int half = bins * (bins + 1) / 2, n = w_slots(bins);
+    for (int k = group_tid<NW>(); k < n; k += NW * 32) {
+        if (!(U[k] | U[k + n] | U[k + 2 * n])) continue;
+        const double l0 = (double)atomicExch(U + k, 0u), l1 = (double)atomicExch(U + k + n, 0u),
+                     l2 = (double)atomicExch(U + k + 2 * n, 0u);
+        const int a = k / half, p = k - a * half;
+        int hi = (int)((sqrtf(8.f * (float)p + 1.f) - 1.f) * 0.5f);  // hi (hi + 1) / 2 <= p, up to rounding
+        if (hi * (hi + 1) / 2 > p) --hi;
+        if ((hi + 1) * (hi + 2) / 2 <= p) ++hi;
+        atomicAdd(g + ((long long)a * bins + (p - hi * (hi + 1) / 2)) * bins + hi,
+                  (l2 * 0x1p64 + (l1 * 0x1p32 + l0)) * unscale);
+    }
+    gsync<NW>();
+}
 
 // Adds U into the u64 histogram g (bins^3, [b_ij][b_ki][b_jk]) and clears it
 // (whole group); returns the triangles this thread added.  SHARED: other groups
@@ -658,7 +699,7 @@ __device__ __forceinline__ void tri_anchor(const TripArgs &A, int i, TripCta<NW>
     // Flush budget of the shared histogram: this anchor adds at most
     // `tests` times.  Flush first if the total could pass the budget; an
     // anchor whose tests alone exceed it counts into global memory.
-    bool smem_hist = !WEIGHTED && A.hist_in_smem;
+    bool smem_hist = A.hist_in_smem;
     if (smem_hist) {
         const unsigned long long tests =
             MIXED ? (unsigned long long)nJ * (unsigned long long)nK
@@ -667,14 +708,15 @@ __device__ __forceinline__ void tri_anchor(const TripArgs &A, int i, TripCta<NW>
             smem_hist = false;
         } else {
             if (C.since + tests > A.flush_budget) {
-                C.n_tri += flush_hist<NW, NW != kTWarps>(C.U, bins, A.g_count);
+                if (WEIGHTED) flush_limbs<NW>(C.U, bins, A.wunscale, A.g_wsum);
+                else C.n_tri += flush_hist<NW, NW != kTWarps>(C.U, bins, A.g_count);
                 C.since = 0;
             }
             C.since += tests;
         }
     }
     // pass 2: pairs of neighbours
-    if (smem_hist) {
+    if (smem_hist && !WEIGHTED) {
         // the lists' address space is fixed per instantiation, so the
         // shared-memory case (all but overflowing anchors) uses shared loads
         if (spill) {
@@ -688,6 +730,8 @@ __device__ __forceinline__ void tri_anchor(const TripArgs &A, int i, TripCta<NW>
         }
         return;
     }
+    auto weight = [&](float w) { return A.wfix ? (double)__float_as_uint(w) : (double)w; };
+    const int nw = WEIGHTED ? w_slots(bins) : 0;
     // rows j dealt to warps in the order 0, n-1, 1, n-2, ... (XXX rows shrink with j)
     for (int rr = warp; rr < nJ; rr += NW) {
         const int half = rr >> 1;
@@ -695,7 +739,9 @@ __device__ __forceinline__ void tri_anchor(const TripArgs &A, int i, TripCta<NW>
         const float4 ej = LJ[jj];
         const int bj = __float_as_int(ej.w) & 255;
         const int jidx = (int)((unsigned)__float_as_int(ej.w) >> 8);
-        const double wij = WEIGHTED ? (double)hw * (double)WJ[jj] : 1.0;
+        const double wij = WEIGHTED ? weight(hw) * weight(WJ[jj]) * (A.wfix ? A.wunscale : 1.0) : 1.0;
+        const unsigned long long qij =
+            WEIGHTED ? (unsigned long long)__float_as_uint(hw) * __float_as_uint(WJ[jj]) : 0ull;
         const int ubase = bj * bins * bins;
         const int k0 = MIXED ? 0 : jj + 1;
         for (int kk = k0 + lane; kk < nK; kk += 32) {
@@ -715,8 +761,25 @@ __device__ __forceinline__ void tri_anchor(const TripArgs &A, int i, TripCta<NW>
                 const int bk = __float_as_int(ek.w) & 255;
                 const int slot = ubase + bk * bins + bjk;
                 ++C.n_tri;
-                if (WEIGHTED) atomicAdd(A.g_wsum + slot, wij * (double)WK[kk]);
-                else atomicAdd(A.g_count + slot, 1ull);
+                if (!WEIGHTED) {
+                    atomicAdd(A.g_count + slot, 1ull);
+                } else if (smem_hist) {
+                    // q_i q_j q_k in three limbs, the carries by the values that the
+                    // adds return (an FP64 add to shared memory is a loop of
+                    // compare-and-swaps, one to global memory queues in L2)
+                    const unsigned qk = __float_as_uint(WK[kk]);
+                    const unsigned long long p0 = (qij & 0xffffffffull) * qk, p1 = (qij >> 32) * qk + (p0 >> 32);
+                    unsigned *u = C.U + w_slot(bins, bj, bk, bjk);
+                    const unsigned l0 = (unsigned)p0, l1 = (unsigned)p1;
+                    const unsigned c0 = atomicAdd(u, l0) > ~l0 ? 1u : 0u;
+                    const unsigned long long m = (unsigned long long)l1 + c0;
+                    const unsigned m0 = (unsigned)m;
+                    const unsigned c1 = atomicAdd(u + nw, m0) > ~m0 ? 1u : 0u;
+                    const unsigned h = (unsigned)(p1 >> 32) + (unsigned)(m >> 32) + c1;
+                    if (h) atomicAdd(u + 2 * nw, h);
+                } else {
+                    atomicAdd(A.g_wsum + slot, wij * weight(WK[kk]));
+                }
             }
         }
     }
@@ -727,7 +790,7 @@ __global__ void __launch_bounds__(kTThreads, 1) k_triplets(const __grid_constant
     constexpr int G = kTWarps / NW;
     extern __shared__ __align__(16) unsigned char smem[];
     const int bins = A.rXX.bins;
-    const size_t u_bytes = A.hist_in_smem ? (((size_t)u_words(bins) * 4 + 15) & ~(size_t)15) : 0;
+    const size_t u_bytes = A.hist_in_smem ? hist_bytes(bins, WEIGHTED) : 0;
     __shared__ ListScratch<NW> s_scr[G];
     __shared__ ChunkBox s_boxes[kMaxBoxes];
     __shared__ uint2 s_queue[64 * kTWarps];
@@ -738,7 +801,7 @@ __global__ void __launch_bounds__(kTThreads, 1) k_triplets(const __grid_constant
                   s_boxes + g * max_boxes<NW>(), s_queue + g * NW * 64, &s_unit[g], (int)blockIdx.x * G + g, 0u,
                   0ull, 0ull};
     if (A.hist_in_smem)
-        for (int k = threadIdx.x; k < u_words(bins); k += kTThreads) C.U[k] = 0u;
+        for (int k = threadIdx.x; k < (int)(u_bytes / 4); k += kTThreads) C.U[k] = 0u;
     if (G > 1) __syncthreads();
     long long taken = 0;  // anchors this group took (iteration cap: nX + 1)
     int ticket = 0;       // thread 0: the next anchor, taken while the last one is counted
@@ -761,7 +824,8 @@ __global__ void __launch_bounds__(kTThreads, 1) k_triplets(const __grid_constant
     }
     if (A.hist_in_smem) {
         if (G > 1) __syncthreads();  // every group's counts are in
-        C.n_tri += flush_hist<kTWarps, (G > 1)>(C.U, bins, A.g_count);
+        if (WEIGHTED) flush_limbs<kTWarps>(C.U, bins, A.wunscale, A.g_wsum);
+        else C.n_tri += flush_hist<kTWarps, (G > 1)>(C.U, bins, A.g_count);
     }
     unsigned long long rr = C.n_rechk, nt = C.n_tri;
     for (int off = 16; off > 0; off >>= 1) {
@@ -803,10 +867,10 @@ __global__ void __launch_bounds__(kTThreads, 1) k_triplets_batch(const __grid_co
     const TripArgs &J0 = B.job[0];
     const int bins = J0.rXX.bins;
     const bool in_smem = J0.hist_in_smem != 0;
-    const size_t u_bytes = in_smem ? (((size_t)u_words(bins) * 4 + 15) & ~(size_t)15) : 0;
+    const size_t u_bytes = in_smem ? hist_bytes(bins, WEIGHTED) : 0;
     TripCta<kTWarps> C{reinterpret_cast<unsigned *>(smem), smem + u_bytes, &s_scr, s_boxes, s_queue, &s_unit, (int)blockIdx.x, 0u, 0ull, 0ull};
     if (in_smem)
-        for (int k = tid; k < u_words(bins); k += kTThreads) C.U[k] = 0u;
+        for (int k = tid; k < (int)(u_bytes / 4); k += kTThreads) C.U[k] = 0u;
     int cur = -1;  // the CTA's current job (uniform: every thread follows s_anchor)
     long long taken = 0, ticket = 0;  // ticket (thread 0): taken while the last anchor is counted
     if (tid == 0) ticket = (long long)atomicAdd(B.counter, 1ull);
@@ -828,7 +892,8 @@ __global__ void __launch_bounds__(kTThreads, 1) k_triplets_batch(const __grid_co
             int j = cur < 0 ? 0 : cur;
             while (j + 1 < B.n_jobs && g >= B.job[j + 1].anchor_begin) ++j;
             if (cur >= 0 && in_smem && C.since) {
-                C.n_tri += flush_hist<kTWarps, false>(C.U, bins, B.job[cur].g_count);
+                if (WEIGHTED) flush_limbs<kTWarps>(C.U, bins, B.job[cur].wunscale, B.job[cur].g_wsum);
+                else C.n_tri += flush_hist<kTWarps, false>(C.U, bins, B.job[cur].g_count);
                 C.since = 0;
             }
             cur = j;
@@ -837,7 +902,8 @@ __global__ void __launch_bounds__(kTThreads, 1) k_triplets_batch(const __grid_co
         tri_anchor<kTWarps, MIXED, WEIGHTED>(A, (int)(g - A.anchor_begin), C);
         __syncthreads();
     }
-    if (in_smem && cur >= 0) C.n_tri += flush_hist<kTWarps, false>(C.U, bins, B.job[cur].g_count);
+    if (WEIGHTED && in_smem && cur >= 0) flush_limbs<kTWarps>(C.U, bins, B.job[cur].wunscale, B.job[cur].g_wsum);
+    else if (in_smem && cur >= 0) C.n_tri += flush_hist<kTWarps, false>(C.U, bins, B.job[cur].g_count);
     unsigned long long rr = C.n_rechk, nt = C.n_tri;
     for (int off = 16; off > 0; off >>= 1) {
         rr += __shfl_down_sync(kFull, rr, off);
@@ -1200,8 +1266,16 @@ static TripCuts trip_cuts(const PairRule &rule, float box, float dmax, bool bpc)
 constexpr size_t kTripSmem = 227 * 1024 - 256 - sizeof(ListScratch<kTWarps>) - sizeof(ChunkBox) * kMaxBoxes -
                              sizeof(uint2) * 64 * kTWarps;
 static size_t trip_hist_bytes(int bins, bool weighted) {
-    const size_t b = ((size_t)u_words(bins) * 4 + 15) & ~(size_t)15;
-    return !weighted && b <= 150 * 1024 ? b : 0;
+    const size_t b = hist_bytes(bins, weighted);
+    return b <= (weighted ? 166 : 150) * 1024 ? b : 0;
+}
+// Adds that a three-limb counter of the weighted counts takes (0: the weights are
+// no exact integers, or their products too large).
+static unsigned long long limb_budget(const pcf_grid *X, const pcf_grid *Y) {
+    if (!X->wfix_ok || (Y && !Y->wfix_ok)) return 0;
+    const double q = (double)X->wqmax * (double)X->wqmax * (double)(Y ? Y : X)->wqmax;
+    const double adds = std::floor(std::ldexp(1.0, 96) / std::max(q, 1.0) * (1.0 - 1e-9));
+    return adds < 262144.0 ? 0 : (unsigned long long)std::min(adds, 2147483648.0);
 }
 
 // Groups of warps per CTA, each with anchors of its own.  Three overlap the
@@ -1211,16 +1285,18 @@ static size_t trip_hist_bytes(int bins, bool weighted) {
 // clustered, XXX, XXY): 1000 points, dmax 45 of 250, 20 bins 42 39 55 -> 29 23 35;
 // 4100: 153 136 254 -> 86 71 176; 16000: 969 817 2848 -> 698 524 1755; 30 bins, dmax 80: 4100: 279
 // 257 852 -> 221 193 567; 8000: 986 883 2939 -> 952 805 2468; 16000, where they
-// spill: 5057 4401 15533 -> 5652 4770 18544.  Weighted counts, bound by their
-// atomics in global memory: 1000 points 53 41 76 -> 78 35 86, 4100 190 131 373 ->
-// 180 73 384, so they keep one.  (Four groups of 6 warps and two of 12 lie between.)
+// spill: 5057 4401 15533 -> 5652 4770 18544.  Weighted counts take three up to half
+// that: 1000 points, 20 bins 45 37 58 -> 32 24 37, 4100 points, dmax 70, 25 bins 412
+// 354 731 -> 377 310 682, 8000: 2133 1732 3980 -> 2111 1618 4036, 30 bins, dmax 80 3568 3104
+// 7501 -> 3901 3058 11834; without exact integer weights, bound by atomics in
+// global memory, one.  (Four groups of 6 warps and two of 12 lie between.)
 static int trip_groups(const pcf_grid *X, const pcf_grid *Y, int bins, float dmax, bool weighted) {
     const size_t hist = trip_hist_bytes(bins, weighted);
-    if (weighted || !hist) return 1;
+    if (!hist || (weighted && !limb_budget(X, Y))) return 1;
     const double L = X->box, in = std::min(1.0, 4.18879 * (double)dmax * dmax * dmax / (L * L * L));
     const double list = Y ? (0.5 * (double)X->n + (double)Y->n) * in : (double)X->n * in;
     constexpr int G = kTWarps / kGroupWarps;
-    return list <= (double)((kTripSmem - hist) / G / 16) ? G : 1;
+    return list <= (double)((kTripSmem - hist) / G / (weighted ? 40 : 16)) ? G : 1;
 }
 
 // Arguments of one isotropic triplet histogram over the cell structures of
@@ -1254,8 +1330,15 @@ static void trip_setup(pcf_ctx *ctx, const pcf_grid *X, const pcf_grid *Y, int P
     A.status = ctx->d_status;
     A.mixed = mixed ? 1 : 0;
     A.fc = trip_cuts(rXX, X->box, dmax, bpc);
-    const size_t hist_b = trip_hist_bytes(bins, weighted);
+    const size_t hist_b = weighted && !limb_budget(X, Y) ? 0 : trip_hist_bytes(bins, weighted);
     A.hist_in_smem = hist_b > 0 ? 1 : 0;
+    if (hist_b && weighted) {
+        A.wfix = 1;
+        A.wunscale = std::ldexp(1.0, -(2 * X->wshift + (mixed ? Y : X)->wshift));
+        A.X.w = reinterpret_cast<const float *>(gx.qw.as<unsigned>());
+        A.Y.w = reinterpret_cast<const float *>(gy.qw.as<unsigned>());
+        A.flush_budget = std::min(A.flush_budget, limb_budget(X, Y));
+    }
     const size_t ent = 16 + (weighted ? 4 : 0);
     const size_t room = (kTripSmem - hist_b) / groups;
     if (mixed && !(A.hist_in_smem && !weighted)) {
