@@ -1417,20 +1417,31 @@ pcf_status stencil_max(pcf_ctx *ctx, const CellGrid &g, const RowDesc *d_rows, i
 // while it holds 6, else 1 (us per DD + DR, isotropic: 300000 points, box 1000,
 // dmax 100: 1325 at 3 cells, 1620 at 4; 10^6 points: 10083 and 9738; 2000 points,
 // box 250, dmax 80: 55, 59, 98 and 136 at 1, 2, 3 and 4).  Triplet counts, where
-// a candidate costs an anchor's CTA more, take 4 or 3 from 6 points on.  A periodic stencil never wraps onto
-// itself (2k + 2 <= P).
+// a candidate costs an anchor's CTA more, take 4 or 3 from 6 points on.  Cells of
+// one dmax that would hold fewer than 5 points grow to 5: a tile spans at most two
+// cells, and a tile costs about 1100 instructions however few points it holds
+// (1.7M and 2.7M points, box 2000, dmax 10.6, us per DD + RR + DR: 4388 at 188 cells per
+// side, 0.4 points each; 2062 at 94; 1925 at 80, 5.2 points; 2201 at 64; 200000 and
+// 300000 points, dmax 20: 565 at 99 cells, 374 at 50, 400 at 40, 366 at 32, weighted
+// 2ani 638, 420, 448, 463; 6M and 9M points, dmax 15: 5517 at 133, 5276 at 120, 5891 at 100).
+// A periodic stencil never wraps onto itself (2k + 2 <= P).
 int choose_partitions(int64_t n, float box, float dmax, int kind, bool bpc, int refine) {
     double least = 6.0;  // points per cell at 3 cells per dmax or more
+    bool grow = false;   // cells of few points
     if (refine <= 0) {
         const char *e = getenv("PCF_REFINE");  // experiment / autotuner override
         refine = e ? atoi(e) : 4;
         if (refine < 1 || refine > 16) refine = 4;
-        if (!e && kind != kTripletCells) least = 12.0;
+        if (!e && kind != kTripletCells) {
+            least = 12.0;
+            grow = true;
+        }
     }
     double L = box, R = dmax;
     auto cells = [&](int r) { return (int)std::floor(L * (r - 1e-4) / (R + 8.0 * L * 1.2e-7) * (1.0 - 1e-9)); };
     int P = cells(refine);
     while (P > 1 && refine > 1 && (double)n / ((double)P * P * P) < (refine > 2 ? least : 6.0)) P = cells(--refine);
+    if (grow && refine == 1) P = std::min(P, (int)std::cbrt((double)n / 5.0));
     P = std::max(1, std::min(P, 256));
     if (bpc) {
         // need 2k+1 <= P with k = ceil(R / (L/P)) (+1 for the tile span)
