@@ -17,7 +17,7 @@
 //   (ru + rv >= rw + h) and (ru + rw >= rv + h) and (rv + rw >= ru + h),
 // every sum rounded as the reference's, and for fixed (u, v) the kept w
 // form one interval (the first clause is decreasing in w, the others
-// increasing).  Each (u, v) then costs two binary searches and two prefix
+// increasing).  Each (u, v) then costs the interval's ends and two prefix
 // sums over w instead of bn_ref corner tests:
 //   sum_w c = (ru+h/2)(rv+h/2) S1,  sum_w f = (ru+h/2)(rv+h/2)[(1+A_u+B_v) S1 + S2]
 // with S1 = sum (rw+h/2), S2 = sum ff_ref[k*bn_ref+w]/3 over the interval.
@@ -140,7 +140,11 @@ __global__ void k_coarse(int bins, double dr, double alpha, const double *ff, do
 
 constexpr int kRefMax = 512;
 
-// One CTA per coarse bin; partial bins refined on the bn_ref^3 sub-grid.
+// One CTA per coarse bin; partial bins refined on the bn_ref^3 sub-grid.  Bound by
+// FP64 issue: everything that depends on u, v or w alone is computed once per CTA,
+// and the ends of a (u, v)'s interval of w are estimated and then checked (two to
+// four tests where the binary searches took sixteen).  20 bins, bn_ref 200: 790 ->
+// 374 us.
 __global__ void __launch_bounds__(256) k_refine(int bins, int bn_ref, double dr, double alpha_ref,
                                                 const double *ffr, const unsigned char *partial,
                                                 double *ddr, double *rrr) {
@@ -151,25 +155,36 @@ __global__ void __launch_bounds__(256) k_refine(int bins, int bn_ref, double dr,
     const double h2 = __dmul_rn(h, 0.5);
     const double ri = __dmul_rn((double)i, dr), rj = __dmul_rn((double)j, dr), rk = __dmul_rn((double)k, dr);
     __shared__ double rw[kRefMax], S1[kRefMax + 1], S2[kRefMax + 1];
+    __shared__ double au_s[kRefMax], av_s[kRefMax], A1[kRefMax], B[kRefMax];  // per u: ru + h/2, 1 + A; per v
     __shared__ double red[2][256];
-    for (int w = threadIdx.x; w < bn_ref; w += blockDim.x) rw[w] = __dadd_rn(rk, __dmul_rn((double)w, h));
+    for (int w = threadIdx.x; w < bn_ref; w += blockDim.x) {
+        rw[w] = __dadd_rn(rk, __dmul_rn((double)w, h));
+        S1[w + 1] = __dadd_rn(rw[w], h2);
+        S2[w + 1] = __ddiv_rn(ffr[(long long)k * bn_ref + w], 3.0);
+        const double au = __dadd_rn(__dadd_rn(ri, __dmul_rn((double)w, h)), h2);
+        const double av = __dadd_rn(__dadd_rn(rj, __dmul_rn((double)w, h)), h2);
+        au_s[w] = au;
+        av_s[w] = av;
+        A1[w] = 1.0 + __ddiv_rn(ffr[(long long)i * bn_ref + w], __dmul_rn(3.0, au));
+        B[w] = __ddiv_rn(ffr[(long long)j * bn_ref + w], __dmul_rn(3.0, av));
+    }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double a = 0.0, b = 0.0;
-        S1[0] = 0.0;
-        S2[0] = 0.0;
-        for (int w = 0; w < bn_ref; ++w) {
-            a += __dadd_rn(rw[w], h2);
-            b += __ddiv_rn(ffr[(long long)k * bn_ref + w], 3.0);
-            S1[w + 1] = a;
-            S2[w + 1] = b;
-        }
+    if (threadIdx.x == 0 || threadIdx.x == 32) {  // prefix sums, in order
+        double *S = threadIdx.x ? S2 : S1, x = 0.0;
+        S[0] = 0.0;
+        for (int w = 1; w <= bn_ref; ++w) S[w] = x += S[w];
     }
     __syncthreads();
     double accS = 0.0, accF = 0.0;
     const int nuv = bn_ref * bn_ref;
-    for (int uv = threadIdx.x; uv < nuv; uv += blockDim.x) {
-        const int u = uv / bn_ref, v = uv % bn_ref;
+    const double inv = 1.0 / h;
+    int u = threadIdx.x / bn_ref, v = threadIdx.x % bn_ref;
+    const int du = blockDim.x / bn_ref, dv = blockDim.x % bn_ref;
+    for (int uv = threadIdx.x; uv < nuv; uv += blockDim.x, u += du, v += dv) {
+        if (v >= bn_ref) {
+            v -= bn_ref;
+            ++u;
+        }
         const double ru = __dadd_rn(ri, __dmul_rn((double)u, h));
         const double rv = __dadd_rn(rj, __dmul_rn((double)v, h));
         const double ruh = __dadd_rn(ru, h), rvh = __dadd_rn(rv, h);
@@ -178,29 +193,19 @@ __global__ void __launch_bounds__(256) k_refine(int bins, int bn_ref, double dr,
         // rv + rw >= ru + h (increasing in w)
         auto D = [&](int w) { return suv >= __dadd_rn(rw[w], h); };
         auto U = [&](int w) { return __dadd_rn(ru, rw[w]) >= rvh && __dadd_rn(rv, rw[w]) >= ruh; };
-        // largest w with D(w)
-        int lo = 0, hi = bn_ref;  // D true on [0, lo), false on [hi, n)
-        while (lo < hi) {
-            const int m = (lo + hi) >> 1;
-            if (D(m)) lo = m + 1; else hi = m;
-        }
-        const int wend = lo;  // exclusive
-        // smallest w with U(w)
-        lo = 0;
-        hi = bn_ref;
-        while (lo < hi) {
-            const int m = (lo + hi) >> 1;
-            if (U(m)) hi = m; else lo = m + 1;
-        }
-        const int wbeg = lo;
+        // the number of w with D(w) and the smallest with U(w): where the unrounded
+        // sums have them, then moved until the rounded tests agree
+        int wend = (int)fmin(fmax((suv - ruh + ru - rk) * inv + 1.0, 0.0), (double)bn_ref);
+        while (wend < bn_ref && D(wend)) ++wend;
+        while (wend > 0 && !D(wend - 1)) --wend;
+        int wbeg = (int)fmin(fmax((fmax(rvh - ru, ruh - rv) - rk) * inv + 0.5, 0.0), (double)bn_ref);
+        while (wbeg > 0 && U(wbeg - 1)) --wbeg;
+        while (wbeg < bn_ref && !U(wbeg)) ++wbeg;
         if (wbeg >= wend) continue;
-        const double au = __dadd_rn(ru, h2), av = __dadd_rn(rv, h2);
-        const double cuv = __dmul_rn(au, av);
+        const double cuv = __dmul_rn(au_s[u], av_s[v]);
         const double s1 = S1[wend] - S1[wbeg], s2 = S2[wend] - S2[wbeg];
-        const double A = __ddiv_rn(ffr[(long long)i * bn_ref + u], __dmul_rn(3.0, au));
-        const double B = __ddiv_rn(ffr[(long long)j * bn_ref + v], __dmul_rn(3.0, av));
         accS += cuv * s1;
-        accF += cuv * ((1.0 + A + B) * s1 + s2);
+        accF += cuv * ((A1[u] + B[v]) * s1 + s2);
     }
     red[0][threadIdx.x] = accS;
     red[1][threadIdx.x] = accF;
@@ -215,6 +220,98 @@ __global__ void __launch_bounds__(256) k_refine(int bins, int bn_ref, double dr,
     if (threadIdx.x == 0 && red[0][0] != 0.0) {
         rrr[t] += red[0][0] * alpha_ref;
         ddr[t] += red[1][0] * alpha_ref;
+    }
+}
+
+// Fine DD histograms (DD2iso_forBPC): each unordered pair's distance by the
+// canonical FP64 rule, at two bin scales, the second's bins behind the first's.
+// At hundreds of thousands of bins every FP32 distance lies in a window, so there
+// is no fast path beyond a test against dmax; a warp takes a home point and walks
+// its stencil's rows, the candidates behind it in cell order.  Two launches of the
+// general pair kernel, which sent each pair to its recheck, took 395 us for 10007
+// points (dmax 60 of 250, 2000 and 400000 bins); this takes 173.
+struct FineArgs {
+    const float *x, *y, *z, *w;
+    const int *cstart;
+    const RowDesc *rows;
+    int n, n_rows, P;
+    float cell, box, hi;
+    PairRule r1, r2;
+    unsigned long long *cnt;
+    double *wsum;
+    unsigned long long *counter;
+    const unsigned *ctrl;
+    unsigned *status;
+};
+template <bool WEIGHTED>
+__global__ void __launch_bounds__(256) k_fine_dd(const FineArgs A) {
+    const int lane = threadIdx.x & 31, P = A.P;
+    for (;;) {
+        long long t = 0;
+        if (lane == 0) t = (long long)atomicAdd(A.counter, 1ull);
+        const long long i = __shfl_sync(0xffffffffu, t, 0);
+        if (i >= A.n) break;
+        if (A.ctrl && ctrl_load(A.ctrl)) {
+            if (A.status && lane == 0) ctrl_store(A.status, PCF_GAVE_UP_ABORT);
+            break;
+        }
+        const float hx = A.x[i], hy = A.y[i], hz = A.z[i];
+        const double hw = WEIGHTED ? (double)A.w[i] : 1.0;
+        const int cix = min(max((int)__fdiv_rn(hx, A.cell), 0), P - 1);
+        const int ciy = min(max((int)__fdiv_rn(hy, A.cell), 0), P - 1);
+        const int ciz = min(max((int)__fdiv_rn(hz, A.cell), 0), P - 1);
+        for (int r0 = 0; r0 < 2 * A.n_rows; r0 += 32) {
+            // one range of cells per lane: a row, or the part of it past a z face
+            const int r = r0 + lane;
+            int a = 0, len = 0;
+            float sx = 0.f, sy = 0.f, sz = 0.f;
+            if (r < 2 * A.n_rows) {
+                const RowDesc rw = A.rows[r >> 1];
+                int nx = cix + rw.dx, ny = ciy + rw.dy;
+                if (nx < 0) { nx += P; sx = -A.box; } else if (nx >= P) { nx -= P; sx = A.box; }
+                if (ny < 0) { ny += P; sy = -A.box; } else if (ny >= P) { ny -= P; sy = A.box; }
+                int zlo = ciz - rw.kz, zhi = ciz + rw.kz;
+                bool ok = true;
+                if (r & 1) {
+                    ok = zlo < 0 || zhi >= P;
+                    if (zlo < 0) { sz = -A.box; zlo += P; zhi = P - 1; } else { sz = A.box; zlo = 0; zhi -= P; }
+                } else {
+                    zlo = max(zlo, 0);
+                    zhi = min(zhi, P - 1);
+                }
+                if (ok) {
+                    const int *cs = A.cstart + (long long)(nx * P + ny) * P;
+                    a = max(cs[zlo], (int)i + 1);
+                    len = max(cs[zhi + 1] - a, 0);
+                }
+            }
+            for (unsigned m = __ballot_sync(0xffffffffu, len > 0); m; m &= m - 1u) {
+                const int q = __ffs(m) - 1;
+                const int a0 = __shfl_sync(0xffffffffu, a, q), n0 = __shfl_sync(0xffffffffu, len, q);
+                const float tx = __shfl_sync(0xffffffffu, sx, q), ty = __shfl_sync(0xffffffffu, sy, q),
+                            tz = __shfl_sync(0xffffffffu, sz, q);
+                for (int c = a0 + lane; c < a0 + n0; c += 32) {
+                    const float px = A.x[c], py = A.y[c], pz = A.z[c];
+                    const float vx = px + tx - hx, vy = py + ty - hy, vz = pz + tz - hz;
+                    if (!(vx * vx + vy * vy + vz * vz < A.hi)) continue;
+                    double dx, dy, dz;
+                    exact_sep(hx, hy, hz, px, py, pz, tx, ty, tz, dx, dy, dz);
+                    const double d2 = exact_d2(dx, dy, dz);
+                    if (!rule_in(d2, A.r1)) continue;
+                    const double d = __dsqrt_rn(d2);
+                    const int b1 = (int)__dmul_rn(d, A.r1.ds), b2 = (int)__dmul_rn(d, A.r2.ds);
+                    const double w = WEIGHTED ? hw * (double)A.w[c] : 1.0;
+                    if (b1 < A.r1.bins) {
+                        if (WEIGHTED) atomicAdd(A.wsum + b1, w);
+                        else atomicAdd(A.cnt + b1, 1ull);
+                    }
+                    if (b2 < A.r2.bins) {
+                        if (WEIGHTED) atomicAdd(A.wsum + A.r1.bins + b2, w);
+                        else atomicAdd(A.cnt + A.r1.bins + b2, 1ull);
+                    }
+                }
+            }
+        }
     }
 }
 
@@ -258,6 +355,7 @@ extern "C" pcf_status pcf_analytic_3iso(pcf_ctx *ctx, const pcf_grid *d_, int bi
         pcf_status s0 = grid_finish(ctx, d_);
         if (s0 != PCF_OK) return s0;
     }
+    if (ctx_abort_requested(ctx) != PCF_OK) return PCF_ERR_TIMEOUT;
     pcf_grid *D = const_cast<pcf_grid *>(d_);
     const float L = D->box;
     if (!(2.0 * (double)dmax < (double)L)) return PCF_ERR_UNSUPPORTED;
@@ -290,14 +388,51 @@ extern "C" pcf_status pcf_analytic_3iso(pcf_ctx *ctx, const pcf_grid *d_, int bi
     double *d_ddr = ffr + (size_t)bins * bn_ref;
     double *d_rrr = d_ddr + n3;
     unsigned char *partial = reinterpret_cast<unsigned char *>(d_rrr + n3);
-    for (int pass = 0; pass < 2; ++pass) {
-        const int64_t nbf = pass ? bn_ffr : bn_ff;
-        const float dsf = (float)nbf / dmax;
-        pcf_stats st{};
-        s = pcf_count_pairs_ds(ctx, D, (int)nbf, dmax, (double)dsf, PCF_BPC | PCF_DEVICE_OUT,
-                               pass ? dd_ffr : dd_ff, stats ? &st : nullptr);  // statistics make a call wait
+    {
+        int P = 0;
+        s = prepare_grids(ctx, D, nullptr, dmax, kTripletCells, true, &P, 0);
         if (s != PCF_OK) return s;
-        kernel_ms += st.kernel_ms;
+        const CellGrid &g = *D->cells;
+        PairPlan plan;
+        plan_pairs(g, L, dmax, false, false, plan, ctx->sm_count * 24);
+        PlanSlot *sl = nullptr;
+        s = stage_plan(ctx, plan, &sl);
+        if (s != PCF_OK) return s;
+        FineArgs A;
+        A.x = g.x();
+        A.y = g.y();
+        A.z = g.z();
+        A.w = g.w();
+        A.cstart = g.cell_start.as<int>();
+        A.rows = sl->rows();
+        A.n = (int)np;
+        A.n_rows = (int)plan.rows.size();
+        A.P = P;
+        A.cell = g.cell;
+        A.box = L;
+        A.r1 = make_pair_rule((int)bn_ff, dmax, PCF_BPC, false, true, false);
+        A.r2 = make_pair_rule((int)bn_ffr, dmax, PCF_BPC, false, true, false);
+        A.r1.ds = (double)((float)bn_ff / dmax);
+        A.r2.ds = (double)((float)bn_ffr / dmax);
+        const double reach = std::sqrt(A.r1.dd) + 4e-6 * (double)L;  // above any FP32 distance in range
+        A.hi = (float)(reach * reach * (1.0 + 1e-5));
+        const bool weighted = !D->unit_weights;
+        const size_t nb = (size_t)(bn_ff + bn_ffr);
+        PCF_CU(ctx, ctx->d_hist.ensure(sizeof(double) * nb));
+        A.cnt = ctx->d_hist.as<unsigned long long>();
+        A.wsum = ctx->d_hist.as<double>();
+        A.counter = sl->counter();
+        A.ctrl = ctx->d_abort;
+        A.status = ctx->d_status;
+        PCF_CU(ctx, cudaMemsetAsync(A.cnt, 0, sizeof(double) * nb, ctx->stream));
+        if (stats) PCF_CU(ctx, cudaEventRecord(ctx->ev0, ctx->stream));
+        (weighted ? k_fine_dd<true> : k_fine_dd<false>)<<<ctx->sm_count * 6, 256, 0, ctx->stream>>>(A);
+        PCF_CU(ctx, cudaGetLastError());
+        if (stats) PCF_CU(ctx, cudaEventRecord(ctx->ev1, ctx->stream));
+        PCF_CU(ctx, cudaEventRecord(sl->done, ctx->stream));
+        ++ctx->launches;
+        s = finalize_hist(ctx, A.cnt, A.wsum, weighted, 2.0, (int)nb, dd_ff, nullptr, nullptr);  // ordered pairs
+        if (s != PCF_OK) return s;
     }
     // analytic RR at the fine binnings (RR2iso_BPC_analytic with alpha_ff*)
     const double alpha_ff = rr_alpha(np, L, dmax, bn_ff);
@@ -328,6 +463,9 @@ extern "C" pcf_status pcf_analytic_3iso(pcf_ctx *ctx, const pcf_grid *d_, int bi
     memcpy(ddr, hb, sizeof(double) * n3);
     memcpy(rrr, hb + sizeof(double) * n3, sizeof(double) * n3);
     if (stats) {
+        float ms = 0.f;
+        cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
+        kernel_ms += ms;
         stats->kernel_ms = kernel_ms;
         stats->partitions = D->cells ? D->cells->P : 0;
     }

@@ -448,16 +448,14 @@ static PairLaunch pair_launch(pcf_ctx *ctx, const pcf_grid *a, const pcf_grid *b
     return pl;
 }
 
-// One pair histogram; ds_override > 0 replaces the bin scale (the fine
-// histograms of the analytic path use (float)bins / dmax).
+// One pair histogram.
 static pcf_status count_pairs_impl(pcf_ctx *ctx, int kind, const pcf_grid *a_, const pcf_grid *b_,
                                    int bins, float dmax, uint32_t flags, double *hist,
-                                   pcf_stats *stats, double ds_override) {
+                                   pcf_stats *stats) {
     if (!ctx || !a_ || !hist || bins < 1 || !(dmax > 0.f) ||
         (kind != PCF_ISO && kind != PCF_ANI && kind != PCF_BOTH))
         return PCF_ERR_INVALID_ARG;
     if (kind != PCF_ISO && (int64_t)bins * bins > (1 << 24)) return PCF_ERR_UNSUPPORTED;
-    if (kind == PCF_BOTH && ds_override > 0) return PCF_ERR_INVALID_ARG;
     if (ctx_abort_requested(ctx) != PCF_OK) return PCF_ERR_TIMEOUT;
     {
         pcf_status s0 = grid_finish(ctx, a_);
@@ -497,10 +495,10 @@ static pcf_status count_pairs_impl(pcf_ctx *ctx, int kind, const pcf_grid *a_, c
     if (both && !one_pass) {
         pcf_stats si{}, sa{};
         pcf_status s = count_pairs_impl(ctx, PCF_ISO, a_, b_, bins, dmax, flags, hist,
-                                        stats ? &si : nullptr, 0.0);
+                                        stats ? &si : nullptr);
         if (s == PCF_OK)
             s = count_pairs_impl(ctx, PCF_ANI, a_, b_, bins, dmax, flags, hist + bins,
-                                 stats ? &sa : nullptr, 0.0);
+                                 stats ? &sa : nullptr);
         if (s == PCF_OK && stats) {
             stats->pairs = si.pairs + sa.pairs;
             stats->candidates = si.candidates + sa.candidates;
@@ -528,7 +526,6 @@ static pcf_status count_pairs_impl(pcf_ctx *ctx, int kind, const pcf_grid *a_, c
     if (s != PCF_OK) return s;
     PairLaunch pl = pair_launch(ctx, a, b, kind, bins, dmax, flags, weighted);
     pl.hist_mode = te.hist_mode;
-    if (ds_override > 0) pl.rule.ds = ds_override;
     pl.count = stats != nullptr && !ctx->tune_timing;
     pl.timed = stats != nullptr;
     pl.tile_cap = tile_cap;
@@ -572,10 +569,6 @@ static pcf_status count_pairs_impl(pcf_ctx *ctx, int kind, const pcf_grid *a_, c
 extern "C" pcf_status pcf_count_pairs(pcf_ctx *ctx, int kind, const pcf_grid *a, const pcf_grid *b,
                                       int bins, float dmax, uint32_t flags, double *hist,
                                       pcf_stats *stats) {
-    return count_pairs_impl(ctx, kind, a, b, bins, dmax, flags, hist, stats, 0.0);
+    return count_pairs_impl(ctx, kind, a, b, bins, dmax, flags, hist, stats);
 }
 
-pcf_status pcf_count_pairs_ds(pcf_ctx *ctx, const pcf_grid *a, int bins, float dmax, double ds,
-                              uint32_t flags, double *hist, pcf_stats *stats) {
-    return count_pairs_impl(ctx, PCF_ISO, a, nullptr, bins, dmax, flags, hist, stats, ds);
-}
