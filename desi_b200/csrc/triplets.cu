@@ -919,7 +919,10 @@ __global__ void __launch_bounds__(kTThreads, 1) k_triplets_batch(const __grid_co
 // triples anchored at point 1 = the anchor i; the lists hold every X (and
 // for XXY every Y) neighbour with its exact side bin and angle bin, and all
 // ordered (j, k), j != k, are counted into the bins^5 histogram
-// [b(d12)][b(d31)][b(d23)][t12][t31] in global memory.
+// [b(d12)][b(d31)][b(d23)][t12][t31] in global memory.  XXX without gates, where
+// (k, j) counts what (j, k) does with points 2 and 3 exchanged: j < k alone, and
+// k_to_double adds the exchanged bin (3000 points, 12 bins, dmax 60: 844 us for
+// DDD and RRR -> 507).
 // GATES (periodic, PCF_REF_NODE_GATES): each ordered triangle counts as many
 // times as the reference's node-gate blocks count it (node_gates.cuh), on the
 // reference's node grid A.gate.  ISO3 (with GATES): the isotropic bins^3
@@ -955,6 +958,7 @@ __global__ void __launch_bounds__(NW * 32, kTWarps / NW) k_triplets_ani(const Tr
     unsigned long long n_tri = 0;
     long long taken = 0;
     const long long B = bins, B2 = B * B, B3 = B2 * B, B4 = B3 * B;
+    constexpr bool HALF = !MIXED && !GATES;
     for (;;) {
         if (tid == 0) {
             s_anchor = (int)atomicAdd(A.counter, 1ull);
@@ -990,7 +994,9 @@ __global__ void __launch_bounds__(NW * 32, kTWarps / NW) k_triplets_ani(const Tr
         const float4 *LK = MIXED ? sK : sJ;
         const unsigned char *AK = MIXED ? aK : aJ;
         const float *WK = MIXED ? swK : swJ;
-        for (int jj = warp; jj < nJ; jj += NW) {
+        for (int rr = warp; rr < nJ; rr += NW) {
+            // HALF: rows in the order 0, n-1, 1, n-2, ... (they shrink with j)
+            const int jj = !HALF ? rr : (rr & 1) ? nJ - 1 - (rr >> 1) : rr >> 1;
             const float4 ej = sJ[jj];
             const int jidx = (int)((unsigned)__float_as_int(ej.w) >> 8);
             const int bj = __float_as_int(ej.w) & 255;
@@ -999,7 +1005,7 @@ __global__ void __launch_bounds__(NW * 32, kTWarps / NW) k_triplets_ani(const Tr
             GateNode n2{};
             if (GATES) n2 = gate_unpack(A.gate, gJ[jj]);
             const unsigned *GK = MIXED ? gK : gJ;
-            for (int kk = lane; kk < nK; kk += 32) {
+            for (int kk = (HALF ? jj + 1 : 0) + lane; kk < nK; kk += 32) {
                 if (!MIXED && kk == jj) continue;
                 const float4 ek = LK[kk];
                 const float dx = ek.x - ej.x, dy = ek.y - ej.y, dz = ek.z - ej.z;
@@ -1167,12 +1173,23 @@ __global__ void __launch_bounds__(NW * 32, kTWarps / NW) k_gate_fix(const __grid
     }
 }
 
+// bins5 > 0: the histogram [b12][b31][b23][t12][t31] holds half the ordered
+// triangles; the others are in the bin with points 2 and 3 exchanged.
 __global__ void k_to_double(const unsigned long long *__restrict__ c, const double *__restrict__ w,
                             int weighted, long long n, double *__restrict__ out,
-                            const unsigned long long *__restrict__ stats, unsigned long long *host_stats) {
+                            const unsigned long long *__restrict__ stats, unsigned long long *host_stats, int bins5) {
     long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t < 4) host_stats[t] = stats[t];
-    if (t < n) out[t] = weighted ? w[t] : (double)c[t];
+    if (t >= n) return;
+    long long u = t;
+    if (bins5) {
+        const long long B = bins5, B2 = B * B;
+        const long long t31 = t % B, t12 = t / B % B, b23 = t / B2 % B, b31 = t / (B2 * B) % B, b12 = t / (B2 * B2);
+        u = ((((b31 * B) + b12) * B + b23) * B + t31) * B + t12;
+        out[t] = weighted ? w[t] + w[u] : (double)(c[t] + c[u]);
+        return;
+    }
+    out[t] = weighted ? w[t] : (double)c[t];
 }
 
 // fix: the node gates' corrections of an unweighted count.
@@ -1850,12 +1867,12 @@ static pcf_status count_triplets_ordered(pcf_ctx *ctx, const pcf_grid *x_, const
     PCF_CU(ctx, cudaGetLastError());
     PCF_CU(ctx, cudaEventRecord(ctx->ev1, ctx->stream));
     PCF_CU(ctx, cudaEventRecord(sl->done, ctx->stream));
-    const bool dev_out = (flags & PCF_DEVICE_OUT) != 0;
+    const bool dev_out = (flags & PCF_DEVICE_OUT) != 0, half = !mixed && !gates;
     OutPath o;
     s = out_open(ctx, n5, dev_out, hist, d_out, &o);
     if (s != PCF_OK) return s;
     k_to_double<<<(unsigned)((n5 + 255) / 256), 256, 0, ctx->stream>>>(A.g_count, A.g_wsum, weighted ? 1 : 0, n5, o.to,
-                                                                       A.g_stats, o.stats);
+                                                                       A.g_stats, o.stats, half ? bins : 0);
     PCF_CU(ctx, cudaGetLastError());
     ctx->launches += 2;
     unsigned long long hs[4];
@@ -1868,7 +1885,7 @@ static pcf_status count_triplets_ordered(pcf_ctx *ctx, const pcf_grid *x_, const
     if (stats) {
         float ms = 0.f;
         cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
-        stats->pairs = (double)hs[2];
+        stats->pairs = (double)hs[2] * (half ? 2 : 1);  // ordered triangles
         stats->rechecks = (double)hs[0];
         stats->candidates = 0;
         stats->kernel_ms = ms;
