@@ -372,7 +372,8 @@ __host__ __device__ __forceinline__ int u_words(int bins) { return bins * bins *
 // b_jk, which the final sums take together.  FP64 adds in global memory queued in
 // L2; FP64 adds to shared memory, loops of compare-and-swaps, lay between (us, XXX
 // clustered, XXX, XXY of 4100 points, 25 bins, dmax 70: 633 424 1316, 557 342 786, and
-// 377 310 682 by limbs; 8000 points 3790 2987 8535, 3222 1861 4779, 2111 1618 3980).
+// 377 310 682 by limbs; 8000 points 3790 2987 8535, 3222 1861 4779, 2111 1618 3980;
+// with XXX rows by ticket since, 309 260 683 and 1587 1237 3978).
 __host__ __device__ __forceinline__ int w_slots(int bins) { return bins * (bins * (bins + 1) / 2); }
 __device__ __forceinline__ int w_slot(int bins, int bij, int bki, int bjk) {
     const int lo = min(bki, bjk), hi = max(bki, bjk);
@@ -732,10 +733,16 @@ __device__ __forceinline__ void tri_anchor(const TripArgs &A, int i, TripCta<NW>
     }
     auto weight = [&](float w) { return A.wfix ? (double)__float_as_uint(w) : (double)w; };
     const int nw = WEIGHTED ? w_slots(bins) : 0;
-    // rows j dealt to warps in the order 0, n-1, 1, n-2, ... (XXX rows shrink with j)
-    for (int rr = warp; rr < nJ; rr += NW) {
-        const int half = rr >> 1;
-        const int jj = MIXED ? rr : ((rr & 1) ? nJ - 1 - half : half);
+    // XXX, whose rows shrink with j: rows by ticket, the longest first.  Dealt out
+    // beforehand (0, n-1, 1, n-2, ...) the warps waited for one another a third of
+    // their time (4100 points, dmax 70, 25 bins, weighted: 377 and 310 -> 320 and
+    // 260 us).  XXY rows are of one length.
+    for (int jj = warp;; jj += NW) {
+        if (!MIXED) {
+            if (lane == 0) jj = atomicAdd(C.s_unit, 1);
+            jj = __shfl_sync(kFull, jj, 0);
+        }
+        if (jj >= nJ) break;
         const float4 ej = LJ[jj];
         const int bj = __float_as_int(ej.w) & 255;
         const int jidx = (int)((unsigned)__float_as_int(ej.w) >> 8);
@@ -922,7 +929,7 @@ __global__ void __launch_bounds__(kTThreads, 1) k_triplets_batch(const __grid_co
 // [b(d12)][b(d31)][b(d23)][t12][t31] in global memory.  XXX without gates, where
 // (k, j) counts what (j, k) does with points 2 and 3 exchanged: j < k alone, and
 // k_to_double adds the exchanged bin (3000 points, 12 bins, dmax 60: 844 us for
-// DDD and RRR -> 507).
+// DDD and RRR -> 507, with rows by ticket 483).
 // GATES (periodic, PCF_REF_NODE_GATES): each ordered triangle counts as many
 // times as the reference's node-gate blocks count it (node_gates.cuh), on the
 // reference's node grid A.gate.  ISO3 (with GATES): the isotropic bins^3
@@ -942,7 +949,7 @@ __global__ void __launch_bounds__(NW * 32, kTWarps / NW) k_triplets_ani(const Tr
     unsigned char *aJ = reinterpret_cast<unsigned char *>(gK + (GATES && MIXED ? A.capK : 0));
     unsigned char *aK = aJ + A.capJ;
     __shared__ ListScratch<NW> s_scr;
-    __shared__ int s_anchor;
+    __shared__ int s_anchor, s_unit;
     __shared__ unsigned s_stop;
     __shared__ GateBlock s_gates[GATES ? 64 : 1];
     __shared__ signed char s_gate_by[GATES ? 64 : 1][2];
@@ -962,6 +969,7 @@ __global__ void __launch_bounds__(NW * 32, kTWarps / NW) k_triplets_ani(const Tr
     for (;;) {
         if (tid == 0) {
             s_anchor = (int)atomicAdd(A.counter, 1ull);
+            s_unit = 0;
             unsigned stop = (A.ctrl && ctrl_load(A.ctrl)) ? PCF_GAVE_UP_ABORT : 0u;
             if (++taken > (long long)A.nX + 1) stop |= PCF_GAVE_UP_CAP;
             if (stop && A.status) ctrl_store(A.status, stop);
@@ -994,9 +1002,12 @@ __global__ void __launch_bounds__(NW * 32, kTWarps / NW) k_triplets_ani(const Tr
         const float4 *LK = MIXED ? sK : sJ;
         const unsigned char *AK = MIXED ? aK : aJ;
         const float *WK = MIXED ? swK : swJ;
-        for (int rr = warp; rr < nJ; rr += NW) {
-            // HALF: rows in the order 0, n-1, 1, n-2, ... (they shrink with j)
-            const int jj = !HALF ? rr : (rr & 1) ? nJ - 1 - (rr >> 1) : rr >> 1;
+        for (int jj = warp;; jj += NW) {
+            if (HALF) {  // rows shrink with j: by ticket, the longest first
+                if (lane == 0) jj = atomicAdd(&s_unit, 1);
+                jj = __shfl_sync(0xffffffffu, jj, 0);
+            }
+            if (jj >= nJ) break;
             const float4 ej = sJ[jj];
             const int jidx = (int)((unsigned)__float_as_int(ej.w) >> 8);
             const int bj = __float_as_int(ej.w) & 255;
