@@ -157,12 +157,9 @@ def tune_step(ctx, D, R, candidates=(8, 9, 10, 11, 12, 13, 14, 16)):
         gd.free()
         gr.free()
     # the tuning table keeps the last candidate's schemes: tune again at the
-    # winner.  A both-kinds call tuned to the default rule (-1) runs the two
-    # single-kind launches, so it needs their entries too; if every one of
-    # the three chose that, the step is the single-kind form.
+    # winner (the default rule, -1, of a both-kinds call of this workload's
+    # exact weights is one pass too)
     _, P, fused, modes = best
-    if fused and all(m < 0 for m in modes.values()):
-        fused = False
     gd, gr = ctx.grid(D, W["box"], partitions=P), ctx.grid(R, W["box"], partitions=P)
     modes = {}
     for ani in ((False, True, "both") if fused else (False, True)):
@@ -253,10 +250,7 @@ def run_ours(args, rank, world, local_rank):
         ctx.set_option(api.PCF_OPT_GRID_DEFER, 1)
     P, fused, tuned = tune_step(ctx, D, R)
     kinds = ("both",) if fused else (False, True)
-    # a both-kinds call tuned to the library's default rule (-1) runs as two
-    # single-kind launches when the isotropic histogram alone gets
-    # lane-private copies (this workload's 30 exact-weight bins)
-    one_pass = [k[:2] for k, m in tuned.items() if k.endswith("both") and m >= 0]
+    one_pass = [k[:2] for k in tuned if k.endswith("both")]
     Dt = torch.from_numpy(D).to(dev)
     Rt = torch.from_numpy(R).to(dev)
     outs = torch.zeros((6, W["bins"] + W["bins"] * W["bins"]), dtype=torch.float64, device=dev)
