@@ -247,7 +247,8 @@ class Context:
                                        float(dmax), f,
                                        dd.ctypes.data_as(ctypes.c_void_p) if dd is not None else None,
                                        rr.ctypes.data_as(ctypes.c_void_p),
-                                       dr.ctypes.data_as(ctypes.c_void_p), ctypes.byref(st))
+                                       dr.ctypes.data_as(ctypes.c_void_p),
+                                       ctypes.byref(st) if stats else None)
         _check(self.handle, rc, "pcf_batch_pairs")
         if both:
             rr, dr = rr.reshape(nr, nb), dr.reshape(nr, nb)
@@ -275,7 +276,7 @@ class Context:
         p = lambda x: x.ctypes.data_as(ctypes.c_void_p)  # noqa: E731
         rc = self._lib.pcf_batch_triplets(self.handle, d.handle, ctypes.cast(arr, ctypes.c_void_p),
                                           nr, int(bins), float(dmax), f, p(ddd), p(rrr), p(ddr),
-                                          p(drr), ctypes.byref(st))
+                                          p(drr), ctypes.byref(st) if stats else None)
         _check(self.handle, rc, "pcf_batch_triplets")
         shp = (nr, bins, bins, bins)
         res = (ddd.reshape(bins, bins, bins), rrr[:nr * n3].reshape(shp), ddr[:nr * n3].reshape(shp),

@@ -148,7 +148,7 @@ extern "C" pcf_status pcf_batch_pairs(pcf_ctx *ctx, int kind, const pcf_grid *d_
     if (use_graph) {
         std::ostringstream os;
         os << kind << ':' << bins << ':' << dmax << ':' << (flags & ~PCF_GRAPH) << ':' << (dd != nullptr)
-           << (rr != nullptr) << (dr != nullptr);
+           << (rr != nullptr) << (dr != nullptr) << (stats != nullptr);
         for (auto &j : js) os << ',' << j.hc->serial << '/' << j.cc->serial;
         key = os.str();
     }
@@ -165,6 +165,7 @@ extern "C" pcf_status pcf_batch_pairs(pcf_ctx *ctx, int kind, const pcf_grid *d_
     pl.weighted = weighted;
     pl.rule = make_pair_rule(bins, dmax, flags, ani, bpc, false);
     pl.mult = 1.0;
+    pl.count = stats != nullptr;
     pl.ctrl = ctx->d_abort;
     pl.status = ctx->d_status;
     {

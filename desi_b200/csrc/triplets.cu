@@ -89,10 +89,7 @@ struct TripArgs {
     unsigned long long flush_budget;
     const unsigned *ctrl;  // abort request, polled with every anchor (null: none)
     unsigned *status;      // where a CTA that gives up records why (null: none)
-    // batched launches (k_triplets_batch): this job's anchors are the
-    // queue's [anchor_begin, anchor_begin + nX); mixed: XXY
-    long long anchor_begin;
-    int mixed;
+    int mixed;  // XXY
     GateGeom gate;  // the reference's node grid (PCF_REF_NODE_GATES)
 };
 
@@ -845,83 +842,6 @@ __global__ void __launch_bounds__(kTThreads, 1) k_triplets(const __grid_constant
     }
 }
 
-// The job table of a batched launch, passed as the kernel's parameter (so
-// job arguments are read from the parameter constant bank, as a single-job
-// launch reads its own; a table in global or shared memory ran the four
-// histograms of the 3iso step 8% slower).
-constexpr int kBatchJobs = 64;
-struct TripBatch {
-    TripArgs job[kBatchJobs];
-    int n_jobs;
-    long long n_anchors;
-    unsigned long long *counter;
-};
-
-// Several isotropic triplet histograms of one kind (XXX, or XXY) in one
-// persistent launch: the jobs' anchors form one queue (job after job); a CTA
-// that crosses into another job flushes its shared histogram into the
-// previous job's histogram.
-template <bool MIXED, bool WEIGHTED>
-__global__ void __launch_bounds__(kTThreads, 1) k_triplets_batch(const __grid_constant__ TripBatch B) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ ListScratch<kTWarps> s_scr;
-    __shared__ ChunkBox s_boxes[kMaxBoxes];
-    __shared__ uint2 s_queue[64 * kTWarps];
-    __shared__ long long s_anchor;
-    __shared__ int s_unit;
-    __shared__ unsigned s_stop;
-    const int tid = threadIdx.x, lane = tid & 31;
-    const TripArgs &J0 = B.job[0];
-    const int bins = J0.rXX.bins;
-    const bool in_smem = J0.hist_in_smem != 0;
-    const size_t u_bytes = in_smem ? hist_bytes(bins, WEIGHTED) : 0;
-    TripCta<kTWarps> C{reinterpret_cast<unsigned *>(smem), smem + u_bytes, &s_scr, s_boxes, s_queue, &s_unit, (int)blockIdx.x, 0u, 0ull, 0ull};
-    if (in_smem)
-        for (int k = tid; k < (int)(u_bytes / 4); k += kTThreads) C.U[k] = 0u;
-    int cur = -1;  // the CTA's current job (uniform: every thread follows s_anchor)
-    long long taken = 0, ticket = 0;  // ticket (thread 0): taken while the last anchor is counted
-    if (tid == 0) ticket = (long long)atomicAdd(B.counter, 1ull);
-    for (;;) {
-        if (tid == 0) {
-            s_anchor = ticket;
-            s_unit = 0;
-            unsigned stop = (J0.ctrl && ctrl_load(J0.ctrl)) ? PCF_GAVE_UP_ABORT : 0u;
-            if (++taken > B.n_anchors + 1) stop |= PCF_GAVE_UP_CAP;
-            if (stop && J0.status) ctrl_store(J0.status, stop);
-            s_stop = stop;
-        }
-        __syncthreads();
-        const long long g = s_anchor;
-        if (g >= B.n_anchors || s_stop) break;
-        if (tid == 0) ticket = (long long)atomicAdd(B.counter, 1ull);
-        // the job of anchor g (a CTA's anchors only move forward in the queue)
-        if (cur < 0 || g >= B.job[cur].anchor_begin + B.job[cur].nX) {
-            int j = cur < 0 ? 0 : cur;
-            while (j + 1 < B.n_jobs && g >= B.job[j + 1].anchor_begin) ++j;
-            if (cur >= 0 && in_smem && C.since) {
-                if (WEIGHTED) flush_limbs<kTWarps>(C.U, bins, B.job[cur].wunscale, B.job[cur].g_wsum);
-                else C.n_tri += flush_hist<kTWarps, false>(C.U, bins, B.job[cur].g_count);
-                C.since = 0;
-            }
-            cur = j;
-        }
-        const TripArgs &A = B.job[cur];
-        tri_anchor<kTWarps, MIXED, WEIGHTED>(A, (int)(g - A.anchor_begin), C);
-        __syncthreads();
-    }
-    if (WEIGHTED && in_smem && cur >= 0) flush_limbs<kTWarps>(C.U, bins, B.job[cur].wunscale, B.job[cur].g_wsum);
-    else if (in_smem && cur >= 0) C.n_tri += flush_hist<kTWarps, false>(C.U, bins, B.job[cur].g_count);
-    unsigned long long rr = C.n_rechk, nt = C.n_tri;
-    for (int off = 16; off > 0; off >>= 1) {
-        rr += __shfl_down_sync(kFull, rr, off);
-        nt += __shfl_down_sync(kFull, nt, off);
-    }
-    if (lane == 0) {
-        if (rr) atomicAdd(J0.g_stats + 0, rr);
-        if (nt) atomicAdd(J0.g_stats + 2, nt);
-    }
-}
-
 // Anisotropic triplets (3ani_k.cuh:8,109; 3aniBPC_k.cuh:210,959): ordered
 // triples anchored at point 1 = the anchor i; the lists hold every X (and
 // for XXY every Y) neighbour with its exact side bin and angle bin, and all
@@ -1381,7 +1301,15 @@ static void trip_setup(pcf_ctx *ctx, const pcf_grid *X, const pcf_grid *Y, int P
     smem = hist_b + (size_t)A.list_bytes * groups;
 }
 
-// Per-CTA overflow lists for lists of up to gcap entries (J, K and weights).
+static void (*trip_kernel(bool mixed, bool weighted, bool several))(const TripArgs) {
+    if (several)
+        return mixed ? (weighted ? k_triplets<true, true, kGroupWarps> : k_triplets<true, false, kGroupWarps>)
+                     : (weighted ? k_triplets<false, true, kGroupWarps> : k_triplets<false, false, kGroupWarps>);
+    return mixed ? (weighted ? k_triplets<true, true, kTWarps> : k_triplets<true, false, kTWarps>)
+                 : (weighted ? k_triplets<false, true, kTWarps> : k_triplets<false, false, kTWarps>);
+}
+
+// Per-group overflow lists for lists of up to gcap entries (J, K and weights).
 static pcf_status trip_overflow(pcf_ctx *ctx, int64_t gmax, bool mixed, bool weighted, int grid,
                                 TripArgs &A) {
     A.gcap = (int)std::min<int64_t>(gmax, 1 << 24);
@@ -1516,11 +1444,7 @@ extern "C" pcf_status pcf_count_triplets(pcf_ctx *ctx, int kind, const pcf_grid 
     // unweighted: the sums' place holds the gates' corrections
     unsigned long long *fix = gates ? reinterpret_cast<unsigned long long *>(A.g_wsum) : nullptr;
 
-    auto pick = [&](auto one, auto several) { return groups > 1 ? several : one; };
-    auto kfn = mixed ? (weighted ? pick(k_triplets<true, true, kTWarps>, k_triplets<true, true, kGroupWarps>)
-                                 : pick(k_triplets<true, false, kTWarps>, k_triplets<true, false, kGroupWarps>))
-                     : (weighted ? pick(k_triplets<false, true, kTWarps>, k_triplets<false, true, kGroupWarps>)
-                                 : pick(k_triplets<false, false, kTWarps>, k_triplets<false, false, kGroupWarps>));
+    const auto kfn = trip_kernel(mixed, weighted, groups > 1);
     PCF_CU(ctx, ensure_smem_limit(reinterpret_cast<const void *>(kfn), ctx->device, smem));
     cudaEvent_t pe0 = nullptr, pe1 = nullptr;
     if (ctx->profile) {
@@ -1578,9 +1502,12 @@ extern "C" pcf_status pcf_count_triplets(pcf_ctx *ctx, int kind, const pcf_grid 
 }
 
 // One data catalog against n_rand random catalogs: DDD once, RRR_i, DDR_i
-// and DRR_i per random catalog, as the jobs of two persistent launches
-// (k_triplets_batch: the XXX jobs, then the XXY jobs).  All grids take one partition count (the one a call
-// on the largest catalog would use; results do not depend on it).
+// and DRR_i per random catalog: their kernels queued one behind the other, one
+// wait for all.  All grids take one partition count (the one a call on the largest
+// catalog would use; results do not depend on it).  (All jobs' anchors as one queue
+// of a persistent launch saved the tails between kernels, but a CTA's groups of
+// warps had to stay in one job: 32768 points against 8 randoms of 4k to 32k, dmax 40 of
+// 250, 20 bins 84.6 ms; 53.7 so.)
 extern "C" pcf_status pcf_batch_triplets(pcf_ctx *ctx, const pcf_grid *d_, const pcf_grid *const *r_,
                                          int n_rand, int bins, float dmax, uint32_t flags, double *ddd,
                                          double *rrr, double *ddr, double *drr, pcf_stats *stats) {
@@ -1639,9 +1566,11 @@ extern "C" pcf_status pcf_batch_triplets(pcf_ctx *ctx, const pcf_grid *d_, const
     }
     const int nj = (int)jobs.size();
     std::vector<TripArgs> args((size_t)nj);
-    size_t smem = 0;
     long long anchors = 0;
     bool any_mixed = false;
+    int n_of[2] = {0, 0}, most = 1;
+    std::vector<size_t> smem((size_t)nj);
+    std::vector<int> groups((size_t)nj);
     int64_t gmax = 0;
     // rows + counters through the plan slot
     PlanSlot *sl = nullptr;
@@ -1660,28 +1589,30 @@ extern "C" pcf_status pcf_batch_triplets(pcf_ctx *ctx, const pcf_grid *d_, const
         gmax = std::max(gmax, b);
     }
     for (int k = 0; k < nj; ++k) {
-        size_t sm = 0;
+        groups[k] = trip_groups(jobs[k].x, jobs[k].y, bins, dmax, weighted);
         trip_setup(ctx, jobs[k].x, jobs[k].y, P, (int)plan.rows.size(), bins, dmax, flags, weighted,
-                   args[k], sm);
-        smem = std::max(smem, sm);
-        args[k].anchor_begin = anchors;
+                   args[k], smem[k], groups[k]);
+        ++n_of[jobs[k].y ? 1 : 0];
+        most = std::max(most, groups[k]);
         anchors += jobs[k].x->n;
         any_mixed = any_mixed || jobs[k].y;
     }
     const int grid = ctx->sm_count;
     TripArgs ov;
-    s = trip_overflow(ctx, gmax + 32, any_mixed, weighted, grid, ov);
+    s = trip_overflow(ctx, gmax + 32, any_mixed, weighted, grid * most, ov);
     if (s != PCF_OK) return s;
+    if ((n_of[0] + 63) / 64 + (n_of[1] + 63) / 64 > 8) return PCF_ERR_UNSUPPORTED;
 
-    // histograms per job
-    const size_t nh = (size_t)nj * n3;
-    PCF_CU(ctx, ctx->d_hist.ensure(nh * 24 + 64));
+    // histograms per job, a counter per job, statistics, results
+    const size_t nh = (size_t)nj * n3, cb = ((size_t)nj * 8 + 63) & ~(size_t)63;
+    PCF_CU(ctx, ctx->d_hist.ensure(nh * 24 + cb + 64));
     char *hp = ctx->d_hist.as<char>();
     unsigned long long *cnt = reinterpret_cast<unsigned long long *>(hp);
     double *wsum = reinterpret_cast<double *>(hp + nh * 8);
-    unsigned long long *gstats = reinterpret_cast<unsigned long long *>(hp + nh * 16);
-    double *d_out = reinterpret_cast<double *>(hp + nh * 16 + 64);
-    PCF_CU(ctx, cudaMemsetAsync(hp, 0, nh * 16 + 64, ctx->stream));
+    unsigned long long *ctr = reinterpret_cast<unsigned long long *>(hp + nh * 16);
+    unsigned long long *gstats = reinterpret_cast<unsigned long long *>(hp + nh * 16 + cb);
+    double *d_out = reinterpret_cast<double *>(hp + nh * 16 + cb + 64);
+    PCF_CU(ctx, cudaMemsetAsync(hp, 0, nh * 16 + cb + 64, ctx->stream));
     for (int k = 0; k < nj; ++k) {
         TripArgs &A = args[k];
         A.gcap = ov.gcap;
@@ -1690,27 +1621,11 @@ extern "C" pcf_status pcf_batch_triplets(pcf_ctx *ctx, const pcf_grid *d_, const
         A.gwJ = ov.gwJ;
         A.gwK = ov.gwK;
         A.rows = sl->rows();
-        A.counter = sl->counter();
+        A.counter = ctr + k;
         A.g_count = cnt + (size_t)k * n3;
         A.g_wsum = wsum + (size_t)k * n3;
         A.g_stats = gstats;
     }
-    // launches per kind (the XXX jobs, then the XXY jobs), each over one
-    // anchor queue of up to kBatchJobs jobs with its own counter
-    std::vector<std::vector<TripArgs>> groups;
-    for (int m = 0; m < 2; ++m) {
-        std::vector<TripArgs> cur;
-        for (int k = 0; k < nj; ++k) {
-            if ((jobs[k].y ? 1 : 0) != m) continue;
-            cur.push_back(args[k]);
-            if ((int)cur.size() == kBatchJobs) {
-                groups.push_back(cur);
-                cur.clear();
-            }
-        }
-        if (!cur.empty()) groups.push_back(cur);
-    }
-    if (groups.size() > 8) return PCF_ERR_UNSUPPORTED;  // counters of the plan slot
     cudaEvent_t pe0 = nullptr, pe1 = nullptr;
     if (ctx->profile) {
         s = profile_events(ctx, &pe0, &pe1);
@@ -1718,24 +1633,10 @@ extern "C" pcf_status pcf_batch_triplets(pcf_ctx *ctx, const pcf_grid *d_, const
         PCF_CU(ctx, cudaEventRecord(pe0, ctx->stream));
     }
     PCF_CU(ctx, cudaEventRecord(ctx->ev0, ctx->stream));
-    unsigned long long *ctr = sl->counter();
-    std::unique_ptr<TripBatch> tb(new TripBatch);
-    for (size_t q = 0; q < groups.size(); ++q) {
-        memset(tb.get(), 0, sizeof(TripBatch));
-        long long a0 = 0;
-        for (size_t k = 0; k < groups[q].size(); ++k) {
-            tb->job[k] = groups[q][k];
-            tb->job[k].anchor_begin = a0;
-            a0 += tb->job[k].nX;
-        }
-        tb->n_jobs = (int)groups[q].size();
-        tb->n_anchors = a0;
-        tb->counter = ctr + q;
-        const bool m = groups[q][0].mixed != 0;
-        auto kfn = m ? (weighted ? k_triplets_batch<true, true> : k_triplets_batch<true, false>)
-                     : (weighted ? k_triplets_batch<false, true> : k_triplets_batch<false, false>);
-        PCF_CU(ctx, ensure_smem_limit(reinterpret_cast<const void *>(kfn), ctx->device, smem));
-        kfn<<<grid, kTThreads, smem, ctx->stream>>>(*tb);
+    for (int k = 0; k < nj; ++k) {
+        const auto kfn = trip_kernel(jobs[k].y != nullptr, weighted, groups[k] > 1);
+        PCF_CU(ctx, ensure_smem_limit(reinterpret_cast<const void *>(kfn), ctx->device, smem[k]));
+        kfn<<<grid, kTThreads, smem[k], ctx->stream>>>(args[k]);
         PCF_CU(ctx, cudaGetLastError());
         ++ctx->launches;
     }
