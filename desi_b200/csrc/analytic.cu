@@ -431,7 +431,7 @@ extern "C" pcf_status pcf_analytic_3iso(pcf_ctx *ctx, const pcf_grid *d_, int bi
         if (stats) PCF_CU(ctx, cudaEventRecord(ctx->ev1, ctx->stream));
         PCF_CU(ctx, cudaEventRecord(sl->done, ctx->stream));
         ++ctx->launches;
-        s = finalize_hist(ctx, A.cnt, A.wsum, weighted, 2.0, (int)nb, dd_ff, nullptr, nullptr);  // ordered pairs
+        s = finalize_hist(ctx, A.cnt, A.wsum, weighted, false, 2.0, (int)nb, dd_ff, nullptr, nullptr);  // ordered pairs
         if (s != PCF_OK) return s;
     }
     // analytic RR at the fine binnings (RR2iso_BPC_analytic with alpha_ff*)

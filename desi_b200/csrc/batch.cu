@@ -173,6 +173,7 @@ extern "C" pcf_status pcf_batch_pairs(pcf_ctx *ctx, int kind, const pcf_grid *d_
         gs.push_back(D);
         set_weight_fix(pl, gs.data(), (int)gs.size());
     }
+    const bool exact = weighted && pair_lean(pl, box);
     if (!bg) {
         bg = std::make_shared<BatchGraph>();
         bg->plan.pool = ctx->pool;
@@ -230,7 +231,7 @@ extern "C" pcf_status pcf_batch_pairs(pcf_ctx *ctx, int kind, const pcf_grid *d_
             j.pad = 0;
             j.P = js[k].P;
             item += (long long)h.n_tiles * j.n_chunks;
-            mult[k] = js[k].mult;
+            mult[k] = js[k].mult * (exact ? j.wunscale : 1.0);
             bg->keep.push_back(js[k].hc);
             bg->keep.push_back(js[k].cc);
         }
@@ -265,7 +266,7 @@ extern "C" pcf_status pcf_batch_pairs(pcf_ctx *ctx, int kind, const pcf_grid *d_
             e = launch_pair_jobs(reinterpret_cast<const PairJob *>(dp + off_j), nslots, item, js[0].P, box, pl,
                                  counter, cnt, ws, stt, st, ctx->sm_count, ctx->device);
             if (e != cudaSuccess) return e;
-            return launch_finalize_slots(cnt, ws, weighted, reinterpret_cast<const double *>(dp + off_m),
+            return launch_finalize_slots(cnt, ws, weighted, exact, reinterpret_cast<const double *>(dp + off_m),
                                          nb, nslots, out, st);
         };
         if (use_graph) {

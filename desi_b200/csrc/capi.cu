@@ -537,7 +537,9 @@ static pcf_status count_pairs_impl(pcf_ctx *ctx, int kind, const pcf_grid *a_, c
     OutPath o;
     s = out_open(ctx, nb, dev_out, hist, d_out, &o);
     if (s != PCF_OK) return s;
-    s = finalize_hist(ctx, d_cnt, d_ws, pl.weighted, pl.mult, nb, o.to, d_stats, stats || !dev_out ? o.stats : nullptr);
+    const bool exact = pl.weighted && pair_lean(pl, a->box);
+    s = finalize_hist(ctx, d_cnt, d_ws, pl.weighted, exact, exact ? pl.mult * pl.wunscale : pl.mult, nb, o.to, d_stats,
+                      stats || !dev_out ? o.stats : nullptr);
     if (s != PCF_OK) return s;
     if (stats || !dev_out) {
         unsigned long long hs[4];

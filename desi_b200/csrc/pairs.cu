@@ -919,6 +919,15 @@ __global__ void __launch_bounds__(kThreads, MinBlocks<KIND, HM, VAR>::value) k_p
 
 #include "pairs_lean.cuh"
 
+// A bin of k_pairs_lean's weighted sums: 128-bit whole numbers, low and high.
+__device__ __forceinline__ double exact_sum(unsigned long long lo, double hi) {
+    return (double)(unsigned long long)__double_as_longlong(hi) * 0x1p64 + (double)lo;
+}
+
+// How a histogram arrives: u64 counts, FP64 sums, or exact sums (whose scale the
+// caller's multiplier includes).
+enum { SUM_COUNTS = 0, SUM_FP64 = 1, SUM_EXACT = 2 };
+
 // Several histograms: out[s*nb + k] = mult[s] * hist[s*nb + k].
 __global__ void k_finalize_slots(const unsigned long long *__restrict__ cnt,
                                  const double *__restrict__ ws, int weighted,
@@ -927,7 +936,7 @@ __global__ void k_finalize_slots(const unsigned long long *__restrict__ cnt,
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= (long long)nb * nslots) return;
     const int s = (int)(t / nb);
-    out[t] = mult[s] * (weighted ? ws[t] : (double)cnt[t]);
+    out[t] = mult[s] * (weighted == SUM_EXACT ? exact_sum(cnt[t], ws[t]) : weighted ? ws[t] : (double)cnt[t]);
 }
 
 // out[k] = mult * hist[k] (u64 counts or FP64 sums); with host_stats, the four
@@ -938,7 +947,7 @@ __global__ void k_finalize(const unsigned long long *__restrict__ cnt, const dou
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (host_stats && k < 4) host_stats[k] = stats[k];
     if (k >= nb) return;
-    double v = weighted ? ws[k] : (double)cnt[k];
+    double v = weighted == SUM_EXACT ? exact_sum(cnt[k], ws[k]) : weighted ? ws[k] : (double)cnt[k];
     out[k] = mult * v;
 }
 
@@ -1473,11 +1482,13 @@ pcf_status launch_pairs(pcf_ctx *ctx, const PairPlan &plan, const CellGrid &home
     return PCF_OK;
 }
 
+static int sum_kind(bool weighted, bool exact) { return !weighted ? SUM_COUNTS : exact ? SUM_EXACT : SUM_FP64; }
+
 cudaError_t launch_finalize_slots(const unsigned long long *d_count, const double *d_wsum,
-                                  bool weighted, const double *d_mult, int nb, int nslots,
+                                  bool weighted, bool exact, const double *d_mult, int nb, int nslots,
                                   double *d_out, cudaStream_t st) {
     const long long n = (long long)nb * nslots;
-    k_finalize_slots<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(d_count, d_wsum, weighted ? 1 : 0,
+    k_finalize_slots<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(d_count, d_wsum, sum_kind(weighted, exact),
                                                                    d_mult, nb, nslots, d_out);
     return cudaGetLastError();
 }
@@ -1489,9 +1500,9 @@ cudaError_t launch_finalize(const unsigned long long *d_count, const double *d_w
 }
 
 pcf_status finalize_hist(pcf_ctx *ctx, const unsigned long long *d_count, const double *d_wsum,
-                         bool weighted, double mult, int nb, double *out, const unsigned long long *d_stats,
-                         unsigned long long *host_stats) {
-    k_finalize<<<(nb + 255) / 256, 256, 0, ctx->stream>>>(d_count, d_wsum, weighted ? 1 : 0, mult,
+                         bool weighted, bool exact, double mult, int nb, double *out,
+                         const unsigned long long *d_stats, unsigned long long *host_stats) {
+    k_finalize<<<(nb + 255) / 256, 256, 0, ctx->stream>>>(d_count, d_wsum, sum_kind(weighted, exact), mult,
                                                           nb, out, d_stats, host_stats);
     PCF_CU(ctx, cudaGetLastError());
     ++ctx->launches;

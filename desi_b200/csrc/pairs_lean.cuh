@@ -224,6 +224,13 @@ __global__ void __launch_bounds__(LeanShape<W>::threads, LeanShape<W>::ctas) k_p
         if (queued) settle(0, queued);
         queued = 0;
     };
+    // Adds an exact weighted sum to a bin: 128 bits in g_count (low) and g_wsum's
+    // place (high), which the finalize kernels convert (exact_sum).
+    auto add_exact = [&](size_t bin, unsigned long long lo, unsigned long long hi) {
+        const unsigned long long old = atomicAdd(A.g_count + bin, lo);
+        hi += old > ~lo ? 1u : 0u;
+        if (hi) atomicAdd(reinterpret_cast<unsigned long long *>(A.g_wsum) + bin, hi);
+    };
     // Adds this warp's isotropic copy into job slot J.slot and clears it.
     auto flush_iso = [&]() {
         if (!DO_I) return;
@@ -251,9 +258,8 @@ __global__ void __launch_bounds__(LeanShape<W>::threads, LeanShape<W>::ctas) k_p
                     lo += __shfl_xor_sync(kFull, lo, o);
                     hi += __shfl_xor_sync(kFull, hi, o);
                 }
-                hi += lo >> 32;  // exact; the double rounds once
-                if ((lane & (NC - 1)) == 0 && (hi | lo))
-                    atomicAdd(A.g_wsum + off + k, ((double)hi * 0x1p32 + (double)(lo & 0xffffffffull)) * J.wunscale);
+                hi += lo >> 32;
+                if ((lane & (NC - 1)) == 0 && (hi | lo)) add_exact(off + k, hi << 32 | (lo & 0xffffffffull), hi >> 32);
             }
         }
         __syncwarp();
@@ -273,9 +279,7 @@ __global__ void __launch_bounds__(LeanShape<W>::threads, LeanShape<W>::ctas) k_p
             } else {
                 const unsigned l0 = c[3 * s], l1 = c[3 * s + 1], l2 = c[3 * s + 2];
                 c[3 * s] = c[3 * s + 1] = c[3 * s + 2] = 0u;
-                if (l0 | l1 | l2)
-                    atomicAdd(A.g_wsum + off + k,
-                              ((double)l2 * 0x1p64 + ((double)l1 * 0x1p32 + (double)l0)) * J.wunscale);
+                if (l0 | l1 | l2) add_exact(off + k, (unsigned long long)l1 << 32 | l0, l2);
             }
         }
     };

@@ -447,8 +447,8 @@ pcf_status launch_pairs(pcf_ctx *ctx, const PairPlan &plan, const CellGrid &home
                         const CellGrid &cand, float box, const PairLaunch &pl,
                         unsigned long long *d_count, double *d_wsum, unsigned long long *d_stats);
 pcf_status finalize_hist(pcf_ctx *ctx, const unsigned long long *d_count, const double *d_wsum,
-                         bool weighted, double mult, int nb, double *out, const unsigned long long *d_stats,
-                         unsigned long long *host_stats);
+                         bool weighted, bool exact, double mult, int nb, double *out,
+                         const unsigned long long *d_stats, unsigned long long *host_stats);
 // One histogram of a pair launch: home / candidate catalogs, stencil rows,
 // and the implicit items [item_begin, item_begin + n_tiles * n_chunks).
 struct PairJob {
@@ -482,7 +482,7 @@ cudaError_t launch_pairs_view(const PairView &home, const PairView &cand, const 
 cudaError_t launch_finalize(const unsigned long long *d_count, const double *d_wsum, bool weighted,
                             double mult, int nb, double *d_out, cudaStream_t st);
 cudaError_t launch_finalize_slots(const unsigned long long *d_count, const double *d_wsum,
-                                  bool weighted, const double *d_mult, int nb, int nslots,
+                                  bool weighted, bool exact, const double *d_mult, int nb, int nslots,
                                   double *d_out, cudaStream_t st);
 unsigned reference_pair_rule(bool ani, bool bpc, bool cross);
 // Counting sort of n points into P^3 cells on explicit buffers; returns the
