@@ -362,7 +362,7 @@ def run_ours(args, rank, world, local_rank):
         except Exception:
             traffic = None
     roofline = {
-        "bound": "fp32", "kernel": "k_pairs",
+        "bound": "fp32", "kernel": "k_pairs_lean",
         "achieved": round(achieved, 4), "peak": round(fp32_peak, 3), "unit": "TFLOP/s",
         "frac": round(achieved / fp32_peak, 5),
         "peak_source": "FP32 FMA-loop microbenchmark of this run (not in MEASURED_PEAKS.json)",
@@ -590,7 +590,7 @@ def run_triplets(ctx, torch, stream, n=32768):
                             "bins, dmax 80, unit weights: DDD, RRR, DDR, DRR",
                 "ms": ms, "triangles": tri, "value": tri / (ms * 1e-3), "unit": "triplets/s",
                 "per_histogram_ms": {k: v["kernel_ms"] for k, v in sts.items()}})
-    # the same four histograms as the jobs of one persistent launch
+    # the same four histograms in one batched call
     batched = lambda: ctx.batch_triplets(gd, [gr], **kw)[1]  # noqa: E731
     batched()
     bms, bst = _timed_ms(torch, stream, batched)

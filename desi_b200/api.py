@@ -150,8 +150,8 @@ class Context:
                     stats: bool = False, out_device_ptr: int | None = None):
         """One pair histogram (DD / RR with b None, else DR).  ani=False:
         isotropic [bins]; True: anisotropic [bins, bins]; "both": the two in
-        one call (one pass over the candidates where the autotuner found that
-        faster), returned as (iso, ani) (a device output then holds bins +
+        one call (one pass over the candidates for unit and exact integer
+        weights), returned as (iso, ani) (a device output then holds bins +
         bins^2 doubles, isotropic first)."""
         both = ani == "both"
         kind = PCF_BOTH if both else (PCF_ANI if ani else PCF_ISO)
@@ -263,8 +263,8 @@ class Context:
 
     def batch_triplets(self, d: "Grid", rands, *, bins: int, dmax: float, bpc: bool = False,
                        flags: int = 0, stats: bool = False):
-        """DDD, and RRR_i, DDR_i, DRR_i per random grid, in one persistent
-        launch (pcf_batch_triplets): (ddd, rrr, ddr, drr), the last three
+        """DDD, and RRR_i, DDR_i, DRR_i per random grid, queued in one
+        call (pcf_batch_triplets): (ddd, rrr, ddr, drr), the last three
         with a leading random-catalog axis."""
         nr = len(rands)
         n3 = bins ** 3

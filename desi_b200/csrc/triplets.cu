@@ -7,10 +7,10 @@
 // *triple* with a global FP64 atomic per triangle and spell out 64 image
 // combinations.  Here:
 //
-//  * A persistent CTA takes one anchor point i at a time.  It lists the point
-//    ranges of the anchor's neighbour rows (the pair stencil, periodic images
-//    by index wrap), deals the candidates of all of them to its warps 32 at a
-//    time, and compacts into shared memory the X neighbours j > i (list J)
+//  * A group of warps of a persistent CTA takes one anchor point i at a time.  It
+//    lists the point ranges of the anchor's neighbour rows (the pair stencil,
+//    periodic images by index wrap), walks the candidates of all of them at
+//    full width, and compacts into shared memory the X neighbours j > i (list J)
 //    and, for XXY, all Y neighbours (list K), each with its FP32 image
 //    displacement from i (in bins) and its exact side bin (FP32 fast path +
 //    FP64 recheck, as in the pair kernel).
@@ -19,16 +19,14 @@
 //    count123 (3isoBPC_k.cuh:56-75) -- tested and binned in FP32 with the
 //    same edge-window recheck.  Each unordered XXX triangle is seen once (i
 //    its lowest index), each unordered XX pair of an XXY triangle once.
-//  * Counts go to a shared u32 histogram (one orientation per triangle); the
-//    finalize pass symmetrises it into the reference's ordered-triple
+//  * Counts go to a shared u32 histogram (one orientation per triangle), exact
+//    weight products to one of three limbs per counter; the finalize pass symmetrises it into the reference's ordered-triple
 //    histogram: XXX sums the 6 axis permutations, XXY the two orders of the
 //    XX pair (b_jk <-> b_ki).
 #include <algorithm>
 #include <cmath>
 #include <cstring>
-#include <map>
 #include <vector>
-#include <type_traits>
 
 #include "pcf_internal.cuh"
 #include "node_gates.cuh"

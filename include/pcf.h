@@ -60,9 +60,9 @@ typedef enum pcf_status {
 
 /* Histogram kinds.  PCF_BOTH (pair counts only): the isotropic and the
  * anisotropic histogram in one call, written as bins doubles (isotropic)
- * followed by bins*bins doubles (anisotropic).  The call runs the two
- * single-kind launches, or one pass over the candidate pairs for both kinds
- * where pcf_autotune_pairs found that faster for the call's class. */
+ * followed by bins*bins doubles (anisotropic).  Unit and exact integer weights
+ * take one pass over the candidate pairs for both kinds; other calls run the two
+ * single-kind launches, or one pass where pcf_autotune_pairs found that faster. */
 enum { PCF_ISO = 0, PCF_ANI = 1, PCF_BOTH = 2 };
 
 /* Flags for the counting calls. */
@@ -207,9 +207,8 @@ pcf_status pcf_batch_pairs(pcf_ctx *ctx, int kind, const pcf_grid *d, const pcf_
 
 /*
  * The 3-point analogue of pcf_batch_pairs: one data catalog against n_rand
- * random catalogs, the isotropic triplet histograms in two persistent
- * launches (DDD and every RRR_i; every DDR_i and DRR_i), each over one
- * (anchor, histogram) work queue.  Writes ddd (bins^3) once
+ * random catalogs, the isotropic triplet histograms' kernels queued one behind
+ * the other with one wait for all.  Writes ddd (bins^3) once
  * and, per random catalog i, rrr / ddr / drr at [i*bins^3 ..]; any of them
  * may be NULL to skip it.  Replaces the per-file loop of pcf_3iso /
  * pcf_3isoBPC over the -rd random directory (cuda/pcf3iso.cuh:101-112).
