@@ -142,12 +142,15 @@ extern "C" pcf_status pcf_batch_pairs(pcf_ctx *ctx, int kind, const pcf_grid *d_
     bool weighted = !D->unit_weights;
     for (auto *g : R) weighted = weighted || !g->unit_weights;
 
-    // cache key of the captured graph: grids (by cell buffers) and parameters
+    // cache key of the captured graph: grids (by cell buffers) and parameters,
+    // dmax by its bits (printed, two that differ past six digits look alike)
     std::string key;
     const bool use_graph = (flags & PCF_GRAPH) != 0;
     if (use_graph) {
+        uint32_t dmax_bits;
+        memcpy(&dmax_bits, &dmax, sizeof(dmax_bits));
         std::ostringstream os;
-        os << kind << ':' << bins << ':' << dmax << ':' << (flags & ~PCF_GRAPH) << ':' << (dd != nullptr)
+        os << kind << ':' << bins << ':' << dmax_bits << ':' << (flags & ~PCF_GRAPH) << ':' << (dd != nullptr)
            << (rr != nullptr) << (dr != nullptr) << (stats != nullptr);
         for (auto &j : js) os << ',' << j.hc->serial << '/' << j.cc->serial;
         key = os.str();
