@@ -124,6 +124,12 @@ extern "C" pcf_status pcf_batch_pairs(pcf_ctx *ctx, int kind, const pcf_grid *d_
         if (rr) add_job(R[i], R[i], true, 2.0);
         if (dr) add_job(D, R[i], false, 1.0);
     }
+    if (bpc)  // as a single call of each job
+        for (const auto &j : js)
+            if (!stencil_fits(box, dmax, j.P)) {
+                ctx->last_error = "dmax too close to box/2 for the periodic stencil";
+                return PCF_ERR_UNSUPPORTED;
+            }
     pcf_status s = PCF_OK;
     // every structure queued before the first is completed, so the builds'
     // host work overlaps the device; each job holds its structures, and a

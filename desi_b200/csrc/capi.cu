@@ -370,6 +370,15 @@ PairRule make_pair_rule(int bins, float dmax, uint32_t flags, bool ani, bool bpc
     return r;
 }
 
+// Whether the stencil of a periodic count keeps from wrapping onto itself at P
+// cells per side: k neighbour cells each way, and home tiles that span two cells.
+// (Past that a tile reaches over both z faces at once, and row_range follows one.)
+bool stencil_fits(float box, float dmax, int P) {
+    const double cell = (double)box / P;
+    const int k = (int)std::ceil(((double)dmax + 1e-4 * cell + 8.0 * box * 1.2e-7) / cell);
+    return 2 * k + 2 <= P;
+}
+
 // Shared validation + re-gridding of the counting calls.
 pcf_status prepare_grids(pcf_ctx *ctx, pcf_grid *a, pcf_grid *b, float dmax, int kind,
                          bool bpc, int *P_out, int refine) {
@@ -384,19 +393,11 @@ pcf_status prepare_grids(pcf_ctx *ctx, pcf_grid *a, pcf_grid *b, float dmax, int
     // grid build, else the tuned or default rule
     int P = 0;
     if (ctx->tune_override.refine <= 0) P = a->user_P > 0 ? a->user_P : (b ? b->user_P : 0);
-    if (P > 0 && bpc) {  // a periodic stencil must not wrap onto itself: else automatic
-        const double cell = (double)box / P;
-        const int k = (int)std::ceil(((double)dmax + 1e-4 * cell + 8.0 * box * 1.2e-7) / cell);
-        if (2 * k + 2 > P) P = 0;
-    }
+    if (P > 0 && bpc && !stencil_fits(box, dmax, P)) P = 0;  // else automatic
     if (P <= 0) P = choose_partitions(n, box, dmax, kind, bpc, refine);
-    if (bpc) {
-        double cell = (double)box / P;
-        int k = (int)std::ceil(((double)dmax + 1e-4 * cell + 8.0 * box * 1.2e-7) / cell);
-        if (2 * k + 2 > P) {
-            ctx->last_error = "dmax too close to box/2 for the periodic stencil";
-            return PCF_ERR_UNSUPPORTED;
-        }
+    if (bpc && !stencil_fits(box, dmax, P)) {
+        ctx->last_error = "dmax too close to box/2 for the periodic stencil";
+        return PCF_ERR_UNSUPPORTED;
     }
     // both structures queued before either is completed: a's host work
     // (cell table, tiles) overlaps b's build on the device

@@ -1425,7 +1425,8 @@ pcf_status stencil_max(pcf_ctx *ctx, const CellGrid &g, const RowDesc *d_rows, i
 // side, 0.4 points each; 2062 at 94; 1925 at 80, 5.2 points; 2201 at 64; 200000 and
 // 300000 points, dmax 20: 565 at 99 cells, 374 at 50, 400 at 40, 366 at 32, weighted
 // 2ani 638, 420, 448, 463; 6M and 9M points, dmax 15: 5517 at 133, 5276 at 120, 5891 at 100).
-// A periodic stencil never wraps onto itself (2k + 2 <= P).
+// A periodic stencil that would wrap onto itself takes more cells, up to 256 (callers
+// refuse what does not fit then).
 int choose_partitions(int64_t n, float box, float dmax, int kind, bool bpc, int refine) {
     double least = 6.0;  // points per cell at 3 cells per dmax or more
     bool grow = false;   // cells of few points
@@ -1444,15 +1445,8 @@ int choose_partitions(int64_t n, float box, float dmax, int kind, bool bpc, int 
     while (P > 1 && refine > 1 && (double)n / ((double)P * P * P) < (refine > 2 ? least : 6.0)) P = cells(--refine);
     if (grow && refine == 1) P = std::min(P, (int)std::cbrt((double)n / 5.0));
     P = std::max(1, std::min(P, 256));
-    if (bpc) {
-        // need 2k+1 <= P with k = ceil(R / (L/P)) (+1 for the tile span)
-        for (;;) {
-            double cell = L / P;
-            int k = (int)std::ceil((R + 1e-4 * cell + 8.0 * L * 1.2e-7) / cell);
-            if (2 * k + 2 <= P || P >= 256) break;
-            ++P;
-        }
-    }
+    if (bpc)
+        while (P < 256 && !stencil_fits(box, dmax, P)) ++P;
     return P;
 }
 

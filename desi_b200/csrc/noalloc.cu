@@ -81,11 +81,7 @@ extern "C" pcf_status pcf_count_pairs_noalloc(const pcf_point *a, int64_t na, co
 
     const int64_t nmax = std::max<int64_t>(na, cross ? nb : 0);
     const int P = choose_partitions(nmax, box, dmax, kind, bpc, 0);
-    if (bpc) {
-        const double cell = (double)box / P;
-        const int k = (int)std::ceil(((double)dmax + 1e-4 * cell + 8.0 * box * 1.2e-7) / cell);
-        if (2 * k + 2 > P) return PCF_ERR_UNSUPPORTED;
-    }
+    if (bpc && !stencil_fits(box, dmax, P)) return PCF_ERR_UNSUPPORTED;
     const int64_t ncell = (int64_t)P * P * P;
     // the same bound as pcf_count_pairs (bins^2 accumulators at most 2^24)
     if (ani && (int64_t)bins * bins > (1 << 24)) return PCF_ERR_UNSUPPORTED;

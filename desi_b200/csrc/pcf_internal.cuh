@@ -363,6 +363,7 @@ pcf_status stencil_max(pcf_ctx *ctx, const CellGrid &g, const RowDesc *d_rows, i
 // kind: a histogram kind, or kTripletCells.
 constexpr int kTripletCells = 3;
 int choose_partitions(int64_t n, float box, float dmax, int kind, bool bpc, int refine);
+bool stencil_fits(float box, float dmax, int P);
 
 // Stencil of one pair launch (host).  Work items are implicit: item i is
 // (tile i / n_chunks, rows [c*rows_per_item, ...) of chunk c = i % n_chunks).
