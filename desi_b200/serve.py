@@ -390,24 +390,28 @@ class PcfServer:
                 s.ctx.close()
 
     # -- a timed stream ----------------------------------------------------
-    def run_stream(self, reqs: list[Request], tick_s: float = 0.005) -> dict:
-        """Submit requests at their arrival times; wait for all; report.
-        Arrivals within tick_s after the one that is due are submitted with
-        it: each wake-up of this thread takes the interpreter lock from the
-        slots, and small requests now take less than a millisecond."""
+    def run_stream(self, reqs: list[Request], tick_s: float = 0.003) -> dict:
+        """Submits requests at their arrival times, waits for all, reports
+        (latencies from each arrival to its result).  A request that arrives
+        waits tick_s for others, and those that arrived meanwhile go with it:
+        each wake-up of this thread takes the interpreter lock from the slots,
+        and small requests take less than a millisecond.  None is submitted
+        before its arrival; tick_s=0 submits each at its arrival."""
         a0 = _lib.alloc_counters()
         t0 = time.perf_counter()
-        due = -1.0
-        for r in sorted(reqs, key=lambda r: r.arrival):
-            if r.arrival > due:
-                due = r.arrival + tick_s
-                delay = t0 + r.arrival - time.perf_counter()
-                if delay > 0:
-                    time.sleep(delay)
-            self.submit(r)
+        order = sorted(reqs, key=lambda r: r.arrival)
+        i = 0
+        while i < len(order):
+            delay = t0 + order[i].arrival + tick_s - time.perf_counter()
+            if delay > 0:
+                time.sleep(delay)
+            now = time.perf_counter() - t0
+            while i < len(order) and order[i].arrival <= now:
+                self.submit(order[i])
+                i += 1
         results = [r.future.result() for r in reqs]
         t1 = time.perf_counter()
-        return self._report(reqs, results, t1 - t0, a0)
+        return self._report(reqs, results, t1 - t0, a0, [t0 + r.arrival for r in reqs])
 
     def run_serial(self, reqs: list[Request]) -> dict:
         """The plain per-call form of the same requests: one at a time, in
@@ -425,8 +429,10 @@ class PcfServer:
         return self._report(order, results, t1 - t0, a0)
 
     @staticmethod
-    def _report(reqs, results, wall, allocs0=None) -> dict:
-        lat = np.array([(r.t_end - r.t_submit) * 1e3 for r in reqs])
+    def _report(reqs, results, wall, allocs0=None, since=None) -> dict:
+        """since: when each request's latency begins (None: its submission)."""
+        since = since or [r.t_submit for r in reqs]
+        lat = np.array([(r.t_end - s) * 1e3 for r, s in zip(reqs, since)])
         units = sum(res.get("_units", 0.0) for res in results)
         tri = sum(res.get("_triangles", 0.0) for res in results)
         busy = {}
