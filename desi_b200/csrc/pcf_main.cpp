@@ -202,8 +202,8 @@ int main(int argc, char **argv) {
             pcfio::save3d("DRR" + sfx + tag + data_name, bn, ddr.data());  // pcf3isoBPC.cuh:340
             pcfio::save3d("RRR" + sfx + tag + data_name, bn, rrr.data());
         } else if (!ani && gR.size() > 1 && !gated) {
-            // -rd: DDD, and RRR / DDR / DRR of every random catalog, in one
-            // persistent launch (the reference launches per file,
+            // -rd: DDD, and RRR / DDR / DRR of every random catalog, queued in
+            // one call (the reference launches per file and waits,
             // cuda/pcf3iso.cuh:101-112)
             const size_t nr = gR.size();
             std::vector<double> rrr(b3 * nr), ddr(b3 * nr), drr(b3 * nr);

@@ -1566,7 +1566,7 @@ extern "C" pcf_status pcf_batch_triplets(pcf_ctx *ctx, const pcf_grid *d_, const
     std::vector<TripArgs> args((size_t)nj);
     long long anchors = 0;
     bool any_mixed = false;
-    int n_of[2] = {0, 0}, most = 1;
+    int most = 1;
     std::vector<size_t> smem((size_t)nj);
     std::vector<int> groups((size_t)nj);
     int64_t gmax = 0;
@@ -1590,7 +1590,6 @@ extern "C" pcf_status pcf_batch_triplets(pcf_ctx *ctx, const pcf_grid *d_, const
         groups[k] = trip_groups(jobs[k].x, jobs[k].y, bins, dmax, weighted);
         trip_setup(ctx, jobs[k].x, jobs[k].y, P, (int)plan.rows.size(), bins, dmax, flags, weighted,
                    args[k], smem[k], groups[k]);
-        ++n_of[jobs[k].y ? 1 : 0];
         most = std::max(most, groups[k]);
         anchors += jobs[k].x->n;
         any_mixed = any_mixed || jobs[k].y;
@@ -1599,7 +1598,6 @@ extern "C" pcf_status pcf_batch_triplets(pcf_ctx *ctx, const pcf_grid *d_, const
     TripArgs ov;
     s = trip_overflow(ctx, gmax + 32, any_mixed, weighted, grid * most, ov);
     if (s != PCF_OK) return s;
-    if ((n_of[0] + 63) / 64 + (n_of[1] + 63) / 64 > 8) return PCF_ERR_UNSUPPORTED;
 
     // histograms per job, a counter per job, statistics, results
     const size_t nh = (size_t)nj * n3, cb = ((size_t)nj * 8 + 63) & ~(size_t)63;
