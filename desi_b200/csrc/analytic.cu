@@ -246,13 +246,21 @@ struct FineArgs {
 template <bool WEIGHTED>
 __global__ void __launch_bounds__(256) k_fine_dd(const FineArgs A) {
     const int lane = threadIdx.x & 31, P = A.P;
-    for (;;) {
+    for (long long taken = 1;; ++taken) {
+        // lane 0 takes the ticket and reads the abort word, which may change at any
+        // time: the warp leaves together
         long long t = 0;
-        if (lane == 0) t = (long long)atomicAdd(A.counter, 1ull);
+        unsigned stop = 0u;
+        if (lane == 0) {
+            t = (long long)atomicAdd(A.counter, 1ull);
+            if (A.ctrl && ctrl_load(A.ctrl)) stop = PCF_GAVE_UP_ABORT;
+            if (taken > (long long)A.n + 1) stop |= PCF_GAVE_UP_CAP;
+        }
         const long long i = __shfl_sync(0xffffffffu, t, 0);
         if (i >= A.n) break;
-        if (A.ctrl && ctrl_load(A.ctrl)) {
-            if (A.status && lane == 0) ctrl_store(A.status, PCF_GAVE_UP_ABORT);
+        stop = __shfl_sync(0xffffffffu, stop, 0);
+        if (stop) {
+            if (A.status && lane == 0) ctrl_store(A.status, stop);
             break;
         }
         const float hx = A.x[i], hy = A.y[i], hz = A.z[i];
