@@ -229,7 +229,11 @@ __global__ void __launch_bounds__(256) k_refine(int bins, int bn_ref, double dr,
 // is no fast path beyond a test against dmax; a warp takes a home point and walks
 // its stencil's rows, the candidates behind it in cell order.  Two launches of the
 // general pair kernel, which sent each pair to its recheck, took 395 us for 10007
-// points (dmax 60 of 250, 2000 and 400000 bins); this takes 173.
+// points (dmax 60 of 250, 2000 and 400000 bins); this takes 173.  A histogram of up
+// to kPairBins bins goes to the pair kernel instead, which counts in shared memory:
+// here every pair's global add queues behind the others of its bin (20 and 20 bins, 30000
+// points, dmax 110 of 250: 73 ms, and 0.84 by the pair kernel).
+constexpr int64_t kPairBins = 255;
 struct FineArgs {
     const float *x, *y, *z, *w;
     const int *cstart;
@@ -403,44 +407,52 @@ extern "C" pcf_status pcf_analytic_3iso(pcf_ctx *ctx, const pcf_grid *d_, int bi
         const CellGrid &g = *D->cells;
         PairPlan plan;
         plan_pairs(g, L, dmax, false, false, plan, ctx->sm_count * 24);
-        PlanSlot *sl = nullptr;
-        s = stage_plan(ctx, plan, &sl);
-        if (s != PCF_OK) return s;
-        FineArgs A;
-        A.x = g.x();
-        A.y = g.y();
-        A.z = g.z();
-        A.w = g.w();
-        A.cstart = g.cell_start.as<int>();
-        A.rows = sl->rows();
-        A.n = (int)np;
-        A.n_rows = (int)plan.rows.size();
-        A.P = P;
-        A.cell = g.cell;
-        A.box = L;
-        A.r1 = make_pair_rule((int)bn_ff, dmax, PCF_BPC, false, true, false);
-        A.r2 = make_pair_rule((int)bn_ffr, dmax, PCF_BPC, false, true, false);
-        A.r1.ds = (double)((float)bn_ff / dmax);
-        A.r2.ds = (double)((float)bn_ffr / dmax);
-        const double reach = std::sqrt(A.r1.dd) + 4e-6 * (double)L;  // above any FP32 distance in range
-        A.hi = (float)(reach * reach * (1.0 + 1e-5));
-        const bool weighted = !D->unit_weights;
-        const size_t nb = (size_t)(bn_ff + bn_ffr);
-        PCF_CU(ctx, ctx->d_hist.ensure(sizeof(double) * nb));
-        A.cnt = ctx->d_hist.as<unsigned long long>();
-        A.wsum = ctx->d_hist.as<double>();
-        A.counter = sl->counter();
-        A.ctrl = ctx->d_abort;
-        A.status = ctx->d_status;
-        PCF_CU(ctx, cudaMemsetAsync(A.cnt, 0, sizeof(double) * nb, ctx->stream));
         if (stats) PCF_CU(ctx, cudaEventRecord(ctx->ev0, ctx->stream));
-        (weighted ? k_fine_dd<true> : k_fine_dd<false>)<<<ctx->sm_count * 6, 256, 0, ctx->stream>>>(A);
-        PCF_CU(ctx, cudaGetLastError());
+        const double ds1 = (double)((float)bn_ff / dmax), ds2 = (double)((float)bn_ffr / dmax);
+        if (bn_ff <= kPairBins && (s = queue_scaled_pairs(ctx, D, (int)bn_ff, dmax, ds1, dd_ff)) != PCF_OK) return s;
+        if (bn_ffr <= kPairBins && (s = queue_scaled_pairs(ctx, D, (int)bn_ffr, dmax, ds2, dd_ffr)) != PCF_OK) return s;
+        if (bn_ffr > kPairBins) {  // (bn_ff is at most bn_ffr)
+            PlanSlot *sl = nullptr;
+            s = stage_plan(ctx, plan, &sl);
+            if (s != PCF_OK) return s;
+            const bool both = bn_ff > kPairBins;
+            FineArgs A;
+            A.x = g.x();
+            A.y = g.y();
+            A.z = g.z();
+            A.w = g.w();
+            A.cstart = g.cell_start.as<int>();
+            A.rows = sl->rows();
+            A.n = (int)np;
+            A.n_rows = (int)plan.rows.size();
+            A.P = P;
+            A.cell = g.cell;
+            A.box = L;
+            A.r1 = make_pair_rule((int)bn_ff, dmax, PCF_BPC, false, true, false);
+            A.r2 = make_pair_rule((int)bn_ffr, dmax, PCF_BPC, false, true, false);
+            A.r1.ds = ds1;
+            A.r2.ds = ds2;
+            if (!both) A.r1.bins = 0;
+            const double reach = std::sqrt(A.r1.dd) + 4e-6 * (double)L;  // above any FP32 distance in range
+            A.hi = (float)(reach * reach * (1.0 + 1e-5));
+            const bool weighted = !D->unit_weights;
+            const size_t nb = (size_t)(A.r1.bins + bn_ffr);
+            PCF_CU(ctx, ctx->d_hist.ensure(sizeof(double) * nb));
+            A.cnt = ctx->d_hist.as<unsigned long long>();
+            A.wsum = ctx->d_hist.as<double>();
+            A.counter = sl->counter();
+            A.ctrl = ctx->d_abort;
+            A.status = ctx->d_status;
+            PCF_CU(ctx, cudaMemsetAsync(A.cnt, 0, sizeof(double) * nb, ctx->stream));
+            (weighted ? k_fine_dd<true> : k_fine_dd<false>)<<<ctx->sm_count * 6, 256, 0, ctx->stream>>>(A);
+            PCF_CU(ctx, cudaGetLastError());
+            PCF_CU(ctx, cudaEventRecord(sl->done, ctx->stream));
+            ++ctx->launches;
+            s = finalize_hist(ctx, A.cnt, A.wsum, weighted, false, 2.0, (int)nb, both ? dd_ff : dd_ffr, nullptr,
+                              nullptr);  // ordered pairs
+            if (s != PCF_OK) return s;
+        }
         if (stats) PCF_CU(ctx, cudaEventRecord(ctx->ev1, ctx->stream));
-        PCF_CU(ctx, cudaEventRecord(sl->done, ctx->stream));
-        ++ctx->launches;
-        s = finalize_hist(ctx, A.cnt, A.wsum, weighted, false, 2.0, (int)nb, dd_ff, nullptr, nullptr);  // ordered pairs
-        if (s != PCF_OK) return s;
     }
     // analytic RR at the fine binnings (RR2iso_BPC_analytic with alpha_ff*)
     const double alpha_ff = rr_alpha(np, L, dmax, bn_ff);

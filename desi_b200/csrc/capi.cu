@@ -449,6 +449,25 @@ static PairLaunch pair_launch(pcf_ctx *ctx, const pcf_grid *a, const pcf_grid *b
     return pl;
 }
 
+// Queues the periodic isotropic XX histogram of a's current cells with the bin
+// scale ds into device memory (ordered pairs); nothing waits for it.
+pcf_status queue_scaled_pairs(pcf_ctx *ctx, const pcf_grid *a, int bins, float dmax, double ds, double *d_out) {
+    PairPlan plan;
+    plan_pairs(*a->cells, a->box, dmax, false, true, plan, ctx->sm_count * 24);
+    unsigned long long *d_cnt, *d_stats;
+    double *d_ws, *unused;
+    pcf_status s = hist_scratch(ctx, bins, &d_cnt, &d_ws, &d_stats, &unused);
+    if (s != PCF_OK) return s;
+    PairLaunch pl = pair_launch(ctx, a, nullptr, PCF_ISO, bins, dmax, PCF_BPC, !a->unit_weights);
+    pl.rule.ds = ds;
+    pl.count = pl.timed = false;
+    s = launch_pairs(ctx, plan, *a->cells, *a->cells, a->box, pl, d_cnt, d_ws, d_stats);
+    if (s != PCF_OK) return s;
+    const bool exact = pl.weighted && pair_lean(pl, a->box);
+    return finalize_hist(ctx, d_cnt, d_ws, pl.weighted, exact, exact ? pl.mult * pl.wunscale : pl.mult, bins, d_out,
+                         nullptr, nullptr);
+}
+
 // One pair histogram.
 static pcf_status count_pairs_impl(pcf_ctx *ctx, int kind, const pcf_grid *a_, const pcf_grid *b_,
                                    int bins, float dmax, uint32_t flags, double *hist,

@@ -523,6 +523,7 @@ PairRule make_pair_rule(int bins, float dmax, uint32_t flags, bool ani, bool bpc
 // pair job at *d_job to a slot, in one copy.
 pcf_status stage_plan(pcf_ctx *ctx, const PairPlan &plan, PlanSlot **out, PairJob *job = nullptr,
                       PairJob **d_job = nullptr);
+pcf_status queue_scaled_pairs(pcf_ctx *ctx, const pcf_grid *a, int bins, float dmax, double ds, double *d_out);
 pcf_status pcf_count_triplets_ani(pcf_ctx *ctx, const pcf_grid *x, const pcf_grid *y, int bins,
                                   float dmax, uint32_t flags, double *hist, pcf_stats *stats);
 pcf_status profile_events(pcf_ctx *ctx, cudaEvent_t *a, cudaEvent_t *b);
