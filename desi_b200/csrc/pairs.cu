@@ -1189,25 +1189,35 @@ static cudaError_t launch_lean(const PairArgs &A, cudaStream_t st, int sm_count,
 }
 
 // Columns per isotropic bin of a lean launch (32, 16 or 8): the most that let
-// two CTAs share an SM, else 8; 0 where not even that fits one CTA.
+// two CTAs share an SM, else 8; 0 where the general kernel is the faster one, which
+// is where too few warps would be left (time of the general kernel over this, 30000
+// + 40000 and 200000 + 267000 points):
+//  * unit weights, fewer than two CTAs of 4 warps (the anisotropic copy, from 153
+//    bins on): 0.99 and 1.19 at 150 bins, 0.61 and 0.63 at 160, 0.61 and 0.63 at 220;
+//  * exact weights, isotropic, one CTA of 8 warps (161 bins on): 1.14 and 1.12 at
+//    160, 0.89 and 0.74 at 165, 0.96 and 0.78 at 255;
+//  * exact weights, anisotropic: one CTA with a copy of up to 110 bins is worth it
+//    (1.64 and 2.05 at 80, 1.01 and 1.19 at 110, 0.84 and 0.91 at 115), and fewer
+//    than 5 bins are not, where the CTA's warps collide on few counters (0.85 and
+//    0.82 at 2, 0.94 and 0.98 at 4, 1.01 and 1.02 at 5).  One pass for both kinds
+//    saves more: one CTA is worth it wherever it fits (1.41 and 1.43 at 100 bins).
 static int lean_columns(const PairLaunch &pl) {
     const int bins = pl.rule.bins;
     const int kLWarps = pl.weighted ? LeanShape<true>::warps : LeanShape<false>::warps;
-    const size_t fixed = sizeof(LeanWarp) * kLWarps + sizeof(PairJob) + 2048;
+    const size_t fixed = sizeof(LeanWarp) * kLWarps + sizeof(PairJob) + 64;  // its static shared memory
     const size_t ani = !pl.ani ? 0 : pl.weighted ? LeanCopies<K_ANI, true, 32>::ani(bins) : LeanCopies<K_ANI, false, 32>::ani(bins);
-    const bool cols = pl.weighted && (!pl.ani || pl.both);
-    for (int nc = 32; nc >= 8; nc >>= 1) {
-        const size_t iso = cols ? (size_t)kLWarps * (bins + 1) * 8 * nc : (size_t)kLWarps * (bins + 1) * 4;
-        const size_t room = nc > 8 && cols ? 114 * 1024 : 227 * 1024;
-        if (fixed + iso + ani <= room) return nc;
-    }
+    const size_t iso = !pl.ani || pl.both ? (size_t)kLWarps * (bins + 1) * 4 : 0;  // (weighted: per limb and column)
+    constexpr size_t two = 113 * 1024;  // what each of two CTAs can have
+    if (!pl.weighted) return fixed + iso + ani <= 110 * 1024 ? 32 : 0;
+    if (!iso) return bins >= 5 && fixed + ani <= 204 * 1024 ? 32 : 0;
+    for (int nc = 32; nc >= 8; nc >>= 1)
+        if (fixed + iso * 2 * nc + ani <= (nc == 8 && pl.ani ? 227 * 1024 : two)) return nc;
     return 0;
 }
 
 // k_pairs_lean takes every launch of unit weights or exact integer weights that
-// its windows and its copies fit, unless a histogram scheme or a kernel variant
-// was asked for: it is the faster one at every size and bin count measured
-// (pairs_lean.cuh has both sides).
+// its windows and its copies fit (lean_columns), unless a histogram scheme or a
+// kernel variant was asked for.
 bool pair_lean(const PairLaunch &pl, float box) {
     if (pl.hist_mode >= 0 || pl.variant != 0 || (pl.weighted && !pl.wfix)) return false;
     return make_cuts(pl.rule, box, std::sqrt((float)pl.rule.dd)).wl[0] != 0 && lean_columns(pl) != 0;

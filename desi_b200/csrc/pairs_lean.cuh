@@ -1,6 +1,7 @@
 // pairs_lean.cuh -- the pair kernel of unit weights and of weights with exact
-// integer images, up to 255 bins (included by pairs.cu, which holds the work
-// items, the windows and the general kernel for everything else).
+// integer images, at the bin counts where its copies leave room for enough warps
+// (lean_columns in pairs.cu, which includes this file and holds the work items, the
+// windows and the general kernel for everything else).
 //
 // Same work items as the general kernel: one warp takes (home tile, stencil
 // rows), one home point per lane, candidates two at a time as packed f32x2.
