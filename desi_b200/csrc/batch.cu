@@ -103,6 +103,25 @@ extern "C" pcf_status pcf_batch_pairs(pcf_ctx *ctx, int kind, const pcf_grid *d_
     }
     const float box = D->box;
     if (bpc && !(2.0 * (double)dmax < (double)box)) return PCF_ERR_UNSUPPORTED;
+    const int nb = ani ? bins * bins : bins;
+    bool weighted = !D->unit_weights;
+    for (auto *g : R) weighted = weighted || !g->unit_weights;
+    PairLaunch pl;
+    pl.ani = ani;
+    pl.bpc = bpc;
+    pl.self = false;
+    pl.weighted = weighted;
+    pl.rule = make_pair_rule(bins, dmax, flags, ani, bpc, false);
+    pl.mult = 1.0;
+    pl.count = stats != nullptr;
+    pl.ctrl = ctx->d_abort;
+    pl.status = ctx->d_status;
+    {
+        std::vector<const pcf_grid *> gs(R.begin(), R.end());
+        gs.push_back(D);
+        set_weight_fix(pl, gs.data(), (int)gs.size());
+    }
+    const bool lean = pair_lean(pl, box), exact = weighted && lean;
     // The jobs: DD, then RR_i and DR_i per random catalog.  Each job gets the
     // partition count a single call would use for its catalogs (small
     // catalogs get coarser cells), and holds the cell structures at that
@@ -117,7 +136,7 @@ extern "C" pcf_status pcf_batch_pairs(pcf_ctx *ctx, int kind, const pcf_grid *d_
     std::vector<J> js;
     auto add_job = [&](pcf_grid *h, pcf_grid *c, bool self, double mult) {
         const int64_t n = std::max<int64_t>(h->n, c->n);
-        js.push_back({h, c, self, mult, choose_partitions(n, box, dmax, kind, bpc, 0), nullptr, nullptr});
+        js.push_back({h, c, self, mult, choose_partitions(n, box, dmax, lean ? kind : kGeneralCells, bpc, 0), nullptr, nullptr});
     };
     if (dd) add_job(D, D, true, 2.0);
     for (int i = 0; i < n_rand; ++i) {
@@ -144,10 +163,6 @@ extern "C" pcf_status pcf_batch_pairs(pcf_ctx *ctx, int kind, const pcf_grid *d_
     for (auto &j : js) {
         if ((s = grid_finish(ctx, j.h)) != PCF_OK || (s = grid_finish(ctx, j.c)) != PCF_OK) return s;
     }
-    const int nb = ani ? bins * bins : bins;
-    bool weighted = !D->unit_weights;
-    for (auto *g : R) weighted = weighted || !g->unit_weights;
-
     // cache key of the captured graph: grids (by cell buffers) and parameters,
     // dmax by its bits (printed, two that differ past six digits look alike)
     std::string key;
@@ -167,22 +182,6 @@ extern "C" pcf_status pcf_batch_pairs(pcf_ctx *ctx, int kind, const pcf_grid *d_
         if (it != ctx->graphs.end()) bg = it->second;
     }
     cudaStream_t st = ctx->stream;
-    PairLaunch pl;
-    pl.ani = ani;
-    pl.bpc = bpc;
-    pl.self = false;
-    pl.weighted = weighted;
-    pl.rule = make_pair_rule(bins, dmax, flags, ani, bpc, false);
-    pl.mult = 1.0;
-    pl.count = stats != nullptr;
-    pl.ctrl = ctx->d_abort;
-    pl.status = ctx->d_status;
-    {
-        std::vector<const pcf_grid *> gs(R.begin(), R.end());
-        gs.push_back(D);
-        set_weight_fix(pl, gs.data(), (int)gs.size());
-    }
-    const bool exact = weighted && pair_lean(pl, box);
     if (!bg) {
         bg = std::make_shared<BatchGraph>();
         bg->plan.pool = ctx->pool;

@@ -506,13 +506,10 @@ static pcf_status count_pairs_impl(pcf_ctx *ctx, int kind, const pcf_grid *a_, c
     // contend for few hot bins, and its extra shared memory can cost resident
     // CTAs (signed weights, 40 bins, 200k points against 32 randoms: 381 vs 133 +
     // 216 ms).
-    bool one_pass = te.hist_mode >= 0;
-    if (both && !one_pass) {
-        PairLaunch pl = pair_launch(ctx, a, b, kind, bins, dmax, flags, weighted);
-        pl.count = stats != nullptr;
-        one_pass = pair_lean(pl, a->box);
-    }
-    if (both && !one_pass) {
+    PairLaunch pl = pair_launch(ctx, a, b, kind, bins, dmax, flags, weighted);
+    pl.hist_mode = te.hist_mode;
+    const bool lean = pair_lean(pl, a->box);
+    if (both && !lean && te.hist_mode < 0) {
         pcf_stats si{}, sa{};
         pcf_status s = count_pairs_impl(ctx, PCF_ISO, a_, b_, bins, dmax, flags, hist,
                                         stats ? &si : nullptr);
@@ -530,7 +527,7 @@ static pcf_status count_pairs_impl(pcf_ctx *ctx, int kind, const pcf_grid *a_, c
         return s;
     }
     int P = 0;
-    pcf_status s = prepare_grids(ctx, a, b, dmax, kind, bpc, &P, te.refine);
+    pcf_status s = prepare_grids(ctx, a, b, dmax, lean ? kind : kGeneralCells, bpc, &P, te.refine);
     if (s != PCF_OK) return s;
     const int tile_cap = te.tile == 16 ? 16 : kTileCap;
     if (tile_cap == 16) {
@@ -544,8 +541,6 @@ static pcf_status count_pairs_impl(pcf_ctx *ctx, int kind, const pcf_grid *a_, c
     double *d_ws, *d_out;
     s = hist_scratch(ctx, nb, &d_cnt, &d_ws, &d_stats, &d_out);
     if (s != PCF_OK) return s;
-    PairLaunch pl = pair_launch(ctx, a, b, kind, bins, dmax, flags, weighted);
-    pl.hist_mode = te.hist_mode;
     pl.count = stats != nullptr && !ctx->tune_timing;
     pl.timed = stats != nullptr;
     pl.tile_cap = tile_cap;
@@ -557,7 +552,7 @@ static pcf_status count_pairs_impl(pcf_ctx *ctx, int kind, const pcf_grid *a_, c
     OutPath o;
     s = out_open(ctx, nb, dev_out, hist, d_out, &o);
     if (s != PCF_OK) return s;
-    const bool exact = pl.weighted && pair_lean(pl, a->box);
+    const bool exact = pl.weighted && lean;
     s = finalize_hist(ctx, d_cnt, d_ws, pl.weighted, exact, exact ? pl.mult * pl.wunscale : pl.mult, nb, o.to, d_stats,
                       stats || !dev_out ? o.stats : nullptr);
     if (s != PCF_OK) return s;

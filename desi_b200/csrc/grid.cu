@@ -1425,25 +1425,36 @@ pcf_status stencil_max(pcf_ctx *ctx, const CellGrid &g, const RowDesc *d_rows, i
 // side, 0.4 points each; 2062 at 94; 1925 at 80, 5.2 points; 2201 at 64; 200000 and
 // 300000 points, dmax 20: 565 at 99 cells, 374 at 50, 400 at 40, 366 at 32, weighted
 // 2ani 638, 420, 448, 463; 6M and 9M points, dmax 15: 5517 at 133, 5276 at 120, 5891 at 100).
+// The general pair kernel has other lines (signed weights, us per DR of n points and
+// 3n / 4, box 1000).  Few cells leave SMs idle, so small catalogs take smaller cells: 3
+// or 4 per dmax from n / 3500 points per cell on (1.25 to 6; n = 4000, dmax 200: 131 at 4 cells
+// per side, 55 at 15; 20000, dmax 200: 265 at 10, 211 at 15; 40000, box 500, dmax 60: 188 at 16, 224
+// at 24), 2 from n / 8000 on (20000, dmax 100: 102 at 10, 81 at 20; 40000: 200 at 9, 159 at 20;
+// 400000, dmax 40: 662 at 24, 740 at 50).  Cells of one dmax grow to 2.5 points (400000, dmax
+// 15: 234 at 43, 200 at 54, 205 at 66; dmax 8: 214 at 43, 182 at 54, 292 at 125).
 // A periodic stencil that would wrap onto itself takes more cells, up to 256 (callers
 // refuse what does not fit then).
 int choose_partitions(int64_t n, float box, float dmax, int kind, bool bpc, int refine) {
-    double least = 6.0;  // points per cell at 3 cells per dmax or more
-    bool grow = false;   // cells of few points
+    double least = 6.0, coarse = 6.0;  // points per cell at 3 cells per dmax or more, at 2
+    double grow = 0.0;                 // ... at 1 (0: any)
     if (refine <= 0) {
         const char *e = getenv("PCF_REFINE");  // experiment / autotuner override
         refine = e ? atoi(e) : 4;
         if (refine < 1 || refine > 16) refine = 4;
-        if (!e && kind != kTripletCells) {
+        if (!e && kind == kGeneralCells) {
+            least = std::min(6.0, std::max(1.25, (double)n / 3500.0));
+            coarse = std::min(6.0, std::max(1.25, (double)n / 8000.0));
+            grow = 2.5;
+        } else if (!e && kind != kTripletCells) {
             least = 12.0;
-            grow = true;
+            grow = 5.0;
         }
     }
     double L = box, R = dmax;
     auto cells = [&](int r) { return (int)std::floor(L * (r - 1e-4) / (R + 8.0 * L * 1.2e-7) * (1.0 - 1e-9)); };
     int P = cells(refine);
-    while (P > 1 && refine > 1 && (double)n / ((double)P * P * P) < (refine > 2 ? least : 6.0)) P = cells(--refine);
-    if (grow && refine == 1) P = std::min(P, (int)std::cbrt((double)n / 5.0));
+    while (P > 1 && refine > 1 && (double)n / ((double)P * P * P) < (refine > 2 ? least : coarse)) P = cells(--refine);
+    if (grow > 0.0 && refine == 1) P = std::min(P, (int)std::cbrt((double)n / grow));
     P = std::max(1, std::min(P, 256));
     if (bpc)
         while (P < 256 && !stencil_fits(box, dmax, P)) ++P;

@@ -360,8 +360,9 @@ pcf_status grid_default_cells(pcf_ctx *ctx, pcf_grid *g);
 pcf_status grid_host_starts(pcf_ctx *ctx, const pcf_grid *g, std::vector<int> &out);
 // Largest stencil population of any cell (rows on the device); waits for it.
 pcf_status stencil_max(pcf_ctx *ctx, const CellGrid &g, const RowDesc *d_rows, int n_rows, bool bpc, int64_t *out);
-// kind: a histogram kind, or kTripletCells.
-constexpr int kTripletCells = 3;
+// kind: a histogram kind (pair counts by k_pairs_lean), or one of these: triplet
+// counts, pair counts by the general kernel.
+constexpr int kTripletCells = 3, kGeneralCells = 4;
 int choose_partitions(int64_t n, float box, float dmax, int kind, bool bpc, int refine);
 bool stencil_fits(float box, float dmax, int P);
 
