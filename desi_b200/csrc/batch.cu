@@ -121,6 +121,27 @@ extern "C" pcf_status pcf_batch_pairs(pcf_ctx *ctx, int kind, const pcf_grid *d_
         gs.push_back(D);
         set_weight_fix(pl, gs.data(), (int)gs.size());
     }
+    // Anisotropic jobs of few pairs: where the warps of a k_pairs_lean CTA, which share
+    // a copy, meet at every job's end, they cost more than the general kernel's (us,
+    // bins 25, dmax 50 of 500, lean and general; unit, exact weights; expected pairs per
+    // job: 201 jobs of 2 thousand 517 346, 774 379; 65 of 60 thousand 355 273, 470 332; 121 of
+    // 130 thousand 816 609, 1176 759; 25 of 310 thousand 255 279, 361 338; 12 catalogs of 80000,
+    // bins 40, dmax 120 of 1000 4458 5478, 7854 13242).
+    int64_t n_jobs = 0;
+    double pairs = 0.0;  // expected of uniform catalogs, all jobs
+    {
+        const double v = (ani ? 2.0 : 4.0 / 3.0) * 3.14159265 * (double)dmax * dmax * dmax / ((double)box * box * box);
+        auto job = [&](const pcf_grid *h, const pcf_grid *c, double half) {
+            pairs += half * (double)h->n * (double)c->n * std::min(1.0, v);
+            ++n_jobs;
+        };
+        if (dd) job(D, D, 0.5);
+        for (auto *g : R) {
+            if (rr) job(g, g, 0.5);
+            if (dr) job(D, g, 1.0);
+        }
+    }
+    pl.small_jobs = n_jobs >= 4 && pairs < 250000.0 * (double)n_jobs;
     const bool lean = pair_lean(pl, box), exact = weighted && lean;
     // The jobs: DD, then RR_i and DR_i per random catalog.  Each job gets the
     // partition count a single call would use for its catalogs (small
@@ -136,7 +157,11 @@ extern "C" pcf_status pcf_batch_pairs(pcf_ctx *ctx, int kind, const pcf_grid *d_
     std::vector<J> js;
     auto add_job = [&](pcf_grid *h, pcf_grid *c, bool self, double mult) {
         const int64_t n = std::max<int64_t>(h->n, c->n);
-        js.push_back({h, c, self, mult, choose_partitions(n, box, dmax, lean ? kind : kGeneralCells, bpc, 0), nullptr, nullptr});
+        // (the general kernel's smaller cells are for calls that would leave SMs idle: 121
+        // jobs of 2000 to 30000 points, signed weights, 820 us with them, 609 without; and
+        // both kinds of a batch share their structures)
+        const int rule = lean || n_jobs >= 4 ? kind : kGeneralCells;
+        js.push_back({h, c, self, mult, choose_partitions(n, box, dmax, rule, bpc, 0), nullptr, nullptr});
     };
     if (dd) add_job(D, D, true, 2.0);
     for (int i = 0; i < n_rand; ++i) {

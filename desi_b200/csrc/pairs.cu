@@ -1194,8 +1194,8 @@ static cudaError_t launch_lean(const PairArgs &A, cudaStream_t st, int sm_count,
 // + 40000 and 200000 + 267000 points):
 //  * unit weights, fewer than two CTAs of 4 warps (the anisotropic copy, from 153
 //    bins on): 0.99 and 1.19 at 150 bins, 0.61 and 0.63 at 160, 0.61 and 0.63 at 220;
-//  * exact weights, isotropic, one CTA of 8 warps (161 bins on): 1.14 and 1.12 at
-//    160, 0.89 and 0.74 at 165, 0.96 and 0.78 at 255;
+//  * exact weights, isotropic, one CTA of 8 warps (160 bins on): 1.22 and 1.13 at
+//    155, 0.89 and 0.74 at 165, 0.96 and 0.78 at 255;
 //  * exact weights, anisotropic: one CTA with a copy of up to 110 bins is worth it
 //    (1.64 and 2.05 at 80, 1.01 and 1.19 at 110, 0.84 and 0.91 at 115), and fewer
 //    than 5 bins are not, where the CTA's warps collide on few counters (0.85 and
@@ -1204,10 +1204,11 @@ static cudaError_t launch_lean(const PairArgs &A, cudaStream_t st, int sm_count,
 static int lean_columns(const PairLaunch &pl) {
     const int bins = pl.rule.bins;
     const int kLWarps = pl.weighted ? LeanShape<true>::warps : LeanShape<false>::warps;
-    const size_t fixed = sizeof(LeanWarp) * kLWarps + sizeof(PairJob) + 64;  // its static shared memory
+    const size_t fixed = sizeof(LeanWarp) * kLWarps + sizeof(PairJob) * (pl.ani ? 1 : kLWarps) + 64;  // its static shared memory
     const size_t ani = !pl.ani ? 0 : pl.weighted ? LeanCopies<K_ANI, true, 32>::ani(bins) : LeanCopies<K_ANI, false, 32>::ani(bins);
     const size_t iso = !pl.ani || pl.both ? (size_t)kLWarps * (bins + 1) * 4 : 0;  // (weighted: per limb and column)
     constexpr size_t two = 113 * 1024;  // what each of two CTAs can have
+    if (pl.ani && pl.small_jobs) return 0;  // pcf_batch_pairs has both sides
     if (!pl.weighted) return fixed + iso + ani <= 110 * 1024 ? 32 : 0;
     if (!iso) return bins >= 5 && fixed + ani <= 204 * 1024 ? 32 : 0;
     for (int nc = 32; nc >= 8; nc >>= 1)

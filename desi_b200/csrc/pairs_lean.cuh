@@ -29,7 +29,7 @@
 //  * Both kinds come from one pass: its candidate tests and products are shared.
 //  * The anisotropic copy is shared by the CTA's warps (a reduction costs the
 //    same whichever warps share a copy), so 16 to 20 warps are resident at any
-//    usual bin count; the warps of a CTA meet where their items leave a job.
+//    usual bin count; the warps of a CTA that has one meet where their items leave a job.
 // What bounds it: instruction issue (62 to 70% of slots at 16 to 20 warps; the
 // general kernel 37 to 61% with half as many instructions again) and, for
 // weighted anisotropic counts, the shared-memory pipe beside it (76 to 86%: two
@@ -191,10 +191,16 @@ __global__ void __launch_bounds__(LeanShape<W>::threads, LeanShape<W>::ctas) k_p
     constexpr unsigned kMask = (1u << FB) - 1u, kBias = (FB == 16 ? 0x43000000u : 0x43800000u) >> FB;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ LeanWarp s_w[kLWarps];
-    __shared__ PairJob J;
+    // The job being counted: the CTA's where its warps share a copy (MEET), else each
+    // warp's own.  A CTA that counts one job at a time leaves most of its warps waiting
+    // where jobs are small: a batch of 100 catalogs of 250 to 940 points, exact weights,
+    // isotropic, took 752 us so, 211 with a job per warp (and the cheaper flush below).
+    constexpr bool MEET = DO_A;
+    __shared__ PairJob s_job[MEET ? 1 : kLWarps];
     __shared__ int s_want[2];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     LeanWarp &ws = s_w[warp];
+    PairJob &J = s_job[MEET ? 0 : warp];
     const int bins = A.rule.bins, row1 = Copies::row(bins);
     const int nbi = bins, nbt = (DO_I ? bins : 0) + (DO_A ? bins * bins : 0);
     unsigned char *iso_copy = smem_raw + warp * Copies::iso_warp(bins);
@@ -245,22 +251,20 @@ __global__ void __launch_bounds__(LeanShape<W>::threads, LeanShape<W>::ctas) k_p
                 if (v) atomicAdd(A.g_count + off + k, (unsigned long long)v);
             }
         } else {
-            unsigned *c = reinterpret_cast<unsigned *>(iso_copy) + (lane & (NC - 1));
-            for (int k0 = 0; k0 < bins; k0 += 32 / NC) {
-                const int k = k0 + lane / NC;
+            // a bin per lane, its columns from a different one on in each lane (a bin
+            // per column group and shuffles took four times the instructions)
+            unsigned *c = reinterpret_cast<unsigned *>(iso_copy);
+            for (int k = lane; k < bins; k += 32) {
                 unsigned long long lo = 0, hi = 0;
-                if (k < bins) {
-                    lo = c[2 * NC * k];
-                    hi = c[2 * NC * k + NC];
-                    c[2 * NC * k] = c[2 * NC * k + NC] = 0u;
-                }
-                #pragma unroll
-                for (int o = NC / 2; o > 0; o >>= 1) {
-                    lo += __shfl_xor_sync(kFull, lo, o);
-                    hi += __shfl_xor_sync(kFull, hi, o);
+                #pragma unroll 4
+                for (int o = 0; o < NC; ++o) {
+                    unsigned *p = c + 2 * NC * k + ((o + lane) & (NC - 1));
+                    lo += p[0];
+                    hi += p[NC];
+                    p[0] = p[NC] = 0u;
                 }
                 hi += lo >> 32;
-                if ((lane & (NC - 1)) == 0 && (hi | lo)) add_exact(off + k, hi << 32 | (lo & 0xffffffffull), hi >> 32);
+                if (hi | lo) add_exact(off + k, hi << 32 | (lo & 0xffffffffull), hi >> 32);
             }
         }
         __syncwarp();
@@ -309,31 +313,33 @@ __global__ void __launch_bounds__(LeanShape<W>::threads, LeanShape<W>::ctas) k_p
     int since_i = 0, since_a = 0;  // adds since this warp's last flush (bounds)
     __syncthreads();
     for (;;) {
-        // the job of this warp's next item (the CTA counts one job at a time)
+        // the job of this warp's next item
         int want = INT_MAX;
         if (it < A.n_items && !stop) {
             want = max(cur, 0);
             while (want + 1 < A.n_jobs && it >= A.jobs[want + 1].item_begin) ++want;
         }
-        if (lane == 0 && want != INT_MAX) atomicMin(&s_want[phase], want);
+        if (MEET && lane == 0 && want != INT_MAX) atomicMin(&s_want[phase], want);
         if (cur >= 0) {
             drain();
             flush_iso();
             since_i = since_a = 0;
         }
-        __syncthreads();
-        const int next = s_want[phase];
+        if (MEET) __syncthreads();
+        const int next = MEET ? s_want[phase] : want;
         if (cur >= 0) flush_ani(tid, kLThreads);
         if (next == INT_MAX) break;
-        __syncthreads();  // J is read by the flush until here
+        if (MEET) __syncthreads();  // J is read by the flush until here
+        else __syncwarp();
         static_assert(sizeof(PairJob) % 4 == 0, "PairJob words");
-        for (int q = tid; q < (int)(sizeof(PairJob) / 4); q += kLThreads)
+        for (int q = MEET ? tid : lane; q < (int)(sizeof(PairJob) / 4); q += MEET ? kLThreads : 32)
             reinterpret_cast<int *>(&J)[q] = reinterpret_cast<const int *>(A.jobs + next)[q];
         if (tid == 0) s_want[phase ^ 1] = INT_MAX;
         phase ^= 1;
         cur = next;
         job_end = cur + 1 < A.n_jobs ? A.jobs[cur + 1].item_begin : A.n_items;
-        __syncthreads();
+        if (MEET) __syncthreads();
+        else __syncwarp();
         while (!stop && it < job_end && it < A.n_items && want == cur) {
             if (!fetched) {  // the ticket after this one (and the abort word with it)
                 if (lane == 0) {

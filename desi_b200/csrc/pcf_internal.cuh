@@ -428,6 +428,7 @@ struct PairLaunch {
     double wunscale = 0.0;  // single-job launches: weight_unscale(home, cand)
     bool count = true;   // weighted launches: count in-range pairs (statistics)
     bool timed = true;   // ctx->ev0 and ev1 around the kernel (statistics)
+    bool small_jobs = false;  // a batch whose jobs hold few pairs (pcf_batch_pairs)
     // queue control (pcf_ctx_abort): the abort word the kernel polls at every
     // ticket and the status word it sets when it gives up; null: no polling
     const unsigned *ctrl = nullptr;
