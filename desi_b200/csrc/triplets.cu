@@ -26,6 +26,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <map>
 #include <vector>
 
 #include "pcf_internal.cuh"
@@ -1153,12 +1154,13 @@ __global__ void k_trip_finalize(const unsigned long long *__restrict__ cnt,
 
 }  // namespace
 
+constexpr int64_t kCheapBound = 8192;
 // Bound of an anchor's list in a catalog of n points gridded as g: n itself
 // up to `cheap` (while overflow lists of that size are small), else the largest stencil
 // population of any cell (memoised per cell structure, dmax and periodicity: the
 // rows are fixed by them and the structure's P).
 static pcf_status list_bound(pcf_ctx *ctx, const CellGrid &g, int64_t n, float dmax, const RowDesc *d_rows, int n_rows,
-                             bool bpc, int64_t *out, int64_t cheap = 8192) {
+                             bool bpc, int64_t *out, int64_t cheap = kCheapBound) {
     *out = n;
     if (n <= cheap) return PCF_OK;
     for (const auto &m : g.stencil_memo)
@@ -1236,13 +1238,28 @@ static unsigned long long limb_budget(const pcf_grid *X, const pcf_grid *Y) {
 // 354 731 -> 377 310 682, 8000: 2133 1732 3980 -> 2111 1618 4036, 30 bins, dmax 80 3568 3104
 // 7501 -> 3901 3058 11834; without exact integer weights, bound by atomics in
 // global memory, one.  (Four groups of 6 warps and two of 12 lie between.)
-static int trip_groups(const pcf_grid *X, const pcf_grid *Y, int bins, float dmax, bool weighted) {
+// The lists meant are those of uniform catalogs.  bx, by: the longest there can be
+// (list_bound), which a dense clump in a large box makes much longer.  Then one group where
+//  * the anchors are few, so that a group more is a tail more (clumps of 800 and
+//    100000 points, dmax 20: 4432 us by one group, 7939 by three; 2000 and 30000, dmax 15:
+//    1722 and 2934; 3000 and 3000: 703 and 582),
+//  * the room for all groups' spilled lists grows past 2 GB (of 148 or 444 lists each), or
+//  * an anchor's tests may pass a third of the shared counters' budget, which sends
+//    its triangles to global memory.
+static int trip_groups(pcf_ctx *ctx, const pcf_grid *X, const pcf_grid *Y, int bins, float dmax, bool weighted,
+                       int64_t bx, int64_t by) {
     const size_t hist = trip_hist_bytes(bins, weighted);
     if (!hist || (weighted && !limb_budget(X, Y))) return 1;
     const double L = X->box, in = std::min(1.0, 4.18879 * (double)dmax * dmax * dmax / (L * L * L));
     const double list = Y ? (0.5 * (double)X->n + (double)Y->n) * in : (double)X->n * in;
     constexpr int G = kTWarps / kGroupWarps;
-    return list <= (double)((kTripSmem - hist) / G / (weighted ? 40 : 16)) ? G : 1;
+    const double room = (double)((kTripSmem - hist) / G / (weighted ? 40 : 16));
+    if (list > room) return 1;
+    const int64_t longest = std::max(X->n > kCheapBound ? bx : 0, Y && Y->n > kCheapBound ? by : 0);
+    if (X->n < (int64_t)6 * G * ctx->sm_count && (double)longest > 2.0 * room) return 1;
+    if ((double)longest * 16.0 * (Y ? 2 : 1) * G * ctx->sm_count > 2147483648.0) return 1;
+    const double tests = Y ? (double)bx * (double)by : 0.5 * (double)bx * (double)bx;
+    return tests <= (double)(1 << 30) / G ? G : 1;
 }
 
 // Arguments of one isotropic triplet histogram over the cell structures of
@@ -1390,19 +1407,19 @@ extern "C" pcf_status pcf_count_triplets(pcf_ctx *ctx, int kind, const pcf_grid 
     if (gates && weighted) return ordered();
     TripArgs A;
     size_t smem = 0;
-    const int groups = trip_groups(X, Y, bins, dmax, weighted);
-    trip_setup(ctx, X, Y, P, (int)plan.rows.size(), bins, dmax, flags, weighted, A, smem, groups);
-    const int n3 = bins * bins * bins;
+    const int n3 = bins * bins * bins, n_rows = (int)plan.rows.size();
     // rows + counter through the plan slot
     PlanSlot *sl = nullptr;
     s = stage_plan(ctx, plan, &sl);
     if (s != PCF_OK) return s;
-    A.rows = sl->rows();
-    A.counter = sl->counter();
     // overflow lists
     int64_t bx = 0, by = 0;
-    s = list_bound(ctx, gx, X->n, dmax, A.rows, A.n_rows, bpc, &bx);
-    if (s == PCF_OK && mixed) s = list_bound(ctx, gy, Y->n, dmax, A.rows, A.n_rows, bpc, &by);
+    s = list_bound(ctx, gx, X->n, dmax, sl->rows(), n_rows, bpc, &bx);
+    if (s == PCF_OK && mixed) s = list_bound(ctx, gy, Y->n, dmax, sl->rows(), n_rows, bpc, &by);
+    const int groups = trip_groups(ctx, X, Y, bins, dmax, weighted, bx, by);
+    trip_setup(ctx, X, Y, P, n_rows, bins, dmax, flags, weighted, A, smem, groups);
+    A.rows = sl->rows();
+    A.counter = sl->counter();
     TripArgs F;  // the gates' corrections
     size_t fix_smem = 0;
     int fix_ctas = kTWarps / kGroupWarps;
@@ -1569,25 +1586,28 @@ extern "C" pcf_status pcf_batch_triplets(pcf_ctx *ctx, const pcf_grid *d_, const
     int most = 1;
     std::vector<size_t> smem((size_t)nj);
     std::vector<int> groups((size_t)nj);
-    int64_t gmax = 0;
     // rows + counters through the plan slot
     PlanSlot *sl = nullptr;
     s = stage_plan(ctx, plan, &sl);
     if (s != PCF_OK) return s;
+    auto bound = [&](const pcf_grid *g, int64_t *b) {
+        return list_bound(ctx, *g->cells, g->n, dmax, sl->rows(), (int)plan.rows.size(), bpc, b);
+    };
+    int64_t gmax = 0, bD = 0;
+    s = bound(D, &bD);
+    if (s != PCF_OK) return s;
+    gmax = bD;
+    std::map<const pcf_grid *, int64_t> bounds{{D, bD}};
     for (pcf_grid *g : R) {
         int64_t b = 0;
-        s = list_bound(ctx, *g->cells, g->n, dmax, sl->rows(), (int)plan.rows.size(), bpc, &b);
+        s = bound(g, &b);
         if (s != PCF_OK) return s;
         gmax = std::max(gmax, b);
-    }
-    {
-        int64_t b = 0;
-        s = list_bound(ctx, *D->cells, D->n, dmax, sl->rows(), (int)plan.rows.size(), bpc, &b);
-        if (s != PCF_OK) return s;
-        gmax = std::max(gmax, b);
+        bounds[g] = b;
     }
     for (int k = 0; k < nj; ++k) {
-        groups[k] = trip_groups(jobs[k].x, jobs[k].y, bins, dmax, weighted);
+        groups[k] = trip_groups(ctx, jobs[k].x, jobs[k].y, bins, dmax, weighted, bounds[jobs[k].x],
+                                jobs[k].y ? bounds[jobs[k].y] : 0);
         trip_setup(ctx, jobs[k].x, jobs[k].y, P, (int)plan.rows.size(), bins, dmax, flags, weighted,
                    args[k], smem[k], groups[k]);
         most = std::max(most, groups[k]);

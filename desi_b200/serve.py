@@ -101,12 +101,12 @@ def request_work(req: Request, sizes: dict, boxes: dict) -> float:
 
 def request_bytes(req: Request, sizes: dict) -> int:
     """HBM footprint of a running request: its two grids (if it has to build
-    them), histograms and scratch (triplet lists spill to per-SM scratch in
+    them), histograms and scratch (triplet lists spill to scratch, three per SM, in
     the worst case)."""
     nb = req.bins ** (3 if req.kind == "3iso" else (2 if req.kind == "2ani" else 1))
     fp = 3 * 24 * nb + (8 << 20) + grid_bytes(sizes[req.data]) + grid_bytes(sizes[req.rand])
     if req.kind == "3iso":
-        fp += 2 * 148 * 16 * max(sizes[req.data], sizes[req.rand])
+        fp += 3 * 2 * 148 * 16 * max(sizes[req.data], sizes[req.rand])
     return fp
 
 
