@@ -287,14 +287,11 @@ pcf_status pcf_grid_info(const pcf_grid *g, int64_t *n, float *box, int *partiti
     if (box) *box = g->box;
     if (partitions) *partitions = g->cells ? g->cells->P : 0;
     if (nonempty_cells) {
-        int64_t c = 0;
+        *nonempty_cells = 0;
         if (g->cells && g->owner) {
-            std::vector<int> h;
-            pcf_status s = grid_host_starts(g->owner, g, h);
+            const pcf_status s = grid_nonempty(g->owner, g, nonempty_cells);
             if (s != PCF_OK) return s;
-            for (size_t i = 0; i + 1 < h.size(); ++i) c += h[i + 1] > h[i];
         }
-        *nonempty_cells = c;
     }
     if (unit_weights) *unit_weights = g->unit_weights ? 1 : 0;
     return PCF_OK;
@@ -328,10 +325,18 @@ pcf_status pcf_grid_download(pcf_ctx *ctx, const pcf_grid *g, pcf_point *pts_out
         }
     }
     if (cell_start_out) {
-        std::vector<int> h;
-        pcf_status s0 = grid_host_starts(ctx, g, h);
-        if (s0 != PCF_OK) return s0;
-        memcpy(cell_start_out, h.data(), sizeof(int) * h.size());
+        const CellGrid &c = *g->cells;
+        const size_t bytes = sizeof(int) * ((size_t)c.P * c.P * c.P + 1);
+        if (bytes <= kStagedOut) {
+            std::vector<char> spill;
+            const char *h = nullptr;
+            const pcf_status s0 = fetch_block(ctx, c.cell_start.p, bytes, spill, &h);
+            if (s0 != PCF_OK) return s0;
+            memcpy(cell_start_out, h, bytes);
+        } else {
+            PCF_CU(ctx, cudaMemcpyAsync(cell_start_out, c.cell_start.p, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+            PCF_CU(ctx, cudaStreamSynchronize(ctx->stream));
+        }
     }
     return PCF_OK;
 }
@@ -399,8 +404,7 @@ pcf_status prepare_grids(pcf_ctx *ctx, pcf_grid *a, pcf_grid *b, float dmax, int
         ctx->last_error = "dmax too close to box/2 for the periodic stencil";
         return PCF_ERR_UNSUPPORTED;
     }
-    // both structures queued before either is completed: a's host work
-    // (cell table, tiles) overlaps b's build on the device
+    // both structures queued before either is waited for
     pcf_status s = grid_ensure_cells(ctx, a, P, b != nullptr);
     if (s != PCF_OK) return s;
     if (b) {

@@ -203,6 +203,7 @@ struct CellGrid {
     // built on first use (-1: not yet)
     int64_t n_tiles_half = -1;
     DevBuf d_tiles_half;
+    mutable int64_t nonempty = -1;  // cells that hold a point (grid_nonempty; -1: not yet counted)
     // largest stencil population of a cell per (dmax, periodic), memoised
     // for the triplet launches
     mutable std::vector<std::pair<std::pair<float, bool>, int64_t>> stencil_memo;
@@ -357,7 +358,7 @@ pcf_status grid_finish(pcf_ctx *ctx, const pcf_grid *g);
 // Copies and checks the caller's points (queued; grid_finish reads the checks).
 pcf_status grid_take(pcf_ctx *ctx, pcf_grid *g, const pcf_point *pts);
 pcf_status grid_default_cells(pcf_ctx *ctx, pcf_grid *g);
-pcf_status grid_host_starts(pcf_ctx *ctx, const pcf_grid *g, std::vector<int> &out);
+pcf_status grid_nonempty(pcf_ctx *ctx, const pcf_grid *g, int64_t *out);
 // Largest stencil population of any cell (rows on the device); waits for it.
 pcf_status stencil_max(pcf_ctx *ctx, const CellGrid &g, const RowDesc *d_rows, int n_rows, bool bpc, int64_t *out);
 // kind: a histogram kind (pair counts by k_pairs_lean), or one of these: triplet
