@@ -37,7 +37,8 @@ struct BatchGraph {
 // Both kinds as two single-kind batches, interleaved into the both-kinds
 // layout: per histogram bins isotropic doubles, then bins^2 anisotropic.
 // (One pass of the general kernel over the candidates was slower: the
-// measurements sit beside count_pairs_impl in capi.cu.)
+// measurements sit beside count_pairs_impl in capi.cu.  One pass of k_pairs_lean
+// is not used here.)
 static pcf_status batch_both_split(pcf_ctx *ctx, const pcf_grid *d, const pcf_grid *const *r,
                                    int n_rand, int bins, float dmax, uint32_t flags, double *dd,
                                    double *rr, double *dr, pcf_stats *stats) {

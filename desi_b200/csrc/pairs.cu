@@ -1320,8 +1320,8 @@ static PairArgs make_args(const PairJob *jobs, int n_jobs, long long n_items,
     A.fast = pl.rule.bins <= 255 ? 1 : 0;
     A.ctrl = pl.ctrl;
     A.status = pl.status;
-    A.max_tickets = n_items + 2;  // refined per launch shape in launch_one
-    A.kchunk = pl.chunk_cap;      // a cap here; launch_one sets the run length
+    A.max_tickets = n_items + 2;  // refined per launch shape in with_tickets
+    A.kchunk = pl.chunk_cap;      // a cap here; with_tickets sets the run length
     return A;
 }
 

@@ -30,7 +30,7 @@
 //  * The anisotropic copy is shared by the CTA's warps (a reduction costs the
 //    same whichever warps share a copy), so 16 to 20 warps are resident at any
 //    usual bin count; the warps of a CTA that has one meet where their items leave a job.
-// What bounds it: instruction issue (62 to 70% of slots at 16 to 20 warps; the
+// What bounds it: instruction issue (67 to 74% of slots at 16 to 20 warps; the
 // general kernel 37 to 61% with half as many instructions again) and, for
 // weighted anisotropic counts, the shared-memory pipe beside it (76 to 86%: two
 // returning adds to scattered counters per pair).

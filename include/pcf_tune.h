@@ -7,7 +7,9 @@
  * scheme (-1: the library's rule; 0: a u32 column per lane; 1: one copy per
  * warp with shared atomics; 3: per-warp fixed-point limbs of the exact
  * weight products; 4: lane-private fixed-point limbs (isotropic); for
- * PCF_BOTH a scheme >= 0 means one pass over the candidates for both kinds)
+ * PCF_BOTH a scheme >= 0 means one pass over the candidates for both kinds;
+ * schemes >= 0 are the general kernel's, so a table saved before the library
+ * had the branch-free one is best made again)
  * and the home-tile size (32 or 16 points per warp item).  The best shape
  * depends on the kind, the bins and the point density, so the tuner times
  * candidates on the caller's own catalogs (every refine x scheme at 32-point
