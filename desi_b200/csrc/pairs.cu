@@ -32,22 +32,12 @@
 //    an exact integer image.
 //  * A launch produces the isotropic histogram, the anisotropic one, or both
 //    from one pass over the candidates (PCF_BOTH).
-#include <algorithm>
-#include <climits>
-#include <cmath>
-#include <cstring>
-#include <map>
-#include <mutex>
-#include <numeric>
-#include <type_traits>
-
-#include "pcf_internal.cuh"
+#include "pairs_lean.cuh"
 
 namespace {
 
 constexpr int kThreads = 128;  // 4 independent warps per CTA
 constexpr int kWarps = kThreads / 32;
-constexpr unsigned kFull = 0xffffffffu;
 constexpr float kMagic = 256.0f;  // r + 256 -> low mantissa bits = round(r * 2^15)
 constexpr int kFracBits = 15;
 constexpr unsigned kFracMask = (1u << kFracBits) - 1u;
@@ -81,53 +71,6 @@ constexpr int kLimbs = 3;
 #ifndef PCF_GROUP_ANI
 #define PCF_GROUP_ANI 2
 #endif
-constexpr int kChunkMax = 8;            // work items per ticket, at most
-constexpr int kLeanWideBins = 120;      // bins up to which k_pairs_lean reads out 16 fraction bits
-
-// Fast-path cut constants for one range type (0: unshifted, 1: image-shifted).
-struct FastCuts {
-    float dsf;        // (float)ds
-    float ds2;        // dsf * dsf
-    float lo[2];      // d2 below lo (and >= tiny) is safely inside dmax
-    float hi[2];      // d2 at or above hi is safely outside dmax
-    unsigned w[2];    // edge window in 2^-15 units of r
-    // k_pairs_lean: the edge window in units of its readout, dmax included; 0
-    // where it does not apply (see make_cuts)
-    unsigned wl[2];
-    float tiny;
-};
-
-struct PairArgs {
-    const PairJob *jobs;  // histograms of this launch, items laid out job after job
-    int n_jobs;
-    long long n_items;
-    unsigned long long *counter;  // work tickets handed out so far
-    long long n_chunked;          // items [0, n_chunked) go out `kchunk` per ticket,
-    long long t_chunked;          // in t_chunked tickets; later tickets: one item each
-    int kchunk;
-    float box;
-    int bpc;
-    float zreach;  // dmax * (1 + 1e-5): the z reach of a home tile's rows
-    PairRule rule;
-    FastCuts fc;
-    unsigned long long *g_count;
-    double *g_wsum;
-    unsigned long long *g_stats;
-    int chunk;   // candidates per budget check (even)
-    int budget;  // adds one shared counter absorbs between flushes
-    int fast;    // 0: every pair in range takes the FP64 rule (bins > 255: r + 256
-                 // no longer has a fixed exponent)
-    const unsigned *ctrl;  // abort request polled at every ticket (null: none)
-    unsigned *status;      // where a warp that gives up records why (null: none)
-    long long max_tickets; // iteration cap: tickets one warp may take
-};
-
-__device__ __forceinline__ float sqrt_approx(float x) {
-    float r;
-    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-}
-
 // Fixed-point readout of r in [0, 256): u = bits(r + 256 + w/2^15), so the
 // low 15 bits are frac(r) + w in 2^-15 units.  The bin (u >> 15, biased) is
 // floor(r) unless r is within w/2^15 of an integer, which this rejects.
@@ -135,12 +78,6 @@ __device__ __forceinline__ bool fix_safe(unsigned u, unsigned w2) {
     return (u & kFracMask) >= w2;
 }
 
-// Shared reductions on 32-bit shared-window addresses.  They are not
-// predicated: a lane without a pair adds 0 to a private dummy slot, which
-// keeps the candidate loop free of branches around memory operations.
-__device__ __forceinline__ void red_s_u32(unsigned a, unsigned v) {
-    asm volatile("red.shared.add.u32 [%0], %1;" :: "r"(a), "r"(v));
-}
 __device__ __forceinline__ void red_s_f64(unsigned a, double v) {
     asm volatile("red.shared.add.f64 [%0], %1;" :: "r"(a), "d"(v));
 }
@@ -199,25 +136,6 @@ struct Sink {
         }
     }
 };
-
-// Point j of a pair-packed view.
-__device__ __forceinline__ void load_point(const float4 *pk, int j, float &x, float &y, float &z, float &w) {
-    const float4 a = __ldg(pk + (j & ~1)), b = __ldg(pk + (j & ~1) + 1);
-    const bool o = j & 1;
-    x = o ? a.y : a.x;
-    y = o ? a.w : a.z;
-    z = o ? b.y : b.x;
-    w = o ? b.w : b.z;
-}
-
-// Canonical FP64 decision for one pair (rare path): histogram slot or -1.
-template <bool ANI>
-__device__ __noinline__ int slow_slot(float hx, float hy, float hz, float cx, float cy, float cz,
-                                      float sx, float sy, float sz, PairRule rule) {
-    double dx, dy, dz;
-    exact_sep(hx, hy, hz, cx, cy, cz, sx, sy, sz, dx, dy, dz);
-    return exact_slot<ANI>(dx, dy, dz, rule);
-}
 
 // Shared-memory words (of the copy's element type) of one warp's copy.
 // Per-warp copies end with a dummy region (never flushed) where each lane
@@ -331,10 +249,6 @@ struct MinBlocks {
                                : HM == H_LFIX ? 4 : HM == H_WFIX ? 5 : PCF_PAIR_MINB;
 };
 
-// Kinds of one launch: the isotropic histogram, the anisotropic one, or both
-// from one pass over the candidates (the anisotropic stencil covers the
-// isotropic one).
-enum { K_ISO = 0, K_ANI = 1, K_BOTH = 2 };
 // Scheme of the isotropic copy of a K_BOTH launch, given the anisotropic one:
 // lane-private counts, four per-warp fixed-point sub-copies, else per-warp
 // copies of the same element type.
@@ -379,15 +293,6 @@ __device__ __forceinline__ void setup_sink(Sink<WEIGHTED, HM> &sk, unsigned ms, 
     }
 }
 
-// Candidate ranges of one stencil row for the current home tile: [a0, b0)
-// unshifted in z, [a1, b1) image-shifted by sz1 (periodic wrap in z); the
-// column's image shift is (sx, sy).  kind 1: forward half of the home column.
-struct RowRange {
-    int a0, b0, a1, b1;
-    float sx, sy, sz1;
-    int kind;
-};
-
 // Per-warp state kept in shared memory, so the candidate loop has the
 // registers to itself.
 struct WarpState {
@@ -398,51 +303,6 @@ struct WarpState {
     long long job_end;
     int cj, slot;
 };
-
-// The candidate ranges of stencil row rw for home tile t of job J, whose
-// points lie in [zmn, zmx].
-__device__ __forceinline__ RowRange row_range(const PairArgs &A, const PairJob &J, const RowDesc rw, const TileDesc &t,
-                                              float zmn, float zmx) {
-    RowRange rr{0, 0, 0, 0, 0.f, 0.f, 0.f, 0};
-    int nx = t.ix + rw.dx, ny = t.iy + rw.dy;
-    const int P = J.P;
-    bool ok = true;
-    if (A.bpc) {
-        if (nx < 0) { nx += P; rr.sx = -A.box; } else if (nx >= P) { nx -= P; rr.sx = A.box; }
-        if (ny < 0) { ny += P; rr.sy = -A.box; } else if (ny >= P) { ny -= P; rr.sy = A.box; }
-    } else if (nx < 0 || nx >= P || ny < 0 || ny >= P) {
-        ok = false;
-    }
-    if (ok) {
-        const int col = (nx * P + ny) * P;
-        // the row's cells, clipped to those the home points reach in z:
-        // a candidate within dmax of a home point has z in (zmn - dmax,
-        // zmx + dmax), so its cell lies in [zcut_lo, zcut_hi] (with
-        // 1e-3 of a cell to spare for the rounding of z / cell here
-        // and in the grid build; the tile's own cells always stay);
-        // periodic images follow the same cell arithmetic past 0 and P
-        const float rcell = (float)P / A.box;
-        const int zcut_lo = min((int)floorf((zmn - A.zreach) * rcell - 1e-3f), (int)t.z0);
-        const int zcut_hi = max((int)floorf((zmx + A.zreach) * rcell + 1e-3f), (int)t.z1);
-        const int zhi = min(t.z1 + rw.kz, zcut_hi);
-        rr.kind = rw.kind;
-        const int *cs = J.cand.cstart;
-        if (rw.kind == 1) {  // forward half of the home column (XX): j > home index
-            rr.a0 = t.start;
-            rr.b0 = cs[col + min(zhi, P - 1) + 1];
-            if (A.bpc && zhi >= P) { rr.a1 = cs[col]; rr.b1 = cs[col + zhi - P + 1]; rr.sz1 = A.box; }
-        } else {
-            const int zlo = max(t.z0 - rw.kz, zcut_lo);
-            rr.a0 = cs[col + max(zlo, 0)];
-            rr.b0 = cs[col + min(zhi, P - 1) + 1];
-            if (A.bpc) {
-                if (zlo < 0) { rr.a1 = cs[col + zlo + P]; rr.b1 = cs[col + P]; rr.sz1 = -A.box; }
-                else if (zhi >= P) { rr.a1 = cs[col]; rr.b1 = cs[col + zhi - P + 1]; rr.sz1 = A.box; }
-            }
-        }
-    }
-    return rr;
-}
 
 // COUNT: also count the in-range pairs (weighted histograms, statistics on).
 // HM is the scheme of the anisotropic copy for K_ANI / K_BOTH launches.
@@ -917,40 +777,6 @@ __global__ void __launch_bounds__(kThreads, MinBlocks<KIND, HM, VAR>::value) k_p
     }
 }
 
-#include "pairs_lean.cuh"
-
-// A bin of k_pairs_lean's weighted sums: 128-bit whole numbers, low and high.
-__device__ __forceinline__ double exact_sum(unsigned long long lo, double hi) {
-    return (double)(unsigned long long)__double_as_longlong(hi) * 0x1p64 + (double)lo;
-}
-
-// How a histogram arrives: u64 counts, FP64 sums, or exact sums (whose scale the
-// caller's multiplier includes).
-enum { SUM_COUNTS = 0, SUM_FP64 = 1, SUM_EXACT = 2 };
-
-// Several histograms: out[s*nb + k] = mult[s] * hist[s*nb + k].
-__global__ void k_finalize_slots(const unsigned long long *__restrict__ cnt,
-                                 const double *__restrict__ ws, int weighted,
-                                 const double *__restrict__ mult, int nb, int nslots,
-                                 double *__restrict__ out) {
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long long)nb * nslots) return;
-    const int s = (int)(t / nb);
-    out[t] = mult[s] * (weighted == SUM_EXACT ? exact_sum(cnt[t], ws[t]) : weighted ? ws[t] : (double)cnt[t]);
-}
-
-// out[k] = mult * hist[k] (u64 counts or FP64 sums); with host_stats, the four
-// statistics words too.
-__global__ void k_finalize(const unsigned long long *__restrict__ cnt, const double *__restrict__ ws,
-                           int weighted, double mult, int nb, double *__restrict__ out,
-                           const unsigned long long *__restrict__ stats, unsigned long long *host_stats) {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (host_stats && k < 4) host_stats[k] = stats[k];
-    if (k >= nb) return;
-    double v = weighted == SUM_EXACT ? exact_sum(cnt[k], ws[k]) : weighted ? ws[k] : (double)cnt[k];
-    out[k] = mult * v;
-}
-
 }  // namespace
 
 // ---------------------------------------------------------------------------
@@ -1077,40 +903,6 @@ static int pair_variant(const PairLaunch &pl, int hm, int n_jobs = 1) {
     return (v == 3 && n_jobs != 1) ? 0 : v;  // shared copies hold one job's adds only
 }
 
-// The ticket shape of a launch of `warps` warps: runs of k items per ticket
-// while a queue holds >= 32 runs per warp (k at most 8, or the tuned cap that
-// A.kchunk carries in).
-static PairArgs with_tickets(const PairArgs &A, long long n_items, long long warps) {
-    PairArgs B = A;
-    const long long cap = A.kchunk > 0 ? std::min<long long>(A.kchunk, kChunkMax) : kChunkMax;
-    B.kchunk = (int)std::max(1LL, std::min<long long>(cap, n_items / (warps * 32)));
-    B.n_chunked = B.kchunk > 1 ? std::max(0LL, n_items - 2 * warps) : 0;
-    B.t_chunked = (B.n_chunked + B.kchunk - 1) / B.kchunk;
-    // a warp can take at most every ticket of the queue plus the one that
-    // finds it empty
-    B.max_tickets = B.t_chunked + (n_items - B.n_chunked) + 2;
-    return B;
-}
-
-// CTAs of `kfn` per SM (occupancy queries cost microseconds: cached per device
-// and shared-memory size, under a lock, as several host threads launch).
-struct OccCache {
-    std::mutex mu;
-    std::map<std::pair<int, size_t>, int> per_sm;
-    cudaError_t get(const void *kfn, int threads, int device, size_t smem, int *out) {
-        std::lock_guard<std::mutex> lk(mu);
-        auto it = per_sm.find({device, smem});
-        if (it == per_sm.end()) {
-            int per = 0;
-            const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kfn, threads, smem);
-            if (e != cudaSuccess) return e;
-            it = per_sm.insert({{device, smem}, std::max(1, per)}).first;
-        }
-        *out = it->second;
-        return cudaSuccess;
-    }
-};
-
 template <int KIND, bool W, int HM, bool C, int VAR = 0>
 static cudaError_t launch_one(const PairArgs &A, size_t smem, long long n_items, cudaStream_t st,
                               int sm_count, int device) {
@@ -1172,22 +964,6 @@ static int pair_scheme(const PairLaunch &pl) {
     return hm;
 }
 
-template <int KIND, bool W, bool C, int FB, int NC>
-static cudaError_t launch_lean(const PairArgs &A, cudaStream_t st, int sm_count, int device) {
-    auto kfn = k_pairs_lean<KIND, W, C, FB, NC>;
-    const size_t smem = (size_t)LeanCopies<KIND, W, NC>::bytes(A.rule.bins);
-    static OccCache occ;
-    cudaError_t e = ensure_smem_limit(reinterpret_cast<const void *>(kfn), device, smem);
-    int per_sm = 0;
-    if (e == cudaSuccess) e = occ.get(reinterpret_cast<const void *>(kfn), LeanShape<W>::threads, device, smem, &per_sm);
-    if (e != cudaSuccess) return e;
-    constexpr int kLWarps = LeanShape<W>::warps;
-    const long long want = (A.n_items + kLWarps - 1) / kLWarps;
-    const int grid = (int)std::max(1LL, std::min<long long>(want, (long long)sm_count * per_sm));
-    kfn<<<grid, LeanShape<W>::threads, smem, st>>>(with_tickets(A, A.n_items, (long long)grid * kLWarps));
-    return cudaGetLastError();
-}
-
 // Columns per isotropic bin of a lean launch (32, 16 or 8): the most that let
 // two CTAs share an SM, else 8; 0 where the general kernel is the faster one, which
 // is where too few warps would be left (time of the general kernel over this, 30000
@@ -1224,32 +1000,13 @@ bool pair_lean(const PairLaunch &pl, float box) {
     return make_cuts(pl.rule, box, std::sqrt((float)pl.rule.dd)).wl[0] != 0 && lean_columns(pl) != 0;
 }
 
-template <int KIND, int FB>
-static cudaError_t dispatch_lean(const PairArgs &A, const PairLaunch &pl, cudaStream_t st, int sm_count, int device) {
-    if (!pl.weighted) return launch_lean<KIND, false, false, FB, 32>(A, st, sm_count, device);
-    const int nc = KIND == K_ANI ? 32 : lean_columns(pl);
-    if (pl.count) {
-        if (nc == 32) return launch_lean<KIND, true, true, FB, 32>(A, st, sm_count, device);
-        if (nc == 16) return launch_lean<KIND, true, true, FB, KIND == K_ANI ? 32 : 16>(A, st, sm_count, device);
-        return launch_lean<KIND, true, true, FB, KIND == K_ANI ? 32 : 8>(A, st, sm_count, device);
-    }
-    if (nc == 32) return launch_lean<KIND, true, false, FB, 32>(A, st, sm_count, device);
-    if (nc == 16) return launch_lean<KIND, true, false, FB, KIND == K_ANI ? 32 : 16>(A, st, sm_count, device);
-    return launch_lean<KIND, true, false, FB, KIND == K_ANI ? 32 : 8>(A, st, sm_count, device);
-}
-
 // Chooses the kernel and histogram mode of one launch and starts it.
 static cudaError_t dispatch_pairs(PairArgs A, const PairLaunch &pl, cudaStream_t st,
                                   int sm_count, int device) {
     if (pair_lean(pl, A.box)) {
         A.budget = pl.weighted ? pl.lean_budget : 1 << 30;  // adds a column absorbs between flushes
-        const bool wide = pl.rule.bins <= kLeanWideBins;
-        if (pl.both) return wide ? dispatch_lean<K_BOTH, 16>(A, pl, st, sm_count, device)
-                                 : dispatch_lean<K_BOTH, 15>(A, pl, st, sm_count, device);
-        if (pl.ani) return wide ? dispatch_lean<K_ANI, 16>(A, pl, st, sm_count, device)
-                                : dispatch_lean<K_ANI, 15>(A, pl, st, sm_count, device);
-        return wide ? dispatch_lean<K_ISO, 16>(A, pl, st, sm_count, device)
-                    : dispatch_lean<K_ISO, 15>(A, pl, st, sm_count, device);
+        return pl.weighted ? launch_lean_weighted(A, pl, lean_columns(pl), st, sm_count, device)
+                           : launch_lean_unit(A, pl, st, sm_count, device);
     }
     const int hm = pair_scheme(pl);
     const size_t smem = hm == H_GLOBAL ? 0 : scheme_bytes(pl, hm, A.n_jobs);
@@ -1493,29 +1250,3 @@ pcf_status launch_pairs(pcf_ctx *ctx, const PairPlan &plan, const CellGrid &home
     return PCF_OK;
 }
 
-static int sum_kind(bool weighted, bool exact) { return !weighted ? SUM_COUNTS : exact ? SUM_EXACT : SUM_FP64; }
-
-cudaError_t launch_finalize_slots(const unsigned long long *d_count, const double *d_wsum,
-                                  bool weighted, bool exact, const double *d_mult, int nb, int nslots,
-                                  double *d_out, cudaStream_t st) {
-    const long long n = (long long)nb * nslots;
-    k_finalize_slots<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(d_count, d_wsum, sum_kind(weighted, exact),
-                                                                   d_mult, nb, nslots, d_out);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_finalize(const unsigned long long *d_count, const double *d_wsum, bool weighted,
-                            double mult, int nb, double *d_out, cudaStream_t st) {
-    k_finalize<<<(nb + 255) / 256, 256, 0, st>>>(d_count, d_wsum, weighted ? 1 : 0, mult, nb, d_out, nullptr, nullptr);
-    return cudaGetLastError();
-}
-
-pcf_status finalize_hist(pcf_ctx *ctx, const unsigned long long *d_count, const double *d_wsum,
-                         bool weighted, bool exact, double mult, int nb, double *out,
-                         const unsigned long long *d_stats, unsigned long long *host_stats) {
-    k_finalize<<<(nb + 255) / 256, 256, 0, ctx->stream>>>(d_count, d_wsum, sum_kind(weighted, exact), mult,
-                                                          nb, out, d_stats, host_stats);
-    PCF_CU(ctx, cudaGetLastError());
-    ++ctx->launches;
-    return PCF_OK;
-}

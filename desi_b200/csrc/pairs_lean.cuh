@@ -1,7 +1,7 @@
 // pairs_lean.cuh -- the pair kernel of unit weights and of weights with exact
 // integer images, at the bin counts where its copies leave room for enough warps
-// (lean_columns in pairs.cu, which includes this file and holds the work items, the
-// windows and the general kernel for everything else).
+// (lean_columns in pairs.cu, which holds the windows and the general kernel for
+// everything else).
 //
 // Same work items as the general kernel: one warp takes (home tile, stencil
 // rows), one home point per lane, candidates two at a time as packed f32x2.
@@ -40,6 +40,22 @@
 // box 1000, 40 bins, dmax 120, weighted, anisotropic: 1488 -> 822; 200001 +
 // 300000 points, periodic, 50 bins, dmax 100, unit weights: isotropic 1013 -> 703,
 // anisotropic 1400 -> 883.
+//
+// Unit and weighted counts are compiled in files of their own (pairs_lean_unit.cu,
+// pairs_lean_weighted.cu): a process loads a file's kernels with the first of them
+// it launches, and with the general kernel and the last kernel of every count they
+// had grown to a 14 MB module, which took the first count of a process 15 ms to
+// load (unit weights, without them: 0.8 ms).
+#pragma once
+
+#include "pairs_common.cuh"
+
+cudaError_t launch_lean_unit(const PairArgs &A, const PairLaunch &pl, cudaStream_t st, int sm_count, int device);
+// nc: lean_columns
+cudaError_t launch_lean_weighted(const PairArgs &A, const PairLaunch &pl, int nc, cudaStream_t st, int sm_count,
+                                 int device);
+
+namespace {
 
 // CTA shapes, steps per vote and resident CTAs.  Weighted: 8 warps, two CTAs at
 // 128 registers (the anisotropic copy is large, so few CTAs share an SM); unit: 4
@@ -664,4 +680,22 @@ __global__ void __launch_bounds__(LeanShape<W>::threads, LeanShape<W>::ctas) k_p
         if (n_cand) atomicAdd(A.g_stats + 1, n_cand);
         if (COUNT && rp) atomicAdd(A.g_stats + 2, rp);
     }
+}
+
+}  // namespace
+
+template <int KIND, bool W, bool C, int FB, int NC>
+static cudaError_t launch_lean(const PairArgs &A, cudaStream_t st, int sm_count, int device) {
+    auto kfn = k_pairs_lean<KIND, W, C, FB, NC>;
+    const size_t smem = (size_t)LeanCopies<KIND, W, NC>::bytes(A.rule.bins);
+    static OccCache occ;
+    cudaError_t e = ensure_smem_limit(reinterpret_cast<const void *>(kfn), device, smem);
+    int per_sm = 0;
+    if (e == cudaSuccess) e = occ.get(reinterpret_cast<const void *>(kfn), LeanShape<W>::threads, device, smem, &per_sm);
+    if (e != cudaSuccess) return e;
+    constexpr int kLWarps = LeanShape<W>::warps;
+    const long long want = (A.n_items + kLWarps - 1) / kLWarps;
+    const int grid = (int)std::max(1LL, std::min<long long>(want, (long long)sm_count * per_sm));
+    kfn<<<grid, LeanShape<W>::threads, smem, st>>>(with_tickets(A, A.n_items, (long long)grid * kLWarps));
+    return cudaGetLastError();
 }
