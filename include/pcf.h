@@ -199,7 +199,8 @@ pcf_status pcf_analytic_3iso(pcf_ctx *ctx, const pcf_grid *d, int bins, float dm
  * persistent launch over a (tile, neighbour rows, catalog) work queue.
  * Writes, per random catalog i: rr[i*nb .. ] and dr[i*nb ..] (nb = bins,
  * bins^2, or bins + bins^2 for PCF_BOTH), and dd (nb) once.  Any of dd / rr
- * / dr may be NULL to skip it.
+ * / dr may be NULL to skip it.  Refuses what a single call of any of its
+ * histograms refuses.
  */
 pcf_status pcf_batch_pairs(pcf_ctx *ctx, int kind, const pcf_grid *d, const pcf_grid *const *r,
                            int n_rand, int bins, float dmax, uint32_t flags, double *dd,
